@@ -463,6 +463,18 @@ struct v3dm_ransac {
   size_t bestEFCap = 0;
   double* dBestRT = nullptr;   // refined R, T per pair (iterative refinement)
   size_t bestRTCap = 0;
+  // the refinement's task lists, results and inlier lists (RsRefineWork)
+  int32_t* dTaskIdx = nullptr;
+  size_t taskIdxCap = 0;
+  int32_t* dTaskN = nullptr;   // nPairs counts, then the number of tasks
+  size_t taskNCap = 0;
+  int2* dTasks = nullptr;
+  size_t tasksCap = 0;
+  RsRefined* dRefined = nullptr;
+  size_t refinedCap = 0;
+  int32_t* dLists = nullptr;
+  size_t listsCap = 0;
+  int numSMs = 148;
   bool refine = false;         // RobustOrientationMode::iterativeRefinement
   double thr = 0.0;            // inlier threshold of the call (pixels)
   unsigned long long* dWork = nullptr;  // candidates, Sampson evaluations of the last call
@@ -514,6 +526,23 @@ int rs_enqueue(v3dm_ransac* r, int nPairs, int nCorrs, int nDraw, int nSamples, 
   V3DM_RS_TRY(rs_grow(r->dBestRT, r->bestRTCap, (size_t)nPairs * 12));
   V3DM_RS_TRY(rs_grow(r->dWork, r->workCap, (size_t)2));
   RsState* state = static_cast<RsState*>(r->dState);
+  RsRefineWork rw{};
+  if (r->refine) {
+    V3DM_RS_TRY(rs_grow(r->dTaskIdx, r->taskIdxCap, (size_t)nPairs * kRsTasks));
+    V3DM_RS_TRY(rs_grow(r->dTaskN, r->taskNCap, (size_t)nPairs + 1));
+    V3DM_RS_TRY(rs_grow(r->dTasks, r->tasksCap, (size_t)nPairs * kRsTasks));
+    rw.ctas = 2 * r->numSMs;  // two CTAs of k_rs_refine fit an SM
+    V3DM_RS_TRY(rs_grow(r->dRefined, r->refinedCap, (size_t)nPairs * kRsTasks + rw.ctas));
+    for (int p = 0; p < nPairs; ++p)
+      rw.listRoom = std::max(rw.listRoom, (long long)(r->hOffsets[p + 1] - r->hOffsets[p]));
+    V3DM_RS_TRY(rs_grow(r->dLists, r->listsCap, (size_t)rw.ctas * (size_t)rw.listRoom));
+    rw.taskIdx = r->dTaskIdx;
+    rw.taskN = r->dTaskN;
+    rw.nTasks = r->dTaskN + nPairs;
+    rw.tasks = r->dTasks;
+    rw.refined = r->dRefined;
+    rw.lists = r->dLists;
+  }
   int launches = 0;
   V3DM_RS_TRY(cudaMemsetAsync(r->dWork, 0, 2 * sizeof(unsigned long long), r->stream));
   if (nCorrs > 0) {
@@ -545,11 +574,11 @@ int rs_enqueue(v3dm_ransac* r, int nPairs, int nCorrs, int nDraw, int nSamples, 
     if (r->refine)
       V3DM_RS_TRY(launch_rs_select_refine(r->dOffsets, nPairs, nDraw, s0, len, r->dCounts, r->dSlotOk, r->dCost,
                                           r->dSlots, state, r->dBestEF, dCorrs, r->dNorm, dSamples, r->dInvK, r->thr,
-                                          thr2, r->dBestRT, r->stream));
+                                          thr2, r->dBestRT, rw, r->stream));
     else
       k_rs_select<<<nPairs, 32, 0, r->stream>>>(r->dOffsets, nPairs, nDraw, s0, len, r->dCounts, r->dSlotOk,
                                                  r->dCost, r->dInl, r->dSlots, state, r->dBestEF);
-    launches += 4;
+    launches += r->refine ? 6 : 4;
   }
   k_rs_finish<<<(nPairs + 127) / 128, 128, 0, r->stream>>>(r->dOffsets, nPairs, nDraw, dSamples, r->dNorm, state,
                                                            r->dBestEF, dOut, r->refine ? 1 : 0, r->dBestRT);
@@ -582,6 +611,7 @@ int v3dm_ransac_create(v3dm_ransac** out, int device) {
   v3dm_ransac* r = new (std::nothrow) v3dm_ransac();
   if (!r) return V3DM_ERR_ARG;
   r->device = device;
+  r->numSMs = prop.multiProcessorCount;
   RsDeviceGuard g(device);
   if (cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete r;
@@ -597,7 +627,7 @@ int v3dm_ransac_destroy(v3dm_ransac* r) {
   cudaStreamSynchronize(r->stream);
   void* bufs[] = {r->dOffsets, r->dCorrs, r->dNorm, r->dInvK, r->dSamples, r->dSlots, r->dSlotOk, r->dCounts,
                   r->dList,    r->dListN, r->dCost, r->dInl,  r->dState,   r->dBestEF, r->dWork,  r->dOut,
-                  r->dFlags,   r->dNIn,   r->dBestRT};
+                  r->dFlags,   r->dNIn,   r->dBestRT, r->dTaskIdx, r->dTaskN, r->dTasks, r->dRefined, r->dLists};
   for (void* b : bufs)
     if (b) cudaFree(b);
   for (int k = 0; k < 2; ++k)

@@ -29,10 +29,31 @@ __device__ __forceinline__ int rs_budget(double outlierRatio) {
   return (int)N;
 }
 
-// The round's selection with mode.iterativeRefinement (v3dm_ransac_refine.cu): one warp per pair.
+// The refined candidates of a round (v3dm_ransac_refine.cu).  Sixteen per pair: the prefix minima of
+// 1280 costs in random order are 7.7 on average, and a full list only moves a refinement to the
+// selecting kernel.
+constexpr int kRsTasks = 16;
+struct RsRefined {
+  double EF[18], RT[12];  // refined E, F and R, T
+  double cost;            // cost of the refined F
+  int nIn, ok;            // its inlier count; 0: the sample does not agree on a pose
+};
+struct RsRefineWork {
+  int32_t* taskIdx;     // nPairs x kRsTasks: candidate of each task, ascending
+  int32_t* taskN;       // nPairs
+  int2* tasks;          // nPairs x kRsTasks: (pair x kRsTasks + task, candidate), any order
+  int* nTasks;
+  RsRefined* refined;   // nPairs x kRsTasks, then one per CTA
+  int32_t* lists;       // ctas x listRoom inlier indices
+  long long listRoom;   // the largest correspondence count of a pair
+  int ctas;             // persistent CTAs
+};
+
+// The round's selection with mode.iterativeRefinement (v3dm_ransac_refine.cu).
 cudaError_t launch_rs_select_refine(const int32_t* offsets, int nPairs, int nDraw, int s0, int len, const int8_t* counts,
                                     const uint8_t* slotOk, const double* cost, const double* slots, RsState* st,
                                     double* bestEF, const float4* corrs, const double4* norm, const int32_t* samples,
-                                    const double* invK, double thr, double thr2, double* bestRT, cudaStream_t stream);
+                                    const double* invK, double thr, double thr2, double* bestRT, const RsRefineWork& w,
+                                    cudaStream_t stream);
 
 }  // namespace v3dm

@@ -9,11 +9,29 @@
 // CPU code (ess::refine_pose restates it and matches it inside the loop on every tested pair):
 //   - it is built without contraction into fused multiply-adds (the reference builds for plain
 //     x86-64), see the Makefile;
-//   - the sums over the inliers run in index order: the lanes of the warp compute the
-//     correspondences' residuals and Jacobian rows 32 at a time, stage them in shared memory,
-//     and lane q then accumulates quantity q (one of the 21 entries of J^T J, 6 of J^T e, and
-//     |e|^2) over them in order -- every sum has the sequential order of the reference's loops;
+//   - the sums over the inliers run in index order: seven warps compute the correspondences'
+//     residuals and Jacobian rows, 224 at a time, into shared memory, and lane q of the eighth
+//     accumulates quantity q (one of the 21 entries of J^T J, 6 of J^T e, the two |e|^2 below)
+//     over the previous 224 in order -- every sum has the sequential order of the reference's loops;
 //   - the rotation update's sin and cos are correctly rounded (ess::pose_update, device path).
+//
+// Which candidates are refined does not have to be known one at a time.  The loop accepts a
+// candidate whose cost lies below every accepted one's min(cost, refined cost), so the candidates
+// it can accept in a round are among the strict prefix minima of the round's raw costs (those
+// below the incoming minimum, in loop order, pose flag set), about ln(candidates) of them.
+//   k_rs_refine_tasks   one warp per pair lists them (kRsTasks per pair and round at most);
+//   k_rs_refine         a persistent CTA per task refines and scores each, all in parallel;
+//   k_rs_select_refine  walks the loop in order and picks up the results; a candidate that has
+//                       none (the list was full, or an earlier one's pose failed the exact test)
+//                       is refined there and then.
+// What bounds k_rs_refine: the order of the sums.  An inlier costs the summing warp two
+// shared-memory loads, a product and a dependent add; the other warps' divisions and square roots
+// run beside it.  A step of the Levenberg-Marquardt loop takes one sweep over the inliers: the
+// sweep that scores the step (weights of the old pose) also forms the normal equations the next
+// step needs if it is accepted (weights of the new pose).
+// On 256 pairs of 500 to 3000 correspondences these kernels take 12.0 ms of a call (k_rs_refine
+// 4.5 ms in the first round, 0.8 to 1.4 ms, a refinement's latency, in each later one); one warp
+// per pair that refined its candidates one after the other, two sweeps per step, took 178 ms.
 #include <cuda_runtime.h>
 
 #include "v3dm_essential.cuh"
@@ -41,23 +59,30 @@ __device__ void rs_fund(const double* invK1, const double* invK2t, const double*
     }
 }
 
-constexpr int kRsQuant = 28;  // 21 entries of J^T J (upper triangle), 6 of J^T e, |e|^2
+constexpr int kRsRefineThreads = 256;           // warp 0 sums, warps 1..7 produce
+constexpr int kRsProducers = kRsRefineThreads - 32;
+constexpr int kRsQuant = 29;   // 21 entries of J^T J (upper triangle), 6 of J^T e, |e|^2 under the new and the old weights
+constexpr int kRsEntry = 9;    // doubles per staged inlier: J (6), e (new weights), e (old weights), padding (odd: no bank conflicts)
+constexpr int kRsRow = 8;      // values of an entry
+static_assert(kRsRow < kRsEntry && kRsQuant <= 32, "entry layout");
 
-// One pass over the inliers of F0 (Sampson distance below thr2: the set the reference hands to
-// refineRelativePose, in index order): RelativePoseMinimizer's weights at pose (Rw, Tw) (from the
-// pixel positions and thr, ess::pose_weighted_residual), the weighted residuals at (R, T) and,
-// with derivs, the normal equations (ess::pose_normal_equations).  Every lane gets the sums.
-__device__ double rs_lm_pass(const float4* __restrict__ px, const double4* __restrict__ nm, int n, const double* F0,
-                             double thr2, const double* invK1, const double* invK2t, double thr, const double* Rw,
-                             const double* Tw, const double* R, const double* T, bool derivs, double* JtJ,
-                             double* Jte, double (*sv)[8]) {
-  const int lane = threadIdx.x & 31;
-  double Ew[9], Fw[9], E[9], inner[9][6], a[3], b[2];
-  ess::pose_essential(Rw, Tw, Ew);
-  rs_fund(invK1, invK2t, Ew, Fw);
-  ess::pose_essential(R, T, E);
-  if (derivs) ess::pose_inner(E, R, inner);
-  // the quantity this lane owns: JtJ[qa][qb] (qa <= qb), Jte[qa], or |e|^2
+struct RsShared {
+  double sv[2][kRsProducers * kRsEntry];  // staged inliers, double-buffered
+  double E[9], Fn[9], Fo[9], inner[9][6];  // the sweep's matrices: E and F at the pose, F of the old weights
+  double R[9], T[3], Rs[9], Ts[3];
+  double JtJ[36], Jte[6], sums[kRsQuant];
+  int warpCnt[kRsRefineThreads / 32];
+  int nIn, flag;
+};
+
+// One pass over the inliers list[0..nIn) at pose (s.R, s.T): the weighted residuals and, in s.sums,
+// the normal equations (ess::pose_jacobian_row, weights from the pixel positions under s.Fn) and
+// |e|^2, and |e|^2 with the weights under s.Fo.  The CTA enters and leaves together; s.E, s.Fn,
+// s.Fo and s.inner are set.
+__device__ void rs_sweep(RsShared& s, const float4* __restrict__ px, const double4* __restrict__ nm,
+                         const int32_t* __restrict__ list, double thr) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the quantity lane `lane` of warp 0 owns
   int qa = 0, qb = 0;
   if (lane < 21) {
     int t = lane;
@@ -68,206 +93,378 @@ __device__ double rs_lm_pass(const float4* __restrict__ px, const double4* __res
     qb = qa + t;
   } else if (lane < 27) {
     qa = lane - 21;
-    qb = 6;  // e
-  } else {
-    qa = 6;
     qb = 6;
+  } else {
+    qa = qb = lane == 28 ? 7 : 6;
   }
-  const bool owns = lane < kRsQuant && (derivs || lane == 27);
+  const int nIn = s.nIn, chunks = (nIn + kRsProducers - 1) / kRsProducers;
   double acc = 0.0;
-  for (int k0 = 0; k0 < n; k0 += 32) {
-    const int k = k0 + lane;
-    double J[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, e = 0.0;
+  for (int c = 0; c <= chunks; ++c) {
+    if (warp > 0) {
+      const int i = (int)threadIdx.x - 32, k = c * kRsProducers + i;
+      if (c < chunks && k < nIn) {
+        double* o = s.sv[c & 1] + i * kRsEntry;
+        const int idx = list[k];
+        const float4 p = px[idx];
+        const double4 q = nm[idx];
+        double a[3], b[2], J[6];
+        const double en = ess::pose_residual(s.Fn, p.x, p.y, p.z, p.w, a, b);
+        const double eo = ess::pose_residual(s.Fo, p.x, p.y, p.z, p.w, a, b);
+        const double wn = (fabs(en) < thr) ? 1.0 : sqrt(thr / fabs(en));
+        const double wo = (fabs(eo) < thr) ? 1.0 : sqrt(thr / fabs(eo));
+        const double f = 0.0 - ess::pose_residual(s.E, q.x, q.y, q.z, q.w, a, b);
+        ess::pose_jacobian_row(s.E, s.inner, q.x, q.y, q.z, q.w, J);
+        for (int j = 0; j < 6; ++j) o[j] = J[j];
+        o[6] = wn * f;
+        o[7] = wo * f;
+      }
+    } else if (c > 0) {
+      const double* v = s.sv[(c - 1) & 1];
+      const int m = min(kRsProducers, nIn - (c - 1) * kRsProducers);
+#pragma unroll 8
+      for (int i = 0; i < m; ++i) acc += v[i * kRsEntry + qa] * v[i * kRsEntry + qb];
+    }
+    __syncthreads();
+  }
+  if (warp == 0 && lane < kRsQuant) s.sums[lane] = acc;
+  __syncthreads();
+}
+
+// s.E, s.inner and s.Fn from the pose (s.R, s.T).
+__device__ void rs_matrices(RsShared& s, const double* invK1, const double* invK2t) {
+  if (threadIdx.x == 0) {
+    double E[9], F[9];
+    ess::pose_essential(s.R, s.T, E);
+    rs_fund(invK1, invK2t, E, F);
+    for (int k = 0; k < 9; ++k) {
+      s.E[k] = E[k];
+      s.Fn[k] = F[k];
+    }
+    ess::pose_inner(E, s.R, s.inner);
+  }
+  __syncthreads();
+}
+
+// refineRelativePose on the inliers of F0 (Sampson distance below thr2, in index order; their
+// indices go to list, room for n): ess::refine_pose's Levenberg-Marquardt loop
+// (SimpleLevenbergOptimizer's damping schedule and stopping rules) from the pose in (s.R, s.T).
+__device__ void rs_refine_cta(RsShared& s, const float4* __restrict__ px, const double4* __restrict__ nm, int n,
+                              const double* F0, double thr2, const double* invK1, const double* invK2t, double thr,
+                              int32_t* __restrict__ list) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int base = 0;
+  for (int k0 = 0; k0 < n; k0 += kRsRefineThreads) {
+    const int k = k0 + (int)threadIdx.x;
     bool in = false;
     if (k < n) {
       const float4 c = px[k];
       in = ess::sampson(F0, c.x, c.y, c.z, c.w) < thr2;
-      if (in) {
-        const double4 q = nm[k];
-        const double ew = ess::pose_residual(Fw, c.x, c.y, c.z, c.w, a, b);
-        const double w = (fabs(ew) < thr) ? 1.0 : sqrt(thr / fabs(ew));
-        e = w * (0.0 - ess::pose_residual(E, q.x, q.y, q.z, q.w, a, b));
-        if (derivs) ess::pose_jacobian_row(E, inner, q.x, q.y, q.z, q.w, J);
-      }
     }
-    const unsigned inMask = __ballot_sync(0xffffffffu, in);
-    __syncwarp();
-    for (int j = 0; j < 6; ++j) sv[lane][j] = J[j];
-    sv[lane][6] = e;
-    __syncwarp();
-    if (owns) {
-      for (unsigned m = inMask; m; m &= m - 1) {  // the inliers of this chunk, in index order
-        const int l = __ffs(m) - 1;
-        acc += sv[l][qa] * sv[l][qb];
-      }
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) s.warpCnt[warp] = __popc(m);
+    __syncthreads();
+    int before = base, total = 0;
+    for (int w = 0; w < kRsRefineThreads / 32; ++w) {
+      if (w < warp) before += s.warpCnt[w];
+      total += s.warpCnt[w];
     }
+    if (in) list[before + __popc(m & ((1u << lane) - 1))] = k;
+    base += total;
+    __syncthreads();
   }
-  if (derivs) {
-    for (int t = 0; t < 21; ++t) {
-      const double v = __shfl_sync(0xffffffffu, acc, t);
-      int i = 0, r = t;
-      while (r >= 6 - i) {
-        r -= 6 - i;
-        ++i;
-      }
-      JtJ[6 * i + i + r] = v;
-      JtJ[6 * (i + r) + i] = v;
-    }
-    for (int t = 0; t < 6; ++t) Jte[t] = __shfl_sync(0xffffffffu, acc, 21 + t);
-  }
-  return __shfl_sync(0xffffffffu, acc, 27);
-}
-
-// refineRelativePose on the inliers of F0: ess::refine_pose's Levenberg-Marquardt loop
-// (SimpleLevenbergOptimizer's damping schedule and stopping rules), warp-uniform.
-__device__ void rs_refine_warp(const float4* __restrict__ px, const double4* __restrict__ nm, int n, const double* F0,
-                               double thr2, const double* invK1, const double* invK2t, double thr, double* R,
-                               double* T, double (*sv)[8]) {
-  double lambda = 1e-3, JtJ[36], Jte[6], N[36], delta[6], Rs[9], Ts[3];
-  bool computeDerivatives = true;
+  if (threadIdx.x == 0) s.nIn = base;
+  rs_matrices(s, invK1, invK2t);
+  if (threadIdx.x < 9) s.Fo[threadIdx.x] = s.Fn[threadIdx.x];
+  __syncthreads();
+  rs_sweep(s, px, nm, list, thr);
+  // the loop's scalars live in thread 0
+  double lambda = 1e-3, err = 0.0, delta[6];
+  bool fresh = true;  // s.sums holds the normal equations at (s.R, s.T)
   for (int it = 0; it < 50; ++it) {
-    const double err =
-        rs_lm_pass(px, nm, n, F0, thr2, invK1, invK2t, thr, R, T, R, T, computeDerivatives, JtJ, Jte, sv);
-    double gmax = 0.0;
-    for (int k = 0; k < 6; ++k) gmax = fmax(gmax, fabs(Jte[k]));
-    if (gmax < 1e-8) return;
-    if (it == 0) {
-      double maxEl = -1e30;
-      for (int k = 0; k < 6; ++k) maxEl = fmax(maxEl, JtJ[7 * k]);
-      lambda = 1e-3 * maxEl;
+    if (threadIdx.x == 0) {
+      if (fresh) {
+        for (int t = 0; t < 21; ++t) {
+          int i = 0, r = t;
+          while (r >= 6 - i) {
+            r -= 6 - i;
+            ++i;
+          }
+          s.JtJ[6 * i + i + r] = s.sums[t];
+          s.JtJ[6 * (i + r) + i] = s.sums[t];
+        }
+        for (int t = 0; t < 6; ++t) s.Jte[t] = s.sums[21 + t];
+        err = s.sums[27];
+      }
+      bool go = true;
+      double gmax = 0.0;
+      for (int k = 0; k < 6; ++k) gmax = fmax(gmax, fabs(s.Jte[k]));
+      if (gmax < 1e-8) go = false;
+      if (go) {
+        if (it == 0) {
+          double maxEl = -1e30;
+          for (int k = 0; k < 6; ++k) maxEl = fmax(maxEl, s.JtJ[7 * k]);
+          lambda = 1e-3 * maxEl;
+        }
+        double N[36];
+        for (int k = 0; k < 36; ++k) N[k] = s.JtJ[k];
+        for (int k = 0; k < 6; ++k) N[7 * k] += lambda;
+        go = ess::cholesky_solve6(N, s.Jte, delta);
+      }
+      if (go) {
+        double dl = 0.0;
+        for (int k = 0; k < 6; ++k) dl += delta[k] * delta[k];
+        dl = sqrt(dl);
+        if (it >= 10 && dl < 1e-8 * (4.0 + 1e-8)) go = false;
+      }
+      if (go) {
+        for (int k = 0; k < 9; ++k) s.Rs[k] = s.R[k];
+        for (int k = 0; k < 3; ++k) s.Ts[k] = s.T[k];
+        ess::pose_update(s.Rs, s.Ts, delta, s.R, s.T);
+      }
+      s.flag = go;
     }
-    for (int k = 0; k < 36; ++k) N[k] = JtJ[k];
-    for (int k = 0; k < 6; ++k) N[7 * k] += lambda;
-    if (!ess::cholesky_solve6(N, Jte, delta)) return;
-    double dl = 0.0;
-    for (int k = 0; k < 6; ++k) dl += delta[k] * delta[k];
-    dl = sqrt(dl);
-    if (it >= 10 && dl < 1e-8 * (4.0 + 1e-8)) return;
-    for (int k = 0; k < 9; ++k) Rs[k] = R[k];
-    for (int k = 0; k < 3; ++k) Ts[k] = T[k];
-    ess::pose_update(Rs, Ts, delta, R, T);
-    const double errNew =
-        rs_lm_pass(px, nm, n, F0, thr2, invK1, invK2t, thr, Rs, Ts, R, T, false, nullptr, nullptr, sv);
-    double rho = err - errNew;
-    double d1 = 0.0, d2 = 0.0;
-    for (int k = 0; k < 6; ++k) {
-      d1 += delta[k] * delta[k];
-      d2 += delta[k] * Jte[k];
+    __syncthreads();
+    if (!s.flag) return;  // uniform
+    rs_matrices(s, invK1, invK2t);  // s.Fo stays: the weights of the pose before the step
+    rs_sweep(s, px, nm, list, thr);
+    if (threadIdx.x == 0) {
+      const double errNew = s.sums[28];
+      double rho = err - errNew;
+      double d1 = 0.0, d2 = 0.0;
+      for (int k = 0; k < 6; ++k) {
+        d1 += delta[k] * delta[k];
+        d2 += delta[k] * s.Jte[k];
+      }
+      rho = rho / (lambda * d1 + d2);
+      fresh = rho > 0;
+      if (fresh) {
+        lambda = fmax(1e-10, lambda * 0.1);
+        for (int k = 0; k < 9; ++k) s.Fo[k] = s.Fn[k];
+      } else {
+        for (int k = 0; k < 9; ++k) s.R[k] = s.Rs[k];
+        for (int k = 0; k < 3; ++k) s.T[k] = s.Ts[k];
+        lambda *= 10.0;
+      }
     }
-    rho = rho / (lambda * d1 + d2);
-    if (rho > 0) {
-      lambda = fmax(1e-10, lambda * 0.1);
-      computeDerivatives = true;
-    } else {
-      for (int k = 0; k < 9; ++k) R[k] = Rs[k];
-      for (int k = 0; k < 3; ++k) T[k] = Ts[k];
-      lambda *= 10.0;
-      computeDerivatives = false;
-    }
+    // thread 0 alone reads s.sums, s.JtJ and the pose until the next barrier
   }
+  __syncthreads();
 }
 
 // sum_i min(d_i, thr2) over all correspondences in index order (the loop's sum, as k_rs_score
-// forms it) and the count of d_i < thr2; every lane gets both.
-__device__ void rs_cost_in_order(const float4* __restrict__ px, int n, const double* F, double thr2, double* cost,
-                                 int* nIn) {
-  const int lane = threadIdx.x & 31;
+// forms it) and the count of d_i < thr2; every thread gets both.
+__device__ void rs_cost_in_order(RsShared& s, const float4* __restrict__ px, int n, const double* F, double thr2,
+                                 double* cost, int* nIn) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunks = (n + kRsProducers - 1) / kRsProducers;
   double sum = 0.0;
   int cnt = 0;
-  for (int k0 = 0; k0 < n; k0 += 32) {
-    double t = 0.0;
-    bool in = false;
-    if (k0 + lane < n) {
-      const float4 c = px[k0 + lane];
-      t = ess::sampson_truncated(F, (double)c.x, (double)c.y, (double)c.z, (double)c.w, thr2, in);
+  for (int c = 0; c <= chunks; ++c) {
+    if (warp > 0) {
+      const int i = (int)threadIdx.x - 32, k = c * kRsProducers + i;
+      if (c < chunks && k < n) {
+        const float4 p = px[k];
+        bool in;
+        s.sv[c & 1][i] = ess::sampson_truncated(F, (double)p.x, (double)p.y, (double)p.z, (double)p.w, thr2, in);
+        cnt += in;
+      }
+    } else if (c > 0) {
+      const double* v = s.sv[(c - 1) & 1];
+      const int m = min(kRsProducers, n - (c - 1) * kRsProducers);
+#pragma unroll 8
+      for (int i = 0; i < m; ++i) sum = ess::dadd(sum, v[i]);
     }
-    cnt += __popc(__ballot_sync(0xffffffffu, in));
-    const int m = min(32, n - k0);
-    for (int l = 0; l < m; ++l) sum = ess::dadd(sum, __shfl_sync(0xffffffffu, t, l));
+    __syncthreads();
   }
-  *cost = sum;
-  *nIn = cnt;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  if (lane == 0) s.warpCnt[warp] = cnt;
+  if (threadIdx.x == 0) s.sums[0] = sum;
+  __syncthreads();
+  *cost = s.sums[0];
+  int total = 0;
+  for (int w = 0; w < kRsRefineThreads / 32; ++w) total += s.warpCnt[w];
+  *nIn = total;
+  __syncthreads();
 }
 
-// One warp per pair: the round's costs and pose flags staged in shared memory, then every lane
-// walks the loop over the round's samples in order (the same decisions on every lane), and the
-// warp refines each accepted pose.
-__global__ void __launch_bounds__(32)
-k_rs_select_refine(const int32_t* __restrict__ offsets, int nDraw, int s0, int len, const int8_t* __restrict__ counts,
-                   const uint8_t* __restrict__ slotOk, const double* __restrict__ cost,
-                   const double* __restrict__ slots, RsState* __restrict__ st, double* __restrict__ bestEF,
-                   const float4* __restrict__ corrs, const double4* __restrict__ norm,
-                   const int32_t* __restrict__ samples, const double* __restrict__ invK, double thr, double thr2,
-                   double* __restrict__ bestRT) {
-  const int p = blockIdx.x;
-  const int lane = threadIdx.x;
-  __shared__ double sCost[kRsRound * kRsMaxSol];
-  __shared__ uint8_t sOk[kRsRound * kRsMaxSol];
-  __shared__ int8_t sCnt[kRsRound];
-  __shared__ double sv[32][8];
-  RsState s = st[p];
-  if (s.done) return;  // uniform over the warp
-  const long long base = (long long)p * kRsRound;
-  for (int j = lane; j < len; j += 32) sCnt[j] = counts[base + j];
-  __syncwarp();
-  for (int idx = lane; idx < len * kRsMaxSol; idx += 32) {
-    const int j = idx / kRsMaxSol, r = idx - j * kRsMaxSol;
-    if (r < sCnt[j]) {
-      sCost[idx] = cost[base * kRsMaxSol + idx];
-      sOk[idx] = slotOk[base * kRsMaxSol + idx];
-    }
-  }
-  __syncwarp();
+// Candidate idx (sample j, solution r) of pair p: its pose on the sample, the refinement on the
+// inliers of its F, the refined model and its cost.  o.ok = 0 when the sample's correspondences
+// do not agree on a pose (the loop skips the candidate).  The CTA enters and leaves together.
+__device__ void rs_refine_candidate(RsShared& s, int p, int idx, const int32_t* __restrict__ offsets, int nDraw,
+                                    int s0, const double* __restrict__ slots, const float4* __restrict__ corrs,
+                                    const double4* __restrict__ norm, const int32_t* __restrict__ samples,
+                                    const double* __restrict__ invK, double thr, double thr2,
+                                    int32_t* __restrict__ list, RsRefined* __restrict__ o) {
   const int b = offsets[p], n = offsets[p + 1] - b;
   double invK1[9], invK2t[9];
   for (int k = 0; k < 9; ++k) invK1[k] = invK[(size_t)p * 18 + k];
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) invK2t[3 * i + j] = invK[(size_t)p * 18 + 9 + 3 * j + i];
-  for (int j = 0; j < len; ++j) {
-    if (s.drawn > s.budget) break;
-    ++s.drawn;
-    const int ns = sCnt[j];
-    for (int r = 0; r < ns; ++r) {
-      const int idx = j * kRsMaxSol + r;
-      if (!(sCost[idx] < s.minError)) continue;
-      if (!sOk[idx]) continue;
-      double EF[kRsSlotDoubles];
-      for (int k = 0; k < kRsSlotDoubles; ++k) EF[k] = slots[(base * kRsMaxSol + idx) * kRsSlotDoubles + k];
-      const int32_t* smp = samples + ((long long)p * nDraw + s0 + j) * 5;
-      double x1[5], y1[5], x2[5], y2[5];
-      for (int k = 0; k < 5; ++k) {
-        const double4 v = norm[b + smp[k]];
-        x1[k] = v.x;
-        y1[k] = v.y;
-        x2[k] = v.z;
-        y2[k] = v.w;
+  const double* EF = slots + ((long long)p * kRsRound * kRsMaxSol + idx) * kRsSlotDoubles;
+  if (threadIdx.x == 0) {
+    const int32_t* smp = samples + ((long long)p * nDraw + s0 + idx / kRsMaxSol) * 5;
+    double x1[5], y1[5], x2[5], y2[5], E[9], R[9], T[3];
+    for (int k = 0; k < 5; ++k) {
+      const double4 v = norm[b + smp[k]];
+      x1[k] = v.x;
+      y1[k] = v.y;
+      x2[k] = v.z;
+      y2[k] = v.w;
+    }
+    for (int k = 0; k < 9; ++k) E[k] = EF[k];
+    s.flag = ess::essential_pose(E, 5, x1, y1, x2, y2, R, T);  // relativePoseFromEssential
+    for (int k = 0; k < 9; ++k) s.R[k] = R[k];
+    for (int k = 0; k < 3; ++k) s.T[k] = T[k];
+  }
+  __syncthreads();
+  const int ok = s.flag;
+  __syncthreads();
+  if (!ok) {
+    if (threadIdx.x == 0) o->ok = 0;
+    return;
+  }
+  double F0[9];
+  for (int k = 0; k < 9; ++k) F0[k] = EF[9 + k];
+  rs_refine_cta(s, corrs + b, norm + b, n, F0, thr2, invK1, invK2t, thr, list);
+  rs_matrices(s, invK1, invK2t);
+  double F[9], cost;
+  int nIn;
+  for (int k = 0; k < 9; ++k) F[k] = s.Fn[k];
+  rs_cost_in_order(s, corrs + b, n, F, thr2, &cost, &nIn);
+  if (threadIdx.x < 9) {
+    o->EF[threadIdx.x] = s.E[threadIdx.x];
+    o->EF[9 + threadIdx.x] = s.Fn[threadIdx.x];
+    o->RT[threadIdx.x] = s.R[threadIdx.x];
+  } else if (threadIdx.x < 12) {
+    o->RT[threadIdx.x] = s.T[threadIdx.x - 9];
+  }
+  if (threadIdx.x == 0) {
+    o->cost = cost;
+    o->nIn = nIn;
+    o->ok = 1;
+  }
+  __syncthreads();
+}
+
+// The round's candidates of a pair in shared memory, in loop order: the cost, or +inf where the
+// slot is empty or its pose flag is not set.
+__device__ void rs_stage_costs(double* sCost, long long base, int len, const int8_t* __restrict__ counts,
+                               const uint8_t* __restrict__ slotOk, const double* __restrict__ cost) {
+  for (int idx = threadIdx.x; idx < kRsRound * kRsMaxSol; idx += blockDim.x) {
+    const int j = idx / kRsMaxSol, r = idx - j * kRsMaxSol;
+    const bool have = j < len && r < counts[base + j] && slotOk[base * kRsMaxSol + idx];
+    sCost[idx] = have ? cost[base * kRsMaxSol + idx] : INFINITY;
+  }
+}
+
+// The samples the loop draws in a round of len: until one more than the budget has been drawn.
+__device__ __forceinline__ int rs_used(const RsState& s, int len) {
+  return len <= s.budget - s.drawn ? len : s.budget - s.drawn + 1;
+}
+
+// The first candidate in [from, limit) whose cost is below minError, or limit.  Whole warps, the
+// same result on every lane.
+__device__ int rs_next_below(const double* sCost, int from, int limit, double minError) {
+  const int lane = threadIdx.x & 31;
+  for (int i0 = from; i0 < limit; i0 += 32) {
+    const unsigned m = __ballot_sync(0xffffffffu, i0 + lane < limit && sCost[i0 + lane] < minError);
+    if (m) return i0 + __ffs(m) - 1;
+  }
+  return limit;
+}
+
+// One warp per pair: the strict prefix minima of the round's costs below the incoming minimum,
+// in loop order, as tasks.
+__global__ void __launch_bounds__(32)
+k_rs_refine_tasks(int len, const int8_t* __restrict__ counts, const uint8_t* __restrict__ slotOk,
+                  const double* __restrict__ cost, const RsState* __restrict__ st, int32_t* __restrict__ taskIdx,
+                  int32_t* __restrict__ taskN, int2* __restrict__ tasks, int* __restrict__ nTasks) {
+  const int p = blockIdx.x, lane = threadIdx.x;
+  __shared__ double sCost[kRsRound * kRsMaxSol];
+  const RsState s = st[p];
+  int n = 0;
+  if (!s.done) {  // uniform over the warp
+    rs_stage_costs(sCost, (long long)p * kRsRound, len, counts, slotOk, cost);
+    __syncwarp();
+    const int limit = rs_used(s, len) * kRsMaxSol;
+    double minError = s.minError;
+    for (int idx = rs_next_below(sCost, 0, limit, minError); idx < limit && n < kRsTasks;
+         idx = rs_next_below(sCost, idx + 1, limit, minError)) {
+      minError = sCost[idx];
+      if (lane == 0) {
+        taskIdx[p * kRsTasks + n] = idx;
+        tasks[atomicAdd(nTasks, 1)] = make_int2(p * kRsTasks + n, idx);
       }
-      double R[9], T[3];
-      if (!ess::essential_pose(EF, 5, x1, y1, x2, y2, R, T)) continue;  // relativePoseFromEssential
-      rs_refine_warp(corrs + b, norm + b, n, EF + 9, thr2, invK1, invK2t, thr, R, T, sv);
-      double Er[9], Fr[9], costR;
-      int nInR;
-      ess::pose_essential(R, T, Er);
-      rs_fund(invK1, invK2t, Er, Fr);
-      rs_cost_in_order(corrs + b, n, Fr, thr2, &costR, &nInR);
-      s.minError = fmin(sCost[idx], costR);
-      s.chosen = s0 + j;
-      const float frac = (float)(nInR - 5) / (float)(n - 5);
-      s.budget = min(s.budget, rs_budget(1.0 - (double)frac));
-      double* ef = bestEF + (size_t)p * kRsSlotDoubles;
-      double* rt = bestRT + (size_t)p * 12;
-      if (lane < 9) {
-        ef[lane] = Er[lane];
-        ef[9 + lane] = Fr[lane];
-        rt[lane] = R[lane];
-      } else if (lane < 12) {
-        rt[lane] = T[lane - 9];
-      }
+      ++n;
     }
   }
-  if (lane == 0) {
-    if (s.drawn > s.budget || s0 + len >= nDraw) s.done = 1;  // the next sample would end the loop
-    st[p] = s;
+  if (lane == 0) taskN[p] = n;
+}
+
+// Persistent CTAs over the tasks; listRoom ints of inlier indices per CTA.
+__global__ void __launch_bounds__(kRsRefineThreads, 2)
+k_rs_refine(const int32_t* __restrict__ offsets, int nDraw, int s0, const double* __restrict__ slots,
+            const float4* __restrict__ corrs, const double4* __restrict__ norm, const int32_t* __restrict__ samples,
+            const double* __restrict__ invK, double thr, double thr2, const int2* __restrict__ tasks,
+            const int* __restrict__ nTasks, int32_t* __restrict__ lists, long long listRoom,
+            RsRefined* __restrict__ refined) {
+  __shared__ RsShared s;
+  const int n = *nTasks;
+  for (int t = blockIdx.x; t < n; t += gridDim.x) {
+    const int2 task = tasks[t];
+    rs_refine_candidate(s, task.x / kRsTasks, task.y, offsets, nDraw, s0, slots, corrs, norm, samples, invK, thr, thr2,
+                        lists + (long long)blockIdx.x * listRoom, refined + task.x);
+  }
+}
+
+// The loop over the round's candidates in order (reconstruction_common.cpp:177-335), a CTA per pair
+// at a time; every warp walks the same decisions.
+__global__ void __launch_bounds__(kRsRefineThreads, 2)
+k_rs_select_refine(const int32_t* __restrict__ offsets, int nPairs, int nDraw, int s0, int len,
+                   const int8_t* __restrict__ counts, const uint8_t* __restrict__ slotOk,
+                   const double* __restrict__ cost, const double* __restrict__ slots, RsState* __restrict__ st,
+                   double* __restrict__ bestEF, const float4* __restrict__ corrs, const double4* __restrict__ norm,
+                   const int32_t* __restrict__ samples, const double* __restrict__ invK, double thr, double thr2,
+                   double* __restrict__ bestRT, const int32_t* __restrict__ taskIdx, const int32_t* __restrict__ taskN,
+                   int32_t* __restrict__ lists, long long listRoom, RsRefined* __restrict__ refined) {
+  __shared__ RsShared sh;
+  __shared__ double sCost[kRsRound * kRsMaxSol];
+  for (int p = blockIdx.x; p < nPairs; p += gridDim.x) {
+    RsState s = st[p];
+    __syncthreads();  // every thread has read the state; sCost is free
+    if (s.done) continue;  // uniform
+    rs_stage_costs(sCost, (long long)p * kRsRound, len, counts, slotOk, cost);
+    __syncthreads();
+    const int n = offsets[p + 1] - offsets[p];
+    const int nt = taskN[p];
+    int t = 0, used = rs_used(s, len);
+    for (int idx = rs_next_below(sCost, 0, used * kRsMaxSol, s.minError); idx < used * kRsMaxSol;
+         idx = rs_next_below(sCost, idx + 1, used * kRsMaxSol, s.minError)) {
+      while (t < nt && taskIdx[p * kRsTasks + t] < idx) ++t;
+      const bool have = t < nt && taskIdx[p * kRsTasks + t] == idx;
+      RsRefined* o = refined + (have ? p * kRsTasks + t : nPairs * kRsTasks + (int)blockIdx.x);
+      if (!have) {
+        rs_refine_candidate(sh, p, idx, offsets, nDraw, s0, slots, corrs, norm, samples, invK, thr, thr2,
+                            lists + (long long)blockIdx.x * listRoom, o);
+        __syncthreads();
+      }
+      if (!o->ok) continue;
+      s.minError = fmin(sCost[idx], o->cost);
+      const int j = idx / kRsMaxSol;
+      s.chosen = s0 + j;
+      const float frac = (float)(o->nIn - 5) / (float)(n - 5);
+      s.budget = min(s.budget, rs_budget(1.0 - (double)frac));
+      used = max(j + 1, rs_used(s, len));
+      if (threadIdx.x < kRsSlotDoubles) bestEF[(size_t)p * kRsSlotDoubles + threadIdx.x] = o->EF[threadIdx.x];
+      if (threadIdx.x < 12) bestRT[(size_t)p * 12 + threadIdx.x] = o->RT[threadIdx.x];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      s.drawn += used;
+      if (s.drawn > s.budget || s0 + len >= nDraw) s.done = 1;  // the next sample would end the loop
+      st[p] = s;
+    }
   }
 }
 
@@ -276,10 +473,17 @@ k_rs_select_refine(const int32_t* __restrict__ offsets, int nDraw, int s0, int l
 cudaError_t launch_rs_select_refine(const int32_t* offsets, int nPairs, int nDraw, int s0, int len, const int8_t* counts,
                                     const uint8_t* slotOk, const double* cost, const double* slots, RsState* st,
                                     double* bestEF, const float4* corrs, const double4* norm, const int32_t* samples,
-                                    const double* invK, double thr, double thr2, double* bestRT, cudaStream_t stream) {
+                                    const double* invK, double thr, double thr2, double* bestRT, const RsRefineWork& w,
+                                    cudaStream_t stream) {
   if (nPairs <= 0) return cudaSuccess;
-  k_rs_select_refine<<<nPairs, 32, 0, stream>>>(offsets, nDraw, s0, len, counts, slotOk, cost, slots, st, bestEF,
-                                                corrs, norm, samples, invK, thr, thr2, bestRT);
+  cudaError_t e = cudaMemsetAsync(w.nTasks, 0, sizeof(int), stream);
+  if (e != cudaSuccess) return e;
+  k_rs_refine_tasks<<<nPairs, 32, 0, stream>>>(len, counts, slotOk, cost, st, w.taskIdx, w.taskN, w.tasks, w.nTasks);
+  k_rs_refine<<<w.ctas, kRsRefineThreads, 0, stream>>>(offsets, nDraw, s0, slots, corrs, norm, samples, invK, thr, thr2,
+                                                       w.tasks, w.nTasks, w.lists, w.listRoom, w.refined);
+  k_rs_select_refine<<<nPairs < w.ctas ? nPairs : w.ctas, kRsRefineThreads, 0, stream>>>(
+      offsets, nPairs, nDraw, s0, len, counts, slotOk, cost, slots, st, bestEF, corrs, norm, samples, invK, thr, thr2,
+      bestRT, w.taskIdx, w.taskN, w.lists, w.listRoom, w.refined);
   return cudaGetLastError();
 }
 
