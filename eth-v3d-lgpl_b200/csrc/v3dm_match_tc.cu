@@ -7,9 +7,10 @@
 //   warp 0      TMA producer: an A group (NB blocks of 128 descriptors x 128 bytes) whenever
 //               the group changes, B tiles (BN x 128 bytes) through a ring of shared-memory
 //               stages, 128-byte swizzle;
-//   warp 1      allocates 512 TMEM columns and issues tcgen05.mma.kind::i8 (u8 x u8 -> s32,
-//               M=128, N=BN, four K=32 steps per block) into 512/(NB*BN) accumulator stages;
-//   warps 2-17  epilogue, four per TMEM lane quadrant.  Lane i of a warp owns A descriptor
+//   warps 1-2   (warp 1 allocates 512 TMEM columns) issue tcgen05.mma.kind::i8 (u8 x u8 -> s32,
+//               M=128, N=BN, four K=32 steps per block) into 512/(NB*BN) accumulator stages,
+//               alternate tiles each;
+//   warps 3-18  epilogue, four per TMEM lane quadrant.  Lane i of a warp owns A descriptor
 //               'row' and reads its scores with tcgen05.ld (32 columns per chunk), hands the
 //               stage back, and per chunk does one of two things:
 //                 - all scores below Smin (the smallest score that can pass the min-score
@@ -33,7 +34,18 @@
 // (TcConfig).  NB=2 keeps 256 A rows resident and halves the B bytes per MMA compared with one
 // 128-row block; more TMEM stages hide the MMA -> epilogue -> MMA hand-off latency.
 // The work is the flattened sequence (A group, B tile); each CTA takes one contiguous range
-// of it.  Every role walks the same range; mbarriers order the hand-offs.  Every mbarrier wait
+// of it.  Every role walks the same range; mbarriers order the hand-offs.
+// What bounds the kernel is each role's own instruction latency per tile, not a pipe: a tile is 512
+// tensor cycles, and a warp's wait, commit or branch is 50 to 100.  So the walk is two loops, an
+// outer one over runs of tiles that share their A group and an inner one over a run's tiles, in
+// which ring slots and parities come from one tile counter; one commit per tile tells the producer
+// and the epilogue; and two issuers share the tiles.  Measured per tile and issuer before: 510
+// cycles in a cursor that was advanced at every tile, 180 in two commits, 120 in each wait, 70 in
+// the MMAs.  32768^2 went from 140 to 97 us (2833 TOPS, 85% of twice the bf16 burst), pass A of 120
+// images (1000 to 12000 features) from 39.1 to 29.3 ms; without the epilogue's filtering a tile takes
+// 523 of its 512 cycles, with it 710, so the epilogue's maxima are what is left.  On 200 images the
+// 1 kW limit holds the SM clock at about 1600 MHz.  Pairs of CTAs on one 256 x 256 tile
+// (cta_group::2) took 190 us for 32768^2, and epilogue groups on alternate tiles 102.  Every mbarrier wait
 // is bounded: on timeout the CTA raises kErrWaitTimeout, drains its own TMA loads and MMAs,
 // frees TMEM and returns.
 #include <cuda.h>
@@ -52,44 +64,44 @@ namespace {
 
 constexpr int BM = 128;          // rows per MMA block (TMEM lanes)
 constexpr int kEpiWarps = 16;    // four per TMEM lane quadrant
-constexpr int kThreads = (2 + kEpiWarps) * 32;
+constexpr int kIssuers = 2;      // MMA issuer warps, taking alternate tiles
+constexpr int kEpiWarp0 = 1 + kIssuers;
+constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;
 constexpr int kTmemCols = 512;
 
-template <int NB_, int BN_, int STAGES_, int ASLOTS_ = 2, int SPLIT_ = 1, int PIPE_ = 0>
+template <int NB_, int BN_, int STAGES_, int ASLOTS_ = 2, int PIPE_ = 0>
 struct TcCfg {
   static constexpr int NB = NB_;                 // 128-row MMA blocks per left group
   static constexpr int BN = BN_;                 // rights per tile
   static constexpr int kStages = STAGES_;        // right-tile ring depth
   static constexpr int kASlots = ASLOTS_;        // left-group buffers (more: short rows prefetch further)
-  // kSplit = 2: each tile is scored as two BN/2-column MMAs into two accumulator stages, so the MMA
-  // can run further ahead of the epilogue (twice the stages of half the width)
-  static constexpr int kSplit = SPLIT_;
   // kPipe = 1: the epilogue loads its second chunk while it filters the first
   static constexpr int kPipe = PIPE_;
   static constexpr int GM = BM * NB;             // left rows per group
   static constexpr int kABytes = GM * kDescBytes;
   static constexpr int kBBytes = BN * kDescBytes;
-  static constexpr int kMmaN = BN / kSplit;      // columns of one MMA / accumulator block
-  static constexpr int kAccCols = NB * kMmaN;    // TMEM columns per accumulator stage
+  static constexpr int kAccCols = NB * BN;       // TMEM columns per accumulator stage
   static constexpr int kAcc = kTmemCols / kAccCols;  // accumulator stages
   // Epilogue split: the four warps of a lane quadrant own (block, column quarter or half) of a
   // stage: with NB == 2 a warp owns one block and half of the columns, with NB == 1 a quarter.
-  static constexpr int kWarpCols = NB == 2 ? kMmaN / 2 : kMmaN / 4;
+  static constexpr int kWarpCols = NB == 2 ? BN / 2 : BN / 4;
   static constexpr int kChunks = kWarpCols / 32;
   static_assert(NB == 1 || NB == 2, "one or two blocks per group");
-  static_assert(kSplit == 1 || (kSplit == 2 && NB == 1), "split tiles with one block per group");
   static_assert(kWarpCols >= 32 && kWarpCols % 32 == 0 && kChunks <= 2 && BN <= 256, "1..2 chunks per warp");
   static_assert(kPipe == 0 || kChunks == 2, "pipelined loads need two chunks");
   static_assert(kAcc >= 2, "at least two accumulator stages");
+  // done[] serves the producer and the epilogue: a stage's next tile must not complete before
+  // every epilogue warp has seen this one, which its accumulator's hand-back ensures
+  static_assert(kStages >= kAcc, "the B ring is at least as deep as the accumulator ring");
 };
 
 template <class C>
 struct Smem {
   uint8_t a[C::kASlots][C::kABytes];
   uint8_t b[C::kStages][C::kBBytes];
-  unsigned long long fullB[C::kStages], emptyB[C::kStages];
+  unsigned long long fullB[C::kStages], done[C::kStages];  // a tile has landed; its MMAs have completed
   unsigned long long fullA[C::kASlots], emptyA[C::kASlots];
-  unsigned long long accFull[C::kAcc], accEmpty[C::kAcc];
+  unsigned long long accEmpty[C::kAcc];
   unsigned long long mmaDone;
   uint32_t tmemBase;
   int abort;
@@ -148,28 +160,32 @@ __device__ __forceinline__ void cta_range(const TcShape& sh, long long& w0, long
   w1 = sh.nWork * (blockIdx.x + 1) / gridDim.x;
 }
 
-// Single pair: walks (group, tile) pairs of a work range with one division at the start, so
-// the per-tile loops of the MMA issuer and the epilogue stay free of 64-bit divisions.
+// Slot and parity of the i-th use of a ring of N.
+template <int N>
+__device__ __forceinline__ uint32_t ring_slot(uint32_t i) {
+  return i % (uint32_t)N;
+}
+template <int N>
+__device__ __forceinline__ uint32_t ring_parity(uint32_t i) {
+  return (i / (uint32_t)N) & 1u;
+}
+
+// Single pair: the runs of a work range, a run being the tiles t0 .. t0 + nT - 1 of one group.
 struct WorkCursor {
-  int g, t, nTiles;
-  long long left;
-  bool fresh;  // first tile of a group
-  bool newA;   // the group's A block differs from the previous one (always, with fresh)
-  __device__ __forceinline__ WorkCursor(long long w0, long long w1, int nT)
-      : nTiles(nT), left(w1 - w0), fresh(true), newA(true) {
-    g = (int)(w0 / nT);
-    t = (int)(w0 - (long long)g * nT);
+  int g, t0, nT, nTiles;
+  int left;     // tiles from this run on
+  static constexpr bool newA = true;  // the run's A block differs from the previous run's
+  __device__ __forceinline__ WorkCursor(long long w0, long long w1, int nT_) : nTiles(nT_), left((int)(w1 - w0)) {
+    g = (int)(w0 / nTiles);
+    t0 = (int)(w0 - (long long)g * nTiles);
+    nT = min(nTiles - t0, left);
   }
   __device__ __forceinline__ bool more() const { return left > 0; }
   __device__ __forceinline__ void next() {
-    --left;
-    fresh = false;
-    if (++t == nTiles) {
-      t = 0;
-      ++g;
-      fresh = true;
-    }
-    newA = fresh;
+    left -= nT;
+    ++g;
+    t0 = 0;
+    nT = min(nTiles, left);
   }
   __device__ __forceinline__ void prefetch_rows() const {}
 };
@@ -203,9 +219,11 @@ constexpr int kRowAhead = 6;    // the producer prefetches the row entry this ma
 // its first row aRow).
 struct BatchCursor {
   const BatchRow* rows;
-  int R, Rend, t, schedule;
+  int R, Rend, schedule;
   BatchRow cur, nxt;
-  bool fresh, newA;
+  static constexpr int t0 = 0;
+  int nT;
+  bool newA;
   __device__ __forceinline__ int step_from(int r) const {
     if (schedule == 0) return r + (int)gridDim.x;
     if (schedule == 1) return r + 1;
@@ -213,7 +231,7 @@ struct BatchCursor {
     return (r % kChunkRows) == 0 ? r + ((int)gridDim.x - 1) * kChunkRows : r;
   }
   __device__ __forceinline__ BatchCursor(const BatchRow* rows_, int nRows, int sch)
-      : rows(rows_), t(0), schedule(sch), fresh(true), newA(true) {
+      : rows(rows_), schedule(sch), newA(true) {
     cur = BatchRow{};
     nxt = BatchRow{};
     if (schedule == 0) {
@@ -229,20 +247,16 @@ struct BatchCursor {
     if (R < Rend) cur = load_row(rows, R);
     const int R1 = step_from(R);
     if (R1 < Rend) nxt = load_row(rows, R1);
+    nT = cur.nTiles;
   }
   __device__ __forceinline__ bool more() const { return R < Rend; }
   __device__ __forceinline__ void next() {
-    fresh = false;
-    newA = false;
-    if (++t == cur.nTiles) {
-      t = 0;
-      R = step_from(R);
-      fresh = true;
-      newA = nxt.aRow != cur.aRow;
-      cur = nxt;
-      const int R1 = step_from(R);
-      if (R1 < Rend) nxt = load_row(rows, R1);
-    }
+    R = step_from(R);
+    newA = nxt.aRow != cur.aRow;
+    cur = nxt;
+    nT = cur.nTiles;
+    const int R1 = step_from(R);
+    if (R1 < Rend) nxt = load_row(rows, R1);
   }
   // The row entry kRowAhead rows ahead, into L1 (the other roles of the CTA read it later).
   __device__ __forceinline__ void prefetch_rows() const {
@@ -273,6 +287,45 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// The chunks of one lane's scores (columns col0 ..) one by one: a chunk with a score >= sminRow goes
+// to the warp's segment as a record (k_records does its exact work), otherwise its maximum is
+// folded into lw.
+template <int CHUNKS>
+__device__ __forceinline__ void filter_chunks(uint32_t (&v)[CHUNKS][32], int colBase, int nB, int bRow0, int orig,
+                                           int32_t sminRow, uint32_t& lw, int& segN, uint4* segBase,
+                                           long long segCap) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const int col0 = colBase + 32 * c;
+    if (col0 >= nB) break;  // chunks past the last B descriptor (warp-uniform)
+    if (col0 + 32 > nB) {
+      // The chunk holding the last B descriptor: the columns past it hold zero fill, zero
+      // padding or the next block's descriptors; a 0 there is <= every real score, so the
+      // chunk maximum stays the maximum of its real scores.
+#pragma unroll
+      for (int k = 0; k < 32; ++k)
+        if (col0 + k >= nB) v[c][k] = 0u;
+    }
+    const uint32_t cm = max32_bits(v[c], lw);  // max(lw, chunk maximum)
+    const bool trig = (int32_t)cm >= sminRow;
+    if (!trig) lw = cm;
+    const unsigned m = __ballot_sync(0xffffffffu, trig);
+    if (m == 0u) continue;
+    if (trig) {
+      const int idx = segN + __popc(m & ((1u << lane) - 1u));
+      if (idx < segCap) {
+        uint4* rec = segBase + (long long)idx * kRecordQuads;
+        rec[0] = make_uint4((uint32_t)orig, (uint32_t)col0, (uint32_t)nB, (uint32_t)bRow0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          rec[1 + k] = make_uint4(v[c][4 * k], v[c][4 * k + 1], v[c][4 * k + 2], v[c][4 * k + 3]);
+      }
+    }
+    segN += __popc(m);
+  }
+}
+
 // kBatch = false: one pair, the flattened (group, tile) range of this CTA (WorkCursor).
 // kBatch = true: rows of a.rows (BatchCursor); a row's state indices are state0 + row.
 // kGather = true (batched pass only): A blocks gathered row by row from a.aSrc (tmA unused).
@@ -293,7 +346,7 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
   if constexpr (kBatch) {
     nRows = a.nRowsPtr ? *a.nRowsPtr : a.nRows;
     if (nRows <= 0) {  // nothing to score: uniform early exit
-      if (warp >= 2 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - 2)] = 0;
+      if (warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
       return;
     }
   } else {
@@ -302,7 +355,7 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
     sh.nTiles = nTiles;
     sh.nWork = (long long)sh.nGroups * nTiles;
     if (sh.nWork == 0) {  // nothing to score (e.g. no right was chosen): uniform early exit
-      if (warp >= 2 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - 2)] = 0;
+      if (warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
       return;
     }
     cta_range(sh, w0, w1);
@@ -315,17 +368,14 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::kStages; ++i) {
       mbar_init(&s.fullB[i], 1);
-      mbar_init(&s.emptyB[i], 1);
+      mbar_init(&s.done[i], 1);
     }
     for (int i = 0; i < C::kASlots; ++i) {
       mbar_init(&s.fullA[i], 1);
-      mbar_init(&s.emptyA[i], 1);
+      mbar_init(&s.emptyA[i], kIssuers);
     }
-    for (int i = 0; i < C::kAcc; ++i) {
-      mbar_init(&s.accFull[i], 1);
-      mbar_init(&s.accEmpty[i], kEpiWarps);
-    }
-    mbar_init(&s.mmaDone, 1);
+    for (int i = 0; i < C::kAcc; ++i) mbar_init(&s.accEmpty[i], kEpiWarps);
+    mbar_init(&s.mmaDone, kIssuers);
     s.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -345,15 +395,13 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
   }
   __syncthreads();
 
+  // Ring uses are numbered from 0 in every role: tile i has B stage i % kStages and accumulator
+  // i % kAcc, the run's A block number j slot j % kASlots.
   if (warp == 0) {
    if constexpr (kGather) {
     // ---------------- producer, gathered A: the whole warp ----------------
     if (!s.abort) {
-      int stage = 0, aBuf = C::kASlots - 1;
-      uint32_t phase = 0, aPhase = 1;
-      uint32_t armedPhase[C::kStages];
-      bool armed[C::kStages];
-      for (int i = 0; i < C::kStages; ++i) armed[i] = false;
+      uint32_t i = 0, j = 0;             // tiles, A blocks
       int pend[kGatherDepth + 1] = {};  // slots whose gather still needs its arrive, oldest first
       int nPend = 0;
       int preRow = -1;                   // A block whose entry indices pre[] holds
@@ -364,8 +412,8 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s.fullA[pend[0]]);
-        for (int i = 1; i <= kGatherDepth; ++i)
-          if (i < nPend) pend[i - 1] = pend[i];
+        for (int k = 1; k <= kGatherDepth; ++k)
+          if (k < nPend) pend[k - 1] = pend[k];
         --nPend;
       };
       auto arrive_all = [&]() {
@@ -381,14 +429,13 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
         if (lane == 0) okl = mbar_wait(bar, par, &s.abort, a.err, lim) ? 1 : 0;
         return __shfl_sync(0xffffffffu, okl, 0) != 0;
       };
-      for (Cursor wc = make_cursor(); wc.more(); wc.next()) {
-        if (wc.fresh && lane == 0) wc.prefetch_rows();
+      bool go = true;
+      for (Cursor wc = make_cursor(); wc.more() && go; wc.next()) {
+        if (lane == 0) wc.prefetch_rows();
         if (wc.newA) {
-          if (++aBuf == C::kASlots) {
-            aBuf = 0;
-            aPhase ^= 1;
-          }
-          if (!wait_slot(&s.emptyA[aBuf], aPhase ^ 1)) break;
+          const uint32_t slot = ring_slot<C::kASlots>(j);
+          if (!wait_slot(&s.emptyA[slot], ring_parity<C::kASlots>(j) ^ 1)) break;
+          ++j;
           const int aRow = wc.cur.aRow, nValid = wc.cur.validRows;
           int src[C::GM / 32];
 #pragma unroll
@@ -396,7 +443,7 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
             const int rr = lane + 32 * k;
             src[k] = aRow == preRow ? pre[k] : (rr < nValid ? __ldg(a.aSrcRow + aRow + rr) : -1);
           }
-          const uint32_t dst0 = smem_u32(s.a[aBuf]);
+          const uint32_t dst0 = smem_u32(s.a[slot]);
 #pragma unroll
           for (int k = 0; k < C::GM / 32; ++k) {
             const int rr = lane + 32 * k;
@@ -416,173 +463,163 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
               pre[k] = rr < wc.nxt.validRows ? __ldg(a.aSrcRow + preRow + rr) : -1;
             }
           }
-          pend[nPend++] = aBuf;
+          pend[nPend++] = (int)slot;
           if (nPend > kGatherDepth) {
             cp_async_wait<kGatherDepth>();
             arrive_oldest();
           }
         }
-        if (!wait_slot(&s.emptyB[stage], phase ^ 1)) break;
-        if (lane == 0) {
-          mbar_expect_tx(&s.fullB[stage], C::kBBytes);
-          int bRow = 0;
-          if constexpr (kBatch) bRow = wc.cur.bRow0 + wc.t * C::BN;
-          tma_load_2d(s.b[stage], &tmB, &s.fullB[stage], 0, bRow);
-        }
-        armed[stage] = true;
-        armedPhase[stage] = phase;
-        if (++stage == C::kStages) {
-          stage = 0;
-          phase ^= 1;
+        for (int t = 0; t < wc.nT; ++t, ++i) {
+          const uint32_t st = ring_slot<C::kStages>(i);
+          if (!wait_slot(&s.done[st], ring_parity<C::kStages>(i) ^ 1)) {
+            go = false;
+            break;
+          }
+          if (lane == 0) {
+            mbar_expect_tx(&s.fullB[st], C::kBBytes);
+            tma_load_2d(s.b[st], &tmB, &s.fullB[st], 0, wc.cur.bRow0 + t * C::BN);
+          }
         }
       }
       // every gather has landed (and is handed over) and every load lane 0 issued has landed
       // before the CTA may exit
       arrive_all();
       if (lane == 0)
-        for (int i = 0; i < C::kStages; ++i)
-          if (armed[i]) {
-            long long t0c = clock64();
-            while (!mbar_try(&s.fullB[i], armedPhase[i]) && clock64() - t0c < kWaitCycles) {
-            }
+        for (uint32_t k = i > (uint32_t)C::kStages ? i - C::kStages : 0u; k < i; ++k) {
+          long long t0c = clock64();
+          while (!mbar_try(&s.fullB[ring_slot<C::kStages>(k)], ring_parity<C::kStages>(k)) &&
+                 clock64() - t0c < kWaitCycles) {
           }
+        }
     }
    } else {
     // ---------------- TMA producer ----------------
     if (lane == 0 && !s.abort) {
-      int stage = 0, aBuf = C::kASlots - 1;
-      uint32_t phase = 0, aPhase = 1;
-      uint32_t armedPhase[C::kStages], armedAPhase[C::kASlots];
-      bool armed[C::kStages], armedA[C::kASlots];
-      int nIssued = 0;  // B tile loads issued (test hook)
-      for (int i = 0; i < C::kStages; ++i) armed[i] = false;
-      for (int i = 0; i < C::kASlots; ++i) armedA[i] = false;
-      for (Cursor wc = make_cursor(); wc.more(); wc.next()) {
-        if (wc.fresh) wc.prefetch_rows();
+      uint32_t i = 0, j = 0;  // tiles, A blocks
+      uint32_t skipped = 0xffffffffu;  // test hook: the tile that was not loaded
+      bool go = true;
+      for (Cursor wc = make_cursor(); wc.more() && go; wc.next()) {
+        wc.prefetch_rows();
         if (wc.newA) {
-          if (++aBuf == C::kASlots) {
-            aBuf = 0;
-            aPhase ^= 1;
-          }
-          if (!mbar_wait(&s.emptyA[aBuf], aPhase ^ 1, &s.abort, a.err, lim)) break;
-          mbar_expect_tx(&s.fullA[aBuf], C::kABytes);
+          const uint32_t slot = ring_slot<C::kASlots>(j);
+          if (!mbar_wait(&s.emptyA[slot], ring_parity<C::kASlots>(j) ^ 1, &s.abort, a.err, lim)) break;
+          mbar_expect_tx(&s.fullA[slot], C::kABytes);
           int aRow;
           if constexpr (kBatch) aRow = wc.cur.aRow;
           else aRow = wc.g * C::GM;
-          tma_load_2d(s.a[aBuf], &tmA, &s.fullA[aBuf], 0, aRow);
-          armedA[aBuf] = true;
-          armedAPhase[aBuf] = aPhase;
+          tma_load_2d(s.a[slot], &tmA, &s.fullA[slot], 0, aRow);
+          ++j;
         }
-        if (!mbar_wait(&s.emptyB[stage], phase ^ 1, &s.abort, a.err, lim)) break;
-        if (a.skipLoad > 0 && blockIdx.x == 0 && ++nIssued == a.skipLoad) {
-          armed[stage] = false;  // test hook: this tile never arrives; the MMA's bounded wait gives up
-        } else {
-          mbar_expect_tx(&s.fullB[stage], C::kBBytes);
-          int bRow;
-          if constexpr (kBatch) bRow = wc.cur.bRow0 + wc.t * C::BN;
-          else bRow = wc.t * C::BN;
-          tma_load_2d(s.b[stage], &tmB, &s.fullB[stage], 0, bRow);
-          armed[stage] = true;
-          armedPhase[stage] = phase;
-        }
-        if (++stage == C::kStages) {
-          stage = 0;
-          phase ^= 1;
+        int bRow;
+        if constexpr (kBatch) bRow = wc.cur.bRow0;
+        else bRow = wc.t0 * C::BN;
+        for (int t = 0; t < wc.nT; ++t, ++i, bRow += C::BN) {
+          const uint32_t st = ring_slot<C::kStages>(i);
+          if (!mbar_wait(&s.done[st], ring_parity<C::kStages>(i) ^ 1, &s.abort, a.err, lim)) {
+            go = false;
+            break;
+          }
+          if (a.skipLoad > 0 && blockIdx.x == 0 && i + 1 == (uint32_t)a.skipLoad) {
+            skipped = i;  // test hook: this tile never arrives; the MMA's bounded wait gives up
+          } else {
+            mbar_expect_tx(&s.fullB[st], C::kBBytes);
+            tma_load_2d(s.b[st], &tmB, &s.fullB[st], 0, bRow);
+          }
         }
       }
       // Drain: every load this thread issued has landed before the CTA may exit.
-      for (int i = 0; i < C::kStages; ++i)
-        if (armed[i]) {
-          long long t0c = clock64();
-          while (!mbar_try(&s.fullB[i], armedPhase[i]) && clock64() - t0c < kWaitCycles) {
-          }
+      for (uint32_t k = i > (uint32_t)C::kStages ? i - C::kStages : 0u; k < i; ++k) {
+        long long t0c = clock64();
+        while (k != skipped && !mbar_try(&s.fullB[ring_slot<C::kStages>(k)], ring_parity<C::kStages>(k)) &&
+               clock64() - t0c < kWaitCycles) {
         }
-      for (int i = 0; i < C::kASlots; ++i)
-        if (armedA[i]) {
-          long long t0c = clock64();
-          while (!mbar_try(&s.fullA[i], armedAPhase[i]) && clock64() - t0c < kWaitCycles) {
-          }
+      }
+      for (uint32_t k = j > (uint32_t)C::kASlots ? j - C::kASlots : 0u; k < j; ++k) {
+        long long t0c = clock64();
+        while (!mbar_try(&s.fullA[ring_slot<C::kASlots>(k)], ring_parity<C::kASlots>(k)) &&
+               clock64() - t0c < kWaitCycles) {
         }
+      }
     }
    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0 && !s.abort) {
-      int stage = 0, acc = 0, aBuf = C::kASlots - 1;
-      bool anyA = false;
-      uint32_t phase = 0, accPhase = 0, aPhase = 1;
-      uint32_t aAddr = 0;
-      for (Cursor wc = make_cursor(); wc.more(); wc.next()) {
+  } else if (warp < kEpiWarp0) {
+    // ---------------- MMA issuers ----------------
+    // The whole warp walks the loop and one elected lane issues: with the loop's values uniform over
+    // the warp the instruction's operands stay in uniform registers.  Issuer w takes the tiles with
+    // i % kIssuers == w.
+    auto wait = [&](unsigned long long* bar, uint32_t par) -> bool {
+      return mbar_wait_warp(bar, par, &s.abort, a.err, lim);
+    };
+    if (!s.abort) {
+      const uint32_t aBase = sdesc_lo(smem_u32(s.a[0])), bBase = sdesc_lo(smem_u32(s.b[0]));
+      const bool leader = elect_one();
+      uint32_t i0 = 0;              // the run's first tile
+      uint32_t i = warp - 1;        // this issuer's next tile
+      uint32_t j = 0;               // A blocks started
+      bool go = true;
+      for (Cursor wc = make_cursor(); wc.more() && go; wc.next()) {
         if (wc.newA) {
-          if (anyA) mma_commit(&s.emptyA[aBuf]);
-          if (++aBuf == C::kASlots) {
-            aBuf = 0;
-            aPhase ^= 1;
-          }
-          if (!mbar_wait(&s.fullA[aBuf], aPhase, &s.abort, a.err, lim)) break;
-          aAddr = smem_u32(s.a[aBuf]);
-          anyA = true;
+          // the block before is done with: each issuer says so once it has issued its MMAs of it.  The
+          // wait comes first and whether or not this issuer has a tile in the run: it keeps an issuer
+          // from counting twice on a slot's barrier before the other has counted once.
+          if (!wait(&s.fullA[ring_slot<C::kASlots>(j)], ring_parity<C::kASlots>(j))) break;
+          if (j > 0 && leader) mma_commit(&s.emptyA[ring_slot<C::kASlots>(j - 1)]);
+          ++j;
         }
-        if (!mbar_wait(&s.fullB[stage], phase, &s.abort, a.err, lim)) break;
-        const uint32_t bAddr = smem_u32(s.b[stage]);
-        bool stop = false;
-#pragma unroll
-        for (int h = 0; h < C::kSplit; ++h) {
-          if (!mbar_wait(&s.accEmpty[acc], accPhase ^ 1, &s.abort, a.err, lim)) {
-            stop = true;
+        i0 += (uint32_t)wc.nT;
+        const uint32_t aSlot = ring_slot<C::kASlots>(j - 1);
+        const uint32_t ad = aBase + aSlot * (uint32_t)(C::kABytes >> 4);
+        for (; i < i0; i += kIssuers) {
+          const uint32_t st = ring_slot<C::kStages>(i), acc = ring_slot<C::kAcc>(i);
+          if (!wait(&s.fullB[st], ring_parity<C::kStages>(i)) ||
+              !wait(&s.accEmpty[acc], ring_parity<C::kAcc>(i) ^ 1)) {
+            go = false;
             break;
           }
           tc_fence_after();
-          // columns h * kMmaN .. of the tile: B rows 128 bytes each, 1024-byte aligned halves
-          const uint32_t bh = bAddr + (uint32_t)(h * C::kMmaN * kDescBytes);
+          const uint32_t bd = bBase + st * (uint32_t)(C::kBBytes >> 4);
+          const uint32_t d = tmem + acc * (uint32_t)C::kAccCols;
+          if (leader) {
 #pragma unroll
-          for (int blk = 0; blk < C::NB; ++blk) {
-            const uint32_t d = tmem + (uint32_t)(acc * C::kAccCols + blk * C::kMmaN);
-            const uint32_t ab = aAddr + (uint32_t)(blk * BM * kDescBytes);
+            for (int blk = 0; blk < C::NB; ++blk) {
 #pragma unroll
-            for (int k = 0; k < kDescBytes / 32; ++k)
-              mma_i8<C::kMmaN>(d, sdesc(ab + 32u * k), sdesc(bh + 32u * k), k > 0 ? 1u : 0u);
-          }
-          mma_commit(&s.accFull[acc]);
-          if (++acc == C::kAcc) {
-            acc = 0;
-            accPhase ^= 1;
+              for (int k = 0; k < kDescBytes / 32; ++k)
+                mma_i8<C::BN>(d + (uint32_t)(blk * C::BN),
+                              sdesc_of(ad + (uint32_t)((blk * BM * kDescBytes + 32 * k) >> 4)),
+                              sdesc_of(bd + (uint32_t)(2 * k)), k > 0 ? 1u : 0u);
+            }
+            mma_commit(&s.done[st]);
           }
         }
-        if (stop) break;
-        mma_commit(&s.emptyB[stage]);
-        if (++stage == C::kStages) {
-          stage = 0;
-          phase ^= 1;
+      }
+      // Every MMA the elected lane issued has completed before TMEM is released.
+      if (leader) {
+        if (j > 0) mma_commit(&s.emptyA[ring_slot<C::kASlots>(j - 1)]);
+        mma_commit(&s.mmaDone);
+        long long t0c = clock64();
+        while (!mbar_try(&s.mmaDone, 0) && clock64() - t0c < kWaitCycles) {
         }
       }
-      if (anyA) mma_commit(&s.emptyA[aBuf]);
-      // Every MMA this thread issued has completed before TMEM is released.
-      mma_commit(&s.mmaDone);
-      long long t0c = clock64();
-      while (!mbar_try(&s.mmaDone, 0) && clock64() - t0c < kWaitCycles) {
-      }
+      __syncwarp();
     }
   } else {
     // ---------------- epilogue ----------------
-    const int e = warp - 2;
+    const int e = warp - kEpiWarp0;
     const int q = warp & 3;                              // TMEM lane quadrant this warp may access
     const int sub = e >> 2;                              // 0..3 within the quadrant
     const int blk = C::NB == 2 ? (sub & 1) : 0;          // A block of the group
     const int colOff = (C::NB == 2 ? (sub >> 1) : sub) * C::kWarpCols;  // first tile column of this warp
     const int rowInGroup = blk * BM + q * 32 + lane;
+    const uint32_t tbase0 = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(blk * C::BN + colOff);
     uint4* const segBase = a.records + (long long)(blockIdx.x * kEpiWarps + e) * a.segCap * kRecordQuads;
     int segN = 0;                                        // warp-uniform count of records written
-    int acc = 0;
-    bool started = false;
-    uint32_t accPhase = 0;
     bool ok = !s.abort;
     bool rowValid = false;
     int orig = 0;
     int aLocal = 0;  // batched pass: index of this lane's A row within its image
     int nB = a.nB;
     int bRow0 = 0;
-    // maximum of this lane's scores in the current unit, chunks with a record excluded; kNoScore
+    // maximum of this lane's scores in the current run, chunks with a record excluded; kNoScore
     // (a negative float, below every score in the max.f32 order) while there is none
     constexpr uint32_t kNoScore = 0xbf800000u;
     uint32_t lw = kNoScore;
@@ -592,97 +629,67 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
       const uint32_t w = lw == kNoScore ? 0u : lw + 1u;  // sec[] holds second + 1
       if (rowValid && w > (uint32_t)a.Tsec) atomicMax(&a.sec[orig], w);
     };
+    uint32_t i = 0;
     for (Cursor wc = make_cursor(); wc.more() && ok; wc.next()) {
-      if (wc.fresh) {
-        if (started) flush();
-        started = true;
-        if constexpr (kBatch) {
-          rowValid = rowInGroup < wc.cur.validRows;
-          if (wc.newA)  // the A block's index map is read once per block, not once per row
-            aLocal = rowValid ? (a.amap ? __ldg(a.amap + wc.cur.aRow + rowInGroup) : rowInGroup) : 0;
-          orig = rowValid ? (int)(wc.cur.state0 + aLocal) : 0;
-          nB = wc.cur.nB;
-          bRow0 = wc.cur.bRow0;
-        } else {
-          const int row = wc.g * C::GM + rowInGroup;
-          rowValid = row < nA;
-          orig = rowValid ? (a.amap ? a.amap[row] : row) : 0;
-        }
-        lw = kNoScore;
-        sminRow = rowValid ? a.Smin : 0x7fffffff;
-      }
-      for (int h = 0; h < C::kSplit; ++h) {
-      const int colBase = wc.t * C::BN + h * C::kMmaN + colOff;
-      ok = mbar_wait(&s.accFull[acc], accPhase, &s.abort, a.err, lim);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t tbase =
-          tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * C::kAccCols + blk * C::kMmaN + colOff);
-      // All of this warp's scores into registers, then hand the stage back at once so the
-      // MMA never waits for the filtering below (kPipe: the second chunk is loaded while the
-      // first is filtered, and the stage handed back after it).
-      uint32_t v[C::kChunks][32];
-      if constexpr (C::kPipe) {
-        tmem_ld32(tbase, v[0]);
-        tmem_wait(v[0]);
-        tmem_ld32(tbase + 32u, v[1]);
+      if constexpr (kBatch) {
+        rowValid = rowInGroup < wc.cur.validRows;
+        if (wc.newA)  // the A block's index map is read once per block, not once per row
+          aLocal = rowValid ? (a.amap ? __ldg(a.amap + wc.cur.aRow + rowInGroup) : rowInGroup) : 0;
+        orig = rowValid ? (int)(wc.cur.state0 + aLocal) : 0;
+        nB = wc.cur.nB;
+        bRow0 = wc.cur.bRow0;
       } else {
+        const int row = wc.g * C::GM + rowInGroup;
+        rowValid = row < nA;
+        orig = rowValid ? (a.amap ? a.amap[row] : row) : 0;
+      }
+      lw = kNoScore;
+      sminRow = rowValid ? a.Smin : 0x7fffffff;
+      int colBase = wc.t0 * C::BN + colOff;
+      for (const uint32_t iEnd = i + (uint32_t)wc.nT; i < iEnd; ++i, colBase += C::BN) {
+        const uint32_t acc = ring_slot<C::kAcc>(i);
+        ok = mbar_wait_warp(&s.done[ring_slot<C::kStages>(i)], ring_parity<C::kStages>(i), &s.abort, a.err, lim);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t tbase = tbase0 + acc * (uint32_t)C::kAccCols;
+        // All of this warp's scores into registers, then hand the stage back at once so the
+        // MMA never waits for the filtering below (kPipe: the second chunk is loaded while the
+        // first is filtered, and the stage handed back after it).
+        uint32_t v[C::kChunks][32];
+        uint32_t cm[C::kChunks];  // max(lw, chunk maximum)
+        if constexpr (C::kPipe) {
+          tmem_ld32(tbase, v[0]);
+          tmem_wait(v[0]);
+          tmem_ld32(tbase + 32u, v[1]);
+          cm[0] = max32_bits(v[0], lw);
+          tmem_wait(v[1]);
+        } else {
 #pragma unroll
-        for (int c = 0; c < C::kChunks; ++c) tmem_ld32(tbase + (uint32_t)(c * 32), v[c]);
+          for (int c = 0; c < C::kChunks; ++c) tmem_ld32(tbase + (uint32_t)(c * 32), v[c]);
 #pragma unroll
-        for (int c = 0; c < C::kChunks; ++c) tmem_wait(v[c]);
+          for (int c = 0; c < C::kChunks; ++c) tmem_wait(v[c]);
+        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s.accEmpty[acc]);
-      }
+        // Whole chunks only (every tile but an image's last): straight-line code, the chunks' maxima
+        // interleaved and one vote for both.  A test for the last B descriptor at every chunk, with
+        // the code that clears the columns past it, cost as much as the filtering itself (32768^2
+        // 137 us with it, 103 us without).
+        if (colBase + C::kChunks * 32 <= nB) {  // warp-uniform
 #pragma unroll
-      for (int c = 0; c < C::kChunks; ++c) {
-        if constexpr (C::kPipe) {
-          if (c == 1) {
-            tmem_wait(v[1]);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s.accEmpty[acc]);
+          for (int c = C::kPipe ? 1 : 0; c < C::kChunks; ++c) cm[c] = max32_bits(v[c], lw);
+          const uint32_t tm = C::kChunks == 2 ? max3_bits(cm[0], cm[C::kChunks - 1], lw) : cm[0];
+          // kNoScore is negative as an int32; an invalid row's lw is never flushed
+          if (!__any_sync(0xffffffffu, (int32_t)tm >= sminRow)) {
+            lw = tm;
+            continue;
           }
         }
-        const int col0 = colBase + 32 * c;
-        if (col0 >= nB) continue;  // chunks past the last B descriptor (warp-uniform)
-        if (col0 + 32 > nB) {
-          // The chunk holding the last B descriptor: the columns past it hold zero fill, zero
-          // padding or the next block's descriptors; a 0 there is <= every real score, so the
-          // chunk maximum stays the maximum of its real scores.
-#pragma unroll
-          for (int k = 0; k < 32; ++k)
-            if (col0 + k >= nB) v[c][k] = 0u;
-        }
-        const uint32_t cm = max32_bits(v[c], lw);  // max(lw, chunk maximum)
-        const bool trig = (int32_t)cm >= sminRow;   // kNoScore is negative as an int32
-        if (!trig) lw = cm;                          // an invalid row's lw is never flushed
-        if (__any_sync(0xffffffffu, trig)) {
-          // rare: hand the chunk to k_records (its exact best, gates and other scores)
-          const unsigned m = __ballot_sync(0xffffffffu, trig);
-          if (trig) {
-            const int idx = segN + __popc(m & ((1u << lane) - 1u));
-            if (idx < a.segCap) {
-              uint4* rec = segBase + (long long)idx * kRecordQuads;
-              rec[0] = make_uint4((uint32_t)orig, (uint32_t)col0, (uint32_t)nB, (uint32_t)bRow0);
-#pragma unroll
-              for (int k = 0; k < 8; ++k)
-                rec[1 + k] = make_uint4(v[c][4 * k], v[c][4 * k + 1], v[c][4 * k + 2], v[c][4 * k + 3]);
-            }
-          }
-          segN += __popc(m);
-        }
+        filter_chunks<C::kChunks>(v, colBase, nB, bRow0, orig, sminRow, lw, segN, segBase, a.segCap);
       }
-      if (++acc == C::kAcc) {
-        acc = 0;
-        accPhase ^= 1;
-      }
-      }
-      if (!ok) break;
+      if (ok) flush();
     }
-    if (started && ok) flush();
     if (lane == 0) a.segCount[blockIdx.x * kEpiWarps + e] = segN;
   }
 
@@ -730,9 +737,9 @@ using Cfg3 = TcCfg<2, 64, 16>;   // 256 x 64 tiles, 4 accumulator stages
 using Cfg4 = TcCfg<1, 256, 6>;   // 128 x 256 tiles, 2 accumulator stages, 6-deep ring
 using Cfg5 = TcCfg<1, 256, 4, 4>;   // as Cfg0 with 4 left-group buffers (rows of few tiles)
 using Cfg6 = TcCfg<1, 128, 6, 6>;   // 128 x 128 tiles, 6 left-group buffers
-using Cfg7 = TcCfg<1, 256, 4, 4, 2>;      // as Cfg5, each tile as two 128-column MMAs (4 accumulator stages)
-using Cfg8 = TcCfg<1, 256, 6, 2, 2>;      // as Cfg4, split the same way
-using Cfg9 = TcCfg<1, 256, 4, 4, 1, 1>;   // as Cfg5 with the epilogue's second chunk loaded while the first is filtered
+using Cfg7 = TcCfg<1, 256, 4, 3>;   // as Cfg5 with 3 left-group buffers
+using Cfg8 = TcCfg<1, 256, 5, 2>;   // as Cfg0 with a 5-deep ring
+using Cfg9 = TcCfg<1, 256, 4, 4, 1>;   // as Cfg5 with the epilogue's second chunk loaded while the first is filtered
 
 template <class C, bool kBatch, bool kGather = false>
 cudaError_t launch_cfg(const CUtensorMap& mA, const CUtensorMap& mB, int nTiles, const SideArgs& a, int grid,

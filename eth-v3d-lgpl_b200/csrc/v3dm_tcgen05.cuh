@@ -73,6 +73,13 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* b, uint32_t parity
   }
 }
 
+// mbar_wait by a whole warp, with a result that is uniform over it.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long* b, uint32_t parity, int* abortFlag, int* err,
+                                               long long limit = kWaitCycles) {
+  if (__all_sync(0xffffffffu, mbar_try(b, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(b, parity, abortFlag, err, limit));
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -86,6 +93,25 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
          (2ull << 61);
+}
+
+// The same in two words: the low one for a shared-memory address (it advances by bytes >> 4), and
+// the descriptor of a low word.
+__device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr) { return ((saddr >> 4) & 0x3FFFu) | (1u << 16); }
+__device__ __forceinline__ uint64_t sdesc_of(uint32_t lo) {
+  constexpr uint64_t hi = ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+  return hi | lo;
+}
+
+// One lane of the warp (the same each time for a full warp).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
 }
 
 __device__ __forceinline__ void mma_commit(unsigned long long* bar) {

@@ -113,6 +113,28 @@ def test_every_config_and_schedule(v3dm_mod, small_set):
     b.close()
 
 
+@pytest.mark.parametrize("counts", [[90] * 40, [64, 300] * 14, [20, 2000, 20, 20, 700] * 6, [256, 257, 512, 513] * 5])
+def test_runs_of_few_tiles(v3dm_mod, oracle_mod, counts):
+    """Rows of one tile and of many, alone and mixed: a left group then changes at nearly every tile,
+    so the two issuers of the side pass and the left-group ring take turns at every step.  Every
+    configuration and schedule gives the first one's triples, and those are the oracle's."""
+    desc, counts, offs = _images(int(sum(counts)), counts)
+    with v3dm_mod.BatchMatching() as b:
+        b.set_images(desc, counts)
+        b.set_pairs(None)
+        pairs = synth.all_pairs(len(counts))
+        ref = b.match(0.7, 0.8)
+        per = b.split_pairs(ref)
+        for k in range(0, len(pairs), max(1, len(pairs) // 60)):
+            i, j = pairs[k]
+            np.testing.assert_array_equal(per[k], oracle_mod.match(_img(desc, offs, i), _img(desc, offs, j), 0.7, 0.8))
+        for cfg in range(v3dm_mod.SIFTMatching().num_configs()):
+            for sch in (0, 1, 2):
+                b.set_config(cfg, sch)
+                for _ in range(3):
+                    np.testing.assert_array_equal(b.match(0.7, 0.8), ref, err_msg=f"cfg {cfg} schedule {sch}")
+
+
 def test_device_call_and_growth(v3dm_mod, oracle_mod):
     """Identical images: every left is accepted in every pair, far beyond the first pass-B
     buffers, so the call overflows once, grows them and is repeated."""
