@@ -196,6 +196,41 @@ constexpr int kVtcBoxRows = 16;
 constexpr int kVtcKeyBox = 128;
 cudaError_t launch_vtc(const VtcArgs& a, const CUtensorMap& nodeMap, const CUtensorMap& keyMap, int grid,
                        cudaStream_t st);
+// Tensor-core descent of float trees (v3dm_voctree_f.cu): a phase as VtcArgs describes it, the items
+// of a single bucket of itemKeys keys each; keys the scores cannot decide are listed (key, node, levels)
+// and resolved in the reference's arithmetic, keys that are not finite in the first phase's `weird`.
+struct VtfArgs {
+  const float* keys;
+  const int32_t* perm;
+  int bf, levels;
+  long long bucketBase;
+  const int4* items;
+  const int* nItems;
+  int singleN, itemKeys;
+  const float* maxNorm;          // the largest node norm
+  const float* childNorm;        // the largest norm among the children of node r at r + 1
+  int final;
+  int32_t* out;
+  int idMode;
+  long long leafBase;
+  int32_t* next;
+  long long nextBase;
+  int* hist;
+  int bins;
+  int4* flagged;
+  int* nFlagged;
+  int32_t* weird;                // null after the first phase
+  int* nWeird;
+  int* err;
+};
+int vtf_levels(int bf);          // levels a phase descends (0: shape not supported)
+constexpr int kVtfRowBytes = 512;  // split node planes per node
+// The split node planes, the norms above (childNorm: rows / bf entries) and the planes' tensor map.
+cudaError_t vtf_prepare(const float* nodes, const float* norm, long long rows, int bf, void* planes, float* childNorm,
+                        float* maxNorm, CUtensorMap* map, cudaStream_t st);
+// The phase and the resolution of what it listed.
+cudaError_t launch_vtf(const VtfArgs& a, const CUtensorMap& m, const float* nodes, unsigned long long* exactCount,
+                       int grid, cudaStream_t st);
 // 2-D map over rows x 128 bytes with a box of boxRows rows and the 128-byte swizzle (v3dm_match_tc.cu).
 cudaError_t tc_rows_map(CUtensorMap* m, const uint8_t* base, int rows, int boxRows);
 

@@ -118,6 +118,7 @@ __global__ void k_vt_f32_to_u8(const float4* __restrict__ src, uint32_t* __restr
 // phase reached.  Between phases the keys are sorted by bucket (a counting sort: k_vt_scan,
 // then k_vt_scatter), and k_vt_scan cuts every bucket into work items of at most kVtItemKeys keys.
 constexpr int kVtItemKeys = 2048;       // keys per work item
+constexpr int kVtMaxPhases = 32;        // phases of the float tensor descent
 constexpr int kVtLocalBins = 16384;     // bucket counts kept in shared memory by k_vt_scatter (2 x 64 KB)
 
 // Bucket offsets and the work items of a phase: (bucket, first key in sorted order, count), at
@@ -220,17 +221,21 @@ __device__ __forceinline__ int seq_best_child(const float* __restrict__ key, con
 // Float descent.  Four threads per key; thread `part` holds key floats q*16 + part*4 .. +3 for
 // q = 0..7, so the four threads of a key read 64 contiguous bytes of a node row per load.
 // nodeNorm[i] >= |node i| (L2).  exactCount (optional) counts the key-levels resolved by the
-// sequential replay.  err gets kErrBadTree when a child block would leave the tree.
+// sequential replay.  err gets kErrBadTree when a child block would leave the tree.  With list, the
+// keys are list[0 .. *listN) instead of 0 .. n - 1.
 __global__ void __launch_bounds__(kVtThreads, 2)
 k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNorm, long long nodeCount, int bf,
               int depth, long long leafBase, const float* __restrict__ keys, int n, int32_t* __restrict__ out,
-              int idMode, unsigned long long* __restrict__ exactCount, int32_t* __restrict__ err) {
+              int idMode, unsigned long long* __restrict__ exactCount, int32_t* __restrict__ err,
+              const int32_t* __restrict__ list, const int* __restrict__ listN) {
   const int gt = blockIdx.x * kVtThreads + threadIdx.x;
-  const int key = gt / kTpk;
   const int part = gt % kTpk;
   const int lane = threadIdx.x & 31;
   const unsigned grp = 0xfu << (lane & ~3);
-  const bool valid = key < n;
+  const int total = list ? *listN : n;
+  for (int at = gt / kTpk; at - lane / kTpk < total; at += gridDim.x * kVtThreads / kTpk) {  // whole warps
+  const bool valid = at < total;
+  const int key = list ? (valid ? list[at] : 0) : at;
   const float* krow = keys + (size_t)(valid ? key : 0) * kDescBytes;
   float4 kv[8];
 #pragma unroll
@@ -306,6 +311,7 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
   if (!ok && part == 0 && valid) atomicOr(err, kErrBadTree);
   if (valid && part == 0) out[key] = (int32_t)(idMode == V3DM_LEAF_LOCAL ? leafId - leafBase : leafId);
   if (exactCount && part == 0 && replays) atomicAdd(exactCount, replays);
+  }
 }
 
 // |node i| rounded up, for the bound above (double sum, then an upward margin).
@@ -387,6 +393,17 @@ struct v3dm_voctree {
   int* dNItems = nullptr;
   int numSMs = 148;
   int lastLaunches = 0;         // kernels launched by the last quantization
+  // tensor-core descent of float trees (fLevels levels per phase; 0: shape not supported)
+  int fLevels = 0, fPhases = 0;
+  long long fMaxBins = 1;       // buckets of its last phase
+  void* dPlanes = nullptr;      // split node planes, kVtfRowBytes per node (valid when planesReady)
+  bool planesReady = false;
+  float* dMaxNorm = nullptr;
+  float* dChildNorm = nullptr;  // in dPlanes' block
+  int4* dFlagged = nullptr;     // nMax
+  int32_t* dWeird = nullptr;    // nMax
+  int* dFCounts = nullptr;      // [0] weird keys, [1 + p] listed keys of phase p
+  CUtensorMap tmPlanes;
   CUtensorMap tmNodes;          // the u8 node rows for the tensor path's TMA loads
   bool tmValid = false;
   CUtensorMap tmKeys;           // the keys of the last call (first phase), for TMA tiles
@@ -414,7 +431,28 @@ void vt_plan(v3dm_voctree* t) {
   for (int k = 0; k < 2 * (t->phases - 1); ++k) bins *= t->bf;
   t->maxBins = bins;
   t->tcPath = vtc_supported(t->bf) && bins <= (1LL << 22);
+  t->fLevels = vtf_levels(t->bf);
+  if (t->fLevels == 0) return;
+  t->fPhases = (t->depth + t->fLevels - 1) / t->fLevels;
+  bins = 1;
+  for (int k = 0; k < t->fLevels * (t->fPhases - 1); ++k) bins *= t->bf;
+  t->fMaxBins = bins;
+  // the node index is an int32 in the lists, and a TMA row coordinate
+  if (bins > (1LL << 22) || t->fPhases > kVtMaxPhases || t->nodeCount > 0x7fffffffLL - 256) t->fLevels = 0;
 }
+
+// Buckets the sorting buffers hold.
+long long vt_bins(const v3dm_voctree* t) {
+  return std::max(t->tcPath ? t->maxBins : 0, t->fLevels ? t->fMaxBins : 0);
+}
+
+// A call of n keys takes the float tensor descent when the last phase has at least kVtMinPerBin keys
+// per bucket: below that the tiles of 128 keys are mostly empty (and the node planes, 512 bytes a node,
+// are not made for trees whose calls cannot reach it).
+constexpr int kVtMinPerBin = 16;
+bool vt_f_wanted(const v3dm_voctree* t, long long n) { return t->fLevels > 0 && n >= kVtMinPerBin * t->fMaxBins; }
+
+int vt_sort(v3dm_voctree* t, int n, long long bins);
 
 int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int idMode) {
   t->lastLaunches = 0;
@@ -466,16 +504,8 @@ int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int i
     const long long nextBins = bins * bf * bf;
     if (p > 0) {
       // keys sorted by the bucket the previous phase reached
-      k_vt_scan<<<1, 1024, 0, t->stream>>>(t->dHist, (int)bins, 0, t->dOff, t->dItems, t->dNItems);
-      if (cudaGetLastError() != cudaSuccess) return V3DM_ERR_CUDA;
-      if (cudaMemsetAsync(t->dHist + t->maxBins, 0, (size_t)bins * sizeof(int), t->stream) != cudaSuccess)
-        return V3DM_ERR_CUDA;
-      const unsigned sg = (unsigned)std::max<long long>(
-          1, std::min<long long>(((long long)n + 4095) / 4096, (long long)t->numSMs * 2));
-      const size_t ssm = bins <= kVtLocalBins ? 2 * (size_t)bins * sizeof(int) : 0;
-      k_vt_scatter<<<sg, kVtScatterThreads, ssm, t->stream>>>(t->dBucket, n, t->dOff, t->dHist + t->maxBins, t->dPerm,
-                                                              (int)bins);
-      if (cudaGetLastError() != cudaSuccess) return V3DM_ERR_CUDA;
+      const int st = vt_sort(t, n, bins);
+      if (st != V3DM_OK) return st;
     }
     if (!last && cudaMemsetAsync(t->dHist, 0, (size_t)nextBins * sizeof(int), t->stream) != cudaSuccess)
       return V3DM_ERR_CUDA;
@@ -493,14 +523,81 @@ int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int i
   return V3DM_OK;
 }
 
+// Keys in bucket order: offsets and work items from the histogram, then the permutation.
+int vt_sort(v3dm_voctree* t, int n, long long bins) {
+  k_vt_scan<<<1, 1024, 0, t->stream>>>(t->dHist, (int)bins, 0, t->dOff, t->dItems, t->dNItems);
+  if (cudaGetLastError() != cudaSuccess) return V3DM_ERR_CUDA;
+  int* cursor = t->dHist + vt_bins(t);
+  if (cudaMemsetAsync(cursor, 0, (size_t)bins * sizeof(int), t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
+  const unsigned sg =
+      (unsigned)std::max<long long>(1, std::min<long long>(((long long)n + 4095) / 4096, (long long)t->numSMs * 2));
+  const size_t ssm = bins <= kVtLocalBins ? 2 * (size_t)bins * sizeof(int) : 0;
+  k_vt_scatter<<<sg, kVtScatterThreads, ssm, t->stream>>>(t->dBucket, n, t->dOff, cursor, t->dPerm, (int)bins);
+  return cudaGetLastError() == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
+}
+
 int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int idMode) {
   t->lastLaunches = 0;
   if (n == 0) return V3DM_OK;
-  t->lastLaunches = 1;
-  long long threads = (long long)n * kTpk;
-  unsigned blocks = (unsigned)((threads + kVtThreads - 1) / kVtThreads);
-  k_voctree_f32<<<blocks, kVtThreads, 0, t->stream>>>(t->dNodesF, t->dNorm, t->nodeCount, t->bf, t->depth,
-                                                      t->leafBase, dKeys, n, dIds, idMode, t->dReplays, t->dErr);
+  if (!vt_f_wanted(t, n) || !t->planesReady || !t->dFlagged || n > t->nMax) {
+    t->lastLaunches = 1;
+    long long threads = (long long)n * kTpk;
+    unsigned blocks = (unsigned)((threads + kVtThreads - 1) / kVtThreads);
+    k_voctree_f32<<<blocks, kVtThreads, 0, t->stream>>>(t->dNodesF, t->dNorm, t->nodeCount, t->bf, t->depth,
+                                                        t->leafBase, dKeys, n, dIds, idMode, t->dReplays, t->dErr,
+                                                        nullptr, nullptr);
+    return cudaGetLastError() == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
+  }
+  if (cudaMemsetAsync(t->dFCounts, 0, (1 + kVtMaxPhases) * sizeof(int), t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
+  VtfArgs va;
+  std::memset(&va, 0, sizeof(va));
+  va.keys = dKeys;
+  va.bf = t->bf;
+  va.items = t->dItems;
+  va.nItems = t->dNItems;
+  va.itemKeys = std::max(128, std::min(kVtItemKeys, (n / t->numSMs + 127) / 128 * 128));
+  va.maxNorm = t->dMaxNorm;
+  va.childNorm = t->dChildNorm;
+  va.out = dIds;
+  va.idMode = idMode;
+  va.leafBase = t->leafBase;
+  va.next = t->dBucket;
+  va.hist = t->dHist;
+  va.flagged = t->dFlagged;
+  va.nWeird = t->dFCounts;
+  va.err = t->dErr;
+  long long bins = 1;
+  for (int p = 0; p < t->fPhases; ++p) {
+    const int d0 = p * t->fLevels;
+    const int levels = std::min(t->fLevels, t->depth - d0);
+    const bool last = p == t->fPhases - 1;
+    long long nextBins = bins;
+    for (int k = 0; k < levels; ++k) nextBins *= t->bf;
+    if (p > 0) {
+      const int st = vt_sort(t, n, bins);
+      if (st != V3DM_OK) return st;
+    }
+    if (!last && cudaMemsetAsync(t->dHist, 0, (size_t)nextBins * sizeof(int), t->stream) != cudaSuccess)
+      return V3DM_ERR_CUDA;
+    va.levels = levels;
+    va.singleN = p == 0 ? n : 0;
+    va.bucketBase = p == 0 ? -1 : level_start(t->bf, d0);
+    va.perm = p == 0 ? nullptr : t->dPerm;
+    va.final = last ? 1 : 0;
+    va.nextBase = last ? 0 : level_start(t->bf, d0 + levels);
+    va.bins = last ? 0 : (int)nextBins;
+    va.nFlagged = t->dFCounts + 1 + p;
+    va.weird = p == 0 ? t->dWeird : nullptr;
+    if (launch_vtf(va, t->tmPlanes, t->dNodesF, t->dReplays, t->numSMs, t->stream) != cudaSuccess)
+      return V3DM_ERR_CUDA;
+    t->lastLaunches += p == 0 ? 2 : 4;
+    bins = nextBins;
+  }
+  // keys that are not finite (or overflow): the whole descent in one kernel, over what the phases wrote
+  k_voctree_f32<<<2 * t->numSMs, kVtThreads, 0, t->stream>>>(t->dNodesF, t->dNorm, t->nodeCount, t->bf, t->depth,
+                                                            t->leafBase, dKeys, n, dIds, idMode, t->dReplays, t->dErr,
+                                                            t->dWeird, t->dFCounts);
+  t->lastLaunches += 1;
   return cudaGetLastError() == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
 }
 
@@ -519,6 +616,8 @@ int vt_to_u8(v3dm_voctree* t, const float* dSrc, size_t count, uint8_t* dst, boo
   *exact = *t->hErr == 0;
   return V3DM_OK;
 }
+
+int vt_planes(v3dm_voctree* t);
 
 // Node norms of the float tree.
 int vt_norms(v3dm_voctree* t) {
@@ -548,6 +647,26 @@ int vt_ensure_float_tree(v3dm_voctree* t) {
   st = vt_norms(t);
   if (st != V3DM_OK) return st;
   t->nodesF = true;
+  return vt_planes(t);
+}
+
+// The split node planes, once the float tree is set and calls can be large enough for them.  A tree
+// whose planes do not fit in memory keeps the one-kernel descent.
+int vt_planes(v3dm_voctree* t) {
+  if (!t->nodesF || t->planesReady || !vt_f_wanted(t, t->nMax)) return V3DM_OK;
+  // one block: the planes, then the children's norms (nodeCount / BF parents, the root among them)
+  const size_t planeBytes = (size_t)t->nodeCount * kVtfRowBytes;
+  if (!t->dPlanes &&
+      cudaMalloc(&t->dPlanes, planeBytes + (size_t)(t->nodeCount / t->bf) * sizeof(float)) != cudaSuccess) {
+    cudaGetLastError();
+    t->dPlanes = nullptr;
+    return V3DM_OK;
+  }
+  t->dChildNorm = reinterpret_cast<float*>(static_cast<uint8_t*>(t->dPlanes) + planeBytes);
+  if (vtf_prepare(t->dNodesF, t->dNorm, t->nodeCount, t->bf, t->dPlanes, t->dChildNorm, t->dMaxNorm, &t->tmPlanes,
+                  t->stream) != cudaSuccess)
+    return V3DM_ERR_CUDA;
+  t->planesReady = true;
   return V3DM_OK;
 }
 
@@ -601,9 +720,11 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
       cudaMalloc(reinterpret_cast<void**>(&t->dReplays), sizeof(unsigned long long)) != cudaSuccess ||
       cudaMemsetAsync(t->dErr, 0, sizeof(int32_t), t->stream) != cudaSuccess ||
       cudaMemsetAsync(t->dReplays, 0, sizeof(unsigned long long), t->stream) != cudaSuccess ||
-      (t->tcPath &&
-       (cudaMalloc(reinterpret_cast<void**>(&t->dHist), 2 * (size_t)t->maxBins * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&t->dOff), ((size_t)t->maxBins + 1) * sizeof(int)) != cudaSuccess ||
+      (vt_bins(t) > 0 &&
+       (cudaMalloc(reinterpret_cast<void**>(&t->dHist), 2 * (size_t)vt_bins(t) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(reinterpret_cast<void**>(&t->dOff), ((size_t)vt_bins(t) + 1) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(reinterpret_cast<void**>(&t->dMaxNorm), sizeof(float)) != cudaSuccess ||
+        cudaMalloc(reinterpret_cast<void**>(&t->dFCounts), (1 + kVtMaxPhases) * sizeof(int)) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&t->dNItems), sizeof(int)) != cudaSuccess ||
         cudaFuncSetAttribute(k_vt_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              2 * kVtLocalBins * (int)sizeof(int)) != cudaSuccess)) ||
@@ -615,6 +736,8 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
     if (t->dHist) cudaFree(t->dHist);
     if (t->dOff) cudaFree(t->dOff);
     if (t->dNItems) cudaFree(t->dNItems);
+    if (t->dMaxNorm) cudaFree(t->dMaxNorm);
+    if (t->dFCounts) cudaFree(t->dFCounts);
     delete t;
     return V3DM_ERR_CUDA;
   }
@@ -636,6 +759,11 @@ int v3dm_voctree_destroy(v3dm_voctree* t) {
   if (t->dBucket) cudaFree(t->dBucket);
   if (t->dPerm) cudaFree(t->dPerm);
   if (t->dItems) cudaFree(t->dItems);
+  if (t->dMaxNorm) cudaFree(t->dMaxNorm);
+  if (t->dFCounts) cudaFree(t->dFCounts);
+  if (t->dFlagged) cudaFree(t->dFlagged);
+  if (t->dWeird) cudaFree(t->dWeird);
+  if (t->dPlanes) cudaFree(t->dPlanes);
   if (t->dKeys) cudaFree(t->dKeys);
   if (t->dStage) cudaFree(t->dStage);
   if (t->dIds) cudaFree(t->dIds);
@@ -656,6 +784,10 @@ int v3dm_voctree_allocate(v3dm_voctree* t, int nMax) {
   if (t->dBucket) cudaFree(t->dBucket);
   if (t->dPerm) cudaFree(t->dPerm);
   if (t->dItems) cudaFree(t->dItems);
+  if (t->dFlagged) cudaFree(t->dFlagged);
+  if (t->dWeird) cudaFree(t->dWeird);
+  t->dFlagged = nullptr;
+  t->dWeird = nullptr;
   t->dKeys = nullptr;
   t->dStage = nullptr;
   t->dIds = nullptr;
@@ -667,14 +799,18 @@ int v3dm_voctree_allocate(v3dm_voctree* t, int nMax) {
       cudaMalloc(reinterpret_cast<void**>(&t->dStage), m * kDescBytes * sizeof(float)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&t->dIds), m * sizeof(int32_t)) != cudaSuccess)
     return V3DM_ERR_CUDA;
-  if (t->tcPath &&
+  if (vt_bins(t) > 0 &&
       (cudaMalloc(reinterpret_cast<void**>(&t->dBucket), m * sizeof(int32_t)) != cudaSuccess ||
        cudaMalloc(reinterpret_cast<void**>(&t->dPerm), m * sizeof(int32_t)) != cudaSuccess ||
-       cudaMalloc(reinterpret_cast<void**>(&t->dItems), (m / kVtItemKeys + t->maxBins + 1) * sizeof(int4)) !=
+       cudaMalloc(reinterpret_cast<void**>(&t->dItems), (m / kVtItemKeys + vt_bins(t) + 1) * sizeof(int4)) !=
            cudaSuccess))
     return V3DM_ERR_CUDA;
+  if (vt_f_wanted(t, nMax) &&
+      (cudaMalloc(reinterpret_cast<void**>(&t->dFlagged), m * sizeof(int4)) != cudaSuccess ||
+       cudaMalloc(reinterpret_cast<void**>(&t->dWeird), m * sizeof(int32_t)) != cudaSuccess))
+    return V3DM_ERR_CUDA;
   t->nMax = nMax;
-  return V3DM_OK;
+  return vt_planes(t);
 }
 
 int v3dm_voctree_set_nodes_u8(v3dm_voctree* t, const uint8_t* nodes) {
@@ -682,7 +818,7 @@ int v3dm_voctree_set_nodes_u8(v3dm_voctree* t, const uint8_t* nodes) {
   DeviceGuardVt g(t->device);
   if (!t->dNodes && cudaMalloc(reinterpret_cast<void**>(&t->dNodes), (size_t)t->nodeCount * kDescBytes) != cudaSuccess)
     return V3DM_ERR_CUDA;
-  t->nodesU8 = t->nodesF = false;
+  t->nodesU8 = t->nodesF = t->planesReady = false;
   if (cudaMemcpyAsync(t->dNodes, nodes, (size_t)t->nodeCount * kDescBytes, cudaMemcpyHostToDevice, t->stream) !=
           cudaSuccess ||
       cudaStreamSynchronize(t->stream) != cudaSuccess)
@@ -694,7 +830,7 @@ int v3dm_voctree_set_nodes_u8(v3dm_voctree* t, const uint8_t* nodes) {
 int v3dm_voctree_set_nodes_f32(v3dm_voctree* t, const float* nodes) {
   if (!t || !nodes) return V3DM_ERR_ARG;
   DeviceGuardVt g(t->device);
-  t->nodesU8 = t->nodesF = false;
+  t->nodesU8 = t->nodesF = t->planesReady = false;
   int st = vt_alloc_float_tree(t);
   if (st != V3DM_OK) return st;
   if (!t->dNodes && cudaMalloc(reinterpret_cast<void**>(&t->dNodes), (size_t)t->nodeCount * kDescBytes) != cudaSuccess)
@@ -709,7 +845,7 @@ int v3dm_voctree_set_nodes_f32(v3dm_voctree* t, const float* nodes) {
   if (st != V3DM_OK) return st;
   t->nodesF = true;
   t->nodesU8 = exact;  // u/512 trees also keep the faster integer descent
-  return V3DM_OK;
+  return vt_planes(t);
 }
 
 int v3dm_voctree_quantize_u8(v3dm_voctree* t, int n, const uint8_t* keys, int32_t* ids, int idMode) {
