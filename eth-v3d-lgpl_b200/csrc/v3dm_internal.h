@@ -201,6 +201,8 @@ cudaError_t launch_vtc(const VtcArgs& a, const CUtensorMap& nodeMap, const CUten
 // and resolved in the reference's arithmetic, keys that are not finite in the first phase's `weird`.
 struct VtfArgs {
   const float* keys;
+  const uint8_t* split;          // split keys, kVtfRowBytes each, and their norms (launch_vtf_split)
+  const float* keyNorm;
   const int32_t* perm;
   int bf, levels;
   long long bucketBase;
@@ -217,17 +219,18 @@ struct VtfArgs {
   long long nextBase;
   int* hist;
   int bins;
-  int4* flagged;
+  int4* flagged;                 // two per listed key: (key, node, levels, 0), the candidate children's mask
   int* nFlagged;
   int32_t* weird;                // null after the first phase
   int* nWeird;
   int* err;
 };
 int vtf_levels(int bf);          // levels a phase descends (0: shape not supported)
-constexpr int kVtfRowBytes = 512;  // split node planes per node
+constexpr int kVtfRowBytes = 512;  // split planes per node or key
 // The split node planes, the norms above (childNorm: rows / bf entries) and the planes' tensor map.
 cudaError_t vtf_prepare(const float* nodes, const float* norm, long long rows, int bf, void* planes, float* childNorm,
                         float* maxNorm, CUtensorMap* map, cudaStream_t st);
+cudaError_t launch_vtf_split(const float* keys, int n, void* split, float* norm, int numSMs, cudaStream_t st);
 // The phase and the resolution of what it listed.
 cudaError_t launch_vtf(const VtfArgs& a, const CUtensorMap& m, const float* nodes, unsigned long long* exactCount,
                        int grid, cudaStream_t st);

@@ -13,7 +13,9 @@
 //     keys scored against its children and grandchildren with tcgen05 int8 GEMMs;
 //   - k_voctree otherwise: one launch, four threads per key (below).
 // Float nodes and keys of any value:
-//   - k_voctree_f32: float nodes and keys (the apps' trees are float k-means
+//   - the tensor-core descent with exact replay of near ties (v3dm_voctree_f.cu) for shapes and
+//     calls with enough keys per bucket (vt_f_wanted);
+//   - k_voctree_f32 otherwise: float nodes and keys (the apps' trees are float k-means
 //     centres of unit-L2 descriptors, v3d_voctree.h:38-52).  The leaf ids equal those of the
 //     reference's CPU tree, VocabularyTree::findBestNodeIndex (v3d_voctree.h:82-99), which sums
 //     key[i] * node[i] sequentially for i = 0..127 in FP32 (one rounded product and one rounded
@@ -118,25 +120,25 @@ __global__ void k_vt_f32_to_u8(const float4* __restrict__ src, uint32_t* __restr
 // phase reached.  Between phases the keys are sorted by bucket (a counting sort: k_vt_scan,
 // then k_vt_scatter), and k_vt_scan cuts every bucket into work items of at most kVtItemKeys keys.
 constexpr int kVtItemKeys = 2048;       // keys per work item
+constexpr int kVtMinItem = 256;         // the smallest setting of the float descent
 constexpr int kVtMaxPhases = 32;        // phases of the float tensor descent
 constexpr int kVtLocalBins = 16384;     // bucket counts kept in shared memory by k_vt_scatter (2 x 64 KB)
 
 // Bucket offsets and the work items of a phase: (bucket, first key in sorted order, count), at
-// most kVtItemKeys keys each.  One block.  With bins == 1 and single > 0, one bucket of `single`
-// keys (the first phase: no histogram).
+// most itemKeys keys each.  One block.
 __global__ void __launch_bounds__(1024)
-k_vt_scan(const int* __restrict__ hist, int bins, int single, int* __restrict__ off, int4* __restrict__ items,
+k_vt_scan(const int* __restrict__ hist, int bins, int itemKeys, int* __restrict__ off, int4* __restrict__ items,
           int* __restrict__ nItems) {
   __shared__ long long sh[1024];
   __shared__ long long shI[1024];
   const int T = blockDim.x, tid = threadIdx.x;
   const int per = (bins + T - 1) / T;
   const int b0 = min(bins, tid * per), b1 = min(bins, b0 + per);
-  auto cnt = [&](int b) { return single > 0 ? single : hist[b]; };
+  auto cnt = [&](int b) { return hist[b]; };
   long long sk = 0, si = 0;
   for (int b = b0; b < b1; ++b) {
     sk += cnt(b);
-    si += (cnt(b) + kVtItemKeys - 1) / kVtItemKeys;
+    si += (cnt(b) + itemKeys - 1) / itemKeys;
   }
   sh[tid] = sk;
   shI[tid] = si;
@@ -152,7 +154,7 @@ k_vt_scan(const int* __restrict__ hist, int bins, int single, int* __restrict__ 
   for (int b = b0; b < b1; ++b) {
     const int c = cnt(b);
     off[b] = (int)k;
-    for (int j = 0; j < c; j += kVtItemKeys) items[it++] = make_int4(b, (int)k + j, min(kVtItemKeys, c - j), 0);
+    for (int j = 0; j < c; j += itemKeys) items[it++] = make_int4(b, (int)k + j, min(itemKeys, c - j), 0);
     k += c;
   }
   if (tid == T - 1) {
@@ -400,7 +402,8 @@ struct v3dm_voctree {
   bool planesReady = false;
   float* dMaxNorm = nullptr;
   float* dChildNorm = nullptr;  // in dPlanes' block
-  int4* dFlagged = nullptr;     // nMax
+  int4* dFlagged = nullptr;     // 2 x nMax
+  void* dSplit = nullptr;       // nMax split keys, then their norms
   int32_t* dWeird = nullptr;    // nMax
   int* dFCounts = nullptr;      // [0] weird keys, [1 + p] listed keys of phase p
   CUtensorMap tmPlanes;
@@ -452,7 +455,7 @@ long long vt_bins(const v3dm_voctree* t) {
 constexpr int kVtMinPerBin = 16;
 bool vt_f_wanted(const v3dm_voctree* t, long long n) { return t->fLevels > 0 && n >= kVtMinPerBin * t->fMaxBins; }
 
-int vt_sort(v3dm_voctree* t, int n, long long bins);
+int vt_sort(v3dm_voctree* t, int n, long long bins, int itemKeys);
 
 int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int idMode) {
   t->lastLaunches = 0;
@@ -504,7 +507,7 @@ int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int i
     const long long nextBins = bins * bf * bf;
     if (p > 0) {
       // keys sorted by the bucket the previous phase reached
-      const int st = vt_sort(t, n, bins);
+      const int st = vt_sort(t, n, bins, kVtItemKeys);
       if (st != V3DM_OK) return st;
     }
     if (!last && cudaMemsetAsync(t->dHist, 0, (size_t)nextBins * sizeof(int), t->stream) != cudaSuccess)
@@ -524,8 +527,8 @@ int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int i
 }
 
 // Keys in bucket order: offsets and work items from the histogram, then the permutation.
-int vt_sort(v3dm_voctree* t, int n, long long bins) {
-  k_vt_scan<<<1, 1024, 0, t->stream>>>(t->dHist, (int)bins, 0, t->dOff, t->dItems, t->dNItems);
+int vt_sort(v3dm_voctree* t, int n, long long bins, int itemKeys) {
+  k_vt_scan<<<1, 1024, 0, t->stream>>>(t->dHist, (int)bins, itemKeys, t->dOff, t->dItems, t->dNItems);
   if (cudaGetLastError() != cudaSuccess) return V3DM_ERR_CUDA;
   int* cursor = t->dHist + vt_bins(t);
   if (cudaMemsetAsync(cursor, 0, (size_t)bins * sizeof(int), t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
@@ -539,7 +542,7 @@ int vt_sort(v3dm_voctree* t, int n, long long bins) {
 int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int idMode) {
   t->lastLaunches = 0;
   if (n == 0) return V3DM_OK;
-  if (!vt_f_wanted(t, n) || !t->planesReady || !t->dFlagged || n > t->nMax) {
+  if (!vt_f_wanted(t, n) || !t->planesReady || !t->dSplit || n > t->nMax) {
     t->lastLaunches = 1;
     long long threads = (long long)n * kTpk;
     unsigned blocks = (unsigned)((threads + kVtThreads - 1) / kVtThreads);
@@ -549,13 +552,20 @@ int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int
     return cudaGetLastError() == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
   }
   if (cudaMemsetAsync(t->dFCounts, 0, (1 + kVtMaxPhases) * sizeof(int), t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
+  float* keyNorm = reinterpret_cast<float*>(static_cast<uint8_t*>(t->dSplit) + (size_t)t->nMax * kVtfRowBytes);
+  if (launch_vtf_split(dKeys, n, t->dSplit, keyNorm, t->numSMs, t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
+  t->lastLaunches += 1;
   VtfArgs va;
   std::memset(&va, 0, sizeof(va));
   va.keys = dKeys;
+  va.split = static_cast<const uint8_t*>(t->dSplit);
+  va.keyNorm = keyNorm;
   va.bf = t->bf;
   va.items = t->dItems;
   va.nItems = t->dNItems;
-  va.itemKeys = std::max(128, std::min(kVtItemKeys, (n / t->numSMs + 127) / 128 * 128));
+  // about eight items per CTA, so that an uneven last one costs little (whole tiles; an item's node
+  // rows are loaded once per item, from L2 for the second item of a bucket)
+  va.itemKeys = std::max(kVtMinItem, std::min(kVtItemKeys, n / (8 * t->numSMs) / 128 * 128));
   va.maxNorm = t->dMaxNorm;
   va.childNorm = t->dChildNorm;
   va.out = dIds;
@@ -574,7 +584,7 @@ int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int
     long long nextBins = bins;
     for (int k = 0; k < levels; ++k) nextBins *= t->bf;
     if (p > 0) {
-      const int st = vt_sort(t, n, bins);
+      const int st = vt_sort(t, n, bins, va.itemKeys);
       if (st != V3DM_OK) return st;
     }
     if (!last && cudaMemsetAsync(t->dHist, 0, (size_t)nextBins * sizeof(int), t->stream) != cudaSuccess)
@@ -762,6 +772,7 @@ int v3dm_voctree_destroy(v3dm_voctree* t) {
   if (t->dMaxNorm) cudaFree(t->dMaxNorm);
   if (t->dFCounts) cudaFree(t->dFCounts);
   if (t->dFlagged) cudaFree(t->dFlagged);
+  if (t->dSplit) cudaFree(t->dSplit);
   if (t->dWeird) cudaFree(t->dWeird);
   if (t->dPlanes) cudaFree(t->dPlanes);
   if (t->dKeys) cudaFree(t->dKeys);
@@ -785,8 +796,10 @@ int v3dm_voctree_allocate(v3dm_voctree* t, int nMax) {
   if (t->dPerm) cudaFree(t->dPerm);
   if (t->dItems) cudaFree(t->dItems);
   if (t->dFlagged) cudaFree(t->dFlagged);
+  if (t->dSplit) cudaFree(t->dSplit);
   if (t->dWeird) cudaFree(t->dWeird);
   t->dFlagged = nullptr;
+  t->dSplit = nullptr;
   t->dWeird = nullptr;
   t->dKeys = nullptr;
   t->dStage = nullptr;
@@ -802,13 +815,17 @@ int v3dm_voctree_allocate(v3dm_voctree* t, int nMax) {
   if (vt_bins(t) > 0 &&
       (cudaMalloc(reinterpret_cast<void**>(&t->dBucket), m * sizeof(int32_t)) != cudaSuccess ||
        cudaMalloc(reinterpret_cast<void**>(&t->dPerm), m * sizeof(int32_t)) != cudaSuccess ||
-       cudaMalloc(reinterpret_cast<void**>(&t->dItems), (m / kVtItemKeys + vt_bins(t) + 1) * sizeof(int4)) !=
+       cudaMalloc(reinterpret_cast<void**>(&t->dItems), (m / kVtMinItem + vt_bins(t) + 1) * sizeof(int4)) !=
            cudaSuccess))
     return V3DM_ERR_CUDA;
+  // the float descent's lists and split keys (548 bytes per key; without them calls take k_voctree_f32)
   if (vt_f_wanted(t, nMax) &&
-      (cudaMalloc(reinterpret_cast<void**>(&t->dFlagged), m * sizeof(int4)) != cudaSuccess ||
-       cudaMalloc(reinterpret_cast<void**>(&t->dWeird), m * sizeof(int32_t)) != cudaSuccess))
-    return V3DM_ERR_CUDA;
+      (cudaMalloc(reinterpret_cast<void**>(&t->dFlagged), 2 * m * sizeof(int4)) != cudaSuccess ||
+       cudaMalloc(reinterpret_cast<void**>(&t->dWeird), m * sizeof(int32_t)) != cudaSuccess ||
+       cudaMalloc(&t->dSplit, m * (kVtfRowBytes + sizeof(float))) != cudaSuccess)) {
+    cudaGetLastError();
+    t->dSplit = nullptr;
+  }
   t->nMax = nMax;
   return vt_planes(t);
 }

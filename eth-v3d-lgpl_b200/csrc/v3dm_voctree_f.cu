@@ -20,15 +20,19 @@
 //   - Keys whose norm times the largest node norm is not below 1e30 (NaN, infinities, overflow) are
 //     listed and descend with k_voctree_f32 at the end, whatever the phases made of them.
 // A phase descends one level (BF <= 128), or two where BF^2 grandchildren and BF children fit 128
-// MMA columns (BF <= 10); between phases k_vt_scan / k_vt_scatter sort the keys by node.
+// MMA columns (BF <= 10); between phases k_vt_scan / k_vt_scatter sort the keys by node.  The keys
+// are split once (k_vtf_split): splitting them in the phases, in the producers' registers, made the
+// phases issue-bound at 2.3 TB/s.
 //
-// Roles (one persistent CTA per SM, 13 warps): warps 0-7 read the tile's key rows (512 bytes each,
-// through the permutation), split them into two BF16 planes each in the MMA's swizzled layout and
-// keep the key's norm; warp 0 also loads an item's node rows with TMA (pre-split planes); warp 8
-// issues; warps 9-12 read the scores, one key per lane.  Every wait is bounded as in k_side.
+// Roles (one persistent CTA per SM, 9 warps): warps 0-3 gather the tile's split key rows (512 bytes
+// each, through the permutation) with cp.async, 16 bytes a lane, into the MMA's swizzled planes, and
+// their norms; warp 0 also loads an item's node rows with TMA (pre-split planes); warp 4 issues;
+// warps 5-8 read the scores, one key per lane.  Every wait is bounded as in k_side.
 //
-// What bounds it: reading the keys once per phase.  300,007 keys on a BF 50, depth 3 tree of 125,000
-// leaves: see vt_launch_f32 for the time against k_voctree_f32.
+// What bounds it: reading the keys once per phase (and writing them once).  300,007 keys on a BF 50,
+// depth 3 tree (125,000 leaves): 184 us a call, 2166 with k_voctree_f32; the split 45 us (6.8 TB/s),
+// the phases 37, 42 and 64 us (4.1 TB/s where the tiles are full; 120 keys per bucket in the last),
+// the lists 17, 11 and 10 us, the two sorts 31 us.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -40,11 +44,12 @@ namespace v3dm {
 
 namespace {
 
-constexpr int kVfProducers = 8;
+constexpr int kVfProducers = 4;
 constexpr int kVfMmaWarp = kVfProducers;
 constexpr int kVfEpiWarp0 = kVfProducers + 1;
 constexpr int kVfThreads = (kVfEpiWarp0 + 4) * 32;
 constexpr int kVfRows = 128;              // keys per tile
+static_assert(kVfProducers * 32 == kVfRows, "a producer warp has 32 rows of a tile, one key index per lane");
 constexpr int kVfPlanes = 4;              // 128-byte K planes per row: hi 0..63, hi 64..127, lo, lo
 constexpr int kVfABytes = kVfPlanes * kVfRows * 128;
 constexpr int kVfBBytes = 65536;          // node planes of up to two items
@@ -84,6 +89,19 @@ __device__ __forceinline__ void vtf_ld16(uint32_t taddr, uint32_t* v) {
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
         "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr));
+}
+
+// 16 (4) bytes to shared memory, asynchronously.
+__device__ __forceinline__ void vtf_cp16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void vtf_cp4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+// Raises the mbarrier's pending count by one now and arrives once every cp.async this thread has
+// issued so far has completed (so the phase cannot complete before the copies have landed).
+__device__ __forceinline__ void vtf_cp_arrive(unsigned long long* bar) {
+  asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // Two values' hi parts and lo parts, packed (the first value in the low half).
@@ -159,7 +177,8 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
   // Tiles are numbered from 0 in every role (i), items likewise (j): A slot i % 2, accumulator and
   // done barrier i % 4, norms i % 8, B buffer j % nBufs.
   if (warp < kVfProducers) {
-    // ---------------- producers: 16 rows of every tile each ----------------
+    // ---------------- producers: 32 rows of every tile each ----------------
+    const int row0 = warp * 32;
     uint32_t i = 0, j = 0;
     bool ok = true;
     for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j) {
@@ -183,19 +202,14 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
         __syncwarp();
       }
       const int tiles = (item.z + kVfRows - 1) / kVfRows;
+      // the lane's row of tile t: its key, -1 past the item's keys
+      auto load_key = [&](int t) -> int {
+        const int pos = t * kVfRows + row0 + lane;
+        if (pos >= item.z) return -1;
+        return a.perm ? __ldg(a.perm + item.y + pos) : item.y + pos;
+      };
+      int mine = load_key(0);
       for (int t = 0; t < tiles; ++t, ++i) {
-        const int row0 = warp * 16;
-        const int left = item.z - t * kVfRows - row0;  // keys of the bucket from this warp's first row on
-        const int pos = item.y + t * kVfRows + row0;
-        int mine = 0;
-        if (lane < 16 && lane < left) mine = a.perm ? __ldg(a.perm + pos + lane) : pos + lane;
-        float4 x[16];
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-          const int key = __shfl_sync(0xffffffffu, mine, r);
-          x[r] = r < left ? __ldg(reinterpret_cast<const float4*>(a.keys + (size_t)key * kDescBytes) + lane)
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
         // the slot's previous tile, i - 2, has been multiplied.  Its norms' slot is free as well: the
         // MMAs of tile i - 2 followed the epilogue's hand-back of tile i - 6, and this tile overwrites
         // the norms of tile i - 8.
@@ -204,43 +218,27 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
           ok = mbar_wait_warp(&s.done[d % kVfAcc], (d / kVfAcc) & 1u, &s.abort, a.err);
           if (!ok) break;
         }
+        const int next = t + 1 < tiles ? load_key(t + 1) : -1;
         const uint32_t slot = i % kVfASlots;
-        const uint32_t base = smem_u32(s.a[slot]) + (uint32_t)(lane >> 4) * (kVfRows * 128);
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-          const int row = row0 + r;
-          uint2 hi, lo;
-          split2(x[r].x, x[r].y, hi.x, lo.x);
-          split2(x[r].z, x[r].w, hi.y, lo.y);
-          // value 4 * lane of the row: plane lane / 16, 16-byte chunk (lane % 16) / 2, swizzled
-          const uint32_t at = base + (uint32_t)row * 128u +
-                              ((((uint32_t)(lane & 15) >> 1) ^ (uint32_t)(row & 7)) << 4) + ((uint32_t)lane & 1u) * 8u;
-          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(hi.x), "r"(hi.y) : "memory");
-          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + 2 * kVfRows * 128), "r"(lo.x), "r"(lo.y)
-                       : "memory");
+        // lane's 16 bytes of a row: plane lane / 8, chunk lane % 8
+        const uint32_t base = smem_u32(s.a[slot]) + (uint32_t)(lane >> 3) * (kVfRows * 128) + (uint32_t)row0 * 128u;
+        const uint32_t ch = (uint32_t)lane & 7u;
+        const int have = min(32, max(0, item.z - t * kVfRows - row0));  // rows past the item keep what is there
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) {
+          const int key = __shfl_sync(0xffffffffu, mine, r);
+          if (r < have)
+            vtf_cp16(base + (uint32_t)r * 128u + ((ch ^ (uint32_t)(r & 7)) << 4),
+                     a.split + (size_t)key * kVtfRowBytes + 16 * lane);
         }
-        // |key|: row r's sum ends in lane r (a butterfly that halves the rows at each step)
-        float ss[16];
-#pragma unroll
-        for (int r = 0; r < 16; ++r)
-          ss[r] = fmaf(x[r].x, x[r].x, fmaf(x[r].y, x[r].y, fmaf(x[r].z, x[r].z, x[r].w * x[r].w)));
-#pragma unroll
-        for (int w = 8; w > 0; w >>= 1) {
-#pragma unroll
-          for (int r = 0; r < 8; ++r) {
-            if (r >= w) break;
-            const bool up = (lane & w) != 0;
-            const float send = up ? ss[r] : ss[r + w], keep = up ? ss[r + w] : ss[r];
-            ss[r] = keep + __shfl_xor_sync(0xffffffffu, send, w);
-          }
-        }
-        ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 16);
-        if (lane < 16) s.norm[i % kVfNorms][row0 + lane] = sqrtf(ss[0]);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (lane < have) vtf_cp4(smem_u32(&s.norm[i % kVfNorms][row0 + lane]), a.keyNorm + mine);
+        vtf_cp_arrive(&s.fullA[slot]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&s.fullA[slot]);
+        mine = next;
       }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     // an item's node planes have landed before the CTA may exit (their bytes are waited for by the
     // issuer, except after an abort)
     if (warp == 0 && lane == 0)
@@ -271,6 +269,9 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
         const uint32_t ad = aBase + (i % kVfASlots) * (uint32_t)(kVfABytes >> 4);
         const uint32_t d = tmem + (i % kVfAcc) * 128u;
         if (leader) {
+          // the rows were written by cp.async (generic proxy); the tensor core reads them through the
+          // async proxy
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 #pragma unroll
           for (int k = 0; k < 24; ++k) {  // hi.hi', lo.hi', hi.lo', eight K steps of 16 values each
             const int prod = k >> 3, half = (k >> 2) & 1, step = k & 3;
@@ -348,28 +349,49 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
             }
           }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s.accEmpty[i % kVfAcc]);
-        if (key < 0) continue;
         const float tiny = 1e-30f * (1.0f + kn + maxNorm);  // underflow
+        const float e1 = kTcRel * kn * childNorm + tiny;
         const bool weird = !(kn * maxNorm < 1e30f);
-        if (weird && a.weird) a.weird[atomicAdd(a.nWeird, 1)] = key;  // first phase: descends by itself at the end
         long long node = g1 + ta.c;
-        int undecided = 0;  // levels left to the replay, from `node`'s parent down
-        long long from = 0;
-        if (!weird) {
-          if (!ta.decided(kTcRel * kn * childNorm + tiny)) {
+        int undecided = 0;  // levels left to the replay, from node `from` down
+        long long from = r;
+        if (key >= 0 && !weird) {
+          if (!ta.decided(e1)) {
             undecided = kBF2 ? 2 : 1;
-            from = r;
           } else if (kBF2 && !tc.decided(kTcRel * kn * __ldg(a.childNorm + node + 1) + tiny)) {
             undecided = 1;
             from = node;
           }
         }
+        // one level: the children whose scores come within twice the bound of the first, the only
+        // ones the sequential rule can choose
+        uint32_t mask[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+        if constexpr (kBF2 == 0) {
+          if (__any_sync(0xffffffffu, undecided)) {
+            const float lead = ta.s1 - 2.0f * e1;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              if (32 * c >= bf) break;
+              uint32_t v[32];
+              tmem_ld32(tb + (uint32_t)(32 * c), v);
+              tmem_wait(v);
+              uint32_t m = 0;
+#pragma unroll
+              for (int k = 0; k < 32; ++k) m |= __uint_as_float(v[k]) >= lead ? 1u << k : 0u;
+              mask[c] = m;
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s.accEmpty[i % kVfAcc]);
+        if (key < 0) continue;
+        if (weird && a.weird) a.weird[atomicAdd(a.nWeird, 1)] = key;  // first phase: descends by itself at the end
         if (kBF2) node = (node + 1) * bf + tc.c;
         if (undecided) {
-          a.flagged[atomicAdd(a.nFlagged, 1)] = make_int4(key, (int)from, undecided, 0);
+          const int at = atomicAdd(a.nFlagged, 1);
+          a.flagged[2 * at] = make_int4(key, (int)from, undecided, 0);
+          a.flagged[2 * at + 1] = make_int4((int)mask[0], (int)mask[1], (int)mask[2], (int)mask[3]);
           continue;
         }
         if (a.final) {
@@ -395,7 +417,8 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-// The listed keys' levels in the reference's arithmetic: a warp per key, a child per lane.
+// The listed keys' levels in the reference's arithmetic: a warp per key, a candidate child per lane
+// (the first level's come as a mask).
 __global__ void __launch_bounds__(256)
 k_vtf_resolve(VtfArgs a, const float* __restrict__ nodes, unsigned long long* __restrict__ exactCount) {
   const int lane = threadIdx.x & 31;
@@ -403,19 +426,29 @@ k_vtf_resolve(VtfArgs a, const float* __restrict__ nodes, unsigned long long* __
   const int bf = a.bf;
   unsigned long long levels = 0;
   for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (gridDim.x * blockDim.x) >> 5) {
-    const int4 f = a.flagged[w];
+    const int4 f = a.flagged[2 * w], fm = a.flagged[2 * w + 1];
     const float4* krow = reinterpret_cast<const float4*>(a.keys + (size_t)f.x * kDescBytes);
     long long node = f.y;
     for (int l = 0; l < f.z; ++l) {
       const long long base = (node + 1) * bf;
+      uint32_t m[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t in = bf >= 32 * (c + 1) ? 0xffffffffu : bf > 32 * c ? (1u << (bf - 32 * c)) - 1u : 0u;
+        m[c] = l == 0 ? in & (uint32_t)(c == 0 ? fm.x : c == 1 ? fm.y : c == 2 ? fm.z : fm.w) : in;
+      }
+      const int total = __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
       float best = -1e30f;
       int bi = -1;
-      for (int c = lane; c < bf; c += 32) {
+      for (int c0 = lane; c0 < total; c0 += 32) {
+        int k = c0, word = 0;  // the k-th candidate of the word
+        while (k >= __popc(m[word])) k -= __popc(m[word++]);
+        const int c = 32 * word + (int)__fns(m[word], 0, k + 1);
         const float4* nrow = reinterpret_cast<const float4*>(nodes + (size_t)(base + c) * kDescBytes);
         float sc = 0.0f;
 #pragma unroll 8
-        for (int k = 0; k < kDescBytes / 4; ++k) {
-          const float4 x = __ldg(krow + k), y = __ldg(nrow + k);
+        for (int q = 0; q < kDescBytes / 4; ++q) {
+          const float4 x = __ldg(krow + q), y = __ldg(nrow + q);
           sc = __fadd_rn(sc, __fmul_rn(x.x, y.x));
           sc = __fadd_rn(sc, __fmul_rn(x.y, y.y));
           sc = __fadd_rn(sc, __fmul_rn(x.z, y.z));
@@ -426,6 +459,7 @@ k_vtf_resolve(VtfArgs a, const float* __restrict__ nodes, unsigned long long* __
           bi = c;
         }
       }
+      __syncwarp();
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {  // the largest score, its first child
         const float so = __shfl_xor_sync(0xffffffffu, best, o);
@@ -453,6 +487,34 @@ k_vtf_resolve(VtfArgs a, const float* __restrict__ nodes, unsigned long long* __
     }
   }
   if (lane == 0 && levels) atomicAdd(exactCount, levels);
+}
+
+// Keys split: per key 512 bytes, BF16 hi of the 128 values and then lo, and the key's norm.  A warp
+// per key.
+__global__ void __launch_bounds__(256)
+k_vtf_split(const float4* __restrict__ keys, int n, uint2* __restrict__ split, float* __restrict__ norm) {
+  const int lane = threadIdx.x & 31;
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, step = (gridDim.x * blockDim.x) >> 5;
+  for (int k0 = 4 * w; k0 < n; k0 += 4 * step) {
+    float4 x[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      x[r] = k0 + r < n ? __ldg(keys + (size_t)(k0 + r) * 32 + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      uint2 hi, lo;
+      split2(x[r].x, x[r].y, hi.x, lo.x);
+      split2(x[r].z, x[r].w, hi.y, lo.y);
+      float ss = fmaf(x[r].x, x[r].x, fmaf(x[r].y, x[r].y, fmaf(x[r].z, x[r].z, x[r].w * x[r].w)));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (k0 + r < n) {
+        split[(size_t)(k0 + r) * 64 + lane] = hi;
+        split[(size_t)(k0 + r) * 64 + 32 + lane] = lo;
+        if (lane == 0) norm[k0 + r] = sqrtf(ss);
+      }
+    }
+  }
 }
 
 // Node rows as four planes of `rows` x 128 bytes: BF16 hi 0..63, hi 64..127, lo 0..63, lo 64..127.
@@ -525,6 +587,14 @@ cudaError_t vtf_prepare(const float* nodes, const float* norm, long long rows, i
   return cudaGetLastError();
 }
 
+cudaError_t launch_vtf_split(const float* keys, int n, void* split, float* norm, int numSMs, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  const int blocks = (n + 31) / 32;  // four keys per warp, eight warps
+  k_vtf_split<<<blocks < 16 * numSMs ? blocks : 16 * numSMs, 256, 0, st>>>(reinterpret_cast<const float4*>(keys), n,
+                                                                        static_cast<uint2*>(split), norm);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_vtf(const VtfArgs& a, const CUtensorMap& m, const float* nodes, unsigned long long* exactCount,
                        int grid, cudaStream_t st) {
   cudaError_t e;
@@ -541,7 +611,7 @@ cudaError_t launch_vtf(const VtfArgs& a, const CUtensorMap& m, const float* node
     default: e = launch_bf2<0>(a, m, grid, st); break;
   }
   if (e != cudaSuccess) return e;
-  k_vtf_resolve<<<4 * grid, 256, 0, st>>>(a, nodes, exactCount);
+  k_vtf_resolve<<<8 * grid, 256, 0, st>>>(a, nodes, exactCount);
   return cudaGetLastError();
 }
 

@@ -143,6 +143,56 @@ def test_float_keys_on_a_byte_tree_and_near_ties(v3dm_mod, oracle_mod):
     t.close()
 
 
+@pytest.mark.parametrize("bf,depth,n,vmax", [(2, 3, 500, 0.0), (3, 5, 20000, 0.01), (9, 4, 12000, 1.0), (10, 3, 1601, 0.0),
+                                             (11, 3, 2100, 1.0), (16, 2, 257, 0.0), (17, 3, 5000, 0.01),
+                                             (64, 2, 1100, 1.0), (100, 2, 1700, 0.01), (128, 2, 2049, 0.0)])
+def test_float_tensor_descent_shapes(v3dm_mod, oracle_mod, bf, depth, n, vmax):
+    """Shapes the float tensor-core descent takes, with one level per phase and two, an odd last
+    level, branching factors at the edges of the 16-column and 32-column steps, few keys per bucket;
+    values of either sign (vmax 0: unit descriptors; 0.01: nodes within 1% of each other, so that
+    most levels are replayed; 1: any sign, some norms huge and tiny), zero, NaN, infinite and
+    overflowing keys, copied nodes (ties).  Ids equal the oracle's sequential FP32 descent; a call
+    above the allocated count and one with few keys take the one-kernel descent, with the same ids."""
+    import torch
+    rng = synth.rng_for(9000 + 100 * bf + depth)
+    count = v3dm_mod.voctree_counts(bf, depth)[0]
+    if vmax == 0.0:
+        nodes, keys = synth.unit_sift(rng, count), synth.unit_sift(rng, n)
+    elif vmax == 0.01:
+        nodes = (synth.unit_sift(rng, 1) * (1 + rng.normal(0, 0.01, (count, 128)))).astype(np.float32)
+        keys = synth.unit_sift(rng, n)
+    else:
+        nodes = rng.normal(0, 1, (count, 128)).astype(np.float32)
+        keys = rng.normal(0, 1, (n, 128)).astype(np.float32)
+        nodes[3] *= 1e4
+        keys[20] *= 1e-6
+        keys[21] *= 1e6
+    nodes[bf // 2] = nodes[0]
+    keys[3] = np.nan
+    keys[4] = 0.0
+    keys[5, 7] = np.inf
+    keys[6] = 3e38
+    keys[9] = -keys[9]
+    exp = oracle_mod.voctree(bf, depth, nodes, keys, True)
+    with v3dm_mod.VocabularyTreeTraversal(bf, depth) as t:
+        t.allocate(n)
+        t.set_nodes(nodes)
+        np.testing.assert_array_equal(t.traverse_tree(keys, v3dm_mod.LEAF_GLOBAL), exp)
+        assert t.last_launches() > 1  # the phases ran
+        np.testing.assert_array_equal(t.traverse_tree(keys[:11], v3dm_mod.LEAF_GLOBAL), exp[:11])
+        np.testing.assert_array_equal(t.traverse_tree(keys, v3dm_mod.LEAF_GLOBAL), exp)
+        d_keys = torch.from_numpy(np.concatenate([keys, keys])).cuda()
+        d_ids = torch.empty(2 * n, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        t.quantize_f32_device(2 * n, d_keys.data_ptr(), d_ids.data_ptr(), v3dm_mod.LEAF_GLOBAL)
+        torch.cuda.synchronize()
+        assert t.last_launches() == 1
+        np.testing.assert_array_equal(d_ids.cpu().numpy(), np.concatenate([exp, exp]))
+        t.set_nodes(nodes[::-1].copy())  # another tree on the same handle
+        np.testing.assert_array_equal(t.traverse_tree(keys, v3dm_mod.LEAF_GLOBAL),
+                                      oracle_mod.voctree(bf, depth, nodes[::-1].copy(), keys, True))
+
+
 def test_config_tree_all_queries(v3dm_mod, oracle_mod):
     """The vocabulary-tree configuration at full size: BF 10, depth 6, HKM centres from 500k
     descriptors, all 2,000,000 queries; leaf ids equal the reference CPU tree's."""
