@@ -21,18 +21,17 @@
 // dot products are exact integers (at most 255 * 255 * 128 < 2^23), so the leaf ids are the
 // reference's whatever the summation order; ties keep the first child.
 //
-// Roles (one persistent CTA per SM, 352 threads):
-//   warps 0-1   producers, alternate tiles: the first phase's keys are consecutive and come as
-//               one TMA tile (128 rows, 128-byte swizzle); later phases gather their rows through
-//               the permutation with cp.async (16-byte chunks into the same swizzle, eight lanes
-//               per row, rows past the bucket zero), each lane's copies completing on the slot's
-//               mbarrier (cp.async.mbarrier.arrive).  Producer 0 also loads every item's
-//               subtree rows with TMA (boxes of 16 rows) into a ring of B buffers; the
-//               rows past the BF children and BF^2 grandchildren that a box brings along only fill
-//               columns the epilogue never reads;
-//   warp 2      allocates 512 TMEM columns and issues the MMAs of a tile into one of
-//               512 / (N2 + 16) accumulator stages;
-//   warps 3-10  epilogue, two warps per TMEM lane quadrant taking alternate tiles.
+// Roles (one persistent CTA per SM, 13 warps):
+//   warps 0-3   producers: the first phase's keys are consecutive and come as one TMA tile (128 rows,
+//               128-byte swizzle) that warp 0 loads; later phases gather their rows through the
+//               permutation with cp.async, 32 rows of a tile per warp (16-byte chunks into the same
+//               swizzle, eight lanes per row), each lane's copies completing on the slot's mbarrier
+//               (cp.async.mbarrier.arrive).  Warp 0 also loads every item's subtree rows with TMA
+//               (boxes of 16 rows) into a ring of B buffers; the rows past the BF children and BF^2
+//               grandchildren that a box brings along only fill columns the epilogue never reads;
+//   warp 4      allocates 512 TMEM columns and issues the MMAs of a tile into one of
+//               512 / (N2 + 16) accumulator stages (the warp walks, one elected lane issues);
+//   warps 5-12  epilogue, two warps per TMEM lane quadrant taking alternate tiles.
 // Every mbarrier wait is bounded (kWaitCycles); on timeout the CTA records kErrWaitTimeout,
 // drains its own copies and MMAs, frees TMEM and returns.
 #include <cuda.h>
@@ -46,13 +45,14 @@ namespace v3dm {
 
 namespace {
 
-constexpr int kVtcProducers = 2;                // producer warps, taking alternate tiles
+constexpr int kVtcProducers = 4;                // producer warps, 32 rows of a tile each
 constexpr int kVtcMmaWarp = kVtcProducers;      // the MMA issuer's warp
 constexpr int kVtcEpiWarp0 = kVtcProducers + 1; // first epilogue warp
 constexpr int kVtcEpiHalves = 2;                // epilogue warps per TMEM lane quadrant
 constexpr int kVtcThreads = (kVtcEpiWarp0 + 4 * kVtcEpiHalves) * 32;
 constexpr int kVtcRows = 128;                   // keys per tile (TMEM lanes)
-constexpr int kVtcASlots = 6;                   // key-tile ring depth
+static_assert(kVtcProducers * 32 == kVtcRows, "a producer warp has 32 rows of a tile, one key index per lane");
+constexpr int kVtcASlots = 8;                   // key-tile ring depth
 constexpr int kVtcTmemCols = 512;
 constexpr int kVtcLocalBins = 4096;             // next-phase histogram kept in shared memory up to this
 constexpr int kVtcItemKeys = 2048;              // keys per implicit item of a single-bucket phase
@@ -77,8 +77,8 @@ struct VtcSmem {
   uint8_t a[kVtcASlots][S::kABytes];
   uint8_t b[S::kBBufs][S::kBBytes];
   int hist[kVtcLocalBins];
-  unsigned long long fullA[kVtcASlots], emptyA[kVtcASlots], fullB[S::kBBufs], emptyB[S::kBBufs];
-  unsigned long long accFull[S::kAcc], accEmpty[S::kAcc], mmaDone;
+  unsigned long long fullA[kVtcASlots], done[kVtcASlots];  // a tile's keys have landed; its MMAs have completed
+  unsigned long long fullB[S::kBBufs], emptyB[S::kBBufs], accEmpty[S::kAcc], mmaDone;
   uint32_t tmemBase;
   int abort;
 };
@@ -99,21 +99,8 @@ __device__ __forceinline__ void vtc_mma(uint32_t dtmem, uint64_t ad, uint64_t bd
       : "memory");
 }
 
-// Non-blocking test of an mbarrier phase.
-__device__ __forceinline__ bool mbar_test(unsigned long long* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ void vtc_cp16(uint32_t dst, const void* src, uint32_t srcBytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(srcBytes) : "memory");
+__device__ __forceinline__ void vtc_cp16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 // Raises the mbarrier's pending count by one now and arrives once every cp.async this thread has
 // issued so far has completed (so the phase cannot complete before the copies have landed).
@@ -131,47 +118,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
         "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr));
 }
-
-// The work walk every role follows: the CTA's items (it = blockIdx.x, += gridDim.x), each cut
-// into tiles of 128 keys.  The next item is loaded one item ahead (small items follow each
-// other quickly).
-struct VtcWalk {
-  const int4* items;
-  int nIt, it, t, single;
-  int4 item, pre;
-  // single > 0: one bucket of `single` keys, cut into items of kVtcItemKeys in order
-  __device__ int4 load(int i) const {
-    if (i >= nIt) return make_int4(0, 0, 0, 0);
-    if (single > 0) return make_int4(0, i * kVtcItemKeys, min(kVtcItemKeys, single - i * kVtcItemKeys), 0);
-    return __ldg(items + i);
-  }
-  __device__ bool start(const int4* its, int n, int singleN) {
-    items = its;
-    nIt = n;
-    single = singleN;
-    it = blockIdx.x;
-    t = 0;
-    if (it >= nIt) return false;
-    item = load(it);
-    pre = load(it + gridDim.x);
-    return true;
-  }
-  __device__ bool first() const { return t == 0; }
-  __device__ bool last() const { return (t + 1) * kVtcRows >= item.z; }
-  // advances; returns false past the last tile
-  __device__ bool next() {
-    if (!last()) {
-      ++t;
-      return true;
-    }
-    it += gridDim.x;
-    t = 0;
-    if (it >= nIt) return false;
-    item = pre;
-    pre = load(it + gridDim.x);
-    return true;
-  }
-};
 
 // First index of the largest of v[0..BF-1] (strict '>': the first wins ties).
 template <int BF>
@@ -196,21 +142,23 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nIt = a.singleN > 0 ? (a.singleN + kVtcItemKeys - 1) / kVtcItemKeys : *a.nItems;
   const bool localHist = !a.final && a.bins <= kVtcLocalBins;
-  const long long lim = kWaitCycles;
+  const bool gathered = a.perm != nullptr;
+  // item `it`: (bucket, first position, keys)
+  auto item_at = [&](int it) -> int4 {
+    if (a.singleN > 0) return make_int4(0, it * kVtcItemKeys, min(kVtcItemKeys, a.singleN - it * kVtcItemKeys), 0);
+    return __ldg(a.items + it);
+  };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kVtcASlots; ++i) {
-      mbar_init(&s.fullA[i], 1);  // the producer's arrival (with a TMA's bytes, or its lanes' copies)
-      mbar_init(&s.emptyA[i], 1);
+      mbar_init(&s.fullA[i], gathered ? kVtcProducers : 1);  // with a TMA's bytes, or every lane's copies
+      mbar_init(&s.done[i], 1);
     }
     for (int i = 0; i < S::kBBufs; ++i) {
       mbar_init(&s.fullB[i], 1);
       mbar_init(&s.emptyB[i], 1);
     }
-    for (int i = 0; i < S::kAcc; ++i) {
-      mbar_init(&s.accFull[i], 1);
-      mbar_init(&s.accEmpty[i], 4);  // the four warps of the half that takes the tile
-    }
+    for (int i = 0; i < S::kAcc; ++i) mbar_init(&s.accEmpty[i], 4);  // the four warps of the half that takes the tile
     mbar_init(&s.mmaDone, 1);
     s.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -232,267 +180,186 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
     s.abort = 1;
   }
   __syncthreads();
+  const bool run = !s.abort;
 
+  // Tiles are numbered from 0 in every role (i), items likewise (j): A slot and done barrier
+  // i % kVtcASlots, accumulator i % kAcc, epilogue half i % 2, B buffer j % kBBufs.  (The walk was a
+  // cursor advanced at every tile, with two producers and a lane-0 issuer: the waits, branches and
+  // operand moves of one tile took longer than its 16 KB of keys.  2M keys on the BF 10, depth 6 tree:
+  // 358 us a call then, 315 now; the streamed phase 54 us, 4.7 TB/s, the gathered ones 103 and 157.)
   if (warp < kVtcProducers) {
-    // ---------------- producers: key tiles and subtree rows (warp p takes tiles p, p + 2, ...) ----
-    // Both walk every tile (the tile number gives the A slot, the item number the B buffer);
-    // producer 0 also loads every item's subtree, so that one warp owns the B ring (and knows,
-    // after an abort, which of its loads may still be in flight).
-    if (!s.abort) {
-      const int p = warp;
-      VtcWalk w;
-      int tn = 0, nItem = 0;
-      bool armedB[S::kBBufs];  // B buffers with a TMA load this warp has not seen land (for an abort)
-      uint32_t armedPar[S::kBBufs];
-#pragma unroll
-      for (int i = 0; i < S::kBBufs; ++i) armedB[i] = false;
-      // gathered keys: the key index of each row this lane copies (row 4 i + lane / 8, chunk
-      // lane % 8), -1 past the bucket; the next own tile's are loaded while this one's copies go out
-      auto tile_keys = [&](const VtcWalk& v, int (&kk)[kVtcRows / 4]) {
-        const int base = v.item.y + v.t * kVtcRows;
-        const int cnt = min(kVtcRows, v.item.z - v.t * kVtcRows);
-#pragma unroll
-        for (int i = 0; i < kVtcRows / 4; ++i) {
-          const int rr = 4 * i + (lane >> 3);
-          kk[i] = rr < cnt ? __ldg(a.perm + base + rr) : -1;
+    // ---------------- producers ----------------
+    const int row0 = warp * 32;
+    uint32_t i = 0, j = 0;
+    bool ok = run;
+    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j) {
+      const int4 item = item_at(it);
+      if (warp == 0) {
+        const uint32_t buf = j % S::kBBufs;
+        ok = mbar_wait_warp(&s.emptyB[buf], ((j / S::kBBufs) & 1u) ^ 1u, &s.abort, a.err);
+        if (!ok) break;
+        if (lane == 0) {
+          // subtree of the item's bucket node r: children from g1 (buffer rows N2 ..), and
+          // grandchildren from g2 (buffer rows 0 .. N2 - 1)
+          const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + item.x;
+          const long long g1 = (r + 1) * BF, g2 = (g1 + 1) * BF;
+          const int boxes = a.levels == 2 ? S::N2 / kVtcBoxRows : 0;
+          mbar_expect_tx(&s.fullB[buf], (uint32_t)((boxes + 1) * kVtcBoxRows * kDescBytes));
+          tma_load_2d(s.b[buf] + S::N2 * kDescBytes, &tmNodes, &s.fullB[buf], 0, (int)g1);
+          for (int x = 0; x < boxes; ++x)
+            tma_load_2d(s.b[buf] + x * kVtcBoxRows * kDescBytes, &tmNodes, &s.fullB[buf], 0,
+                        (int)(g2 + x * kVtcBoxRows));
         }
-      };
-      // bounded wait by lane 0, the result broadcast
-      auto wait_free = [&](unsigned long long* bar, uint32_t par) -> bool {
-        int okl = 1;
-        if (lane == 0) okl = mbar_wait(bar, par, &s.abort, a.err, lim) ? 1 : 0;
-        return __shfl_sync(0xffffffffu, okl, 0) != 0;
-      };
-      const bool gathered = a.perm != nullptr;
-      int keysCur[kVtcRows / 4], keysNext[kVtcRows / 4];
-      bool more = w.start(a.items, nIt, a.singleN);
-      if (gathered) {  // the first own tile's keys
-        VtcWalk v = w;
-        bool m = more;
-        for (int k = 0; k < p && m; ++k) m = v.next();
-        if (m) tile_keys(v, keysNext);
+        __syncwarp();
       }
-      bool ok = true;
-      for (; more && ok; more = w.next(), ++tn) {
-        const bool mine = (tn % kVtcProducers) == p;
-        if (w.first()) {
-          const int buf = nItem % S::kBBufs;
-          const uint32_t use = (uint32_t)(nItem / S::kBBufs);
-          ++nItem;
-          if (p == 0) {
-            if (!wait_free(&s.emptyB[buf], (use & 1u) ^ 1u)) break;
+      const int tiles = (item.z + kVtcRows - 1) / kVtcRows;
+      if (!gathered) {
+        if (warp == 0)  // consecutive keys: one TMA tile (rows past the last key read as zero)
+          for (int t = 0; t < tiles; ++t, ++i) {
+            const uint32_t slot = i % kVtcASlots;
+            ok = mbar_wait_warp(&s.done[slot], ((i / kVtcASlots) & 1u) ^ 1u, &s.abort, a.err);
+            if (!ok) break;
             if (lane == 0) {
-              // subtree of the item's bucket node r: children from g1 (buffer rows N2 ..), and
-              // grandchildren from g2 (buffer rows 0 .. N2 - 1)
-              const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + w.item.x;
-              const long long g1 = (r + 1) * BF, g2 = (g1 + 1) * BF;
-              const int boxes = a.levels == 2 ? S::N2 / kVtcBoxRows : 0;
-              mbar_expect_tx(&s.fullB[buf], (uint32_t)((boxes + 1) * kVtcBoxRows * kDescBytes));
-              tma_load_2d(s.b[buf] + S::N2 * kDescBytes, &tmNodes, &s.fullB[buf], 0, (int)g1);
-              for (int x = 0; x < boxes; ++x)
-                tma_load_2d(s.b[buf] + x * kVtcBoxRows * kDescBytes, &tmNodes, &s.fullB[buf], 0,
-                            (int)(g2 + x * kVtcBoxRows));
+              mbar_expect_tx(&s.fullA[slot], (uint32_t)S::kABytes);
+              tma_load_2d(s.a[slot], &tmKeys, &s.fullA[slot], 0, item.y + t * kVtcRows);
             }
-            armedB[buf] = true;
-            armedPar[buf] = use & 1u;
+            __syncwarp();
           }
-        }
-        if (!mine) continue;
-        if (gathered) {
+        continue;
+      }
+      // the lane's row of tile t: its key
+      auto load_key = [&](int t) -> int {
+        const int pos = t * kVtcRows + row0 + lane;
+        return pos < item.z ? __ldg(a.perm + item.y + pos) : 0;
+      };
+      int mine = load_key(0);
+      for (int t = 0; t < tiles; ++t, ++i) {
+        const uint32_t slot = i % kVtcASlots;
+        const int next = t + 1 < tiles ? load_key(t + 1) : 0;
+        ok = mbar_wait_warp(&s.done[slot], ((i / kVtcASlots) & 1u) ^ 1u, &s.abort, a.err);
+        if (!ok) break;
+        // eight lanes per 128-byte row, four rows per instruction; rows past the item keep what is there
+        const int have = item.z - t * kVtcRows - row0;
+        const uint32_t base = smem_u32(s.a[slot]) + (uint32_t)row0 * 128u;
+        const int ch = lane & 7;
 #pragma unroll
-          for (int k = 0; k < kVtcRows / 4; ++k) keysCur[k] = keysNext[k];
-          VtcWalk v = w;
-          bool m = true;
-          for (int k = 0; k < kVtcProducers && m; ++k) m = v.next();
-          if (m) tile_keys(v, keysNext);
+        for (int k = 0; k < 8; ++k) {
+          const int rr = 4 * k + (lane >> 3);
+          const int key = __shfl_sync(0xffffffffu, mine, rr);
+          if (rr < have)
+            vtc_cp16(base + (uint32_t)rr * 128u + (uint32_t)((ch ^ (rr & 7)) << 4),
+                     a.keys + (size_t)key * kDescBytes + 16 * ch);
         }
-        const int slot = tn % kVtcASlots;
-        const uint32_t phaseA = (uint32_t)(tn / kVtcASlots) & 1u;
-        if (!wait_free(&s.emptyA[slot], phaseA ^ 1)) {
-          ok = false;
-          break;
-        }
-        if (!gathered) {
-          // consecutive keys: one TMA tile (rows past the last key read as zero)
-          if (lane == 0) {
-            mbar_expect_tx(&s.fullA[slot], (uint32_t)S::kABytes);
-            tma_load_2d(s.a[slot], &tmKeys, &s.fullA[slot], 0, w.item.y + w.t * kVtcRows);
-          }
-        } else {
-          // eight lanes per 128-byte row, four rows per instruction; each lane's copies are
-          // tracked by the slot's mbarrier, then lane 0 adds the producer's own arrival
-          const uint32_t d0 = smem_u32(s.a[slot]);
-          const int ch = lane & 7;
-#pragma unroll
-          for (int i = 0; i < kVtcRows / 4; ++i) {
-            const int rr = 4 * i + (lane >> 3);
-            const int key = keysCur[i];
-            const uint8_t* g = a.keys + (key >= 0 ? (size_t)key * kDescBytes + 16 * ch : (size_t)0);
-            vtc_cp16(d0 + (uint32_t)rr * 128u + (uint32_t)((ch ^ (rr & 7)) << 4), g, key >= 0 ? 16u : 0u);
-          }
-          vtc_cp_arrive(&s.fullA[slot]);
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&s.fullA[slot]);
+        vtc_cp_arrive(&s.fullA[slot]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s.fullA[slot]);
+        mine = next;
+      }
+    }
+    vtc_wait_all();
+    // after an abort, the TMA loads still in flight land before the CTA exits
+    if (warp == 0 && lane == 0) {
+      for (uint32_t k = j > (uint32_t)S::kBBufs ? j - S::kBBufs : 0u; k < j; ++k) {
+        const long long t0 = clock64();
+        while (!mbar_try(&s.fullB[k % S::kBBufs], (k / S::kBBufs) & 1u) && clock64() - t0 < kWaitCycles) {
         }
       }
-      vtc_wait_all();
-      // after an abort, the TMA loads still in flight land before the CTA exits
-      if (lane == 0)
-        for (int i = 0; i < S::kBBufs; ++i)
-          if (armedB[i]) {
-            long long t0 = clock64();
-            while (!mbar_try(&s.fullB[i], armedPar[i]) && clock64() - t0 < kWaitCycles) {
-            }
-          }
+      for (uint32_t k = i > (uint32_t)kVtcASlots ? i - kVtcASlots : 0u; !gathered && k < i; ++k) {
+        const long long t0 = clock64();
+        while (!mbar_try(&s.fullA[k % kVtcASlots], (k / kVtcASlots) & 1u) && clock64() - t0 < kWaitCycles) {
+        }
+      }
     }
   } else if (warp == kVtcMmaWarp) {
-    // ---------------- MMA issuer (lane 0) ----------------
-    // A tile is one chain of four dependent MMAs (K = 32 each) into its accumulator stage.  When
-    // the next tile is ready as well, the two chains are issued interleaved so that the tensor
-    // core overlaps them.
-    if (lane == 0 && !s.abort) {
-      struct Tile {
-        int slot, acc, buf;
-        bool last;
-      };
-      VtcWalk w;
-      int slot = 0, acc = 0, nItem = 0, buf = 0;
-      uint32_t phaseA = 0, accPhase = 0;
-      bool any = false;
-      // the tile at v: blocking waits (false: abort), or a non-blocking check (false: not ready)
-      auto acquire = [&](const VtcWalk& v, bool block, Tile& t) -> bool {
-        int b = buf;
-        if (v.first()) {
-          b = nItem % S::kBBufs;
-          const uint32_t par = (uint32_t)(nItem / S::kBBufs) & 1u;
-          if (block ? !mbar_wait(&s.fullB[b], par, &s.abort, a.err, lim) : !mbar_test(&s.fullB[b], par)) return false;
-        }
-        if (block ? !mbar_wait(&s.fullA[slot], phaseA, &s.abort, a.err, lim) : !mbar_test(&s.fullA[slot], phaseA))
-          return false;
-        if (block ? !mbar_wait(&s.accEmpty[acc], accPhase ^ 1, &s.abort, a.err, lim)
-                  : !mbar_test(&s.accEmpty[acc], accPhase ^ 1))
-          return false;
-        if (v.first()) {
-          buf = b;
-          ++nItem;
-        }
-        t.slot = slot;
-        t.acc = acc;
-        t.buf = buf;
-        t.last = v.last();
-        if (++slot == kVtcASlots) {
-          slot = 0;
-          phaseA ^= 1;
-        }
-        if (++acc == S::kAcc) {
-          acc = 0;
-          accPhase ^= 1;
-        }
-        return true;
-      };
-      auto mma_k = [&](const Tile& t, int k) {
-        const uint32_t aAddr = smem_u32(s.a[t.slot]), bAddr = smem_u32(s.b[t.buf]);
-        const uint32_t d2 = tmem + (uint32_t)(t.acc * S::kAccCols), d1 = d2 + S::N2;
-        if (a.levels == 2)  // grandchildren and children: one chain over all kRowsB rows
-          vtc_mma<S::kRowsB>(d2, sdesc(aAddr + 32u * k), sdesc(bAddr + 32u * k), k > 0 ? 1u : 0u);
-        else
-          vtc_mma<S::N1>(d1, sdesc(aAddr + 32u * k), sdesc(bAddr + (uint32_t)(S::N2 * kDescBytes) + 32u * k),
-                         k > 0 ? 1u : 0u);
-      };
-      auto commit = [&](const Tile& t) {
-        mma_commit(&s.accFull[t.acc]);
-        mma_commit(&s.emptyA[t.slot]);
-        if (t.last) mma_commit(&s.emptyB[t.buf]);
-      };
-      bool more = w.start(a.items, nIt, a.singleN);
-      while (more) {
-        Tile t0, t1;
-        if (!acquire(w, true, t0)) break;
-        VtcWalk w1 = w;
-        const bool more1 = w1.next();
-        const bool pair = more1 && acquire(w1, false, t1);
-        // the key rows were written by cp.async (generic proxy); the tensor core reads them
-        // through the async proxy
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // ---------------- MMA issuer ----------------
+    const bool leader = elect_one();
+    const uint32_t aBase = sdesc_lo(smem_u32(s.a[0])), bBase = sdesc_lo(smem_u32(s.b[0]));
+    uint32_t i = 0, j = 0;
+    bool ok = run;
+    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j) {
+      const int4 item = item_at(it);
+      const uint32_t buf = j % S::kBBufs;
+      ok = mbar_wait_warp(&s.fullB[buf], (j / S::kBBufs) & 1u, &s.abort, a.err);
+      const uint32_t bd = bBase + buf * (uint32_t)(S::kBBytes >> 4);
+      const uint32_t iEnd = i + (uint32_t)((item.z + kVtcRows - 1) / kVtcRows);
+      for (; i < iEnd && ok; ++i) {
+        const uint32_t slot = i % kVtcASlots, acc = i % S::kAcc;
+        ok = mbar_wait_warp(&s.fullA[slot], (i / kVtcASlots) & 1u, &s.abort, a.err) &&
+             mbar_wait_warp(&s.accEmpty[acc], ((i / S::kAcc) & 1u) ^ 1u, &s.abort, a.err);
+        if (!ok) break;
         tc_fence_after();
+        const uint32_t ad = aBase + slot * (uint32_t)(S::kABytes >> 4);
+        const uint32_t d2 = tmem + acc * (uint32_t)S::kAccCols;
+        if (leader) {
+          // the gathered key rows were written by cp.async (generic proxy); the tensor core reads
+          // them through the async proxy
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 #pragma unroll
-        for (int k = 0; k < kDescBytes / 32; ++k) {
-          mma_k(t0, k);
-          if (pair) mma_k(t1, k);
+          for (int k = 0; k < kDescBytes / 32; ++k) {
+            if (a.levels == 2)  // grandchildren and children: one chain over all kRowsB rows
+              vtc_mma<S::kRowsB>(d2, sdesc_of(ad + 2u * k), sdesc_of(bd + 2u * k), k > 0 ? 1u : 0u);
+            else
+              vtc_mma<S::N1>(d2 + S::N2, sdesc_of(ad + 2u * k),
+                             sdesc_of(bd + (uint32_t)(S::N2 * kDescBytes >> 4) + 2u * k), k > 0 ? 1u : 0u);
+          }
+          mma_commit(&s.done[slot]);
         }
-        any = true;
-        commit(t0);
-        if (pair) {
-          commit(t1);
-          w = w1;
-        }
-        more = w.next();
       }
-      if (any) {  // every MMA issued has completed before TMEM is released
-        mma_commit(&s.mmaDone);
-        long long t0 = clock64();
-        while (!mbar_try(&s.mmaDone, 0) && clock64() - t0 < kWaitCycles) {
-        }
+      if (leader) mma_commit(&s.emptyB[buf]);
+    }
+    if (leader) {  // every MMA issued has completed before TMEM is released
+      mma_commit(&s.mmaDone);
+      const long long t0 = clock64();
+      while (!mbar_try(&s.mmaDone, 0) && clock64() - t0 < kWaitCycles) {
       }
     }
+    __syncwarp();
   } else {
     // ---------------- epilogue: one key per thread ----------------
     const int q = warp & 3;                  // TMEM lane quadrant this warp may access
-    const int half = (warp - kVtcEpiWarp0) >> 2;  // the tiles it takes: every other one
+    const uint32_t half = (uint32_t)(warp - kVtcEpiWarp0) >> 2;  // the tiles it takes: every other one
     const int row = q * 32 + lane;
-    VtcWalk w;
-    int acc = 0, tn = 0;
-    uint32_t accPhase = 0;
-    for (bool more = w.start(a.items, nIt, a.singleN); more; more = w.next(), ++tn) {
-      if ((tn % kVtcEpiHalves) != half) {
-        if (++acc == S::kAcc) {
-          acc = 0;
-          accPhase ^= 1;
-        }
-        continue;
-      }
+    uint32_t i0 = 0;                         // the item's first tile
+    bool ok = run;
+    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x) {
+      const int4 item = item_at(it);
+      const int tiles = (item.z + kVtcRows - 1) / kVtcRows;
+      const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + item.x;
+      const long long g1 = (r + 1) * BF;
+      for (int t = (int)((i0 ^ half) & 1u); t < tiles; t += 2) {
+      const uint32_t i = i0 + (uint32_t)t, acc = i % S::kAcc;
       // this row's key index, loaded before the wait for the accumulator
-      const int pos = w.t * kVtcRows + row;
-      const int key = pos < w.item.z ? (a.perm ? __ldg(a.perm + w.item.y + pos) : w.item.y + pos) : -1;
-      if (!mbar_wait(&s.accFull[acc], accPhase, &s.abort, a.err, lim)) break;
+      const int pos = t * kVtcRows + row;
+      const int key = pos < item.z ? (gathered ? __ldg(a.perm + item.y + pos) : item.y + pos) : -1;
+      ok = mbar_wait_warp(&s.done[i % kVtcASlots], (i / kVtcASlots) & 1u, &s.abort, a.err);
+      if (!ok) break;
       tc_fence_after();
       const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * S::kAccCols);
-      uint32_t v[S::kAccCols];  // D2 in columns 0 .. N2 - 1, D1 in N2 .. N2 + 15
+      // D2 in columns 0 .. N2 - 1, D1 in N2 .. N2 + 15
+      uint32_t d1[16];
+      tmem_ld16(tb + S::N2, d1);
+      tmem_wait(d1);
+      const int c1 = vtc_argmax<BF>(d1);
+      uint32_t g[BF];  // the chosen child's BF children: columns BF c1 .. BF c1 + BF - 1 of D2
       if (a.levels == 2) {
 #pragma unroll
-        for (int c = 0; c < S::kAccCols / 32; ++c) tmem_ld32(tb + (uint32_t)(32 * c), v + 32 * c);
-        if constexpr (S::kAccCols % 32 != 0) tmem_ld16(tb + (uint32_t)(S::kAccCols - 16), v + S::kAccCols - 16);
-      } else {
-        tmem_ld16(tb + S::N2, v + S::N2);
+        for (int k = 0; k < BF; ++k) g[k] = 0u;
+#pragma unroll
+        for (int c0 = 0; c0 < BF * BF; c0 += 64) {
+          uint32_t v[64];
+          tmem_ld32(tb + (uint32_t)c0, v);
+          if (c0 + 32 < BF * BF) tmem_ld32(tb + (uint32_t)(c0 + 32), v + 32);
+          tmem_wait(v);
+#pragma unroll
+          for (int k = 0; k < 64; ++k)
+            if (c0 + k < BF * BF) g[(c0 + k) % BF] = c1 == (c0 + k) / BF ? v[k] : g[(c0 + k) % BF];
+        }
       }
-      tmem_wait(v);
-      const uint32_t* d1 = v + S::N2;
-      const uint32_t* d2 = v;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.accEmpty[acc]);
-      if (++acc == S::kAcc) {
-        acc = 0;
-        accPhase ^= 1;
-      }
       if (key < 0) continue;
-      const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + w.item.x;
-      const long long g1 = (r + 1) * BF;
-      const int c1 = vtc_argmax<BF>(d1);
-      long long node = g1 + c1;
-      if (a.levels == 2) {
-        // the chosen child's BF children: columns BF c1 .. BF c1 + BF - 1 of D2
-        uint32_t g[BF];
-#pragma unroll
-        for (int k = 0; k < BF; ++k) g[k] = d2[k];
-#pragma unroll
-        for (int c = 1; c < BF; ++c) {
-          const bool p = c1 == c;
-#pragma unroll
-          for (int k = 0; k < BF; ++k) g[k] = p ? d2[BF * c + k] : g[k];
-        }
-        node = (g1 + 1) * BF + (long long)BF * c1 + vtc_argmax<BF>(g);
-      }
+      const long long node = a.levels == 2 ? (g1 + 1) * BF + (long long)BF * c1 + vtc_argmax<BF>(g) : g1 + c1;
       if (a.final) {
         a.out[key] = (int32_t)(a.idMode == V3DM_LEAF_LOCAL ? node - a.leafBase : node);
       } else {
@@ -502,6 +369,8 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
         const unsigned peers = __match_any_sync(__activemask(), bkt);
         if (lane == __ffs(peers) - 1) atomicAdd(localHist ? &s.hist[bkt] : &a.hist[bkt], __popc(peers));
       }
+      }
+      i0 += (uint32_t)tiles;
     }
   }
 
