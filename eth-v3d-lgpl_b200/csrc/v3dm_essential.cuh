@@ -468,6 +468,18 @@ V3DM_HD double sampson_truncated(const double* F, double p0, double p1, double q
   return thr2 < d ? thr2 : d;  // std::min(d, thr2)
 }
 
+// The numerator and denominator of the Sampson error, in the same order.
+V3DM_HD void sampson_parts(const double* F, double p0, double p1, double q0, double q1, double& num, double& denom) {
+  const double Fp0 = dadd(dadd(F[2], dmul(F[0], p0)), dmul(F[1], p1));
+  const double Fp1 = dadd(dadd(F[5], dmul(F[3], p0)), dmul(F[4], p1));
+  const double Fp2 = dadd(dadd(F[8], dmul(F[6], p0)), dmul(F[7], p1));
+  const double Ftq0 = dadd(dadd(F[6], dmul(F[0], q0)), dmul(F[3], q1));
+  const double Ftq1 = dadd(dadd(F[7], dmul(F[1], q0)), dmul(F[4], q1));
+  const double tmp = dadd(dadd(dmul(q0, Fp0), dmul(q1, Fp1)), Fp2);
+  num = dmul(tmp, tmp);
+  denom = dadd(dadd(dadd(dmul(Fp0, Fp0), dmul(Fp1, Fp1)), dmul(Ftq0, Ftq0)), dmul(Ftq1, Ftq1));
+}
+
 // C = A B for row-major 3 x 3 matrices, each entry summed over k = 0, 1, 2 in order.
 V3DM_HD void mat3_mul(const double* A, const double* B, double* C) {
   for (int i = 0; i < 3; ++i)
@@ -686,6 +698,8 @@ V3DM_HD void sincos_dd(double x, double* sn, double* cs) {
       c = dd_add(c, tc);
       s = dd_add(s, ts);
     }
+    // what follows is below 2^-115 of either sum: it changes neither's rounding to double
+    if (fabs(ts.hi) <= 2.4e-35 * fabs(s.hi) && fabs(tc.hi) <= 2.4e-35 * fabs(c.hi)) break;
   }
   *sn = s.hi + s.lo;
   *cs = c.hi + c.lo;
@@ -838,28 +852,37 @@ V3DM_HD void pose_normal_equations(const PoseCorr* c, int n, const double* R, co
 }
 
 // x = N^-1 b for a symmetric positive definite 6 x 6 N (Cholesky); false if not positive definite.
+// (Unrolled: one device thread solves while its block waits, and arrays indexed at run time would sit
+// in local memory: 12,000 cycles a solve.)
 V3DM_HD bool cholesky_solve6(const double* N, const double* b, double* x) {
   double L[36];
-  for (int k = 0; k < 36; ++k) L[k] = 0.0;
+#pragma unroll
   for (int j = 0; j < 6; ++j) {
     double d = N[6 * j + j];
+#pragma unroll
     for (int k = 0; k < j; ++k) d -= L[6 * j + k] * L[6 * j + k];
     if (!(d > 0.0)) return false;
     L[6 * j + j] = sqrt(d);
+#pragma unroll
     for (int i = j + 1; i < 6; ++i) {
       double v = N[6 * i + j];
+#pragma unroll
       for (int k = 0; k < j; ++k) v -= L[6 * i + k] * L[6 * j + k];
       L[6 * i + j] = v / L[6 * j + j];
     }
   }
   double y[6];
+#pragma unroll
   for (int i = 0; i < 6; ++i) {
     double v = b[i];
+#pragma unroll
     for (int k = 0; k < i; ++k) v -= L[6 * i + k] * y[k];
     y[i] = v / L[6 * i + i];
   }
+#pragma unroll
   for (int i = 5; i >= 0; --i) {
     double v = y[i];
+#pragma unroll
     for (int k = i + 1; k < 6; ++k) v -= L[6 * k + i] * x[k];
     x[i] = v / L[6 * i + i];
   }

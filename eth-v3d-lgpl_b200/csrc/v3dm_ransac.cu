@@ -12,14 +12,24 @@
 // Here all pairs and all samples run at once:
 //   k_rs_normalize  correspondences normalised by K^-1 (the solver's input);
 //   k_rs_draw       (optional) 5 distinct correspondences per sample from a counter-based hash;
-// then rounds of 128 samples per pair (pairs whose loop has ended are skipped):
-//   k_rs_hyp        one thread per sample: five-point solver, F, pose consistency -> slots;
-//   k_rs_compact    one CTA per pair: the round's candidates in loop order, densely;
-//   k_rs_score      a CTA per (pair, 128 candidates): the pair's correspondences staged in
-//                   shared memory, one candidate per thread, cost and inlier count in double;
-//   k_rs_select     one warp per pair: the round's candidates staged in shared memory, then the
-//                   loop's sequential rule (strictly lower cost, pose consistent, adaptive sample
-//                   budget) over them in loop order, its state carried to the next round;
+// then rounds (pairs whose loop has ended take no work):
+//   k_rs_plan       the round's samples: 128 per pair at first, then what the budgets still allow, up to
+//                   four times the round before and an equal share of the slots (a kernel of a round lasts
+//                   as long as one thread's work however few samples it has, so few long rounds are
+//                   better than many short ones; what a pair's loop does not draw of them is not used.
+//                   1001 draws on 256 pairs: three rounds, 2.7 ms of k_rs_hyp; eight of 128 took 5.3);
+//   k_rs_hyp        one thread per sample: five-point solver, F -> slots;
+//   k_rs_compact    one CTA per pair: the round's candidates in loop order, densely, cut into items of
+//                   128 for the two kernels after it;
+//   k_rs_pose       one thread per candidate: pose consistency on its sample;
+//   k_rs_score      a CTA per item: the pair's correspondences staged in shared memory, one candidate per
+//                   thread, cost and inlier count in double; a candidate whose partial sum (of terms that
+//                   are not negative) has reached the pair's best cost cannot be accepted and stops.
+//                   FP64-bound: the pipe is 74% busy, 3.5 ms on those pairs (6.3 ms with one term at a
+//                   time and every sum finished);
+//   k_rs_select     one warp per pair: the loop's sequential rule (strictly lower cost, pose consistent,
+//                   adaptive sample budget) over the round's candidates in loop order, its state carried
+//                   to the next round;
 // and at the end
 //   k_rs_finish     pose, error and inlier flags of the chosen candidate.
 // With the loop's iterative refinement (mode.iterativeRefinement, v3dm_ransac_set_refinement),
@@ -45,7 +55,9 @@ using namespace v3dm;
 namespace {
 
 constexpr int kRsScoreThreads = 128;
+constexpr int kRsMinSlots = 131072;  // sample slots of a round at least (190 MB)
 constexpr int kRsStage = 1024;       // correspondences staged at a time in k_rs_score
+constexpr int kRsUnroll = 4;         // correspondences a thread of k_rs_score scores at a time
 
 struct RsDeviceGuard {
   int prev = -1;
@@ -136,22 +148,64 @@ __global__ void k_rs_init(const int32_t* __restrict__ offsets, int nPairs, int n
   st[p] = s;
 }
 
-// One thread per (pair, sample of this round): candidates into the round's slots (pair, j, r),
-// their count and pose flag.  Pairs whose loop has ended are skipped.
-__global__ void __launch_bounds__(64)
-k_rs_hyp(const int32_t* __restrict__ offsets, int nPairs, int nDraw, int s0, int len,
-         const int32_t* __restrict__ samples, const double4* __restrict__ norm, const double* __restrict__ invK,
-         const RsState* __restrict__ st, double* __restrict__ slots, uint8_t* __restrict__ slotOk,
-         int8_t* __restrict__ counts) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // p * kRsRound + j
-  const int p = (int)(t / kRsRound), j = (int)(t % kRsRound);
-  if (p >= nPairs) return;
-  if (j >= len || st[p].done) {
-    counts[t] = 0;
-    return;
+// The round's plan: pair p takes min(what its budget and its draws leave, limit, an equal share of the
+// cap sample slots) samples.  One block.
+__global__ void __launch_bounds__(1024)
+k_rs_plan(int nPairs, int nDraw, int cap, int limit, const RsState* __restrict__ st, int* __restrict__ start,
+          int* __restrict__ len, int* __restrict__ nItems) {
+  __shared__ int sh[32];
+  __shared__ int sAlive, sBase;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid == 0) sAlive = sBase = *nItems = 0;
+  __syncthreads();
+  int alive = 0;
+  for (int p = tid; p < nPairs; p += 1024) alive += !st[p].done;
+  alive = __reduce_add_sync(0xffffffffu, alive);
+  if (lane == 0 && alive) atomicAdd(&sAlive, alive);
+  __syncthreads();
+  const int share = min(limit, max(kRsRound, cap / max(1, sAlive)));  // cap >= kRsRound * nPairs
+  for (int p0 = 0; p0 < nPairs; p0 += 1024) {
+    const int p = p0 + tid;
+    int want = 0;
+    if (p < nPairs) {
+      const RsState s = st[p];
+      if (!s.done) want = rs_used(s, min(share, nDraw - s.drawn));
+    }
+    int inc = want;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    if (lane == 31) sh[wid] = inc;
+    __syncthreads();
+    int before = sBase, total = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < wid) before += sh[w];
+      total += sh[w];
+    }
+    if (p < nPairs) {
+      start[p] = before + inc - want;
+      len[p] = want;
+    }
+    __syncthreads();
+    if (tid == 0) sBase += total;
+    __syncthreads();
   }
+  if (tid == 0) start[nPairs] = sBase;
+}
+
+// One thread per sample of the round: its candidates into its slots, their count.
+__global__ void __launch_bounds__(64)
+k_rs_hyp(const int32_t* __restrict__ offsets, int nPairs, int nDraw, RsRoundPlan plan,
+         const int32_t* __restrict__ samples, const double4* __restrict__ norm, const double* __restrict__ invK,
+         const RsState* __restrict__ st, double* __restrict__ slots, int8_t* __restrict__ counts) {
+  const int total = plan.start[nPairs];
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  const int p = rs_pair_of(plan.start, nPairs, (int)t), j = (int)t - plan.start[p];
   const int b = offsets[p], n = offsets[p + 1] - b;
-  const int32_t* s = samples + ((long long)p * nDraw + s0 + j) * 5;
+  const int32_t* s = samples + ((long long)p * nDraw + st[p].drawn + j) * 5;
   bool valid = n >= 5;
   for (int k = 0; k < 5 && valid; ++k) valid = s[k] >= 0 && s[k] < n;
   if (!valid) {
@@ -175,14 +229,13 @@ k_rs_hyp(const int32_t* __restrict__ offsets, int nPairs, int nDraw, int s0, int
     for (int c = 0; c < 3; ++c) iK2t[3 * a + c] = iK2[3 * c + a];
   for (int r = 0; r < ns; ++r) {
     double* slot = slots + (t * kRsMaxSol + r) * kRsSlotDoubles;
-    double tmp[9], F[9], R[9], T[3];
+    double tmp[9], F[9];
     ess::mat3_mul(iK2t, Es[r], tmp);  // F = K2^-T E K1^-1
     ess::mat3_mul(tmp, iK1, F);
     for (int k = 0; k < 9; ++k) {
       slot[k] = Es[r][k];
       slot[9 + k] = F[k];
     }
-    slotOk[t * kRsMaxSol + r] = ess::essential_pose(Es[r], 5, x1, y1, x2, y2, R, T) ? 1 : 0;
   }
   counts[t] = (int8_t)ns;
 }
@@ -200,138 +253,186 @@ __global__ void k_rs_five_point(int n, const double* __restrict__ pts, double* _
   counts[t] = ns;
 }
 
-// One CTA per pair: the round's candidate slots (j * 10 + r) in loop order; work counters.
-__global__ void k_rs_compact(const int32_t* __restrict__ offsets, const int8_t* __restrict__ counts,
-                             int32_t* __restrict__ list, int32_t* __restrict__ listN,
-                             unsigned long long* __restrict__ work) {
-  static_assert(kRsRound <= 1024, "one thread per sample of the round");
+// One CTA per pair: the round's candidate slots (j * 10 + r) in loop order, and the items of
+// kRsScoreThreads candidates each; work counters.
+__global__ void __launch_bounds__(kRsRound)
+k_rs_compact(const int32_t* __restrict__ offsets, RsRoundPlan plan, const int8_t* __restrict__ counts,
+             int32_t* __restrict__ list, int32_t* __restrict__ listN, int2* __restrict__ items,
+             int* __restrict__ nItems, unsigned long long* __restrict__ work) {
   const int p = blockIdx.x;
+  const int start = plan.start[p], len = plan.len[p];
   __shared__ int warpSum[32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int j = threadIdx.x;
-  const int c = j < kRsRound ? counts[(long long)p * kRsRound + j] : 0;
-  int inc = c;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kRsRound >> 5;
+  int32_t* out = list + (long long)start * kRsMaxSol;
+  int base = 0;
+  for (int w0 = 0; w0 < len; w0 += kRsRound) {
+    const int j = w0 + threadIdx.x;
+    const int c = j < len ? counts[start + j] : 0;
+    int inc = c;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    if (lane == 31) warpSum[wid] = inc;
+    __syncthreads();
+    int before = base, total = 0;
+    for (int w = 0; w < nw; ++w) {
+      if (w < wid) before += warpSum[w];
+      total += warpSum[w];
+    }
+    for (int r = 0; r < c; ++r) out[before + inc - c + r] = j * kRsMaxSol + r;
+    base += total;
+    __syncthreads();
   }
-  if (lane == 31) warpSum[wid] = inc;
-  __syncthreads();
-  int before = 0;
-  for (int w = 0; w < wid; ++w) before += warpSum[w];
-  int32_t* out = list + (long long)p * kRsRound * kRsMaxSol;
-  for (int r = 0; r < c; ++r) out[before + inc - c + r] = j * kRsMaxSol + r;
   if (threadIdx.x == 0) {
-    int total = 0;
-    for (int w = 0; w < nw; ++w) total += warpSum[w];
-    listN[p] = total;
-    if (total) {
-      atomicAdd(&work[0], (unsigned long long)total);
-      atomicAdd(&work[1], (unsigned long long)total * (unsigned long long)(offsets[p + 1] - offsets[p]));
+    listN[p] = base;
+    if (base) {
+      const int n = (base + kRsScoreThreads - 1) / kRsScoreThreads, at = atomicAdd(nItems, n);
+      for (int k = 0; k < n; ++k) items[at + k] = make_int2(p, k * kRsScoreThreads);
+      atomicAdd(&work[0], (unsigned long long)base);
+      atomicAdd(&work[1], (unsigned long long)base * (unsigned long long)(offsets[p + 1] - offsets[p]));
     }
   }
 }
 
-// CTA (pair, chunk): cost = sum_i min(d_i, thr2) and the count of d_i < thr2 for 128 candidates.
+// Pose consistency of every candidate on its sample (the pose itself is recovered again for the few
+// candidates that are chosen).
 __global__ void __launch_bounds__(kRsScoreThreads)
-k_rs_score(const int32_t* __restrict__ offsets, const float4* __restrict__ corrs, const int32_t* __restrict__ list,
-           const int32_t* __restrict__ listN, const double* __restrict__ slots, double thr2,
-           double* __restrict__ cost, int32_t* __restrict__ inl) {
-  const int p = blockIdx.x;
-  const int h = blockIdx.y * kRsScoreThreads + threadIdx.x;
-  const int H = listN[p];
-  if (blockIdx.y * kRsScoreThreads >= H) return;  // uniform over the CTA
+k_rs_pose(const int32_t* __restrict__ offsets, int nDraw, RsRoundPlan plan, const RsState* __restrict__ st,
+          const int32_t* __restrict__ samples, const double4* __restrict__ norm, const int32_t* __restrict__ list,
+          const int32_t* __restrict__ listN, const int2* __restrict__ items, const int* __restrict__ nItems,
+          const double* __restrict__ slots, uint8_t* __restrict__ slotOk) {
+  const int n = *nItems;
+  for (int it = blockIdx.x; it < n; it += gridDim.x) {
+    const int p = items[it].x, h = items[it].y + (int)threadIdx.x;
+    if (h >= listN[p]) continue;
+    const long long base = (long long)plan.start[p] * kRsMaxSol;
+    const int idx = list[base + h];
+    const int32_t* s = samples + ((long long)p * nDraw + st[p].drawn + idx / kRsMaxSol) * 5;
+    double E[9], x1[5], y1[5], x2[5], y2[5], R[9], T[3];
+    for (int k = 0; k < 9; ++k) E[k] = slots[(base + idx) * kRsSlotDoubles + k];
+    for (int k = 0; k < 5; ++k) {
+      const double4 o = norm[offsets[p] + s[k]];
+      x1[k] = o.x;
+      y1[k] = o.y;
+      x2[k] = o.z;
+      y2[k] = o.w;
+    }
+    slotOk[base + idx] = ess::essential_pose(E, 5, x1, y1, x2, y2, R, T) ? 1 : 0;
+  }
+}
+
+// CTA per item: cost = sum_i min(d_i, thr2) and the count of d_i < thr2 for its candidates, or, for a
+// candidate whose partial sum reaches the pair's best cost, that partial sum.
+__global__ void __launch_bounds__(kRsScoreThreads)
+k_rs_score(const int32_t* __restrict__ offsets, const float4* __restrict__ corrs, RsRoundPlan plan,
+           const RsState* __restrict__ states, const int32_t* __restrict__ list, const int32_t* __restrict__ listN,
+           const int2* __restrict__ items, const int* __restrict__ nItems, const double* __restrict__ slots,
+           double thr2, double* __restrict__ cost, int32_t* __restrict__ inl) {
   __shared__ double4 st[kRsStage];  // the positions converted once per CTA
+  const int total = *nItems;
+  for (int it = blockIdx.x; it < total; it += gridDim.x) {
+  const int p = items[it].x;
+  const int h = items[it].y + (int)threadIdx.x;
   const int b = offsets[p], n = offsets[p + 1] - b;
-  const bool mine = h < H;
+  const bool mine = h < listN[p];
+  const double bound = states[p].minError;
   long long slot = 0;
   double F[9];
   if (mine) {
-    slot = (long long)p * kRsRound * kRsMaxSol + list[(long long)p * kRsRound * kRsMaxSol + h];
+    slot = (long long)plan.start[p] * kRsMaxSol + list[(long long)plan.start[p] * kRsMaxSol + h];
     for (int k = 0; k < 9; ++k) F[k] = slots[slot * kRsSlotDoubles + 9 + k];
   }
   double sum = 0.0;
   int cnt = 0;
+  bool open = mine;  // the candidate can still be accepted
   for (int c0 = 0; c0 < n; c0 += kRsStage) {
     const int m = min(kRsStage, n - c0);
-    __syncthreads();
+    if (!__syncthreads_or(open)) break;
     for (int k = threadIdx.x; k < m; k += blockDim.x) {
       const float4 c = corrs[b + c0 + k];
       st[k] = make_double4(c.x, c.y, c.z, c.w);
     }
     __syncthreads();
-    if (mine)
-      for (int k = 0; k < m; ++k) {
+    if (open) {
+      // kRsUnroll terms at a time: their operations are independent and hide each other's latency.  The
+      // division is unconditional: among a warp's 32 candidates one nearly always needs it, and a branch
+      // around it would order the terms one after the other (6.3 ms of scoring in a 256-pair call).
+      int k = 0;
+      for (; k + kRsUnroll <= m; k += kRsUnroll) {
+        double num[kRsUnroll], den[kRsUnroll], d[kRsUnroll];
+#pragma unroll
+        for (int u = 0; u < kRsUnroll; ++u) {
+          const double4 c = st[k + u];
+          ess::sampson_parts(F, c.x, c.y, c.z, c.w, num[u], den[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kRsUnroll; ++u) d[u] = ess::ddiv(num[u], den[u]);
+#pragma unroll
+        for (int u = 0; u < kRsUnroll; ++u) {
+          cnt += d[u] < thr2;
+          sum = ess::dadd(sum, thr2 < d[u] ? thr2 : d[u]);  // std::min(d, thr2)
+        }
+        if ((k & 31) == 0 && !(sum < bound)) {  // the terms to come only add to it
+          open = false;
+          break;
+        }
+      }
+      for (; open && k < m; ++k) {
         const double4 c = st[k];
         bool in;
         sum = ess::dadd(sum, ess::sampson_truncated(F, c.x, c.y, c.z, c.w, thr2, in));
         cnt += in;
       }
+    }
   }
   if (mine) {
     cost[slot] = sum;
     inl[slot] = cnt;
   }
+  }
 }
 
-// One warp per pair: the round's costs, pose flags and inlier counts staged in shared memory by
-// the warp (coalesced), then lane 0 walks the loop over the round's samples in order (the rule of
-// reconstruction_common.cpp:177-335 without refinement); the last accepted candidate's E and F are
-// kept (the warp copies them).  With refinement the selection is k_rs_select_refine
+// One warp per pair: the loop over the round's samples in order (the rule of
+// reconstruction_common.cpp:177-335 without refinement) on the costs staged in shared memory; the
+// last accepted candidate's E and F are kept.  With refinement the selection is k_rs_select_refine
 // (v3dm_ransac_refine.cu).
 __global__ void __launch_bounds__(32)
-k_rs_select(const int32_t* __restrict__ offsets, int nPairs, int nDraw, int s0, int len,
-            const int8_t* __restrict__ counts, const uint8_t* __restrict__ slotOk, const double* __restrict__ cost,
-            const int32_t* __restrict__ inl, const double* __restrict__ slots, RsState* __restrict__ st,
-            double* __restrict__ bestEF) {
+k_rs_select(const int32_t* __restrict__ offsets, int nDraw, RsRoundPlan plan, const int8_t* __restrict__ counts,
+            const uint8_t* __restrict__ slotOk, const double* __restrict__ cost, const int32_t* __restrict__ inl,
+            const double* __restrict__ slots, RsState* __restrict__ st, double* __restrict__ bestEF) {
   const int p = blockIdx.x;
   const int lane = threadIdx.x;
   __shared__ double sCost[kRsRound * kRsMaxSol];
-  __shared__ int32_t sInl[kRsRound * kRsMaxSol];
-  __shared__ uint8_t sOk[kRsRound * kRsMaxSol];
-  __shared__ int8_t sCnt[kRsRound];
-  __shared__ int sAccepted;
+  const int len = plan.len[p];
+  if (len == 0) return;  // uniform over the warp
   RsState s = st[p];
-  if (s.done) return;  // uniform over the warp
-  const long long base = (long long)p * kRsRound;
-  for (int j = lane; j < len; j += 32) sCnt[j] = counts[base + j];
-  __syncwarp();
-  for (int idx = lane; idx < len * kRsMaxSol; idx += 32) {
-    const int j = idx / kRsMaxSol, r = idx - j * kRsMaxSol;
-    if (r < sCnt[j]) {
-      sCost[idx] = cost[base * kRsMaxSol + idx];
-      sInl[idx] = inl[base * kRsMaxSol + idx];
-      sOk[idx] = slotOk[base * kRsMaxSol + idx];
+  const int n = offsets[p + 1] - offsets[p];
+  const int s0 = s.drawn;
+  const long long base = (long long)plan.start[p] * kRsMaxSol;
+  int accepted = -1, used = rs_used(s, len);
+  for (int w0 = 0; w0 < used; w0 += kRsRound) {
+    __syncwarp();
+    rs_stage_costs(sCost, (long long)plan.start[p] + w0, min(kRsRound, used - w0), counts, slotOk, cost);
+    __syncwarp();
+    auto limit = [&]() { return min(kRsRound, used - w0) * kRsMaxSol; };
+    for (int idx = rs_next_below(sCost, 0, limit(), s.minError); idx < limit();
+         idx = rs_next_below(sCost, idx + 1, limit(), s.minError)) {
+      const int at = w0 * kRsMaxSol + idx, j = at / kRsMaxSol;
+      s.minError = sCost[idx];
+      s.chosen = s0 + j;
+      accepted = at;
+      const float frac = (float)(inl[base + at] - 5) / (float)(n - 5);
+      s.budget = min(s.budget, rs_budget(1.0 - (double)frac));
+      used = max(j + 1, rs_used(s, len));
     }
   }
-  __syncwarp();
-  if (lane == 0) {
-    const int n = offsets[p + 1] - offsets[p];
-    int accepted = -1;
-    for (int j = 0; j < len; ++j) {
-      if (s.drawn > s.budget) break;
-      ++s.drawn;
-      const int ns = sCnt[j];
-      for (int r = 0; r < ns; ++r) {
-        const int idx = j * kRsMaxSol + r;
-        if (!(sCost[idx] < s.minError)) continue;
-        if (!sOk[idx]) continue;
-        s.minError = sCost[idx];
-        s.chosen = s0 + j;
-        accepted = idx;
-        const float frac = (float)(sInl[idx] - 5) / (float)(n - 5);
-        s.budget = min(s.budget, rs_budget(1.0 - (double)frac));
-      }
-    }
-    if (s.drawn > s.budget || s0 + len >= nDraw) s.done = 1;  // the next sample would end the loop
-    st[p] = s;
-    sAccepted = accepted;
-  }
-  __syncwarp();
-  const int accepted = sAccepted;
+  s.drawn += used;
+  if (s.drawn > s.budget || s.drawn >= nDraw) s.done = 1;  // the next sample would end the loop
+  if (lane == 0) st[p] = s;
   if (accepted >= 0 && lane < kRsSlotDoubles)
-    bestEF[(size_t)p * kRsSlotDoubles + lane] = slots[(base * kRsMaxSol + accepted) * kRsSlotDoubles + lane];
+    bestEF[(size_t)p * kRsSlotDoubles + lane] = slots[(base + accepted) * kRsSlotDoubles + lane];
 }
 
 // One thread per pair: E, F, R, T and error of the choice.
@@ -466,7 +567,7 @@ struct v3dm_ransac {
   // the refinement's task lists, results and inlier lists (RsRefineWork)
   int32_t* dTaskIdx = nullptr;
   size_t taskIdxCap = 0;
-  int32_t* dTaskN = nullptr;   // nPairs counts, then the number of tasks
+  int32_t* dTaskN = nullptr;   // nPairs counts, then RsRefineWork::nTasks
   size_t taskNCap = 0;
   int2* dTasks = nullptr;
   size_t tasksCap = 0;
@@ -474,6 +575,10 @@ struct v3dm_ransac {
   size_t refinedCap = 0;
   int32_t* dLists = nullptr;
   size_t listsCap = 0;
+  int* dPlan = nullptr;        // the round's plan: start (nPairs + 1), item count, len (nPairs)
+  size_t planCap = 0;
+  int2* dItems = nullptr;      // the round's items (pair, first candidate)
+  size_t itemsCap = 0;
   int numSMs = 148;
   bool refine = false;         // RobustOrientationMode::iterativeRefinement
   double thr = 0.0;            // inlier threshold of the call (pixels)
@@ -508,7 +613,14 @@ cudaError_t rs_mark(v3dm_ransac* r, int k) {
 // Everything from normalisation to inlier flags, on r's stream; inputs already on the device.
 int rs_enqueue(v3dm_ransac* r, int nPairs, int nCorrs, int nDraw, int nSamples, bool draw, uint64_t seed,
                double thr2, const float4* dCorrs, int32_t* dSamples, double* dOut, int32_t* dNIn, uint8_t* dFlags) {
-  const size_t nR = (size_t)nPairs * kRsRound;  // sample slots of one round
+  // sample slots of one round: 128 per pair, and enough for the later rounds of few pairs
+  const size_t nR = std::max((size_t)nPairs * kRsRound, (size_t)kRsMinSlots);
+  const size_t maxItems = nR * kRsMaxSol / kRsScoreThreads + (size_t)nPairs;
+  V3DM_RS_TRY(rs_grow(r->dPlan, r->planCap, 2 * (size_t)nPairs + 2));
+  V3DM_RS_TRY(rs_grow(r->dItems, r->itemsCap, maxItems));
+  int* start = r->dPlan;
+  int* nItems = start + nPairs + 1;
+  const RsRoundPlan plan{start, nItems + 1};
   V3DM_RS_TRY(rs_grow(r->dNorm, r->normCap, (size_t)nCorrs));
   V3DM_RS_TRY(rs_grow(r->dSlots, r->slotCap, nR * kRsMaxSol * kRsSlotDoubles));
   V3DM_RS_TRY(rs_grow(r->dSlotOk, r->okCap, nR * kRsMaxSol));
@@ -529,7 +641,7 @@ int rs_enqueue(v3dm_ransac* r, int nPairs, int nCorrs, int nDraw, int nSamples, 
   RsRefineWork rw{};
   if (r->refine) {
     V3DM_RS_TRY(rs_grow(r->dTaskIdx, r->taskIdxCap, (size_t)nPairs * kRsTasks));
-    V3DM_RS_TRY(rs_grow(r->dTaskN, r->taskNCap, (size_t)nPairs + 1));
+    V3DM_RS_TRY(rs_grow(r->dTaskN, r->taskNCap, (size_t)nPairs + 3));
     V3DM_RS_TRY(rs_grow(r->dTasks, r->tasksCap, (size_t)nPairs * kRsTasks));
     rw.ctas = 2 * r->numSMs;  // two CTAs of k_rs_refine fit an SM
     V3DM_RS_TRY(rs_grow(r->dRefined, r->refinedCap, (size_t)nPairs * kRsTasks + rw.ctas));
@@ -557,28 +669,35 @@ int rs_enqueue(v3dm_ransac* r, int nPairs, int nCorrs, int nDraw, int nSamples, 
   }
   k_rs_init<<<(nPairs + 127) / 128, 128, 0, r->stream>>>(r->dOffsets, nPairs, nSamples, state);
   ++launches;
-  // rounds of kRsRound samples per pair; pairs whose loop has ended are skipped
-  for (int s0 = 0; s0 < nDraw; s0 += kRsRound) {
-    const int len = std::min(kRsRound, nDraw - s0);
+  // rounds until every pair's draws are covered, however few slots a pair gets (128 at least)
+  int covered = 0, limit = kRsRound;
+  const int share = (int)std::min<size_t>(nR / (size_t)nPairs, 0x7fffffff);
+  while (covered < nDraw) {
     V3DM_RS_TRY(rs_mark(r, 0));
-    k_rs_hyp<<<(unsigned)((nR + 63) / 64), 64, 0, r->stream>>>(r->dOffsets, nPairs, nDraw, s0, len, dSamples,
-                                                                r->dNorm, r->dInvK, state, r->dSlots, r->dSlotOk,
-                                                                r->dCounts);
+    k_rs_plan<<<1, 1024, 0, r->stream>>>(nPairs, nDraw, (int)std::min<size_t>(nR, 0x7fffffff), limit, state, start,
+                                         nItems + 1, nItems);
+    k_rs_hyp<<<(unsigned)((nR + 63) / 64), 64, 0, r->stream>>>(r->dOffsets, nPairs, nDraw, plan, dSamples, r->dNorm,
+                                                                r->dInvK, state, r->dSlots, r->dCounts);
     V3DM_RS_TRY(rs_mark(r, 0));
-    k_rs_compact<<<nPairs, kRsRound, 0, r->stream>>>(r->dOffsets, r->dCounts, r->dList, r->dListN, r->dWork);
-    const unsigned chunks = (unsigned)((kRsRound * kRsMaxSol + kRsScoreThreads - 1) / kRsScoreThreads);
+    k_rs_compact<<<nPairs, kRsRound, 0, r->stream>>>(r->dOffsets, plan, r->dCounts, r->dList, r->dListN, r->dItems,
+                                                     nItems, r->dWork);
+    const unsigned grid = (unsigned)std::min<size_t>(maxItems, (size_t)r->numSMs * 16);
+    k_rs_pose<<<grid, kRsScoreThreads, 0, r->stream>>>(r->dOffsets, nDraw, plan, state, dSamples, r->dNorm, r->dList,
+                                                       r->dListN, r->dItems, nItems, r->dSlots, r->dSlotOk);
     V3DM_RS_TRY(rs_mark(r, 1));
-    k_rs_score<<<dim3(nPairs, chunks), kRsScoreThreads, 0, r->stream>>>(r->dOffsets, dCorrs, r->dList, r->dListN,
-                                                                       r->dSlots, thr2, r->dCost, r->dInl);
+    k_rs_score<<<grid, kRsScoreThreads, 0, r->stream>>>(r->dOffsets, dCorrs, plan, state, r->dList, r->dListN,
+                                                        r->dItems, nItems, r->dSlots, thr2, r->dCost, r->dInl);
     V3DM_RS_TRY(rs_mark(r, 1));
     if (r->refine)
-      V3DM_RS_TRY(launch_rs_select_refine(r->dOffsets, nPairs, nDraw, s0, len, r->dCounts, r->dSlotOk, r->dCost,
+      V3DM_RS_TRY(launch_rs_select_refine(r->dOffsets, nPairs, nDraw, plan, r->dCounts, r->dSlotOk, r->dCost,
                                           r->dSlots, state, r->dBestEF, dCorrs, r->dNorm, dSamples, r->dInvK, r->thr,
                                           thr2, r->dBestRT, rw, r->stream));
     else
-      k_rs_select<<<nPairs, 32, 0, r->stream>>>(r->dOffsets, nPairs, nDraw, s0, len, r->dCounts, r->dSlotOk,
-                                                 r->dCost, r->dInl, r->dSlots, state, r->dBestEF);
-    launches += r->refine ? 6 : 4;
+      k_rs_select<<<nPairs, 32, 0, r->stream>>>(r->dOffsets, nDraw, plan, r->dCounts, r->dSlotOk, r->dCost, r->dInl,
+                                                 r->dSlots, state, r->dBestEF);
+    launches += r->refine ? 8 : 6;
+    covered += std::min(limit, std::max(kRsRound, share));
+    limit = std::min(4 * limit, 1 << 20);
   }
   k_rs_finish<<<(nPairs + 127) / 128, 128, 0, r->stream>>>(r->dOffsets, nPairs, nDraw, dSamples, r->dNorm, state,
                                                            r->dBestEF, dOut, r->refine ? 1 : 0, r->dBestRT);
@@ -627,7 +746,8 @@ int v3dm_ransac_destroy(v3dm_ransac* r) {
   cudaStreamSynchronize(r->stream);
   void* bufs[] = {r->dOffsets, r->dCorrs, r->dNorm, r->dInvK, r->dSamples, r->dSlots, r->dSlotOk, r->dCounts,
                   r->dList,    r->dListN, r->dCost, r->dInl,  r->dState,   r->dBestEF, r->dWork,  r->dOut,
-                  r->dFlags,   r->dNIn,   r->dBestRT, r->dTaskIdx, r->dTaskN, r->dTasks, r->dRefined, r->dLists};
+                  r->dFlags,   r->dNIn,   r->dBestRT, r->dTaskIdx, r->dTaskN, r->dTasks, r->dRefined, r->dLists,
+                  r->dPlan,    r->dItems};
   for (void* b : bufs)
     if (b) cudaFree(b);
   for (int k = 0; k < 2; ++k)

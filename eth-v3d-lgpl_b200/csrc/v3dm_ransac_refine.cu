@@ -29,9 +29,10 @@
 // run beside it.  A step of the Levenberg-Marquardt loop takes one sweep over the inliers: the
 // sweep that scores the step (weights of the old pose) also forms the normal equations the next
 // step needs if it is accepted (weights of the new pose).
-// On 256 pairs of 500 to 3000 correspondences these kernels take 12.0 ms of a call (k_rs_refine
-// 4.5 ms in the first round, 0.8 to 1.4 ms, a refinement's latency, in each later one); one warp
-// per pair that refined its candidates one after the other, two sweeps per step, took 178 ms.
+// On 256 pairs of 500 to 3000 correspondences these kernels take 5.5 ms of a 12.1 ms call: an inlier
+// costs a sweep 22 cycles, a step 17,000 more in the solve, the update and their barriers.  One warp
+// per pair that refined its candidates one after the other, two sweeps per step, took 178 ms;
+// tasks dealt out in a fixed order 1.5 ms more than taken as CTAs become free.
 #include <cuda_runtime.h>
 
 #include "v3dm_essential.cuh"
@@ -60,6 +61,7 @@ __device__ void rs_fund(const double* invK1, const double* invK2t, const double*
 }
 
 constexpr int kRsRefineThreads = 256;           // warp 0 sums, warps 1..7 produce
+constexpr int kRsRefineCtas = 2;                // per SM
 constexpr int kRsProducers = kRsRefineThreads - 32;
 constexpr int kRsQuant = 29;   // 21 entries of J^T J (upper triangle), 6 of J^T e, |e|^2 under the new and the old weights
 constexpr int kRsEntry = 9;    // doubles per staged inlier: J (6), e (new weights), e (old weights), padding (odd: no bank conflicts)
@@ -183,16 +185,13 @@ __device__ void rs_refine_cta(RsShared& s, const float4* __restrict__ px, const 
   for (int it = 0; it < 50; ++it) {
     if (threadIdx.x == 0) {
       if (fresh) {
-        for (int t = 0; t < 21; ++t) {
-          int i = 0, r = t;
-          while (r >= 6 - i) {
-            r -= 6 - i;
-            ++i;
-          }
-          s.JtJ[6 * i + i + r] = s.sums[t];
-          s.JtJ[6 * (i + r) + i] = s.sums[t];
-        }
-        for (int t = 0; t < 6; ++t) s.Jte[t] = s.sums[21 + t];
+        int t = 0;
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+#pragma unroll
+          for (int j = i; j < 6; ++j, ++t) s.JtJ[6 * i + j] = s.JtJ[6 * j + i] = s.sums[t];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s.Jte[k] = s.sums[21 + k];
         err = s.sums[27];
       }
       bool go = true;
@@ -205,10 +204,15 @@ __device__ void rs_refine_cta(RsShared& s, const float4* __restrict__ px, const 
           for (int k = 0; k < 6; ++k) maxEl = fmax(maxEl, s.JtJ[7 * k]);
           lambda = 1e-3 * maxEl;
         }
-        double N[36];
+        double N[36], g[6];
+#pragma unroll
         for (int k = 0; k < 36; ++k) N[k] = s.JtJ[k];
-        for (int k = 0; k < 6; ++k) N[7 * k] += lambda;
-        go = ess::cholesky_solve6(N, s.Jte, delta);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          N[7 * k] += lambda;
+          g[k] = s.Jte[k];
+        }
+        go = ess::cholesky_solve6(N, g, delta);
       }
       if (go) {
         double dl = 0.0;
@@ -288,11 +292,11 @@ __device__ void rs_cost_in_order(RsShared& s, const float4* __restrict__ px, int
   __syncthreads();
 }
 
-// Candidate idx (sample j, solution r) of pair p: its pose on the sample, the refinement on the
+// Candidate idx (sample j of the round, solution r) of pair p: its pose on the sample, the refinement on the
 // inliers of its F, the refined model and its cost.  o.ok = 0 when the sample's correspondences
 // do not agree on a pose (the loop skips the candidate).  The CTA enters and leaves together.
 __device__ void rs_refine_candidate(RsShared& s, int p, int idx, const int32_t* __restrict__ offsets, int nDraw,
-                                    int s0, const double* __restrict__ slots, const float4* __restrict__ corrs,
+                                    RsRoundPlan plan, const RsState* st, const double* __restrict__ slots, const float4* __restrict__ corrs,
                                     const double4* __restrict__ norm, const int32_t* __restrict__ samples,
                                     const double* __restrict__ invK, double thr, double thr2,
                                     int32_t* __restrict__ list, RsRefined* __restrict__ o) {
@@ -301,9 +305,9 @@ __device__ void rs_refine_candidate(RsShared& s, int p, int idx, const int32_t* 
   for (int k = 0; k < 9; ++k) invK1[k] = invK[(size_t)p * 18 + k];
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) invK2t[3 * i + j] = invK[(size_t)p * 18 + 9 + 3 * j + i];
-  const double* EF = slots + ((long long)p * kRsRound * kRsMaxSol + idx) * kRsSlotDoubles;
+  const double* EF = slots + ((long long)plan.start[p] * kRsMaxSol + idx) * kRsSlotDoubles;
   if (threadIdx.x == 0) {
-    const int32_t* smp = samples + ((long long)p * nDraw + s0 + idx / kRsMaxSol) * 5;
+    const int32_t* smp = samples + ((long long)p * nDraw + st[p].drawn + idx / kRsMaxSol) * 5;
     double x1[5], y1[5], x2[5], y2[5], E[9], R[9], T[3];
     for (int k = 0; k < 5; ++k) {
       const double4 v = norm[b + smp[k]];
@@ -347,81 +351,67 @@ __device__ void rs_refine_candidate(RsShared& s, int p, int idx, const int32_t* 
   __syncthreads();
 }
 
-// The round's candidates of a pair in shared memory, in loop order: the cost, or +inf where the
-// slot is empty or its pose flag is not set.
-__device__ void rs_stage_costs(double* sCost, long long base, int len, const int8_t* __restrict__ counts,
-                               const uint8_t* __restrict__ slotOk, const double* __restrict__ cost) {
-  for (int idx = threadIdx.x; idx < kRsRound * kRsMaxSol; idx += blockDim.x) {
-    const int j = idx / kRsMaxSol, r = idx - j * kRsMaxSol;
-    const bool have = j < len && r < counts[base + j] && slotOk[base * kRsMaxSol + idx];
-    sCost[idx] = have ? cost[base * kRsMaxSol + idx] : INFINITY;
-  }
-}
-
-// The samples the loop draws in a round of len: until one more than the budget has been drawn.
-__device__ __forceinline__ int rs_used(const RsState& s, int len) {
-  return len <= s.budget - s.drawn ? len : s.budget - s.drawn + 1;
-}
-
-// The first candidate in [from, limit) whose cost is below minError, or limit.  Whole warps, the
-// same result on every lane.
-__device__ int rs_next_below(const double* sCost, int from, int limit, double minError) {
-  const int lane = threadIdx.x & 31;
-  for (int i0 = from; i0 < limit; i0 += 32) {
-    const unsigned m = __ballot_sync(0xffffffffu, i0 + lane < limit && sCost[i0 + lane] < minError);
-    if (m) return i0 + __ffs(m) - 1;
-  }
-  return limit;
-}
-
 // One warp per pair: the strict prefix minima of the round's costs below the incoming minimum,
 // in loop order, as tasks.
 __global__ void __launch_bounds__(32)
-k_rs_refine_tasks(int len, const int8_t* __restrict__ counts, const uint8_t* __restrict__ slotOk,
+k_rs_refine_tasks(RsRoundPlan plan, const int8_t* __restrict__ counts, const uint8_t* __restrict__ slotOk,
                   const double* __restrict__ cost, const RsState* __restrict__ st, int32_t* __restrict__ taskIdx,
                   int32_t* __restrict__ taskN, int2* __restrict__ tasks, int* __restrict__ nTasks) {
   const int p = blockIdx.x, lane = threadIdx.x;
   __shared__ double sCost[kRsRound * kRsMaxSol];
   const RsState s = st[p];
+  const int len = plan.len[p], used = len > 0 ? rs_used(s, len) : 0;  // uniform over the warp
+  double minError = s.minError;
   int n = 0;
-  if (!s.done) {  // uniform over the warp
-    rs_stage_costs(sCost, (long long)p * kRsRound, len, counts, slotOk, cost);
+  for (int w0 = 0; w0 < used && n < kRsTasks; w0 += kRsRound) {
+    const int have = min(kRsRound, used - w0), limit = have * kRsMaxSol;
     __syncwarp();
-    const int limit = rs_used(s, len) * kRsMaxSol;
-    double minError = s.minError;
+    rs_stage_costs(sCost, (long long)plan.start[p] + w0, have, counts, slotOk, cost);
+    __syncwarp();
     for (int idx = rs_next_below(sCost, 0, limit, minError); idx < limit && n < kRsTasks;
          idx = rs_next_below(sCost, idx + 1, limit, minError)) {
       minError = sCost[idx];
-      if (lane == 0) {
-        taskIdx[p * kRsTasks + n] = idx;
-        tasks[atomicAdd(nTasks, 1)] = make_int2(p * kRsTasks + n, idx);
-      }
+      if (lane == 0) taskIdx[p * kRsTasks + n] = w0 * kRsMaxSol + idx;
       ++n;
     }
   }
+  __syncwarp();
   if (lane == 0) taskN[p] = n;
+  if (lane < n) {
+    const int2 task = make_int2(p * kRsTasks + lane, taskIdx[p * kRsTasks + lane]);
+    // the last two have the lowest costs, so the most inliers to refine on: they start first
+    if (lane >= n - 2) tasks[atomicAdd(&nTasks[0], 1)] = task;
+    else tasks[gridDim.x * kRsTasks - 1 - atomicAdd(&nTasks[1], 1)] = task;
+  }
 }
 
-// Persistent CTAs over the tasks; listRoom ints of inlier indices per CTA.
-__global__ void __launch_bounds__(kRsRefineThreads, 2)
-k_rs_refine(const int32_t* __restrict__ offsets, int nDraw, int s0, const double* __restrict__ slots,
-            const float4* __restrict__ corrs, const double4* __restrict__ norm, const int32_t* __restrict__ samples,
-            const double* __restrict__ invK, double thr, double thr2, const int2* __restrict__ tasks,
-            const int* __restrict__ nTasks, int32_t* __restrict__ lists, long long listRoom,
-            RsRefined* __restrict__ refined) {
+// Persistent CTAs that take the next task when they are done (a refinement lasts from 4 to 50 steps
+// on 10 to 1000s of inliers); listRoom ints of inlier indices per CTA.
+__global__ void __launch_bounds__(kRsRefineThreads, kRsRefineCtas)
+k_rs_refine(const int32_t* __restrict__ offsets, int nDraw, RsRoundPlan plan, const RsState* __restrict__ st,
+            const double* __restrict__ slots, const float4* __restrict__ corrs, const double4* __restrict__ norm,
+            const int32_t* __restrict__ samples, const double* __restrict__ invK, double thr, double thr2,
+            const int2* __restrict__ tasks, int* __restrict__ nTasks, int cap, int32_t* __restrict__ lists,
+            long long listRoom, RsRefined* __restrict__ refined) {
   __shared__ RsShared s;
-  const int n = *nTasks;
-  for (int t = blockIdx.x; t < n; t += gridDim.x) {
-    const int2 task = tasks[t];
-    rs_refine_candidate(s, task.x / kRsTasks, task.y, offsets, nDraw, s0, slots, corrs, norm, samples, invK, thr, thr2,
-                        lists + (long long)blockIdx.x * listRoom, refined + task.x);
+  __shared__ int sNext;
+  const int first = nTasks[0], n = first + nTasks[1];
+  while (true) {
+    __syncthreads();
+    if (threadIdx.x == 0) sNext = atomicAdd(&nTasks[2], 1);
+    __syncthreads();
+    const int t = sNext;
+    if (t >= n) break;
+    const int2 task = tasks[t < first ? t : cap - 1 - (t - first)];
+    rs_refine_candidate(s, task.x / kRsTasks, task.y, offsets, nDraw, plan, st, slots, corrs, norm, samples, invK, thr,
+                        thr2, lists + (long long)blockIdx.x * listRoom, refined + task.x);
   }
 }
 
 // The loop over the round's candidates in order (reconstruction_common.cpp:177-335), a CTA per pair
 // at a time; every warp walks the same decisions.
-__global__ void __launch_bounds__(kRsRefineThreads, 2)
-k_rs_select_refine(const int32_t* __restrict__ offsets, int nPairs, int nDraw, int s0, int len,
+__global__ void __launch_bounds__(kRsRefineThreads, kRsRefineCtas)
+k_rs_select_refine(const int32_t* __restrict__ offsets, int nPairs, int nDraw, RsRoundPlan plan,
                    const int8_t* __restrict__ counts, const uint8_t* __restrict__ slotOk,
                    const double* __restrict__ cost, const double* __restrict__ slots, RsState* __restrict__ st,
                    double* __restrict__ bestEF, const float4* __restrict__ corrs, const double4* __restrict__ norm,
@@ -431,38 +421,45 @@ k_rs_select_refine(const int32_t* __restrict__ offsets, int nPairs, int nDraw, i
   __shared__ RsShared sh;
   __shared__ double sCost[kRsRound * kRsMaxSol];
   for (int p = blockIdx.x; p < nPairs; p += gridDim.x) {
+    const int len = plan.len[p];
+    if (len == 0) continue;  // uniform
     RsState s = st[p];
-    __syncthreads();  // every thread has read the state; sCost is free
-    if (s.done) continue;  // uniform
-    rs_stage_costs(sCost, (long long)p * kRsRound, len, counts, slotOk, cost);
-    __syncthreads();
     const int n = offsets[p + 1] - offsets[p];
     const int nt = taskN[p];
+    const int s0 = s.drawn;
     int t = 0, used = rs_used(s, len);
-    for (int idx = rs_next_below(sCost, 0, used * kRsMaxSol, s.minError); idx < used * kRsMaxSol;
-         idx = rs_next_below(sCost, idx + 1, used * kRsMaxSol, s.minError)) {
-      while (t < nt && taskIdx[p * kRsTasks + t] < idx) ++t;
-      const bool have = t < nt && taskIdx[p * kRsTasks + t] == idx;
-      RsRefined* o = refined + (have ? p * kRsTasks + t : nPairs * kRsTasks + (int)blockIdx.x);
-      if (!have) {
-        rs_refine_candidate(sh, p, idx, offsets, nDraw, s0, slots, corrs, norm, samples, invK, thr, thr2,
-                            lists + (long long)blockIdx.x * listRoom, o);
+    for (int w0 = 0; w0 < used; w0 += kRsRound) {
+      __syncthreads();  // sCost is free
+      rs_stage_costs(sCost, (long long)plan.start[p] + w0, min(kRsRound, used - w0), counts, slotOk, cost);
+      __syncthreads();
+      auto limit = [&]() { return min(kRsRound, used - w0) * kRsMaxSol; };
+      for (int idx = rs_next_below(sCost, 0, limit(), s.minError); idx < limit();
+           idx = rs_next_below(sCost, idx + 1, limit(), s.minError)) {
+        const int at = w0 * kRsMaxSol + idx;
+        while (t < nt && taskIdx[p * kRsTasks + t] < at) ++t;
+        const bool have = t < nt && taskIdx[p * kRsTasks + t] == at;
+        RsRefined* o = refined + (have ? p * kRsTasks + t : nPairs * kRsTasks + (int)blockIdx.x);
+        if (!have) {
+          rs_refine_candidate(sh, p, at, offsets, nDraw, plan, st, slots, corrs, norm, samples, invK, thr, thr2,
+                              lists + (long long)blockIdx.x * listRoom, o);
+          __syncthreads();
+        }
+        if (!o->ok) continue;
+        s.minError = fmin(sCost[idx], o->cost);
+        const int j = at / kRsMaxSol;
+        s.chosen = s0 + j;
+        const float frac = (float)(o->nIn - 5) / (float)(n - 5);
+        s.budget = min(s.budget, rs_budget(1.0 - (double)frac));
+        used = max(j + 1, rs_used(s, len));
+        if (threadIdx.x < kRsSlotDoubles) bestEF[(size_t)p * kRsSlotDoubles + threadIdx.x] = o->EF[threadIdx.x];
+        if (threadIdx.x < 12) bestRT[(size_t)p * 12 + threadIdx.x] = o->RT[threadIdx.x];
         __syncthreads();
       }
-      if (!o->ok) continue;
-      s.minError = fmin(sCost[idx], o->cost);
-      const int j = idx / kRsMaxSol;
-      s.chosen = s0 + j;
-      const float frac = (float)(o->nIn - 5) / (float)(n - 5);
-      s.budget = min(s.budget, rs_budget(1.0 - (double)frac));
-      used = max(j + 1, rs_used(s, len));
-      if (threadIdx.x < kRsSlotDoubles) bestEF[(size_t)p * kRsSlotDoubles + threadIdx.x] = o->EF[threadIdx.x];
-      if (threadIdx.x < 12) bestRT[(size_t)p * 12 + threadIdx.x] = o->RT[threadIdx.x];
-      __syncthreads();
     }
+    __syncthreads();  // every thread is done with the state
     if (threadIdx.x == 0) {
       s.drawn += used;
-      if (s.drawn > s.budget || s0 + len >= nDraw) s.done = 1;  // the next sample would end the loop
+      if (s.drawn > s.budget || s.drawn >= nDraw) s.done = 1;  // the next sample would end the loop
       st[p] = s;
     }
   }
@@ -470,19 +467,20 @@ k_rs_select_refine(const int32_t* __restrict__ offsets, int nPairs, int nDraw, i
 
 }  // namespace
 
-cudaError_t launch_rs_select_refine(const int32_t* offsets, int nPairs, int nDraw, int s0, int len, const int8_t* counts,
+cudaError_t launch_rs_select_refine(const int32_t* offsets, int nPairs, int nDraw, RsRoundPlan plan, const int8_t* counts,
                                     const uint8_t* slotOk, const double* cost, const double* slots, RsState* st,
                                     double* bestEF, const float4* corrs, const double4* norm, const int32_t* samples,
                                     const double* invK, double thr, double thr2, double* bestRT, const RsRefineWork& w,
                                     cudaStream_t stream) {
   if (nPairs <= 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(w.nTasks, 0, sizeof(int), stream);
+  cudaError_t e = cudaMemsetAsync(w.nTasks, 0, 3 * sizeof(int), stream);
   if (e != cudaSuccess) return e;
-  k_rs_refine_tasks<<<nPairs, 32, 0, stream>>>(len, counts, slotOk, cost, st, w.taskIdx, w.taskN, w.tasks, w.nTasks);
-  k_rs_refine<<<w.ctas, kRsRefineThreads, 0, stream>>>(offsets, nDraw, s0, slots, corrs, norm, samples, invK, thr, thr2,
-                                                       w.tasks, w.nTasks, w.lists, w.listRoom, w.refined);
+  k_rs_refine_tasks<<<nPairs, 32, 0, stream>>>(plan, counts, slotOk, cost, st, w.taskIdx, w.taskN, w.tasks, w.nTasks);
+  k_rs_refine<<<w.ctas, kRsRefineThreads, 0, stream>>>(offsets, nDraw, plan, st, slots, corrs, norm, samples, invK, thr,
+                                                       thr2, w.tasks, w.nTasks, nPairs * kRsTasks, w.lists, w.listRoom,
+                                                       w.refined);
   k_rs_select_refine<<<nPairs < w.ctas ? nPairs : w.ctas, kRsRefineThreads, 0, stream>>>(
-      offsets, nPairs, nDraw, s0, len, counts, slotOk, cost, slots, st, bestEF, corrs, norm, samples, invK, thr, thr2,
+      offsets, nPairs, nDraw, plan, counts, slotOk, cost, slots, st, bestEF, corrs, norm, samples, invK, thr, thr2,
       bestRT, w.taskIdx, w.taskN, w.lists, w.listRoom, w.refined);
   return cudaGetLastError();
 }
