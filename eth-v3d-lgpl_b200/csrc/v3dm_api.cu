@@ -77,16 +77,16 @@ struct v3dm_matcher {
   bool countWritten = false;      // the last enqueue wrote *countOut itself
   int lastLaunches = 0;
   // Float descriptors that are not u/512 (tcgen05 kernel): BF16 hi/lo operand layouts
-  // (v3dm_match_f.cu), 6 planes of cap rows x 128 bytes each.
+  // (v3dm_match_f.cu), 4 planes of cap rows x 128 bytes each.
   bool floatL = false, floatR = false;  // the side's current descriptors are float
   int capFL = 0, capFR = 0;
-  uint8_t* dLfA = nullptr;  // lefts, A layout (pass A operand)
-  uint8_t* dLfB = nullptr;  // lefts, B layout (pass B operand)
-  uint8_t* dRfA = nullptr;  // rights, A layout (gathered into dRcf)
-  uint8_t* dRfB = nullptr;  // rights, B layout (pass A operand)
-  uint8_t* dRcf = nullptr;  // chosen rights, A layout (pass B operand)
+  uint8_t* dLf = nullptr;   // lefts
+  uint8_t* dRf = nullptr;   // rights
+  uint8_t* dRcf = nullptr;  // chosen rights (pass-B operand)
+  uint32_t* dFPartial = nullptr;  // segment merges of the side passes
+  int* dFCount = nullptr;
   bool fBound = false;
-  CUtensorMap fmA_A, fmA_B, fmB_A, fmB_B;
+  CUtensorMap fmL, fmR, fmRc;
   int numSMs = 148;
   // Optional CUDA-event timing of the fused matching kernel (v3dm_matcher_profile).
   bool profile = false;
@@ -152,11 +152,11 @@ void free_buffers(v3dm_matcher* h) {
   dfree(h->dFlagA);
   dfree(h->dFlagB);
   h->dCounters = nullptr;  // points into dInfo
-  dfree(h->dLfA);
-  dfree(h->dLfB);
-  dfree(h->dRfA);
-  dfree(h->dRfB);
+  dfree(h->dLf);
+  dfree(h->dRf);
   dfree(h->dRcf);
+  dfree(h->dFPartial);
+  dfree(h->dFCount);
   h->floatL = h->floatR = false;
   h->capFL = h->capFR = 0;
   h->fBound = false;
@@ -482,24 +482,24 @@ int set_features_u8(v3dm_matcher* h, bool left, int n, const uint8_t* desc, bool
 
 // Float operand layouts of both sides (allocated on first use, kept until deallocate).
 cudaError_t alloc_float(v3dm_matcher* h) {
-  if (h->dLfA) return cudaSuccess;
+  if (h->dLf) return cudaSuccess;
   const int capL = std::max(256, (h->nMaxL + 255) / 256 * 256), capR = std::max(256, (h->nMaxR + 255) / 256 * 256);
-  cudaError_t e = dalloc(&h->dLfA, (size_t)capL * kFloatRowBytes);
-  if (e == cudaSuccess) e = dalloc(&h->dLfB, (size_t)capL * kFloatRowBytes);
-  if (e == cudaSuccess) e = dalloc(&h->dRfA, (size_t)capR * kFloatRowBytes);
-  if (e == cudaSuccess) e = dalloc(&h->dRfB, (size_t)capR * kFloatRowBytes);
+  const size_t counts = f_count_words(h->numSMs);
+  cudaError_t e = dalloc(&h->dLf, (size_t)capL * kFloatRowBytes);
+  if (e == cudaSuccess) e = dalloc(&h->dRf, (size_t)capR * kFloatRowBytes);
   if (e == cudaSuccess) e = dalloc(&h->dRcf, (size_t)capR * kFloatRowBytes);
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->dLfA, 0, (size_t)capL * kFloatRowBytes, h->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->dLfB, 0, (size_t)capL * kFloatRowBytes, h->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->dRfA, 0, (size_t)capR * kFloatRowBytes, h->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->dRfB, 0, (size_t)capR * kFloatRowBytes, h->stream);
+  if (e == cudaSuccess) e = dalloc(&h->dFPartial, f_partial_words(h->numSMs));
+  if (e == cudaSuccess) e = dalloc(&h->dFCount, counts);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->dLf, 0, (size_t)capL * kFloatRowBytes, h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->dRf, 0, (size_t)capR * kFloatRowBytes, h->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->dRcf, 0, (size_t)capR * kFloatRowBytes, h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->dFCount, 0, counts * sizeof(int), h->stream);
   if (e != cudaSuccess) {
-    dfree(h->dLfA);
-    dfree(h->dLfB);
-    dfree(h->dRfA);
-    dfree(h->dRfB);
+    dfree(h->dLf);
+    dfree(h->dRf);
     dfree(h->dRcf);
+    dfree(h->dFPartial);
+    dfree(h->dFCount);
     return e;
   }
   h->capFL = capL;
@@ -512,8 +512,8 @@ cudaError_t alloc_float(v3dm_matcher* h) {
 int stage_to_float(v3dm_matcher* h, bool left, int n) {
   V3DM_CUDA_TRY(alloc_float(h));
   V3DM_CUDA_TRY(cudaMemsetAsync(h->dInfo + kInfoErr, 0, sizeof(int32_t), h->stream));
-  V3DM_CUDA_TRY(launch_hilo(h->dStage, nullptr, n, left ? h->capFL : h->capFR, left ? h->dLfA : h->dRfA,
-                            left ? h->dLfB : h->dRfB, h->dInfo + kInfoErr, h->stream));
+  V3DM_CUDA_TRY(launch_hilo(h->dStage, nullptr, n, left ? h->capFL : h->capFR, left ? h->dLf : h->dRf,
+                            h->dInfo + kInfoErr, h->stream));
   V3DM_CUDA_TRY(cudaMemcpyAsync(h->hInfo + kInfoErr, h->dInfo + kInfoErr, sizeof(int32_t), cudaMemcpyDeviceToHost,
                                 h->stream));
   V3DM_CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -808,65 +808,55 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
   return V3DM_OK;
 }
 
-// Float path (either side holds float descriptors): the same two side passes and decisions with
-// BF16 hi/lo scores (v3dm_match_f.cu).  A side holding u/512 descriptors gets its float layouts
-// from its uint8 values, which is exact.
+// The float layouts and their tensor maps; a side holding u/512 descriptors gets its layout from its
+// uint8 values, which is exact.
+int bind_float(v3dm_matcher* h) {
+  V3DM_CUDA_TRY(alloc_float(h));
+  if (!h->floatL) V3DM_CUDA_TRY(launch_hilo(nullptr, h->dL, h->nL, h->capFL, h->dLf, h->dInfo + kInfoErr, h->stream));
+  if (!h->floatR) V3DM_CUDA_TRY(launch_hilo(nullptr, h->dR, h->nR, h->capFR, h->dRf, h->dInfo + kInfoErr, h->stream));
+  if (!h->fBound) {
+    V3DM_CUDA_TRY(f_map(&h->fmL, h->dLf, h->capFL));
+    V3DM_CUDA_TRY(f_map(&h->fmR, h->dRf, h->capFR));
+    V3DM_CUDA_TRY(f_map(&h->fmRc, h->dRcf, h->capFR));
+    h->fBound = true;
+  }
+  return V3DM_OK;
+}
+
+// Float path (either side holds float descriptors): the same two side passes with BF16 hi/lo scores
+// (v3dm_match_f.cu), which decide their rows themselves, the call's gates applied.
 int enqueue_match_f(v3dm_matcher* h, float minScore, float minRatio, int32_t* dPairs) {
   const float Tf = host_float_threshold(minScore, minRatio);
-  V3DM_CUDA_TRY(alloc_float(h));
-  if (!h->floatL)
-    V3DM_CUDA_TRY(launch_hilo(nullptr, h->dL, h->nL, h->capFL, h->dLfA, h->dLfB, h->dInfo + kInfoErr, h->stream));
-  if (!h->floatR)
-    V3DM_CUDA_TRY(launch_hilo(nullptr, h->dR, h->nR, h->capFR, h->dRfA, h->dRfB, h->dInfo + kInfoErr, h->stream));
-  if (!h->fBound) {
-    V3DM_CUDA_TRY(f_maps(&h->fmA_A, h->dLfA, h->capFL, &h->fmA_B, h->dRfB, h->capFR));
-    V3DM_CUDA_TRY(f_maps(&h->fmB_A, h->dRcf, h->capFR, &h->fmB_B, h->dLfB, h->capFL));
-    h->fBound = true;
+  {
+    const int st = bind_float(h);
+    if (st != V3DM_OK) return st;
   }
   SideArgs sa;
   std::memset(&sa, 0, sizeof(sa));
-  sa.records = h->dRecords;
-  sa.segCount = h->dSegCount;
-  sa.segCap = h->segCap;
-  sa.nSeg = h->nSeg;
   sa.err = h->dInfo + kInfoErr;
-  PostArgs pa;
-  std::memset(&pa, 0, sizeof(pa));
-  pa.records = h->dRecords;
-  pa.segCount = h->dSegCount;
-  pa.segCap = h->segCap;
-  pa.nSeg = f_segments(h->numSMs);
-  pa.nGates = h->nGates;
-  pa.gatesDev = h->dGates;
-  pa.minScore = minScore;
-  pa.minRatio = minRatio;
-  pa.err = h->dInfo + kInfoErr;
+  sa.nGates = h->nGates;
+  sa.gatesDev = h->dGates;
+  sa.minScore = minScore;
+  sa.minRatio = minRatio;
+  sa.fPartial = h->dFPartial;
+  sa.fCount = h->dFCount;
+  // the passes leave the counters zero; a pass that gave up on a wait may not have
+  V3DM_CUDA_TRY(cudaMemsetAsync(h->dFCount, 0, f_count_words(h->numSMs) * sizeof(int), h->stream));
   cudaEvent_t evA[2], evB[2];
   // pass A: every left against every right
   sa.nA = h->nL;
   sa.nB = h->nR;
   sa.aIsLeft = 1;
-  sa.best = h->dLBest;
-  sa.sec = h->dLSec;
+  sa.decision = h->dLeftDec;
   if (h->profile) {
     int e = event_pair(h, 0, evA);
     if (e != V3DM_OK) return e;
     V3DM_CUDA_TRY(cudaEventRecord(evA[0], h->stream));
   }
-  // Each CTA scores whole rows (128 lefts against every right) and decides them from the exact
-  // best and second it keeps in registers, the call's gates applied where a score could enter
-  // them; no chunk records for pass A.
-  sa.rows = nullptr;
-  sa.nGates = h->nGates;
-  sa.gatesDev = h->dGates;
-  sa.decision = h->dLeftDec;
-  sa.minScore = minScore;
-  sa.minRatio = minRatio;
-  V3DM_CUDA_TRY(launch_side_f_batch(h->fmA_A, h->fmA_B, sa, Tf, h->numSMs, h->stream));
-  sa.decision = nullptr;
+  V3DM_CUDA_TRY(launch_side_f(h->fmL, h->fmR, sa, Tf, nullptr, h->numSMs, h->stream));
   if (h->profile) V3DM_CUDA_TRY(cudaEventRecord(evA[1], h->stream));
-  // the accepted rights, once each, gathered (six planes) for pass B
-  V3DM_CUDA_TRY(launch_choose_planes(h->dLeftDec, h->nL, h->dChosenFlag, h->dChosenList, h->dCounters, h->dRfA,
+  // the accepted rights, once each, gathered (four planes) for pass B
+  V3DM_CUDA_TRY(launch_choose_planes(h->dLeftDec, h->nL, h->dChosenFlag, h->dChosenList, h->dCounters, h->dRf,
                                      h->dRcf, kFloatRowBytes / kDescBytes, h->capFR, h->capFR, h->stream));
   // pass B: the chosen rights against every left
   sa.nAptr = h->dCounters;
@@ -874,27 +864,18 @@ int enqueue_match_f(v3dm_matcher* h, float minScore, float minRatio, int32_t* dP
   sa.nB = h->nL;
   sa.amap = h->dChosenList;
   sa.aIsLeft = 0;
-  sa.best = h->dRBest;
-  sa.sec = h->dRSec;
+  sa.decision = h->dRightDec;
   if (h->profile) {
     int e = event_pair(h, 1, evB);
     if (e != V3DM_OK) return e;
     V3DM_CUDA_TRY(cudaEventRecord(evB[0], h->stream));
   }
-  V3DM_CUDA_TRY(launch_side_f(h->fmB_A, h->fmB_B, sa, Tf, nullptr, h->numSMs, h->stream));
+  V3DM_CUDA_TRY(launch_side_f(h->fmRc, h->fmL, sa, Tf, nullptr, h->numSMs, h->stream));
   if (h->profile) V3DM_CUDA_TRY(cudaEventRecord(evB[1], h->stream));
-  pa.nRows = h->nR;
-  pa.rowsPtr = h->dCounters;
-  pa.amap = h->dChosenList;
-  pa.aIsLeft = 0;
-  pa.best = h->dRBest;
-  pa.sec = h->dRSec;
-  pa.decision = h->dRightDec;
-  V3DM_CUDA_TRY(launch_post_f(pa, Tf, h->stream));
   V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->dRightDec, h->dChosenFlag, h->dScratch,
                               reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, h->stream));
   h->countWritten = h->countOut != nullptr;
-  h->lastLaunches = (h->floatL ? 0 : 1) + (h->floatR ? 0 : 1) + 7;
+  h->lastLaunches = (h->floatL ? 0 : 1) + (h->floatR ? 0 : 1) + 5;
   return V3DM_OK;
 }
 
@@ -1047,30 +1028,22 @@ int v3dm_scores_f32(v3dm_matcher* h, float* scores) {
   if (n == 0) return V3DM_OK;
   DeviceGuard g(h->device);
   V3DM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  V3DM_CUDA_TRY(alloc_float(h));
-  if (!h->floatL)
-    V3DM_CUDA_TRY(launch_hilo(nullptr, h->dL, h->nL, h->capFL, h->dLfA, h->dLfB, h->dInfo + kInfoErr, h->stream));
-  if (!h->floatR)
-    V3DM_CUDA_TRY(launch_hilo(nullptr, h->dR, h->nR, h->capFR, h->dRfA, h->dRfB, h->dInfo + kInfoErr, h->stream));
-  if (!h->fBound) {
-    V3DM_CUDA_TRY(f_maps(&h->fmA_A, h->dLfA, h->capFL, &h->fmA_B, h->dRfB, h->capFR));
-    V3DM_CUDA_TRY(f_maps(&h->fmB_A, h->dRcf, h->capFR, &h->fmB_B, h->dLfB, h->capFL));
-    h->fBound = true;
+  {
+    const int st = bind_float(h);
+    if (st != V3DM_OK) return st;
   }
   float* dS = nullptr;
   V3DM_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&dS), (size_t)n * sizeof(float)));
   SideArgs sa;
   std::memset(&sa, 0, sizeof(sa));
-  sa.records = h->dRecords;
-  sa.segCount = h->dSegCount;
-  sa.segCap = h->segCap;
-  sa.nSeg = h->nSeg;
   sa.err = h->dInfo + kInfoErr;
   sa.nA = h->nL;
   sa.nB = h->nR;
   sa.aIsLeft = 1;
-  // Tf = +inf: no chunk is handed over, only the dump is written
-  cudaError_t e = launch_side_f(h->fmA_A, h->fmA_B, sa, INFINITY, dS, h->numSMs, h->stream);
+  sa.fPartial = h->dFPartial;
+  sa.fCount = h->dFCount;
+  // only the dump is written
+  cudaError_t e = launch_side_f(h->fmL, h->fmR, sa, INFINITY, dS, h->numSMs, h->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(scores, dS, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);

@@ -195,7 +195,7 @@ k_bscan(const int* __restrict__ cnt, int nPairs, const BImage* __restrict__ im, 
 
 // Gathers, per pair and in ascending left order, the right named by every accepted left into
 // the pass-B operand buffer, with its (pair, left, right) identity.  A row is 'planes' blocks of
-// 128 bytes, block p of row r at (p * planeRows + r) * 128 (one block: uint8 descriptors; six:
+// 128 bytes, block p of row r at (p * planeRows + r) * 128 (one block: uint8 descriptors; four:
 // the planar BF16 hi/lo layout).
 __global__ void __launch_bounds__(kChooseThreads)
 k_bchoose(const BPair* __restrict__ pairs, int nPairs, const BImage* __restrict__ im,
@@ -907,20 +907,19 @@ struct v3dm_batch {
   long long pairAuxCap = 0;
   int* dFlag = nullptr;             // flagged states of one pass
   long long flagCap = 0;
-  // float descriptors not all of the form u/512: BF16 hi/lo layouts (6 planes of fRows x 128 B)
+  // float descriptors not all of the form u/512: BF16 hi/lo layout (4 planes of fRows x 128 B)
   bool floatMode = false;
   int numSMs = 0;
   float* dStageF = nullptr;         // the caller's floats, staged
   long long stageFCap = 0;          // floats
   int* dRowOffI = nullptr;          // per image: first row (device copy of rowOff)
   long long rowOffCap = 0;
-  uint8_t* dFA = nullptr;           // A layout of every image: [hi | lo | hi]
-  uint8_t* dFB = nullptr;           // B layout of every image: [hi | hi | lo]
-  long long fImgCapA = 0, fImgCapB = 0;  // bytes
-  int fRows = 0;                    // rows per plane of dFA / dFB
+  uint8_t* dF = nullptr;            // BF16 hi/lo layout of every image
+  long long fImgCap = 0;            // bytes
+  int fRows = 0;                    // rows per plane of dF
   uint8_t* dFAB = nullptr;          // pass-B A operand: the chosen rights' A rows, capRowsB rows per plane
   long long fabCap = 0;             // bytes
-  CUtensorMap fmA_A, fmA_B, fmB_A, fmB_B;
+  CUtensorMap fmImg, fmAB;
   bool fMapsValid = false;
   // profiling
   bool profile = false;
@@ -1213,16 +1212,16 @@ int enqueue_batch_f(v3dm_batch* b, float minScore, float minRatio, bool withEven
   sa.minScore = minScore;
   sa.minRatio = minRatio;
   if (bg) sa.bg = *bg;
-  // ---- pass A: every (pair, group of 128 lefts) against the pair's right image
+  // ---- pass A: every (pair, group of lefts) against the pair's right image
   sa.aIsLeft = 1;
   sa.rows = b->dRowsA;
   sa.nRows = b->nRowsA;
   sa.decision = b->dDecA;
   if (withEvents) V3DM_BTRY(cudaEventRecord(b->ev[0], b->stream));
-  V3DM_BTRY(launch_side_f_batch(b->fmA_A, b->fmA_B, sa, Tf, b->numSMs, b->stream));
+  V3DM_BTRY(launch_side_f(b->fmImg, b->fmImg, sa, Tf, nullptr, b->numSMs, b->stream));
   if (withEvents) V3DM_BTRY(cudaEventRecord(b->ev[1], b->stream));
   launches += b->nRowsA > 0;
-  // ---- pass-B layout: the chosen rights' A rows (six planes)
+  // ---- pass-B layout: the chosen rights' rows (four planes)
   const int chooseGrid = std::max(1, std::min(b->nPairs, 4 * 148));
   k_bcount<<<chooseGrid, kChooseThreads, 0, b->stream>>>(b->dPairs, b->nPairs, b->dDecA, b->dCnt);
   V3DM_BTRY(cudaGetLastError());
@@ -1231,7 +1230,7 @@ int enqueue_batch_f(v3dm_batch* b, float minScore, float minRatio, bool withEven
                                              b->dCounters);
   V3DM_BTRY(cudaGetLastError());
   k_bchoose<<<chooseGrid, kChooseThreads, 0, b->stream>>>(b->dPairs, b->nPairs, b->dImages, b->dImgB, b->dPrefC,
-                                                          b->dDecA, b->dFA, b->dFAB, b->dChosenLeft, b->dChosenRight,
+                                                          b->dDecA, b->dF, b->dFAB, b->dChosenLeft, b->dChosenRight,
                                                           b->dChosenPair, b->dCounters, kFloatRowBytes / kDescBytes,
                                                           b->fRows, b->capRowsB);
   V3DM_BTRY(cudaGetLastError());
@@ -1243,7 +1242,7 @@ int enqueue_batch_f(v3dm_batch* b, float minScore, float minRatio, bool withEven
   sa.nRows = (int)std::min<long long>(b->capTableB, 0x7fffffff);
   sa.decision = b->dDecB;
   if (withEvents) V3DM_BTRY(cudaEventRecord(b->ev[2], b->stream));
-  V3DM_BTRY(launch_side_f_batch(b->fmB_A, b->fmB_B, sa, Tf, b->numSMs, b->stream));
+  V3DM_BTRY(launch_side_f(b->fmAB, b->fmImg, sa, Tf, nullptr, b->numSMs, b->stream));
   if (withEvents) V3DM_BTRY(cudaEventRecord(b->ev[3], b->stream));
   launches += 1;
   // ---- mutual filter, ordered triples
@@ -1274,8 +1273,8 @@ int prepare_float(v3dm_batch* b) {
     b->fMapsValid = false;
   }
   if (!b->fMapsValid) {
-    V3DM_BTRY(f_maps(&b->fmA_A, b->dFA, b->fRows, &b->fmA_B, b->dFB, b->fRows));
-    V3DM_BTRY(f_maps(&b->fmB_A, b->dFAB, (int)b->capRowsB, &b->fmB_B, b->dFB, b->fRows));
+    V3DM_BTRY(f_map(&b->fmImg, b->dF, b->fRows));
+    V3DM_BTRY(f_map(&b->fmAB, b->dFAB, (int)b->capRowsB));
     b->fMapsValid = true;
   }
   return V3DM_OK;
@@ -1828,8 +1827,7 @@ void free_all(v3dm_batch* b) {
   bfree(b->dFlag);
   bfree(b->dStageF);
   bfree(b->dRowOffI);
-  bfree(b->dFA);
-  bfree(b->dFB);
+  bfree(b->dF);
   bfree(b->dFAB);
   b->dCounters = nullptr;  // points into dInfo
   bfree(b->dInfo);
@@ -1978,16 +1976,14 @@ int set_images_f32(v3dm_batch* b, int nImages, const int32_t* counts, const floa
   set_float_mode(b, true);
   b->fMapsValid = false;  // re-encoded before the next call (same buffers: same maps)
   const int fRows = (int)std::max<long long>(b->totalRows, 256);
-  const uint8_t* oldA = b->dFA;
-  const uint8_t* oldB = b->dFB;
-  V3DM_BTRY(ensure(&b->dFA, &b->fImgCapA, (long long)fRows * kFloatRowBytes));
-  V3DM_BTRY(ensure(&b->dFB, &b->fImgCapB, (long long)fRows * kFloatRowBytes));
-  if (b->dFA != oldA || b->dFB != oldB || b->fRows != fRows) drop_graph(b);  // the graph's maps name the buffers
+  const uint8_t* old = b->dF;
+  V3DM_BTRY(ensure(&b->dF, &b->fImgCap, (long long)fRows * kFloatRowBytes));
+  if (b->dF != old || b->fRows != fRows) drop_graph(b);  // the graph's maps name the buffer
   b->fRows = fRows;
   V3DM_BTRY(ensure(&b->dRowOffI, &b->rowOffCap, std::max(nImages, 1)));
   V3DM_BTRY(cudaMemcpyAsync(b->dRowOffI, b->rowOff.data(), (size_t)nImages * sizeof(int), cudaMemcpyHostToDevice,
                             b->stream));
-  V3DM_BTRY(launch_hilo_images(src, total, b->dSrcOff, b->dRowOffI, nImages, fRows, b->dFA, b->dFB, err, b->stream));
+  V3DM_BTRY(launch_hilo_images(src, total, b->dSrcOff, b->dRowOffI, nImages, fRows, b->dF, err, b->stream));
   V3DM_BTRY(cudaMemcpyAsync(b->hInfo + kInfoErr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, b->stream));
   V3DM_BTRY(cudaStreamSynchronize(b->stream));
   if (b->hInfo[kInfoErr]) {  // a value that is not finite

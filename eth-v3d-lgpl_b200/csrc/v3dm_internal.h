@@ -123,10 +123,12 @@ struct SideArgs {
   // gathered A (launch_side_gather): A row e of the row table is descriptor aSrcRow[e] of aSrc
   const uint8_t* aSrc;
   const int* aSrcRow;
-  // batched float pass (launch_side_f_batch): decisions written per state, the float rules
+  // float pass (launch_side_f): decisions written per state, the float rules
   int32_t* decision;
   float minScore, minRatio;
   BatchGateArgs bg;              // batched float pass of a guided call: each pair's gate (on = 0: none)
+  uint32_t* fPartial;            // float pass of one pair: best and second of its rows' segments
+  int* fCount;
   // failure-path test hooks (zero in production): the bounded waits give up after waitLimit
   // cycles (0: the default), and CTA 0's producer does not issue its skipLoad-th B tile load
   // (0: none), so that the consumer's bounded wait for it runs out
@@ -265,15 +267,12 @@ struct PostArgs {
   int* flaggedCount;
   int* err;
   // Optional (pass A of one pair): every accepted partner is also 'chosen' right here -- flagged,
-  // listed once, and its descriptor row gathered for pass B (planar BF16 rows when choosePlanes
-  // is 6, else 128-byte rows).
+  // listed once, and its descriptor row gathered for pass B.
   int* chooseFlag;
   int* chooseList;
   int* chooseCount;
   const uint8_t* chooseSrc;
   uint8_t* chooseDst;
-  int chooseCapSrc, chooseCapDst;
-  int choosePlanes;
 };
 cudaError_t launch_post(const PostArgs& a, cudaStream_t s);
 // u8 re-quantisation of nValues floats (a multiple of 4), v3dm_features.cu.
@@ -281,28 +280,28 @@ cudaError_t launch_quantize_u8(const float* d_x, long long nValues, uint8_t* d_o
                                int* d_inexact = nullptr);
 
 // ---- float descriptors: BF16 hi/lo scores (v3dm_match_f.cu) ------------------------------
-// Operand layouts: 6 planes of rowsCap x 128 bytes (64 BF16 values of a K slice per row).
-constexpr int kFloatRowBytes = 768;
-int f_segments(int numSMs);
-cudaError_t f_maps(CUtensorMap* mA, const void* dA, int rowsA, CUtensorMap* mB, const void* dB, int rowsB);
+// Operand layout, of either side: 4 planes of rowsCap x 128 bytes (64 BF16 values of a K slice per
+// row: hi, hi, lo, lo).
+constexpr int kFloatRowBytes = 512;
+constexpr int kFMaxSegments = 32;  // segments of one pair's row
+cudaError_t f_map(CUtensorMap* m, const void* base, int rows);
+// Float side pass, one persistent launch.  Over a.rows (a.nRows, or *a.nRowsPtr rows), interleaved
+// over the CTAs: A groups of f_group_rows() rows, B tiles of f_tile_cols() columns.  With a.rows null:
+// one pair, a.nA (or *a.nAptr) A rows against a.nB B rows, a.fPartial and a.fCount (zero, and left
+// zero) for the merges; row r's state is amap[r], or r.  Writes the decision of every state to
+// a.decision (the float rules with a.minScore, a.minRatio, the call's gates and the candidate
+// threshold Tf).  With dump, every score to dump[state * nB + column] as well.
 cudaError_t launch_side_f(const CUtensorMap& mA, const CUtensorMap& mB, const SideArgs& a, float Tf, float* dump,
                           int numSMs, cudaStream_t st);
-// Batched float side pass over a.rows (a.nRows, or *a.nRowsPtr rows), rows interleaved over the
-// persistent CTAs; A groups of f_group_rows() rows, B tiles of f_tile_cols() columns.  Writes
-// the decision of every state of the rows to a.decision (the float rules with a.minScore,
-// a.minRatio and the candidate threshold Tf); no chunk records.  With a.rows null: one pair,
-// a.nA A rows against a.nB B rows, decisions indexed by A row.
-cudaError_t launch_side_f_batch(const CUtensorMap& mA, const CUtensorMap& mB, const SideArgs& a, float Tf,
-                                int numSMs, cudaStream_t st);
 int f_group_rows();
 int f_tile_cols();
-cudaError_t launch_post_f(const PostArgs& a, float Tf, cudaStream_t s);
-cudaError_t launch_hilo(const float* f, const uint8_t* u, int n, int rowsCap, void* la, void* lb, int* err,
-                        cudaStream_t s);
-// The same layouts for the n concatenated descriptors of nImages images: image i (first
+size_t f_partial_words(int numSMs);
+size_t f_count_words(int numSMs);
+cudaError_t launch_hilo(const float* f, const uint8_t* u, int n, int rowsCap, void* planes, int* err, cudaStream_t s);
+// The same layout for the n concatenated descriptors of nImages images: image i (first
 // descriptor srcOff[i], ascending) goes to rows rowOff[i] onwards of the rowsCap-row planes.
 cudaError_t launch_hilo_images(const float* f, long long n, const long long* srcOff, const int* rowOff, int nImages,
-                               int rowsCap, void* la, void* lb, int* err, cudaStream_t s);
+                               int rowsCap, void* planes, int* err, cudaStream_t s);
 float host_float_threshold(float minScore, float minRatio);
 // Exact re-score of the flagged descriptors of side A against side B.
 struct RescoreArgs {

@@ -105,19 +105,10 @@ __device__ __forceinline__ void clear_segments(const PostArgs& a) {
 // Copies right r's descriptor row to slot k of the pass-B operand.
 __device__ __forceinline__ void gather_chosen(const PostArgs& a, int r, int k) {
   a.chooseList[k] = r;
-  if (a.choosePlanes) {
-    for (int p = 0; p < a.choosePlanes; ++p) {
-      const uint4* src = reinterpret_cast<const uint4*>(a.chooseSrc + ((size_t)p * a.chooseCapSrc + r) * 128);
-      uint4* dst = reinterpret_cast<uint4*>(a.chooseDst + ((size_t)p * a.chooseCapDst + k) * 128);
+  const uint4* src = reinterpret_cast<const uint4*>(a.chooseSrc + (size_t)r * kDescBytes);
+  uint4* dst = reinterpret_cast<uint4*>(a.chooseDst + (size_t)k * kDescBytes);
 #pragma unroll
-      for (int w = 0; w < 8; ++w) dst[w] = src[w];
-    }
-  } else {
-    const uint4* src = reinterpret_cast<const uint4*>(a.chooseSrc + (size_t)r * kDescBytes);
-    uint4* dst = reinterpret_cast<uint4*>(a.chooseDst + (size_t)k * kDescBytes);
-#pragma unroll
-    for (int w = 0; w < kDescBytes / 16; ++w) dst[w] = src[w];
-  }
+  for (int w = 0; w < kDescBytes / 16; ++w) dst[w] = src[w];
 }
 
 // Decisions of the pass's descriptors; flags the ones whose gated bound straddles the
