@@ -103,6 +103,8 @@ struct Smem {
   unsigned long long fullA[C::kASlots], emptyA[C::kASlots];
   unsigned long long accEmpty[C::kAcc];
   unsigned long long mmaDone;
+  unsigned long long runFull[32];  // batched pass: the ring of runs (kRunRing)
+  int4 runs[2 * 32];
   uint32_t tmemBase;
   int abort;
 };
@@ -187,25 +189,31 @@ struct WorkCursor {
     t0 = 0;
     nT = min(nTiles, left);
   }
-  __device__ __forceinline__ void prefetch_rows() const {}
 };
 
-__device__ __forceinline__ BatchRow load_row(const BatchRow* rows, int r) {
-  const int4* p = reinterpret_cast<const int4*>(rows + r);
-  const int4 x = __ldg(p), y = __ldg(p + 1);
-  BatchRow b;
-  b.aRow = x.x;
-  b.validRows = x.y;
-  b.bRow0 = x.z;
-  b.nB = x.w;
-  b.nTiles = max(y.x, 1);  // every row advances the cursor by at least one tile
-  b.pad = y.y;
-  b.state0 = (long long)(((unsigned long long)(uint32_t)y.w << 32) | (uint32_t)y.z);
-  return b;
-}
+// A row entry as loaded.  Nothing is computed from it before its turn: the loads take some 800 cycles
+// and any use, were it only the lower limit of nTiles, would wait for them where they are issued.
+struct RawRow {
+  int4 x, y;
+  __device__ __forceinline__ void load(const BatchRow* rows, int r) {
+    const int4* p = reinterpret_cast<const int4*>(rows + r);
+    x = __ldg(p);
+    y = __ldg(p + 1);
+  }
+  __device__ __forceinline__ BatchRow row() const {
+    BatchRow b;
+    b.aRow = x.x;
+    b.validRows = x.y;
+    b.bRow0 = x.z;
+    b.nB = x.w;
+    b.nTiles = y.x;
+    b.pad = y.y;
+    b.state0 = (long long)(((unsigned long long)(uint32_t)y.w << 32) | (uint32_t)y.z);
+    return b;
+  }
+};
 
 constexpr int kChunkRows = 32;  // schedule 2: rows per chunk
-constexpr int kRowAhead = 6;    // the producer prefetches the row entry this many rows ahead
 
 // Batched pass: walks the rows of a row table, every tile of a row in order.  Schedule 0
 // gives CTA b the rows b, b + grid, b + 2 grid, ...: the CTAs then work on neighbouring rows
@@ -213,15 +221,14 @@ constexpr int kRowAhead = 6;    // the producer prefetches the row entry this ma
 // each CTA one contiguous range of rows.  Schedule 2 deals out chunks of kChunkRows
 // consecutive rows the way schedule 0 deals out rows: consecutive rows that share their A
 // block (short rows of one left block against many right blocks) keep it in shared memory,
-// and the CTAs still work on neighbouring rows.  The next row's entry is loaded a row ahead;
-// the producer also prefetches entries kRowAhead rows ahead into L1.  newA says whether the
-// current row's A block differs from the previous row's (a row's A block is identified by
-// its first row aRow).
+// and the CTAs still work on neighbouring rows.  The next row's entry is loaded a row ahead.
+// newA says whether the current row's A block differs from the previous row's (a row's A block
+// is identified by its first row aRow).
 struct BatchCursor {
   const BatchRow* rows;
   int R, Rend, schedule;
-  BatchRow cur, nxt;
-  static constexpr int t0 = 0;
+  BatchRow cur;
+  RawRow raw;  // the next row
   int nT;
   bool newA;
   __device__ __forceinline__ int step_from(int r) const {
@@ -233,7 +240,7 @@ struct BatchCursor {
   __device__ __forceinline__ BatchCursor(const BatchRow* rows_, int nRows, int sch)
       : rows(rows_), schedule(sch), newA(true) {
     cur = BatchRow{};
-    nxt = BatchRow{};
+    raw = RawRow{};
     if (schedule == 0) {
       R = blockIdx.x;
       Rend = nRows;
@@ -244,28 +251,84 @@ struct BatchCursor {
       R = blockIdx.x * kChunkRows;
       Rend = nRows;
     }
-    if (R < Rend) cur = load_row(rows, R);
+    if (R < Rend) raw.load(rows, R);
+    take();
+  }
+  __device__ __forceinline__ void take() {
+    cur = raw.row();
+    nT = cur.nTiles = max(cur.nTiles, 1);  // every row advances the cursor by at least one tile
     const int R1 = step_from(R);
-    if (R1 < Rend) nxt = load_row(rows, R1);
-    nT = cur.nTiles;
+    if (R1 < Rend) raw.load(rows, R1);
   }
   __device__ __forceinline__ bool more() const { return R < Rend; }
   __device__ __forceinline__ void next() {
     R = step_from(R);
-    newA = nxt.aRow != cur.aRow;
-    cur = nxt;
-    nT = cur.nTiles;
-    const int R1 = step_from(R);
-    if (R1 < Rend) nxt = load_row(rows, R1);
+    newA = raw.x.x != cur.aRow;
+    take();
   }
-  // The row entry kRowAhead rows ahead, into L1 (the other roles of the CTA read it later).
-  __device__ __forceinline__ void prefetch_rows() const {
-    int r = R;
-#pragma unroll
-    for (int i = 0; i < kRowAhead; ++i) r = step_from(r);
-    if (r < Rend) asm volatile("prefetch.global.L1 [%0];" ::"l"(rows + r));
+  __device__ __forceinline__ int next_a_row() const { return raw.x.x; }
+  __device__ __forceinline__ int next_valid_rows() const { return raw.x.y; }
+};
+
+// The other roles of a batched pass read each run from a ring in shared memory, where the producer
+// puts its row (newA in the entry's last word) before the row's first load; a row of no tiles ends
+// the walk.  Walking the table themselves cost every epilogue warp the table's loads or, loaded a
+// row ahead, spills: 860 cycles per run, as much as a tile's filtering (runs of one or two tiles:
+// the pass over a cell's rights of the candidate proposal; a proposal call over 60 images of 8000
+// took 8.0 ms, 7.4 with the ring, and 200 images of 8192, whose runs are long, 89 and 84.5: the
+// spills).  A slot is not written again before
+// every role has read it: the producer's tiles are at most kStages + kAcc ahead of the slowest
+// warp, and a run has a tile or more.
+constexpr int kRunRing = 32;
+struct RunCursor {
+  const int4* ring;
+  unsigned long long* full;
+  uint32_t r = 0;
+  BatchRow cur;
+  static constexpr int t0 = 0;
+  int nT;
+  bool newA;
+  int* abortFlag;
+  int* err;
+  long long lim;
+  __device__ __forceinline__ RunCursor(const int4* ring_, unsigned long long* full_, int* abort_, int* err_,
+                                       long long lim_)
+      : ring(ring_), full(full_), abortFlag(abort_), err(err_), lim(lim_) {
+    load();
+  }
+  __device__ __forceinline__ void load() {
+    const uint32_t slot = r % kRunRing;
+    if (!mbar_wait_warp(&full[slot], (r / kRunRing) & 1u, abortFlag, err, lim)) {
+      nT = 0;
+      return;
+    }
+    RawRow raw;
+    raw.x = ring[2 * slot];
+    raw.y = ring[2 * slot + 1];
+    cur = raw.row();
+    nT = cur.nTiles;
+    newA = cur.pad != 0;
+  }
+  __device__ __forceinline__ bool more() const { return nT > 0; }
+  __device__ __forceinline__ void next() {
+    ++r;
+    load();
   }
 };
+// The producer's side: the row of its r-th run, or the end (row null).
+__device__ __forceinline__ void put_run(int4* ring, unsigned long long* full, uint32_t r, const BatchRow* row,
+                                        bool newA) {
+  const uint32_t slot = r % kRunRing;
+  if (row) {
+    ring[2 * slot] = make_int4(row->aRow, row->validRows, row->bRow0, row->nB);
+    ring[2 * slot + 1] = make_int4(row->nTiles, newA ? 1 : 0, (int)(uint32_t)row->state0,
+                                   (int)(uint32_t)((unsigned long long)row->state0 >> 32));
+  } else {
+    ring[2 * slot] = make_int4(0, 0, 0, 0);
+    ring[2 * slot + 1] = make_int4(0, 0, 0, 0);
+  }
+  mbar_arrive(&full[slot]);
+}
 
 // Gathered A blocks (kGather): the producer warp copies each A row from a.aSrc (row
 // a.aSrcRow[entry]) into the 128-byte-swizzled shared layout the TMA would write (16-byte
@@ -339,7 +402,9 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
   extern __shared__ uint8_t smemRaw[];
   Smem<C>& s = *reinterpret_cast<Smem<C>*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  using Cursor = typename std::conditional<kBatch, BatchCursor, WorkCursor>::type;
+  static_assert(C::kStages + C::kAcc + 2 <= kRunRing, "the producer does not lap a reader of the ring of runs");
+  using ProducerCursor = typename std::conditional<kBatch, BatchCursor, WorkCursor>::type;
+  using Cursor = typename std::conditional<kBatch, RunCursor, WorkCursor>::type;
   int nA = 0, nRows = 0;
   TcShape sh{};
   long long w0 = 0, w1 = 0;
@@ -360,8 +425,12 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
     }
     cta_range(sh, w0, w1);
   }
-  auto make_cursor = [&]() -> Cursor {
+  auto producer_cursor = [&]() -> ProducerCursor {
     if constexpr (kBatch) return BatchCursor(a.rows, nRows, a.schedule);
+    else return WorkCursor(w0, w1, sh.nTiles);
+  };
+  auto make_cursor = [&]() -> Cursor {
+    if constexpr (kBatch) return RunCursor(s.runs, s.runFull, &s.abort, a.err, lim);
     else return WorkCursor(w0, w1, sh.nTiles);
   };
 
@@ -376,6 +445,8 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
     }
     for (int i = 0; i < C::kAcc; ++i) mbar_init(&s.accEmpty[i], kEpiWarps);
     mbar_init(&s.mmaDone, kIssuers);
+    if (kBatch)
+      for (int i = 0; i < kRunRing; ++i) mbar_init(&s.runFull[i], 1);
     s.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -430,8 +501,10 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
         return __shfl_sync(0xffffffffu, okl, 0) != 0;
       };
       bool go = true;
-      for (Cursor wc = make_cursor(); wc.more() && go; wc.next()) {
-        if (lane == 0) wc.prefetch_rows();
+      uint32_t r = 0;                    // runs
+      for (ProducerCursor wc = producer_cursor(); wc.more() && go; wc.next()) {
+        if (lane == 0) put_run(s.runs, s.runFull, r, &wc.cur, wc.newA);
+        ++r;
         if (wc.newA) {
           const uint32_t slot = ring_slot<C::kASlots>(j);
           if (!wait_slot(&s.emptyA[slot], ring_parity<C::kASlots>(j) ^ 1)) break;
@@ -455,12 +528,12 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
           }
           cp_async_commit();
           // the next row's entry indices, read now and used at its turn (the loads overlap)
-          if (wc.nxt.aRow != aRow) {
-            preRow = wc.nxt.aRow;
+          if (wc.next_a_row() != aRow) {
+            preRow = wc.next_a_row();
 #pragma unroll
             for (int k = 0; k < C::GM / 32; ++k) {
               const int rr = lane + 32 * k;
-              pre[k] = rr < wc.nxt.validRows ? __ldg(a.aSrcRow + preRow + rr) : -1;
+              pre[k] = rr < wc.next_valid_rows() ? __ldg(a.aSrcRow + preRow + rr) : -1;
             }
           }
           pend[nPend++] = (int)slot;
@@ -481,6 +554,7 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
           }
         }
       }
+      if (lane == 0) put_run(s.runs, s.runFull, r, nullptr, false);
       // every gather has landed (and is handed over) and every load lane 0 issued has landed
       // before the CTA may exit
       arrive_all();
@@ -498,8 +572,9 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
       uint32_t i = 0, j = 0;  // tiles, A blocks
       uint32_t skipped = 0xffffffffu;  // test hook: the tile that was not loaded
       bool go = true;
-      for (Cursor wc = make_cursor(); wc.more() && go; wc.next()) {
-        wc.prefetch_rows();
+      uint32_t r = 0;  // runs
+      for (ProducerCursor wc = producer_cursor(); wc.more() && go; wc.next()) {
+        if constexpr (kBatch) put_run(s.runs, s.runFull, r++, &wc.cur, wc.newA);
         if (wc.newA) {
           const uint32_t slot = ring_slot<C::kASlots>(j);
           if (!mbar_wait(&s.emptyA[slot], ring_parity<C::kASlots>(j) ^ 1, &s.abort, a.err, lim)) break;
@@ -527,6 +602,7 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
           }
         }
       }
+      if constexpr (kBatch) put_run(s.runs, s.runFull, r, nullptr, false);
       // Drain: every load this thread issued has landed before the CTA may exit.
       for (uint32_t k = i > (uint32_t)C::kStages ? i - C::kStages : 0u; k < i; ++k) {
         long long t0c = clock64();
