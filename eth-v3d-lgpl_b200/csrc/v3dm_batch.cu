@@ -82,16 +82,28 @@ constexpr int kChoosePer = 4;     // lefts per thread and step in k_bchoose
 constexpr int kBMutThreads = 256;
 constexpr int kBMutPerBlock = 2048;
 
-// Copies each image's descriptors to its padded place and zeroes its padding rows.
-__global__ void k_bscatter(const uint8_t* __restrict__ src, const long long* __restrict__ srcOff,
-                           const BImage* __restrict__ im, int nImages, uint8_t* __restrict__ dst) {
-  for (int i = blockIdx.x; i < nImages; i += gridDim.x) {
+// Copies each image's descriptors to its padded place and zeroes its padding rows.  Block (x, y):
+// rows 256 x .. of image y, eight loads of a thread in flight (one block per image was bound by its
+// own SM: 24 images 44 us, 200 images 226 us).
+__global__ void __launch_bounds__(256)
+k_bscatter(const uint8_t* __restrict__ src, const long long* __restrict__ srcOff, const BImage* __restrict__ im,
+           int nImages, uint8_t* __restrict__ dst) {
+  constexpr int kQuads = kDescBytes / 16;
+  for (int i = blockIdx.y; i < nImages; i += gridDim.y) {
     const BImage m = im[i];
-    const long long nq = (long long)m.n * (kDescBytes / 16);
-    const long long pq = (long long)((m.n + 255) & ~255) * (kDescBytes / 16);
-    const uint4* s = reinterpret_cast<const uint4*>(src + srcOff[i] * kDescBytes);
-    uint4* d = reinterpret_cast<uint4*>(dst + (size_t)m.rowOff * kDescBytes);
-    for (long long k = threadIdx.x; k < pq; k += blockDim.x) d[k] = k < nq ? s[k] : make_uint4(0u, 0u, 0u, 0u);
+    const int r0 = blockIdx.x * 256;
+    if (r0 >= m.n) continue;  // padding ends with the 256 rows that hold the last descriptor
+    const int valid = min(256, m.n - r0) * kQuads;
+    const uint4* s = reinterpret_cast<const uint4*>(src + (srcOff[i] + r0) * kDescBytes);
+    uint4* d = reinterpret_cast<uint4*>(dst + ((size_t)m.rowOff + r0) * kDescBytes);
+    uint4 v[kQuads];
+#pragma unroll
+    for (int k = 0; k < kQuads; ++k) {
+      const int at = threadIdx.x + 256 * k;
+      v[k] = at < valid ? s[at] : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int k = 0; k < kQuads; ++k) d[threadIdx.x + 256 * k] = v[k];
   }
 }
 
@@ -204,6 +216,7 @@ k_bchoose(const BPair* __restrict__ pairs, int nPairs, const BImage* __restrict_
           int* __restrict__ chosenRight, int* __restrict__ chosenPair, const int* __restrict__ counters, int planes,
           long long srcPlaneRows, long long dstPlaneRows) {
   __shared__ int wsum[kChooseThreads / 32];
+  __shared__ int taken[kChooseThreads * kChoosePer];  // the step's rights, in order
   if (counters[kCntOverflow]) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int p = blockIdx.x; p < nPairs; p += gridDim.x) {
@@ -245,14 +258,19 @@ k_bchoose(const BPair* __restrict__ pairs, int nPairs, const BImage* __restrict_
         chosenLeft[st] = lb + i;
         chosenRight[st] = d[i];
         chosenPair[st] = q.orig;
-        for (int pl = 0; pl < planes; ++pl) {
-          const uint4* src =
-              reinterpret_cast<const uint4*>(img + ((size_t)pl * srcPlaneRows + rRowOff + d[i]) * kDescBytes);
-          uint4* dst = reinterpret_cast<uint4*>(dAB + ((size_t)pl * dstPlaneRows + rowBase + k) * kDescBytes);
-#pragma unroll
-          for (int x = 0; x < kDescBytes / 16; ++x) dst[x] = src[x];
-        }
+        taken[k - run] = d[i];
         ++k;
+      }
+      __syncthreads();
+      // the rows, eight lanes to a block of 128 bytes
+      const int x = threadIdx.x & 7;
+#pragma unroll 4
+      for (int e = threadIdx.x >> 3; e < tot * planes; e += kChooseThreads / 8) {
+        const int t = e / planes, pl = e - t * planes;
+        const uint4* src =
+            reinterpret_cast<const uint4*>(img + ((size_t)pl * srcPlaneRows + rRowOff + taken[t]) * kDescBytes);
+        uint4* dst = reinterpret_cast<uint4*>(dAB + ((size_t)pl * dstPlaneRows + rowBase + run + t) * kDescBytes);
+        dst[x] = src[x];
       }
       run += tot;
       __syncthreads();
@@ -434,48 +452,61 @@ __global__ void k_pcount(const BImage* __restrict__ im, int nImages, const uint8
   }
 }
 
-// Block offsets of the A and B layouts (exclusive prefix sums over (image, cell)).  One block.
+// Block offsets of the A and B layouts (exclusive prefix sums over (image, cell)), and the cursors
+// that k_pscatter takes places from.  One block.
 __global__ void __launch_bounds__(kScanThreads)
 k_pscan_cells(const int* __restrict__ cntA, const int* __restrict__ cntB, int n, int* __restrict__ offA,
-              int* __restrict__ offB) {
+              int* __restrict__ offB, int* __restrict__ curA, int* __restrict__ curB) {
   __shared__ long long sh[kScanThreads];
-  block_scan(n, [&](int i) { return (long long)cntA[i]; }, [&](int i, long long x) { offA[i] = (int)x; }, sh);
-  block_scan(n, [&](int i) { return (long long)cntB[i]; }, [&](int i, long long x) { offB[i] = (int)x; }, sh);
+  block_scan(n, [&](int i) { return (long long)cntA[i]; }, [&](int i, long long x) { offA[i] = curA[i] = (int)x; }, sh);
+  block_scan(n, [&](int i) { return (long long)cntB[i]; }, [&](int i, long long x) { offB[i] = curB[i] = (int)x; }, sh);
 }
 
 // Copies the descriptors into the A and B layouts (order within a block is arbitrary: every
-// result depends on the index maps, not on the order).
-__global__ void k_pscatter(const BImage* __restrict__ im, int nImages, const uint8_t* __restrict__ cell, int probes,
-                           int probesL, int probesR, int C, const int* __restrict__ offA, const int* __restrict__ offB,
-                           const uint8_t* __restrict__ img, uint8_t* __restrict__ la, int* __restrict__ mapA,
-                           uint8_t* __restrict__ lb, int* __restrict__ mapB) {
+// result depends on the index maps, not on the order).  Block (x, y): rows 256 x .. of image y.  It
+// counts its rows per cell, takes the places of each cell with one atomic, and copies each row with
+// eight lanes, read once and written probesL + probesR times.  What bounds it is the writes; one
+// block per image, a thread per row, took 480 us for 60 images of 8000 with 4 + 4 probes, 2.2 GB/ms.
+constexpr int kPScatterRows = 256;
+__global__ void __launch_bounds__(kPScatterRows)
+k_pscatter(const BImage* __restrict__ im, int nImages, const uint8_t* __restrict__ cell, int probes, int probesL,
+           int probesR, int C, int* __restrict__ curA, int* __restrict__ curB, const uint8_t* __restrict__ img,
+           uint8_t* __restrict__ la, int* __restrict__ mapA, uint8_t* __restrict__ lb, int* __restrict__ mapB) {
   extern __shared__ int psSh[];
-  for (int i = blockIdx.x; i < nImages; i += gridDim.x) {
-    for (int t = threadIdx.x; t < 2 * C; t += blockDim.x) psSh[t] = 0;
-    __syncthreads();
+  int* const base = psSh;          // per side and cell: count, then first place
+  int* const pos = psSh + 2 * C;   // per probe and row: place
+  const int tid = threadIdx.x, both = probesL + probesR;
+  for (int i = blockIdx.y; i < nImages; i += gridDim.y) {
     const BImage m = im[i];
-    for (int r = threadIdx.x; r < m.n; r += blockDim.x) {
-      const uint8_t* cr = cell + (size_t)(m.rowOff + r) * probes;
-      const uint4* src = reinterpret_cast<const uint4*>(img + (size_t)(m.rowOff + r) * kDescBytes);
-      uint4 d[kDescBytes / 16];
-#pragma unroll
-      for (int x = 0; x < kDescBytes / 16; ++x) d[x] = src[x];
-      for (int q = 0; q < probesL; ++q) {
-        const int c = cr[q];
-        const int pos = offA[i * C + c] + atomicAdd(&psSh[c], 1);
-        uint4* dst = reinterpret_cast<uint4*>(la + (size_t)pos * kDescBytes);
-#pragma unroll
-        for (int x = 0; x < kDescBytes / 16; ++x) dst[x] = d[x];
-        mapA[pos] = r;
+    const int r0 = blockIdx.x * kPScatterRows, n = min(kPScatterRows, m.n - r0);
+    if (n <= 0) continue;  // uniform over the block
+    for (int t = tid; t < 2 * C; t += kPScatterRows) base[t] = 0;
+    __syncthreads();
+    const uint8_t* cr = cell + (size_t)(m.rowOff + r0 + tid) * probes;
+    if (tid < n)
+      for (int q = 0; q < both; ++q) {
+        const int side = q >= probesL;
+        pos[q * kPScatterRows + tid] = atomicAdd(&base[side * C + cr[side ? q - probesL : q]], 1);
       }
-      for (int q = 0; q < probesR; ++q) {
-        const int c = cr[q];
-        const int pos = offB[i * C + c] + atomicAdd(&psSh[C + c], 1);
-        uint4* dst = reinterpret_cast<uint4*>(lb + (size_t)pos * kDescBytes);
-#pragma unroll
-        for (int x = 0; x < kDescBytes / 16; ++x) dst[x] = d[x];
-        mapB[pos] = r;
+    __syncthreads();
+    for (int t = tid; t < 2 * C; t += kPScatterRows)
+      if (base[t] > 0) base[t] = atomicAdd(t < C ? &curA[i * C + t] : &curB[i * C + t - C], base[t]);
+    __syncthreads();
+    if (tid < n)
+      for (int q = 0; q < both; ++q) {
+        const int side = q >= probesL;
+        const int at = pos[q * kPScatterRows + tid] + base[side * C + cr[side ? q - probesL : q]];
+        pos[q * kPScatterRows + tid] = at;
+        (side ? mapB : mapA)[at] = r0 + tid;
       }
+    __syncthreads();
+    const uint4* src = reinterpret_cast<const uint4*>(img + (size_t)(m.rowOff + r0) * kDescBytes);
+    const int x = tid & 7;
+#pragma unroll 2
+    for (int r = tid >> 3; r < n; r += kPScatterRows / 8) {
+      const uint4 v = src[r * 8 + x];
+      for (int q = 0; q < both; ++q)
+        reinterpret_cast<uint4*>((q >= probesL ? lb : la) + (size_t)pos[q * kPScatterRows + r] * kDescBytes)[x] = v;
     }
     __syncthreads();
   }
@@ -598,12 +629,21 @@ k_pchoose(const BPair* __restrict__ pairs, int nPairs, const long long* __restri
     if (prefC[p + 1] == s0) continue;
     const BPair q = pairs[p];
     int run = 0;
-    for (int l0 = 0; l0 < q.nL; l0 += kChooseThreads) {
-      const int l = l0 + threadIdx.x;
-      const int d = l < q.nL ? decA[q.stateA0 + l] : -1;
-      const bool acc = d >= 0;
-      const unsigned m = __ballot_sync(0xffffffffu, acc);
-      if (lane == 0) wsum[w] = __popc(m);
+    for (int l0 = 0; l0 < q.nL; l0 += kChooseThreads * kChoosePer) {
+      const int lb = l0 + threadIdx.x * kChoosePer;
+      int d[kChoosePer];
+#pragma unroll
+      for (int i = 0; i < kChoosePer; ++i) d[i] = lb + i < q.nL ? decA[q.stateA0 + lb + i] : -1;
+      int c = 0;
+#pragma unroll
+      for (int i = 0; i < kChoosePer; ++i) c += d[i] >= 0;
+      int inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (lane == 31) wsum[w] = inc;
       __syncthreads();
       int before = 0, tot = 0;
 #pragma unroll
@@ -611,12 +651,15 @@ k_pchoose(const BPair* __restrict__ pairs, int nPairs, const long long* __restri
         before += k < w ? wsum[k] : 0;
         tot += wsum[k];
       }
-      if (acc) {
-        const long long st = s0 + run + before + __popc(m & ((1u << lane) - 1u));
-        chosenLeft[st] = l;
-        chosenRight[st] = d;
+      long long st = s0 + run + before + inc - c;
+#pragma unroll
+      for (int i = 0; i < kChoosePer; ++i) {
+        if (d[i] < 0) continue;
+        chosenLeft[st] = lb + i;
+        chosenRight[st] = d[i];
         chosenPair[st] = q.orig;
         chosenSorted[st] = p;
+        ++st;
       }
       run += tot;
       __syncthreads();
@@ -639,12 +682,15 @@ k_pchoose(const BPair* __restrict__ pairs, int nPairs, const long long* __restri
 // lefts that pass A did not accept.  V-left entries are the states grouped by right image (a
 // counting sort); V-right entries are the states themselves, already grouped by left image.
 
-// V-left, pass 1: states per right image.
-__global__ void k_vcount(const BPair* __restrict__ pairs, const int* __restrict__ chosenSorted,
+// V-left, pass 1: states per right image.  A pair's states are consecutive and share its right
+// image, so a pair counts at once.
+__global__ void k_vcount(const BPair* __restrict__ pairs, int nPairs, const long long* __restrict__ prefC,
                          const int* __restrict__ counters, int* __restrict__ cntJ) {
-  const int n = counters[kCntStates];  // 0 after a state overflow
-  for (int st = blockIdx.x * blockDim.x + threadIdx.x; st < n; st += gridDim.x * blockDim.x)
-    atomicAdd(&cntJ[pairs[chosenSorted[st]].ri], 1);
+  if (counters[kCntStates] == 0) return;  // 0 after a state overflow
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nPairs; p += gridDim.x * blockDim.x) {
+    const int c = (int)(prefC[p + 1] - prefC[p]);
+    if (c > 0) atomicAdd(&cntJ[pairs[p].ri], c);
+  }
 }
 
 // Entry offsets per right image and row starts of both verification passes (exclusive prefix
@@ -680,17 +726,27 @@ k_vscan(const int* __restrict__ cntJ, const BImage* __restrict__ im, int nImages
 }
 
 // V-left, pass 2: every state's entry (its left's descriptor row in the image buffer), grouped
-// by right image.  Counts cntJ down to zero for the next call.
-__global__ void k_vscatter(const BPair* __restrict__ pairs, const BImage* __restrict__ im,
-                           const int* __restrict__ chosenLeft, const int* __restrict__ chosenSorted,
+// by right image: a warp per pair takes the places of the pair's states with one atomic (an atomic
+// per state, on as many addresses as there are images, took 115 us for 430000 states, and as much
+// again in pass 1).  Counts cntJ down to zero for the next call.
+__global__ void k_vscatter(const BPair* __restrict__ pairs, const BImage* __restrict__ im, int nPairs,
+                           const long long* __restrict__ prefC, const int* __restrict__ chosenLeft,
                            const int* __restrict__ counters, const int* __restrict__ offJ, int* __restrict__ cntJ,
                            int* __restrict__ srcRow, int* __restrict__ stateOf) {
-  const int n = counters[kCntStates];
-  for (int st = blockIdx.x * blockDim.x + threadIdx.x; st < n; st += gridDim.x * blockDim.x) {
-    const BPair q = pairs[chosenSorted[st]];
-    const int pos = offJ[q.ri] + atomicSub(&cntJ[q.ri], 1) - 1;
-    srcRow[pos] = im[q.li].rowOff + chosenLeft[st];
-    stateOf[pos] = st;
+  if (counters[kCntStates] == 0) return;
+  const int lane = threadIdx.x & 31;
+  for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < nPairs; p += (gridDim.x * blockDim.x) >> 5) {
+    const int s0 = (int)prefC[p], c = (int)prefC[p + 1] - s0;
+    if (c == 0) continue;
+    const BPair q = pairs[p];
+    int pos = 0;
+    if (lane == 0) pos = offJ[q.ri] + atomicSub(&cntJ[q.ri], c) - c;
+    pos = __shfl_sync(0xffffffffu, pos, 0);
+    const int row0 = im[q.li].rowOff;
+    for (int k = lane; k < c; k += 32) {
+      srcRow[pos + k] = row0 + chosenLeft[s0 + k];
+      stateOf[pos + k] = s0 + k;
+    }
   }
 }
 
@@ -851,6 +907,8 @@ struct v3dm_batch {
   int* dCntB = nullptr;
   int* dOffA = nullptr;
   int* dOffB = nullptr;
+  int* dCurA = nullptr;
+  int* dCurB = nullptr;
   long long cellTabCap = 0;
   uint8_t* dLA = nullptr;           // A layout: every descriptor once per probed cell
   long long laCap = 0;              // bytes
@@ -1463,16 +1521,20 @@ int prepare_proposal(v3dm_batch* b, int probesL, int probesR, int C) {
   V3DM_BTRY(ensure(&b->dCell, &b->cellCap, std::max<long long>(b->totalRows, 1) * probes));
   const long long tab = (long long)std::max(b->nImages, 1) * C;
   if (tab > b->cellTabCap) {
-    long long c0 = 0, c1 = 0, c2 = 0, c3 = 0;
+    long long c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0, c5 = 0;
     bfree(b->dCntA);
     bfree(b->dCntB);
     bfree(b->dOffA);
     bfree(b->dOffB);
+    bfree(b->dCurA);
+    bfree(b->dCurB);
     b->cellTabCap = 0;
     V3DM_BTRY(ensure(&b->dCntA, &c0, tab));
     V3DM_BTRY(ensure(&b->dCntB, &c1, tab));
     V3DM_BTRY(ensure(&b->dOffA, &c2, tab));
     V3DM_BTRY(ensure(&b->dOffB, &c3, tab));
+    V3DM_BTRY(ensure(&b->dCurA, &c4, tab));
+    V3DM_BTRY(ensure(&b->dCurB, &c5, tab));
     b->cellTabCap = tab;
   }
   V3DM_BTRY(ensure(&b->dLA, &b->laCap, laRows * kDescBytes));
@@ -1556,11 +1618,13 @@ int enqueue_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL, in
   k_pcount<<<imgGrid, 256, 2 * C * sizeof(int), b->stream>>>(b->dImages, nI, b->dCell, probes, probesL, probesR, C,
                                                              b->dCntA, b->dCntB);
   V3DM_BTRY(cudaGetLastError());
-  k_pscan_cells<<<1, kScanThreads, 0, b->stream>>>(b->dCntA, b->dCntB, nI * C, b->dOffA, b->dOffB);
+  k_pscan_cells<<<1, kScanThreads, 0, b->stream>>>(b->dCntA, b->dCntB, nI * C, b->dOffA, b->dOffB, b->dCurA, b->dCurB);
   V3DM_BTRY(cudaGetLastError());
-  k_pscatter<<<imgGrid, 256, 2 * C * sizeof(int), b->stream>>>(b->dImages, nI, b->dCell, probes, probesL, probesR, C,
-                                                               b->dOffA,
-                                                               b->dOffB, b->dImg, b->dLA, b->dMapA, b->dLB, b->dMapB);
+  const int mostRows = nI > 0 ? *std::max_element(b->counts.begin(), b->counts.end()) : 0;
+  const dim3 scatterGrid(std::max(1, (mostRows + kPScatterRows - 1) / kPScatterRows), std::max(1, std::min(nI, 65535)));
+  k_pscatter<<<scatterGrid, kPScatterRows, (2 * C + (probesL + probesR) * kPScatterRows) * sizeof(int), b->stream>>>(
+      b->dImages, nI, b->dCell, probes, probesL, probesR, C, b->dCurA, b->dCurB, b->dImg, b->dLA, b->dMapA, b->dLB,
+      b->dMapB);
   V3DM_BTRY(cudaGetLastError());
   const int unitGrid = std::max(1, std::min((nI * C + 7) / 8, 4 * 148));
   k_prowcount<<<unitGrid, 256, 0, b->stream>>>(b->dPairs, b->dImages, nI, C, GM, b->dCntA, b->dCntB, b->dRowCnt,
@@ -1625,13 +1689,15 @@ int enqueue_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL, in
   const int GR = tc_gather_rows(), BNG = tc_gather_cols();
   const int stateGrid = 4 * 148;
   const int imgBlocks = std::max(1, (nI + 255) / 256);
-  k_vcount<<<stateGrid, 256, 0, b->stream>>>(b->dPairs, b->dChosenSorted, b->dCounters, b->dCntE);
+  k_vcount<<<std::max(1, std::min((b->nPairs + 255) / 256, stateGrid)), 256, 0, b->stream>>>(
+      b->dPairs, b->nPairs, b->dPrefC, b->dCounters, b->dCntE);
   V3DM_BTRY(cudaGetLastError());
   k_vscan<<<1, kScanThreads, 0, b->stream>>>(b->dCntE, b->dImages, nI, b->dPrefC, GR, b->rowsPBCap, b->dOffE,
                                              b->dRowStartE, b->dRowStartR, b->dCounters);
   V3DM_BTRY(cudaGetLastError());
-  k_vscatter<<<stateGrid, 256, 0, b->stream>>>(b->dPairs, b->dImages, b->dChosenLeft, b->dChosenSorted, b->dCounters,
-                                               b->dOffE, b->dCntE, b->dSrcRowE, b->dStateE);
+  k_vscatter<<<std::max(1, std::min((b->nPairs + 7) / 8, stateGrid)), 256, 0, b->stream>>>(
+      b->dPairs, b->dImages, b->nPairs, b->dPrefC, b->dChosenLeft, b->dCounters, b->dOffE, b->dCntE, b->dSrcRowE,
+      b->dStateE);
   V3DM_BTRY(cudaGetLastError());
   k_vrows_left<<<imgBlocks, 256, 0, b->stream>>>(b->dImages, nI, GR, BNG, b->dOffE, b->dRowStartE, b->dCounters,
                                                  b->dRowsPB);
@@ -1802,6 +1868,8 @@ void free_all(v3dm_batch* b) {
   bfree(b->dCntB);
   bfree(b->dOffA);
   bfree(b->dOffB);
+  bfree(b->dCurA);
+  bfree(b->dCurB);
   bfree(b->dLA);
   bfree(b->dMapA);
   bfree(b->dLB);
@@ -1845,8 +1913,17 @@ void set_float_mode(v3dm_batch* b, bool on) {
   b->fMapsValid = false;
 }
 
-// Layout of the images: padded row offsets, per-image table.
-int set_images(v3dm_batch* b, int nImages, const int32_t* counts, const uint8_t* desc, bool onDevice) {
+cudaError_t launch_bscatter(v3dm_batch* b, const uint8_t* src, int nImages) {
+  const int most = *std::max_element(b->counts.begin(), b->counts.end());
+  const dim3 grid((most + 255) / 256, std::min(nImages, 65535));
+  k_bscatter<<<grid, 256, 0, b->stream>>>(src, b->dSrcOff, b->dImages, nImages, b->dImg);
+  return cudaGetLastError();
+}
+
+// Layout of the images: padded row offsets, per-image table.  With scatter false the descriptors
+// themselves are not copied (float images, whose own layout follows).
+int set_images(v3dm_batch* b, int nImages, const int32_t* counts, const uint8_t* desc, bool onDevice,
+               bool scatter = true) {
   if (!b || nImages < 0 || (nImages > 0 && !counts)) return V3DM_ERR_ARG;
   long long total = 0, rows = 0;
   for (int i = 0; i < nImages; ++i) {
@@ -1865,15 +1942,14 @@ int set_images(v3dm_batch* b, int nImages, const int32_t* counts, const uint8_t*
   // valid, only the descriptors change (the graph reads them from the same buffer).
   const bool sameLayout = b->haveImages && nImages == b->nImages && std::equal(counts, counts + nImages, b->counts.begin());
   if (sameLayout) {
-    if (total > 0) {
+    if (total > 0 && scatter) {
       const uint8_t* src = desc;
       if (!onDevice) {
         V3DM_BTRY(ensure(&b->dStage, &b->stageCap, total * kDescBytes));
         V3DM_BTRY(cudaMemcpyAsync(b->dStage, desc, (size_t)total * kDescBytes, cudaMemcpyHostToDevice, b->stream));
         src = b->dStage;
       }
-      k_bscatter<<<std::min(nImages, 1024), 256, 0, b->stream>>>(src, b->dSrcOff, b->dImages, nImages, b->dImg);
-      V3DM_BTRY(cudaGetLastError());
+      V3DM_BTRY(launch_bscatter(b, src, nImages));
     }
     V3DM_BTRY(cudaStreamSynchronize(b->stream));
     return V3DM_OK;
@@ -1914,15 +1990,14 @@ int set_images(v3dm_batch* b, int nImages, const int32_t* counts, const uint8_t*
     V3DM_BTRY(cudaMemcpyAsync(b->dImages, b->bim.data(), (size_t)nImages * sizeof(BImage), cudaMemcpyHostToDevice,
                               b->stream));
   }
-  if (total > 0) {
+  if (total > 0 && scatter) {
     const uint8_t* src = desc;
     if (!onDevice) {
       V3DM_BTRY(ensure(&b->dStage, &b->stageCap, total * kDescBytes));
       V3DM_BTRY(cudaMemcpyAsync(b->dStage, desc, (size_t)total * kDescBytes, cudaMemcpyHostToDevice, b->stream));
       src = b->dStage;
     }
-    k_bscatter<<<std::min(nImages, 1024), 256, 0, b->stream>>>(src, b->dSrcOff, b->dImages, nImages, b->dImg);
-    V3DM_BTRY(cudaGetLastError());
+    V3DM_BTRY(launch_bscatter(b, src, nImages));
   }
   V3DM_BTRY(cudaStreamSynchronize(b->stream));  // host vectors and the caller's buffer may change after return
   b->haveImages = true;
@@ -1966,7 +2041,7 @@ int set_images_f32(v3dm_batch* b, int nImages, const int32_t* counts, const floa
     V3DM_BTRY(cudaMemsetAsync(err, 0, sizeof(int32_t), b->stream));
   }
   // the layout (and, for exact descriptors, the integer operand) from the uint8 staging buffer
-  int st = set_images(b, nImages, counts, total > 0 ? b->dStage : nullptr, true);
+  int st = set_images(b, nImages, counts, total > 0 ? b->dStage : nullptr, true, exact);
   if (st != V3DM_OK) return st;
   if (exact) {
     set_float_mode(b, false);

@@ -170,15 +170,26 @@ __device__ __forceinline__ uint32_t f32_to_u8_checked(float v, bool& ok) {
   return (uint32_t)(u & 255);
 }
 
-__global__ void k_f32_to_u8(const float4* __restrict__ src, uint32_t* __restrict__ dst, long long n4, int* err) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n4) return;
-  float4 v = src[i];
+// Four float4 of a thread in flight.  Once some value is known not to be of the form u/512 the result
+// is of no use (the caller takes the float path), so blocks that start later leave at once, and a
+// warp reports with one atomic: 180000 such descriptors took 130 us with an atomic per thread.
+constexpr int kF32PerThread = 4;
+__global__ void __launch_bounds__(256)
+k_f32_to_u8(const float4* __restrict__ src, uint32_t* __restrict__ dst, long long n4, int* err) {
+  if (__any_sync(0xffffffffu, *(volatile const int*)err & kErrNotU8)) return;
+  const long long i0 = (long long)blockIdx.x * (256 * kF32PerThread) + threadIdx.x;
+  float4 v[kF32PerThread];
+#pragma unroll
+  for (int k = 0; k < kF32PerThread; ++k)
+    v[k] = i0 + 256 * k < n4 ? src[i0 + 256 * k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   bool ok = true;
-  uint32_t w = f32_to_u8_checked(v.x, ok) | (f32_to_u8_checked(v.y, ok) << 8) | (f32_to_u8_checked(v.z, ok) << 16) |
-               (f32_to_u8_checked(v.w, ok) << 24);
-  dst[i] = w;
-  if (!ok) atomicOr(err, kErrNotU8);
+#pragma unroll
+  for (int k = 0; k < kF32PerThread; ++k) {
+    const uint32_t w = f32_to_u8_checked(v[k].x, ok) | (f32_to_u8_checked(v[k].y, ok) << 8) |
+                       (f32_to_u8_checked(v[k].z, ok) << 16) | (f32_to_u8_checked(v[k].w, ok) << 24);
+    if (i0 + 256 * k < n4) dst[i0 + 256 * k] = w;
+  }
+  if (__any_sync(0xffffffffu, !ok) && (threadIdx.x & 31) == 0) atomicOr(err, kErrNotU8);
 }
 
 }  // namespace
@@ -217,7 +228,8 @@ cudaError_t launch_gate_precompute(int type, const double* m, const float* dLPos
 cudaError_t launch_f32_to_u8(const float* src, uint8_t* dst, int n, int* err, cudaStream_t s) {
   long long n4 = (long long)n * (kDescBytes / 4);
   if (n4 == 0) return cudaSuccess;
-  k_f32_to_u8<<<(unsigned)((n4 + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float4*>(src),
+  constexpr int kPerBlock = 256 * kF32PerThread;
+  k_f32_to_u8<<<(unsigned)((n4 + kPerBlock - 1) / kPerBlock), 256, 0, s>>>(reinterpret_cast<const float4*>(src),
                                                             reinterpret_cast<uint32_t*>(dst), n4, err);
   return cudaGetLastError();
 }
