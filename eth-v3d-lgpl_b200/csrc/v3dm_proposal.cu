@@ -18,6 +18,7 @@
 // Flat parameter layout (V3DM_PROJ_PARAMS floats): W1 [64][128], b1 [64], W2 [32][64], b2 [32].
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -37,122 +38,220 @@ static_assert(kParams == V3DM_PROJ_PARAMS, "parameter count");
 constexpr int kFwdThreads = 128;
 constexpr float kNormEps = 1e-12f;
 
-// One thread per descriptor.  The weights are read from shared memory as FP32 values of the
-// BF16 weights; the hidden layer is accumulated k-outer so the descriptor is unpacked once.
-// Training stores the hidden activations, the normalised output and the norm; inference may
-// instead (or also) assign the descriptor to its 'probes' best cells.
+// Two sums at once: fma.rn.f32x2 rounds each half as fmaf does.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(F2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+constexpr int kCellStep = 8;  // cells scored at a time
+
+// kPer descriptors per thread (every sum in the same order whatever kPer).  The weights are read from
+// shared memory as FP32 values of the BF16 weights; the hidden layer is accumulated k-outer so the
+// descriptor is unpacked once.  Training stores the hidden activations, the normalised output and the
+// norm; inference may instead (or also) assign the descriptor to its 'probes' best cells
+// (probes <= kProbes).
+// What bounds it: 14000 FMAs per descriptor with 128 cells (190 us for 480000), a shared load for every
+// four of them and the sorted list's compares and selects.  Pairs of sums (f32x2) halve the FMAs' issue,
+// the list has four or eight places by what is asked for, bytes become floats through the mantissa:
+// 607 -> 499 us, 87% of the shared-memory rate.  Two descriptors per thread halve the shared loads:
+// 430 us (without the pairs of sums they were slower, 640 us).
+template <int kProbes, int kPer>
 __global__ void __launch_bounds__(kFwdThreads)
 k_proj_forward(const uint8_t* __restrict__ x, int n, const __nv_bfloat16* __restrict__ w1b, const float* __restrict__ b1,
                const __nv_bfloat16* __restrict__ w2b, const float* __restrict__ b2, float* __restrict__ hOut,
                float* __restrict__ zOut, float* __restrict__ normOut, const float* __restrict__ cells, int nCells,
                int probes, uint8_t* __restrict__ cellOut) {
   extern __shared__ float4 projSmem[];
-  auto sW1 = reinterpret_cast<float4(*)[kHid / 4]>(projSmem);                 // W1[:, k] per k, 32 KB
-  auto sW2 = reinterpret_cast<float4(*)[kOut / 4]>(projSmem + kIn * kHid / 4);  // W2[:, j] per j, 8 KB
-  auto sC = reinterpret_cast<float4(*)[kOut / 4]>(projSmem + kIn * kHid / 4 + kHid * kOut / 4);
-  float* sB1 = reinterpret_cast<float*>(projSmem + kIn * kHid / 4 + kHid * kOut / 4 + V3DM_PROJ_MAX_CELLS * kOut / 4);
+  auto sW1 = reinterpret_cast<ulonglong2(*)[kHid / 4]>(projSmem);                 // W1[:, k] per k, 32 KB
+  auto sW2 = reinterpret_cast<ulonglong2(*)[kOut / 4]>(projSmem + kIn * kHid / 4);  // W2[:, j] per j, 8 KB
+  float* sC = reinterpret_cast<float*>(projSmem + kIn * kHid / 4 + kHid * kOut / 4);  // cells[:, o] per o
+  float* sB1 = sC + V3DM_PROJ_MAX_CELLS * kOut;
   float* sB2 = sB1 + kHid;
-  for (int i = threadIdx.x; i < kHid * kIn; i += kFwdThreads) {
-    const int j = i / kIn, k = i % kIn;  // W1[j][k]
-    reinterpret_cast<float*>(sW1)[k * kHid + j] = __bfloat162float(w1b[i]);
+  const int cellPitch = (nCells + kCellStep - 1) / kCellStep * kCellStep;
+  for (int i = threadIdx.x; i < kHid * kIn; i += kFwdThreads) {  // consecutive threads write consecutive words
+    const int j = i % kHid, k = i / kHid;  // W1[j][k]
+    reinterpret_cast<float*>(sW1)[i] = __bfloat162float(w1b[j * kIn + k]);
   }
   for (int i = threadIdx.x; i < kOut * kHid; i += kFwdThreads) {
-    const int o = i / kHid, j = i % kHid;  // W2[o][j]
-    reinterpret_cast<float*>(sW2)[j * kOut + o] = __bfloat162float(w2b[i]);
+    const int o = i % kOut, j = i / kOut;  // W2[o][j]
+    reinterpret_cast<float*>(sW2)[i] = __bfloat162float(w2b[o * kHid + j]);
   }
   if (threadIdx.x < kHid) sB1[threadIdx.x] = b1[threadIdx.x];
   if (threadIdx.x < kOut) sB2[threadIdx.x] = b2[threadIdx.x];
-  for (int i = threadIdx.x; i < nCells * kOut; i += kFwdThreads) reinterpret_cast<float*>(sC)[i] = cells[i];
+  for (int i = threadIdx.x; i < cellPitch * kOut; i += kFwdThreads) {
+    const int o = i / cellPitch, c = i - o * cellPitch;
+    sC[i] = c < nCells ? cells[c * kOut + o] : 0.0f;
+  }
   __syncthreads();
-  for (int d = blockIdx.x * kFwdThreads + threadIdx.x; d < n; d += gridDim.x * kFwdThreads) {
-    float h[kHid];
+  constexpr int kTile = kFwdThreads * kPer;
+  for (long long d0 = (long long)blockIdx.x * kTile + threadIdx.x; d0 < n; d0 += (long long)gridDim.x * kTile) {
+    // descriptors d0, d0 + kFwdThreads; one past the end is the last one again and stores nothing
+    int d[kPer];
+    bool in[kPer];
 #pragma unroll
-    for (int j = 0; j < kHid; ++j) h[j] = sB1[j];
-    const uint4* xd = reinterpret_cast<const uint4*>(x + (size_t)d * kIn);
+    for (int p = 0; p < kPer; ++p) {
+      in[p] = d0 + p * kFwdThreads < n;
+      d[p] = (int)min(d0 + p * kFwdThreads, (long long)n - 1);
+    }
+    F2 h[kPer][kHid / 2];
+#pragma unroll
+    for (int j = 0; j < kHid / 2; ++j)
+#pragma unroll
+      for (int p = 0; p < kPer; ++p) h[p][j] = f2_pack(sB1[2 * j], sB1[2 * j + 1]);
 #pragma unroll 1
     for (int q = 0; q < kIn / 16; ++q) {
-      const uint4 xw = __ldg(xd + q);
-      const uint32_t words[4] = {xw.x, xw.y, xw.z, xw.w};
+      uint32_t words[kPer][4];
+#pragma unroll
+      for (int p = 0; p < kPer; ++p) {
+        const uint4 xw = __ldg(reinterpret_cast<const uint4*>(x + (size_t)d[p] * kIn) + q);
+        words[p][0] = xw.x, words[p][1] = xw.y, words[p][2] = xw.z, words[p][3] = xw.w;
+      }
 #pragma unroll
       for (int wi = 0; wi < 4; ++wi) {
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
           const int k = q * 16 + wi * 4 + b;
-          const float xk = (float)((words[wi] >> (8 * b)) & 255u) * (1.0f / 512.0f);
+          F2 x2[kPer];
+#pragma unroll
+          for (int p = 0; p < kPer; ++p) {
+            // (2^23 + u) / 512 - 2^23 / 512 = u / 512, exactly
+            const float m = __uint_as_float(__byte_perm(words[p][wi], 0x4b000000u, 0x7440u + (uint32_t)b));
+            const float xk = fmaf(m, 1.0f / 512.0f, -16384.0f);
+            x2[p] = f2_pack(xk, xk);
+          }
 #pragma unroll
           for (int j4 = 0; j4 < kHid / 4; ++j4) {
-            const float4 w = sW1[k][j4];
-            h[4 * j4 + 0] = fmaf(w.x, xk, h[4 * j4 + 0]);
-            h[4 * j4 + 1] = fmaf(w.y, xk, h[4 * j4 + 1]);
-            h[4 * j4 + 2] = fmaf(w.z, xk, h[4 * j4 + 2]);
-            h[4 * j4 + 3] = fmaf(w.w, xk, h[4 * j4 + 3]);
+            const ulonglong2 w = sW1[k][j4];
+#pragma unroll
+            for (int p = 0; p < kPer; ++p) {
+              h[p][2 * j4] = f2_fma(w.x, x2[p], h[p][2 * j4]);
+              h[p][2 * j4 + 1] = f2_fma(w.y, x2[p], h[p][2 * j4 + 1]);
+            }
           }
         }
       }
     }
-    float z[kOut];
+    F2 z2[kPer][kOut / 2];
 #pragma unroll
-    for (int o = 0; o < kOut; ++o) z[o] = sB2[o];
+    for (int o = 0; o < kOut / 2; ++o)
+#pragma unroll
+      for (int p = 0; p < kPer; ++p) z2[p][o] = f2_pack(sB2[2 * o], sB2[2 * o + 1]);
 #pragma unroll
     for (int j = 0; j < kHid; ++j) {
-      const float hj = fmaxf(h[j], 0.0f);
-      if (hOut) hOut[(size_t)d * kHid + j] = hj;
+      F2 hj2[kPer];
+#pragma unroll
+      for (int p = 0; p < kPer; ++p) {
+        const float2 hp = f2_unpack(h[p][j / 2]);
+        const float hj = fmaxf(j & 1 ? hp.y : hp.x, 0.0f);
+        if (hOut && in[p]) hOut[(size_t)d[p] * kHid + j] = hj;
+        hj2[p] = f2_pack(hj, hj);
+      }
 #pragma unroll
       for (int o4 = 0; o4 < kOut / 4; ++o4) {
-        const float4 w = sW2[j][o4];
-        z[4 * o4 + 0] = fmaf(w.x, hj, z[4 * o4 + 0]);
-        z[4 * o4 + 1] = fmaf(w.y, hj, z[4 * o4 + 1]);
-        z[4 * o4 + 2] = fmaf(w.z, hj, z[4 * o4 + 2]);
-        z[4 * o4 + 3] = fmaf(w.w, hj, z[4 * o4 + 3]);
+        const ulonglong2 w = sW2[j][o4];
+#pragma unroll
+        for (int p = 0; p < kPer; ++p) {
+          z2[p][2 * o4] = f2_fma(w.x, hj2[p], z2[p][2 * o4]);
+          z2[p][2 * o4 + 1] = f2_fma(w.y, hj2[p], z2[p][2 * o4 + 1]);
+        }
       }
     }
-    float ss = 0.0f;
+    float z[kPer][kOut];
 #pragma unroll
-    for (int o = 0; o < kOut; ++o) ss = fmaf(z[o], z[o], ss);
-    const float nrm = sqrtf(ss);
-    const float inv = 1.0f / fmaxf(nrm, kNormEps);
+    for (int p = 0; p < kPer; ++p) {
 #pragma unroll
-    for (int o = 0; o < kOut; ++o) z[o] *= inv;
-    if (normOut) normOut[d] = nrm;
-    if (zOut) {
-      float4* zo = reinterpret_cast<float4*>(zOut + (size_t)d * kOut);
+      for (int o = 0; o < kOut / 2; ++o) {
+        const float2 v = f2_unpack(z2[p][o]);
+        z[p][2 * o] = v.x;
+        z[p][2 * o + 1] = v.y;
+      }
+      float ss = 0.0f;
 #pragma unroll
-      for (int o4 = 0; o4 < kOut / 4; ++o4) zo[o4] = make_float4(z[4 * o4], z[4 * o4 + 1], z[4 * o4 + 2], z[4 * o4 + 3]);
+      for (int o = 0; o < kOut; ++o) ss = fmaf(z[p][o], z[p][o], ss);
+      const float nrm = sqrtf(ss);
+      const float inv = 1.0f / fmaxf(nrm, kNormEps);
+#pragma unroll
+      for (int o = 0; o < kOut; ++o) z[p][o] *= inv;
+      if (normOut && in[p]) normOut[d[p]] = nrm;
+      if (zOut && in[p]) {
+        float4* zo = reinterpret_cast<float4*>(zOut + (size_t)d[p] * kOut);
+#pragma unroll
+        for (int o4 = 0; o4 < kOut / 4; ++o4)
+          zo[o4] = make_float4(z[p][4 * o4], z[p][4 * o4 + 1], z[p][4 * o4 + 2], z[p][4 * o4 + 3]);
+      }
     }
     if (cellOut) {
       // the 'probes' best cells by z . c, in order; ties keep the lower cell
-      float bs[V3DM_PROJ_MAX_PROBES];
-      int bc[V3DM_PROJ_MAX_PROBES];
+      float bs[kPer][kProbes];
+      int bc[kPer][kProbes];
 #pragma unroll
-      for (int i = 0; i < V3DM_PROJ_MAX_PROBES; ++i) {
-        bs[i] = -INFINITY;
-        bc[i] = 0;
-      }
-      for (int c = 0; c < nCells; ++c) {
-        float s = 0.0f;
+      for (int p = 0; p < kPer; ++p)
 #pragma unroll
-        for (int o4 = 0; o4 < kOut / 4; ++o4) {
-          const float4 w = sC[c][o4];
-          s = fmaf(w.x, z[4 * o4], s);
-          s = fmaf(w.y, z[4 * o4 + 1], s);
-          s = fmaf(w.z, z[4 * o4 + 2], s);
-          s = fmaf(w.w, z[4 * o4 + 3], s);
+        for (int i = 0; i < kProbes; ++i) {
+          bs[p][i] = -INFINITY;
+          bc[p][i] = 0;
         }
-        // insertion into the sorted top list (strict '>' keeps earlier cells first on ties)
-        int cc = c;
+      for (int c0 = 0; c0 < nCells; c0 += kCellStep) {
+        F2 s2[kPer][kCellStep / 2];
 #pragma unroll
-        for (int i = 0; i < V3DM_PROJ_MAX_PROBES; ++i) {
-          if (i < probes && s > bs[i]) {
-            const float ts = bs[i];
-            const int tc = bc[i];
-            bs[i] = s;
-            bc[i] = cc;
-            s = ts;
-            cc = tc;
+        for (int p = 0; p < kPer; ++p)
+#pragma unroll
+          for (int i = 0; i < kCellStep / 2; ++i) s2[p][i] = 0ull;
+#pragma unroll
+        for (int o = 0; o < kOut; ++o) {
+          const ulonglong2* w = reinterpret_cast<const ulonglong2*>(sC + o * cellPitch + c0);
+#pragma unroll
+          for (int i = 0; i < kCellStep / 4; ++i) {
+            const ulonglong2 wv = w[i];
+#pragma unroll
+            for (int p = 0; p < kPer; ++p) {
+              const F2 zo = f2_pack(z[p][o], z[p][o]);
+              s2[p][2 * i] = f2_fma(wv.x, zo, s2[p][2 * i]);
+              s2[p][2 * i + 1] = f2_fma(wv.y, zo, s2[p][2 * i + 1]);
+            }
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < kCellStep; ++t) {
+          if (c0 + t >= nCells) break;
+#pragma unroll
+          for (int p = 0; p < kPer; ++p) {
+            const float2 sp = f2_unpack(s2[p][t / 2]);
+            float s = t & 1 ? sp.y : sp.x;
+            // insertion into the sorted top list (strict '>' keeps earlier cells first on ties)
+            int cc = c0 + t;
+#pragma unroll
+            for (int i = 0; i < kProbes; ++i) {
+              if (s > bs[p][i]) {
+                const float ts = bs[p][i];
+                const int tc = bc[p][i];
+                bs[p][i] = s;
+                bc[p][i] = cc;
+                s = ts;
+                cc = tc;
+              }
+            }
           }
         }
       }
-      for (int i = 0; i < probes; ++i) cellOut[(size_t)d * probes + i] = (uint8_t)bc[i];
+#pragma unroll
+      for (int p = 0; p < kPer; ++p)
+#pragma unroll
+        for (int i = 0; i < kProbes; ++i)
+          if (i < probes && in[p]) cellOut[(size_t)d[p] * probes + i] = (uint8_t)bc[p][i];
     }
   }
 }
@@ -169,15 +268,23 @@ cudaError_t launch_forward(const uint8_t* x, long long n, const __nv_bfloat16* w
   if (e0 != cudaSuccess) return e0;
   if (dev < 0 || dev >= 128) return cudaErrorInvalidDevice;
   if (!attrSet[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_proj_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
+    cudaError_t e = cudaSuccess;
+    for (auto f : {k_proj_forward<4, 1>, k_proj_forward<4, 2>, k_proj_forward<V3DM_PROJ_MAX_PROBES, 1>,
+                   k_proj_forward<V3DM_PROJ_MAX_PROBES, 2>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
     if (e != cudaSuccess) return e;
     attrSet[dev] = true;
   }
   if (n <= 0) return cudaSuccess;
-  long long blocks = (n + kFwdThreads - 1) / kFwdThreads;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  k_proj_forward<<<(unsigned)blocks, kFwdThreads, kFwdSmem, s>>>(x, (int)n, w1b, b1, w2b, b2, hOut, zOut, normOut,
-                                                                 cells, nCells, probes, cellOut);
+  // Two descriptors per thread once that still gives every SM the two blocks it holds; below that more
+  // threads matter more.  As many blocks as are resident at once: each stages the weights.
+  const bool two = n >= 148LL * 2 * 2 * kFwdThreads;
+  const int tile = kFwdThreads * (two ? 2 : 1);
+  const long long blocks = std::min((n + tile - 1) / tile, 148LL * (two ? 2 : 3));
+  auto f = probes <= 4 ? (two ? k_proj_forward<4, 2> : k_proj_forward<4, 1>)
+                       : (two ? k_proj_forward<V3DM_PROJ_MAX_PROBES, 2> : k_proj_forward<V3DM_PROJ_MAX_PROBES, 1>);
+  f<<<(unsigned)blocks, kFwdThreads, kFwdSmem, s>>>(x, (int)n, w1b, b1, w2b, b2, hOut, zOut, normOut, cells, nCells,
+                                                    probes, cellOut);
   return cudaGetLastError();
 }
 
