@@ -52,8 +52,11 @@ static_assert(kFABase + kFGroups * kFACols <= kFTmemCols, "accumulators and the 
 constexpr int kFEpiWarp0 = 2;
 constexpr int kFThreads = (kFEpiWarp0 + 4 * kFGroups) * 32;
 
+constexpr int kFWait = 16;  // guided: scores a lane keeps until their gates are tested together
+
 struct SmemF {
   uint8_t b[kFStages][kFStageBytes];
+  uint2 waiting[4 * kFGroups][kFWait][32];  // score and column, per epilogue warp, place and lane
   unsigned long long full[kFStages], empty[kFStages];
   unsigned long long accFull[kFGroups], accEmpty[kFGroups];
   unsigned long long mmaDone;
@@ -171,17 +174,16 @@ struct GateLane {
   int type, aIsLeft;
 };
 
-// Whether the gate masks (A descriptor of the lane, column col of the B image).  Called only for
-// scores that could enter the lane's top two, so it stays out of line.
-__device__ __noinline__ bool gate_rejects_col(GateLane gl, int col) {
+// Whether the gate masks (A descriptor of the lane, column col of the B image).
+__device__ __forceinline__ bool gate_rejects_col(GateLane gl, int col) {
   const float2 pb = gl.bPos[col];
   if (gl.aIsLeft) return gate_rejects_terms(gl.type, gl.m[9], gl.aT, gate_right_terms(gl.type, gl.m, pb));
   return gate_rejects_terms(gl.type, gl.m[9], gate_left_terms(gl.type, gl.m, pb), gl.aT);
 }
 
 // Whether any of the single-pair matcher's gates (compounding since the last putative call) masks
-// (left l, right r); out of line for the same reason.
-__device__ __noinline__ bool gates_reject(const GateParams* gates, int n, int l, int r) {
+// (left l, right r).
+__device__ __forceinline__ bool gates_reject(const GateParams* gates, int n, int l, int r) {
   for (int g = 0; g < n; ++g)
     if (gate_rejects(gates[g], l, r)) return true;
   return false;
@@ -198,7 +200,8 @@ __device__ __noinline__ bool gates_reject(const GateParams* gates, int n, int l,
 // Before, with 128-row groups and the hi planes stored twice (96 KB of L2 reads per block and tile
 // against 32), a lane-0 issuer (145 cycles per MMA) and a branch per score in the epilogue, it took
 // 3480.  A call over 40 images of 1000 - 8000 descriptors went from 13.9 to 8.9 ms, a guided pair of
-// 7013 x 6450 from the host from 1.14 to 0.90 ms (its rows, 55 before, now fill every SM).
+// 7013 x 6450 from the host from 1.14 to 0.90 ms (its rows, 55 before, now fill every SM; 0.78 with the
+// guided epilogue's waiting scores).
 template <bool kGated>
 __global__ void __launch_bounds__(kFThreads, 1)
 k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, SideArgs a, float Tf,
@@ -322,13 +325,16 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
   } else {
     // ---------------- epilogue ----------------
     const int q = warp & 3, g = (warp - kFEpiWarp0) >> 2;
+    uint2* const waiting = &s.waiting[warp - kFEpiWarp0][0][lane];
     uint32_t i = 0;
     bool ok = true;
     // Scores below Tf change no decision, so the top two start just below it (-0 ranks below +0 but
     // equals it), and a group of eight scores whose maximum is below every lane's second is passed
     // over: on SIFT-like data a lane enters 0.6% of the groups.  All groups' maxima come first and one
-    // vote tells which to enter, so that no branch waits for another's outcome.  In a guided call the
-    // gate is tested for scores that matter only.
+    // vote tells which to enter, so that no branch waits for another's outcome.  In a guided call a
+    // score that could enter waits in shared memory until some lane has several: testing each gate when
+    // its score came up cost 300 cycles for every score of a group in turn (7013 x 6450 with F: the
+    // two guided passes 224 us, 111 now).
     const uint32_t floorKey = f32_order(Tf == 0.0f ? -0.0f : Tf) - 1u;
     GateLane gl{};
     for (FWalk wk = start; wk.more() && ok; wk.next()) {
@@ -351,6 +357,24 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
         gl.bPos = a.bg.pos + a.bg.posOff[bImg];
       }
       const int nB = wk.nB;
+      // Guided: the gates of every lane's waiting scores, in column order.  A masked score counts as none
+      // (the reference's -1e20 is below Tf).
+      int nWait = 0;
+      auto test_waiting = [&]() {
+        for (int k = 0; __any_sync(0xffffffffu, k < nWait); ++k) {
+          if (k >= nWait) continue;
+          const uint2 w = waiting[32 * k];
+          const uint32_t key = f32_order(__uint_as_float(w.x));
+          const int col = (int)w.y;
+          if (key <= b2) continue;
+          const bool masked = a.bg.on ? gate_rejects_col(gl, col)
+                                      : gates_reject(a.gatesDev, a.nGates, a.aIsLeft ? (int)st : col,
+                                                     a.aIsLeft ? col : (int)st);
+          if (!masked) top2_push(key, col, b1, b2, c1);
+        }
+        nWait = 0;
+        if (st >= 0) enter = f32_unorder(b2);
+      };
       for (int t = 0; t < wk.nT; ++t, ++i) {
         ok = mbar_wait_warp(&s.accFull[g], i & 1u, &s.abort, a.err);
         if (!ok) break;
@@ -382,22 +406,23 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
 #pragma unroll
           for (int k8 = 0; k8 < 4; ++k8) {
             if (!(mask & (1u << (4 * c + k8)))) continue;  // warp-uniform
+            if (kGated && __any_sync(0xffffffffu, nWait > kFWait - 8)) test_waiting();
 #pragma unroll
             for (int k = 8 * k8; k < 8 * k8 + 8; ++k) {
               const int col = col0 + 32 * c + k;
-              uint32_t key = 32 * c + k < nB - col0 ? f32_order(__uint_as_float(v[c][k])) : 0u;
-              if (kGated && key > b2) {  // a masked score counts as none (the reference's -1e20 is below Tf)
-                const bool masked = a.bg.on ? gate_rejects_col(gl, col)
-                                            : gates_reject(a.gatesDev, a.nGates, a.aIsLeft ? (int)st : col,
-                                                           a.aIsLeft ? col : (int)st);
-                if (masked) key = 0;
+              if (kGated) {
+                if (32 * c + k < nB - col0 && !(__uint_as_float(v[c][k]) < enter))
+                  waiting[32 * nWait++] = make_uint2(v[c][k], (uint32_t)col);
+              } else {
+                const uint32_t key = 32 * c + k < nB - col0 ? f32_order(__uint_as_float(v[c][k])) : 0u;
+                top2_push(key, col, b1, b2, c1);
               }
-              top2_push(key, col, b1, b2, c1);
             }
           }
         if (st >= 0) enter = f32_unorder(b2);
       }
       if (!ok) break;
+      if (kGated) test_waiting();
       bool decide = true;
       if (wk.nSeg > 1) {
         // a row in segments: this warp's 32 top twos to the row's place, and whichever warp comes last

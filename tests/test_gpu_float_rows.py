@@ -47,3 +47,20 @@ def test_edges_of_rows_tiles_and_segments(v3dm_mod, oracle_mod, nL, nR):
         np.testing.assert_array_equal(m.scores_f32(), exact)
     finally:
         m.close()
+
+
+@pytest.mark.parametrize("nL,nR,ms", [(127, 129, 0.0), (300, 1000, 0.1), (1500, 1400, 0.3)])
+def test_guided_with_most_scores_above_the_threshold(v3dm_mod, oracle_mod, nL, nR, ms):
+    """Low thresholds: nearly every score is tested against the gate, many per descriptor and tile."""
+    L, R, lp, rp, F = features(nL, nR)
+    m = v3dm_mod.SIFTMatching(0, v3dm_mod.KERNEL_TCGEN05)
+    m.allocate(nL, nR, True)
+    try:
+        m.set_left_features_bf16x3(L.astype(np.float32) / 512)
+        m.set_right_features_bf16x3(R.astype(np.float32) / 512)
+        for thr in (2.0, 400.0):  # 400: half of them pass
+            oracle = oracle_mod.match(L, R, ms, 1.0, gates=[("F", F, thr)], lpos=lp, rpos=rp)
+            np.testing.assert_array_equal(m.run_guided_matching(F, thr, lp, rp, ms, 1.0), oracle)
+            m.find_putative_matches(ms, 1.0)  # drops the gate
+    finally:
+        m.close()
