@@ -686,7 +686,36 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
   sa.nB = h->nR;
   sa.aIsLeft = 1;
   sa.best = h->dLBest;
-  if (!reuseA) {
+  // Without gates a pass over few tiles merges its scores itself, which saves the record kernel's launch
+  // and latency (two passes of 512 x 480: 63.5 us a call with records, 53.6 without; 4096 x 4096: 73 and
+  // 63.5); over many, the merging in the epilogue costs more than the kernel (8192 x 8192, 14 tiles per
+  // SM: 75.8 and 75.5; 16384 x 16384, 55 per SM: 101 and 103.5).  Pass A merges only when no guided call
+  // can come for its records.
+  constexpr int kMergeTiles = 16;  // per SM
+  int GM = 0, BN = 0;
+  tc_config_shape(cfg, &GM, &BN);
+  auto few = [&](int nA, int nB) {
+    return (long long)((nA + GM - 1) / GM) * ((nB + BN - 1) / BN) <= (long long)kMergeTiles * h->numSMs;
+  };
+  const bool mergeA = !gated && !h->guidedAlloc && few(h->nL, h->nR);
+  const bool mergeB = !gated && few(h->nR, h->nL);
+  if (mergeA) {
+    sa.merge = 1;
+    sa.sec = h->dLSec;
+    if (h->profile) {
+      int e = event_pair(h, 0, evA);
+      if (e != V3DM_OK) return e;
+      V3DM_CUDA_TRY(cudaEventRecord(evA[0], h->stream));
+    }
+    sa.waitLimit = h->testWaitLimit;
+    sa.skipLoad = h->testSkipLoad;
+    V3DM_CUDA_TRY(launch_side(h->tc, h->mapsA, sa, h->stream));
+    sa.waitLimit = 0;
+    sa.skipLoad = 0;
+    if (h->profile) V3DM_CUDA_TRY(cudaEventRecord(evA[1], h->stream));
+    h->passAValid = false;
+    h->lastLaunches += 1;
+  } else if (!reuseA) {
     // bounds below the smaller of the ungated and gated thresholds of these parameters are
     // dropped, so the guided calls that follow can use this pass
     int32_t tu = 0, tg = 0;
@@ -717,10 +746,14 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
   sa.records = h->dRecords;
   sa.segCount = h->dSegCount;
   sa.Tsec = tNeed;
-  pa.records = h->dRecordsA;
-  pa.segCount = segCountA;
-  pa.keepSegments = 1;
-  pa.secBound = boundA;
+  if (mergeA) {
+    pa.nSeg = 0;
+  } else {
+    pa.records = h->dRecordsA;
+    pa.segCount = segCountA;
+    pa.keepSegments = 1;
+    pa.secBound = boundA;
+  }
   pa.nRows = h->nL;
   pa.nB = h->nR;
   pa.aIsLeft = 1;
@@ -742,7 +775,7 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
   pa.segCount = h->dSegCount;
   pa.keepSegments = 0;
   pa.secBound = nullptr;
-  h->lastLaunches += 2;
+  h->lastLaunches += mergeA ? 1 : 2;
   if (gated) {
     ra.descA = h->dL;
     ra.descB = h->dR;
@@ -769,6 +802,8 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
   sa.aIsLeft = 0;
   sa.best = h->dRBest;
   sa.sec = h->dRSec;
+  sa.merge = mergeB ? 1 : 0;
+  pa.nSeg = mergeB ? 0 : h->nSeg;
   if (h->profile) {
     int e = event_pair(h, 1, evB);
     if (e != V3DM_OK) return e;
@@ -787,7 +822,7 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
   pa.flagged = h->dFlagB;
   pa.flaggedCount = h->dCounters + 2;
   V3DM_CUDA_TRY(launch_post(pa, h->stream));
-  h->lastLaunches += 3;
+  h->lastLaunches += mergeB ? 2 : 3;
   if (gated) {
     ra.descA = h->dR;
     ra.descB = h->dL;
@@ -804,7 +839,7 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
   V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->dRightDec, h->dChosenFlag, h->dScratch,
                               reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, h->stream));
   h->countWritten = h->countOut != nullptr;
-  h->lastLaunches += 2;
+  h->lastLaunches += mutual_launches(h->nL);
   return V3DM_OK;
 }
 
@@ -875,7 +910,7 @@ int enqueue_match_f(v3dm_matcher* h, float minScore, float minRatio, int32_t* dP
   V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->dRightDec, h->dChosenFlag, h->dScratch,
                               reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, h->stream));
   h->countWritten = h->countOut != nullptr;
-  h->lastLaunches = (h->floatL ? 0 : 1) + (h->floatR ? 0 : 1) + 5;
+  h->lastLaunches = (h->floatL ? 0 : 1) + (h->floatR ? 0 : 1) + 3 + mutual_launches(h->nL);
   return V3DM_OK;
 }
 

@@ -111,6 +111,7 @@ struct SideArgs {
   int* segCount;                 // per segment: records written
   long long segCap;              // records per segment
   int nSeg;
+  int merge;                     // 1: one pair without gates: best[] and sec[] are merged, no records
   int* err;
   int nGates;
   const GateParams* gatesDev;    // device array of the call's gates
@@ -331,6 +332,7 @@ cudaError_t launch_choose_planes(const int32_t* leftDec, int nL, int* chosenFlag
 // The pair count goes to info[kInfoPairs] and, when countOut is set, to *countOut.
 cudaError_t launch_mutual(const int32_t* leftDec, int nL, const int32_t* rightDec, int* chosenFlag, int* blockCount,
                           int2* pairs, int32_t* info, int32_t* countOut, cudaStream_t s);
+int mutual_launches(int nL);  // kernels of launch_mutual
 
 // Candidate threshold (v3dm_api.cu).
 int host_candidate_threshold(float minScore, float minRatio, bool gated, int32_t* T);

@@ -350,13 +350,20 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Best and second of one lane's row over the chunks of a run that hold a score >= Smin (kMerge).
+struct LaneTop {
+  uint32_t best = 0;  // largest score + 1, 0: none
+  int col = 0;        // its first column
+  uint32_t next = 0;  // largest other score + 1, 0: none
+};
+
 // The chunks of one lane's scores (columns col0 ..) one by one: a chunk with a score >= sminRow goes
-// to the warp's segment as a record (k_records does its exact work), otherwise its maximum is
-// folded into lw.
-template <int CHUNKS>
+// to the warp's segment as a record (k_records does its exact work) or, with kMerge, into the lane's
+// top; otherwise its maximum is folded into lw.
+template <int CHUNKS, bool kMerge>
 __device__ __forceinline__ void filter_chunks(uint32_t (&v)[CHUNKS][32], int colBase, int nB, int bRow0, int orig,
                                            int32_t sminRow, uint32_t& lw, int& segN, uint4* segBase,
-                                           long long segCap) {
+                                           long long segCap, LaneTop& top) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {
@@ -375,6 +382,25 @@ __device__ __forceinline__ void filter_chunks(uint32_t (&v)[CHUNKS][32], int col
     if (!trig) lw = cm;
     const unsigned m = __ballot_sync(0xffffffffu, trig);
     if (m == 0u) continue;
+    if constexpr (kMerge) {
+      if (trig) {  // cm is the chunk's maximum: lw is below sminRow
+        uint32_t eq = 0, w = 0;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+          eq |= v[c][k] == cm ? 1u << k : 0u;
+          w = max(w, v[c][k] == cm ? 0u : v[c][k]);
+        }
+        if (eq & (eq - 1u)) w = cm;
+        uint32_t next = nB - col0 > 1 ? w + 1u : 0u;  // the zeros past nB are no scores
+        const bool first = cm + 1u > top.best;
+        top.next = max(top.next, max(next, first ? top.best : cm + 1u));
+        if (first) {
+          top.best = cm + 1u;
+          top.col = col0 + __ffs(eq) - 1;
+        }
+      }
+      continue;
+    }
     if (trig) {
       const int idx = segN + __popc(m & ((1u << lane) - 1u));
       if (idx < segCap) {
@@ -391,8 +417,10 @@ __device__ __forceinline__ void filter_chunks(uint32_t (&v)[CHUNKS][32], int col
 
 // kBatch = false: one pair, the flattened (group, tile) range of this CTA (WorkCursor).
 // kBatch = true: rows of a.rows (BatchCursor); a row's state indices are state0 + row.
+// kMerge = true (one pair, no gates): no records.  A lane keeps its row's best and second over a run
+// and merges them into best[] and sec[] at its end, which saves a small pair the record kernel.
 // kGather = true (batched pass only): A blocks gathered row by row from a.aSrc (tmA unused).
-template <class C, bool kBatch, bool kGather = false>
+template <class C, bool kBatch, bool kGather = false, bool kMerge = false>
 __global__ void __launch_bounds__(kThreads, 1)
 k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int nTiles, SideArgs a) {
   static_assert(!kGather || kBatch, "gathered A blocks only in the batched pass");
@@ -411,7 +439,7 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
   if constexpr (kBatch) {
     nRows = a.nRowsPtr ? *a.nRowsPtr : a.nRows;
     if (nRows <= 0) {  // nothing to score: uniform early exit
-      if (warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
+      if (!kMerge && warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
       return;
     }
   } else {
@@ -420,7 +448,7 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
     sh.nTiles = nTiles;
     sh.nWork = (long long)sh.nGroups * nTiles;
     if (sh.nWork == 0) {  // nothing to score (e.g. no right was chosen): uniform early exit
-      if (warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
+      if (!kMerge && warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
       return;
     }
     cta_range(sh, w0, w1);
@@ -699,10 +727,16 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
     // (a negative float, below every score in the max.f32 order) while there is none
     constexpr uint32_t kNoScore = 0xbf800000u;
     uint32_t lw = kNoScore;
+    LaneTop top;
     int32_t sminRow = 0x7fffffff;  // Smin for a valid row, above every score otherwise
     // a bound below Tsec cannot change the decision: no atomic for it
     auto flush = [&]() {
-      const uint32_t w = lw == kNoScore ? 0u : lw + 1u;  // sec[] holds second + 1
+      uint32_t w = lw == kNoScore ? 0u : lw + 1u;  // sec[] holds second + 1
+      if constexpr (kMerge) {
+        if (rowValid && top.best) merge_chunk_best(&a.best[orig], &a.sec[orig], best_key((int32_t)top.best - 1, top.col));
+        w = max(w, top.next);
+        top = LaneTop{};
+      }
       if (rowValid && w > (uint32_t)a.Tsec) atomicMax(&a.sec[orig], w);
     };
     uint32_t i = 0;
@@ -762,11 +796,11 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
             continue;
           }
         }
-        filter_chunks<C::kChunks>(v, colBase, nB, bRow0, orig, sminRow, lw, segN, segBase, a.segCap);
+        filter_chunks<C::kChunks, kMerge>(v, colBase, nB, bRow0, orig, sminRow, lw, segN, segBase, a.segCap, top);
       }
       if (ok) flush();
     }
-    if (lane == 0) a.segCount[blockIdx.x * kEpiWarps + e] = segN;
+    if (!kMerge && lane == 0) a.segCount[blockIdx.x * kEpiWarps + e] = segN;
   }
 
   tc_fence_before();
@@ -817,17 +851,17 @@ using Cfg7 = TcCfg<1, 256, 4, 3>;   // as Cfg5 with 3 left-group buffers
 using Cfg8 = TcCfg<1, 256, 5, 2>;   // as Cfg0 with a 5-deep ring
 using Cfg9 = TcCfg<1, 256, 4, 4, 1>;   // as Cfg5 with the epilogue's second chunk loaded while the first is filtered
 
-template <class C, bool kBatch, bool kGather = false>
+template <class C, bool kBatch, bool kGather = false, bool kMerge = false>
 cudaError_t launch_cfg(const CUtensorMap& mA, const CUtensorMap& mB, int nTiles, const SideArgs& a, int grid,
                        cudaStream_t st, bool& attrSet) {
   const size_t smem = sizeof(Smem<C>) + 1024;
+  auto kernel = k_side<C, kBatch, kGather, kMerge>;
   if (!attrSet) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_side<C, kBatch, kGather>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     attrSet = true;
   }
-  return launch_pdl(k_side<C, kBatch, kGather>, dim3(grid), dim3(kThreads), smem, st, mA, mB, nTiles, a);
+  return launch_pdl(kernel, dim3(grid), dim3(kThreads), smem, st, mA, mB, nTiles, a);
 }
 
 constexpr int kNumCfg = 10;
@@ -844,6 +878,7 @@ struct TcPlan {
   int numSMs = 148;
   int cfg = kDefaultCfg;
   bool attrSet[kNumCfg] = {};
+  bool attrSetMerge[kNumCfg] = {};
   bool attrSetBatch[kNumCfg] = {};
   bool attrSetGather = false;
 };
@@ -889,6 +924,17 @@ cudaError_t tc_side_maps(TcPlan* p, TcMaps* m, const uint8_t* dA, int rowsA, con
   return cudaSuccess;
 }
 
+namespace {
+
+template <class C>
+cudaError_t launch_pair(const TcMaps& m, int nTiles, const SideArgs& a, int grid, cudaStream_t st, bool& attrSet,
+                        bool& attrSetMerge) {
+  if (a.merge) return launch_cfg<C, false, false, true>(m.a, m.b, nTiles, a, grid, st, attrSetMerge);
+  return launch_cfg<C, false>(m.a, m.b, nTiles, a, grid, st, attrSet);
+}
+
+}  // namespace
+
 cudaError_t launch_side(TcPlan* p, const TcMaps& m, const SideArgs& a, cudaStream_t st) {
   const int c = m.cfg;
   const int bn = kCfgBN[c];
@@ -899,16 +945,16 @@ cudaError_t launch_side(TcPlan* p, const TcMaps& m, const SideArgs& a, cudaStrea
   int grid = (int)std::min<long long>(p->numSMs, std::max<long long>(1, maxWork));
   if (grid * kEpiWarps > a.nSeg) return cudaErrorInvalidValue;
   switch (c) {
-    case 0: return launch_cfg<Cfg0, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[0]);
-    case 1: return launch_cfg<Cfg1, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[1]);
-    case 2: return launch_cfg<Cfg2, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[2]);
-    case 3: return launch_cfg<Cfg3, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[3]);
-    case 4: return launch_cfg<Cfg4, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[4]);
-    case 5: return launch_cfg<Cfg5, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[5]);
-    case 6: return launch_cfg<Cfg6, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[6]);
-    case 7: return launch_cfg<Cfg7, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[7]);
-    case 8: return launch_cfg<Cfg8, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[8]);
-    default: return launch_cfg<Cfg9, false>(m.a, m.b, nTiles, a, grid, st, p->attrSet[9]);
+    case 0: return launch_pair<Cfg0>(m, nTiles, a, grid, st, p->attrSet[0], p->attrSetMerge[0]);
+    case 1: return launch_pair<Cfg1>(m, nTiles, a, grid, st, p->attrSet[1], p->attrSetMerge[1]);
+    case 2: return launch_pair<Cfg2>(m, nTiles, a, grid, st, p->attrSet[2], p->attrSetMerge[2]);
+    case 3: return launch_pair<Cfg3>(m, nTiles, a, grid, st, p->attrSet[3], p->attrSetMerge[3]);
+    case 4: return launch_pair<Cfg4>(m, nTiles, a, grid, st, p->attrSet[4], p->attrSetMerge[4]);
+    case 5: return launch_pair<Cfg5>(m, nTiles, a, grid, st, p->attrSet[5], p->attrSetMerge[5]);
+    case 6: return launch_pair<Cfg6>(m, nTiles, a, grid, st, p->attrSet[6], p->attrSetMerge[6]);
+    case 7: return launch_pair<Cfg7>(m, nTiles, a, grid, st, p->attrSet[7], p->attrSetMerge[7]);
+    case 8: return launch_pair<Cfg8>(m, nTiles, a, grid, st, p->attrSet[8], p->attrSetMerge[8]);
+    default: return launch_pair<Cfg9>(m, nTiles, a, grid, st, p->attrSet[9], p->attrSetMerge[9]);
   }
 }
 
