@@ -20,6 +20,11 @@
 
 using namespace v3dm;
 
+// Results a call leaves in pinned memory: its info block and up to kHostPairs pairs, which a host
+// call then takes without asking for a copy (the two copies, each waited for, were 20 us of a small call).
+constexpr int kHostPairs = 16384;
+constexpr int kHostResultWords = kInfoWords + 2 * kHostPairs;
+
 struct v3dm_matcher {
   int device = 0;
   unsigned kernel = V3DM_KERNEL_TCGEN05;
@@ -52,7 +57,10 @@ struct v3dm_matcher {
   int32_t* dScratch = nullptr;    // nMaxR + nMaxL ints of finalize scratch
   int32_t* dPairs = nullptr;      // 2 * min(nMaxL, nMaxR)
   int32_t* dInfo = nullptr;       // kInfoWords: pair count, error flags, largest segment
-  int32_t* hInfo = nullptr;       // pinned mirror of dInfo
+  int32_t* hInfo = nullptr;       // pinned mirror of dInfo, then a call's results (kHostResultWords)
+  bool resInHost = false;         // the last enqueue writes its results there itself
+  bool pairsToHost = false;       // the call's pairs go to the host
+  int lastPairs = 0;              // pairs of the last call, once read_info has returned
   bool pendingCheck = false;      // a device-only call whose info block was not read yet
   float* dLPos = nullptr;         // positions upload (interleaved x, y)
   float* dRPos = nullptr;
@@ -408,7 +416,8 @@ int v3dm_allocate(v3dm_matcher* h, int nMaxL, int nMaxR, int useGuided) {
             dalloc(&h->dRBest, (size_t)nMaxR + 1) == cudaSuccess && dalloc(&h->dRSec, (size_t)nMaxR + 1) == cudaSuccess &&
             dalloc(&h->dScratch, (size_t)nMaxL + nMaxR + 1) == cudaSuccess &&
             dalloc(&h->dPairs, 2 * (size_t)nMin + 2) == cudaSuccess && dalloc(&h->dInfo, kInfoWords + 4) == cudaSuccess &&
-            cudaMallocHost(reinterpret_cast<void**>(&h->hInfo), kInfoWords * sizeof(int32_t)) == cudaSuccess;
+            cudaMallocHost(reinterpret_cast<void**>(&h->hInfo),
+                           (kInfoWords + kHostResultWords) * sizeof(int32_t)) == cudaSuccess;
   if (ok && h->guidedAlloc)
     ok = dalloc(&h->dLPos, 2 * (size_t)nMaxL + 2) == cudaSuccess && dalloc(&h->dRPos, 2 * (size_t)nMaxR + 2) == cudaSuccess &&
          dalloc(&h->dGateL, (size_t)V3DM_MAX_GATES * nMaxL + 1) == cudaSuccess &&
@@ -626,6 +635,11 @@ int enqueue_match_simt(v3dm_matcher* h, float minScore, float minRatio, int32_t*
   return V3DM_OK;
 }
 
+HostResult host_result(v3dm_matcher* h) {
+  int32_t* r = h->hInfo + kInfoWords;
+  return {r, h->pairsToHost ? reinterpret_cast<int2*>(r + kInfoWords) : nullptr, kHostPairs};
+}
+
 // tcgen05 path: side pass lefts x rights, decisions of the lefts, the chosen rights, side
 // pass chosen rights x lefts, their decisions, mutual filter.
 int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* dPairs) {
@@ -837,7 +851,8 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
     h->lastLaunches += 2;
   }
   V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->dRightDec, h->dChosenFlag, h->dScratch,
-                              reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, h->stream));
+                              reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, host_result(h), h->stream));
+  h->resInHost = true;
   h->countWritten = h->countOut != nullptr;
   h->lastLaunches += mutual_launches(h->nL);
   return V3DM_OK;
@@ -908,7 +923,8 @@ int enqueue_match_f(v3dm_matcher* h, float minScore, float minRatio, int32_t* dP
   V3DM_CUDA_TRY(launch_side_f(h->fmRc, h->fmL, sa, Tf, nullptr, h->numSMs, h->stream));
   if (h->profile) V3DM_CUDA_TRY(cudaEventRecord(evB[1], h->stream));
   V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->dRightDec, h->dChosenFlag, h->dScratch,
-                              reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, h->stream));
+                              reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, host_result(h), h->stream));
+  h->resInHost = true;
   h->countWritten = h->countOut != nullptr;
   h->lastLaunches = (h->floatL ? 0 : 1) + (h->floatR ? 0 : 1) + 3 + mutual_launches(h->nL);
   return V3DM_OK;
@@ -919,6 +935,7 @@ int enqueue_match_f(v3dm_matcher* h, float minScore, float minRatio, int32_t* dP
 int enqueue_match(v3dm_matcher* h, float minScore, float minRatio, int32_t* dPairs) {
   h->lastLaunches = 0;
   h->countWritten = false;
+  h->resInHost = false;
   // the info block and, right after it on the tcgen05 path, the call's counters
   V3DM_CUDA_TRY(cudaMemsetAsync(h->dInfo, 0, (h->dCounters ? kInfoWords + 4 : kInfoWords) * sizeof(int32_t),
                                 h->stream));
@@ -942,16 +959,21 @@ int enqueue_match(v3dm_matcher* h, float minScore, float minRatio, int32_t* dPai
 // Reads the info block of the last call.  Returns V3DM_OK, an error, or -1 when the
 // candidate list overflowed (the list has been grown and the call must be repeated).
 int read_info(v3dm_matcher* h) {
-  V3DM_CUDA_TRY(cudaMemcpyAsync(h->hInfo, h->dInfo, kInfoWords * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+  const int32_t* info = h->hInfo + kInfoWords;
+  if (!h->resInHost) {
+    V3DM_CUDA_TRY(cudaMemcpyAsync(h->hInfo, h->dInfo, kInfoWords * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+    info = h->hInfo;
+  }
   V3DM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->pendingCheck = false;
-  int err = h->hInfo[kInfoErr];
+  h->lastPairs = info[kInfoPairs];
+  int err = info[kInfoErr];
   if (err & kErrWaitTimeout) {
     h->passAValid = false;  // the pass stopped early: its records are incomplete
     return V3DM_ERR_TIMEOUT;
   }
   if (err) return V3DM_ERR_CUDA;
-  long long need = h->hInfo[kInfoMaxSeg];
+  long long need = info[kInfoMaxSeg];
   if (need > h->segCap) {
     V3DM_CUDA_TRY(alloc_candidates(h, h->nSeg, need + need / 4 + 1024));
     return -1;
@@ -962,15 +984,19 @@ int read_info(v3dm_matcher* h) {
 // Runs one matching call with host output, repeating it once the candidate list has grown.
 int run_host(v3dm_matcher* h, float minScore, float minRatio, int32_t* pairs, int cap, int* nOut) {
   for (int attempt = 0; attempt < 4; ++attempt) {
+    h->pairsToHost = true;
     int st = enqueue_match(h, minScore, minRatio, h->dPairs);
+    h->pairsToHost = false;
     if (st != V3DM_OK) return st;
     st = read_info(h);
     if (st == -1) continue;
     if (st != V3DM_OK) return st;
-    int n = h->hInfo[kInfoPairs];
+    int n = h->lastPairs;
     if (nOut) *nOut = n;
     int ncopy = n < cap ? n : cap;
-    if (ncopy > 0) {
+    if (h->resInHost && ncopy <= kHostPairs) {
+      if (ncopy > 0) std::memcpy(pairs, h->hInfo + 2 * kInfoWords, (size_t)ncopy * 2 * sizeof(int32_t));
+    } else if (ncopy > 0) {
       V3DM_CUDA_TRY(cudaMemcpyAsync(pairs, h->dPairs, (size_t)ncopy * 2 * sizeof(int32_t), cudaMemcpyDeviceToHost,
                                     h->stream));
       V3DM_CUDA_TRY(cudaStreamSynchronize(h->stream));

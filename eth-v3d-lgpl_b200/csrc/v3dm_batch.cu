@@ -75,6 +75,14 @@ constexpr int kCntNeedTable = 6;
 constexpr int kCntFlagA = 7;      // guided call: pass-A states flagged for an exact re-score
 constexpr int kCntFlagB = 12;     // and pass-B states
 constexpr int kCntAll = 16;      // batch and proposal counter words
+static_assert(kInfoWords + kCntAll <= 32, "one warp hands them to the host");
+
+// The kernel that ends a call leaves its info and counter words, and the first kHostTriples triples, in
+// pinned memory, where a host call takes them without asking for a copy (each copy that is waited for
+// is 10 - 15 us; 65536 take 16 us to cross PCIe either way, and of a call with more of them the copy is
+// a few per cent).
+constexpr int kHostTriples = 65536;
+constexpr size_t kHostInfoBytes = 128;  // the words, then the triples
 
 constexpr int kScanThreads = 1024;
 constexpr int kChooseThreads = 256;
@@ -302,9 +310,10 @@ k_bmutual_count(const int* __restrict__ counters, const int32_t* __restrict__ de
 
 // Pass 2: ordered write of the (pair, left, right) triples.
 __global__ void __launch_bounds__(kBMutThreads)
-k_bmutual_write(int* __restrict__ counters, const int32_t* __restrict__ decB, const int* __restrict__ chosenLeft,
+k_bmutual_write(int* counters, const int32_t* __restrict__ decB, const int* __restrict__ chosenLeft,
                 const int* __restrict__ chosenRight, const int* __restrict__ chosenPair,
-                const int* __restrict__ blockCount, int nBlocks, int3* __restrict__ out, int32_t* __restrict__ info) {
+                const int* __restrict__ blockCount, int nBlocks, int3* out, int32_t* info,
+                int32_t* hostInfo, int3* hostOut) {
   __shared__ int blockOff;
   __shared__ int wsum[kBMutThreads / 32];
   const int n = counters[kCntStates];
@@ -319,6 +328,10 @@ k_bmutual_write(int* __restrict__ counters, const int32_t* __restrict__ decB, co
         counters[kCntOut] = t + blockCount[blockIdx.x];
         info[kInfoPairs] = t + blockCount[blockIdx.x];
       }
+    }
+    if (blockIdx.x == nBlocks - 1) {  // the call ends here: its info and counter words, for the host
+      __syncwarp();
+      if (threadIdx.x < kInfoWords + kCntAll) hostInfo[threadIdx.x] = info[threadIdx.x];
     }
   }
   constexpr int kPer = kBMutPerBlock / kBMutThreads;
@@ -349,6 +362,16 @@ k_bmutual_write(int* __restrict__ counters, const int32_t* __restrict__ decB, co
       const int s = beg + i;
       out[off++] = make_int3(chosenPair[s], chosenLeft[s], chosenRight[s]);
     }
+  // the block's triples that go to the host, word by word in order: whole lines over PCIe (triples
+  // stored by the threads that found them took 40 us for 16384)
+  const int first = blockOff;
+  if (first >= kHostTriples) return;
+  int total = 0;
+  for (int k = 0; k < kBMutThreads / 32; ++k) total += wsum[k];
+  __syncthreads();
+  const int end = 3 * min(first + total, kHostTriples);
+  for (int w = 3 * first + threadIdx.x; w < end; w += kBMutThreads)
+    reinterpret_cast<int32_t*>(hostOut)[w] = reinterpret_cast<const int32_t*>(out)[w];
 }
 
 // Exact second values of the flagged states of a guided pass (k_decide flagged the states whose
@@ -890,7 +913,7 @@ struct v3dm_batch {
   // call state
   int* dCounters = nullptr;
   int32_t* dInfo = nullptr;
-  int32_t* hInfo = nullptr;         // pinned: info words then counter words
+  int32_t* hInfo = nullptr;         // pinned: info words, counter words, triples (kHostInfoBytes in)
   TcMaps mapsA, mapsB;
   bool mapsValid = false;
   int lastLaunches = 0;
@@ -1136,6 +1159,22 @@ int ensure_maps(v3dm_batch* b) {
   return V3DM_OK;
 }
 
+int3* host_triples(v3dm_batch* b) {
+  return reinterpret_cast<int3*>(reinterpret_cast<uint8_t*>(b->hInfo) + kHostInfoBytes);
+}
+
+// The first m triples of a call that the stream has finished.
+int copy_triples(v3dm_batch* b, int32_t* triples, long long m) {
+  if (m <= 0) return V3DM_OK;
+  if (m <= kHostTriples) {
+    std::memcpy(triples, host_triples(b), (size_t)m * sizeof(int3));
+    return V3DM_OK;
+  }
+  V3DM_BTRY(cudaMemcpyAsync(triples, b->dOut, (size_t)m * sizeof(int3), cudaMemcpyDeviceToHost, b->stream));
+  V3DM_BTRY(cudaStreamSynchronize(b->stream));
+  return V3DM_OK;
+}
+
 // Enqueues one batch call (all launches read their sizes from device memory).  With bg set, the
 // call is guided: every pair's gate applies, and flagged states are re-scored exactly.
 int enqueue_batch(v3dm_batch* b, float minScore, float minRatio, bool withEvents,
@@ -1243,11 +1282,9 @@ int enqueue_batch(v3dm_batch* b, float minScore, float minRatio, bool withEvents
   V3DM_BTRY(cudaGetLastError());
   k_bmutual_write<<<mutBlocks, kBMutThreads, 0, b->stream>>>(b->dCounters, b->dDecB, b->dChosenLeft,
                                                              b->dChosenRight, b->dChosenPair, b->dBlockCount,
-                                                             mutBlocks, b->dOut, b->dInfo);
+                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, host_triples(b));
   V3DM_BTRY(cudaGetLastError());
   launches += 2;
-  V3DM_BTRY(cudaMemcpyAsync(b->hInfo, b->dInfo, (kInfoWords + kCntAll) * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                            b->stream));
   b->lastLaunches = launches;
   return V3DM_OK;
 }
@@ -1309,11 +1346,9 @@ int enqueue_batch_f(v3dm_batch* b, float minScore, float minRatio, bool withEven
   V3DM_BTRY(cudaGetLastError());
   k_bmutual_write<<<mutBlocks, kBMutThreads, 0, b->stream>>>(b->dCounters, b->dDecB, b->dChosenLeft,
                                                              b->dChosenRight, b->dChosenPair, b->dBlockCount,
-                                                             mutBlocks, b->dOut, b->dInfo);
+                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, host_triples(b));
   V3DM_BTRY(cudaGetLastError());
   launches += 2;
-  V3DM_BTRY(cudaMemcpyAsync(b->hInfo, b->dInfo, (kInfoWords + kCntAll) * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                            b->stream));
   b->lastLaunches = launches;
   return V3DM_OK;
 }
@@ -1766,11 +1801,9 @@ int enqueue_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL, in
   V3DM_BTRY(cudaGetLastError());
   k_bmutual_write<<<mutBlocks, kBMutThreads, 0, b->stream>>>(b->dCounters, b->dDecB, b->dChosenLeft,
                                                              b->dChosenRight, b->dChosenPair, b->dBlockCount,
-                                                             mutBlocks, b->dOut, b->dInfo);
+                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, host_triples(b));
   V3DM_BTRY(cudaGetLastError());
   launches += 5;  // pass-B states (count, scan, choose), mutual filter (two)
-  V3DM_BTRY(cudaMemcpyAsync(b->hInfo, b->dInfo, (kInfoWords + kCntAll) * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                            b->stream));
   b->lastLaunches = launches;
   return V3DM_OK;
 }
@@ -2090,7 +2123,8 @@ int v3dm_batch_create(v3dm_batch** out, int device) {
   bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess &&
             tc_plan_create(&b->tc, device) == cudaSuccess &&
             cudaMalloc(reinterpret_cast<void**>(&b->dInfo), (kInfoWords + kCntAll) * sizeof(int32_t)) == cudaSuccess &&
-            cudaMallocHost(reinterpret_cast<void**>(&b->hInfo), (kInfoWords + kCntAll) * sizeof(int32_t)) == cudaSuccess;
+            cudaMallocHost(reinterpret_cast<void**>(&b->hInfo), kHostInfoBytes + kHostTriples * sizeof(int3)) ==
+                cudaSuccess;
   if (ok) {
     b->dCounters = b->dInfo + kInfoWords;  // the counter words follow the info words
     ok = alloc_records(b, 256) == cudaSuccess;
@@ -2249,11 +2283,8 @@ int v3dm_batch_match(v3dm_batch* b, float minScore, float minRatio, int32_t* tri
   if (st != V3DM_OK) return st;
   const long long n = b->hInfo[kInfoWords + kCntOut];
   *nOut = n;
-  const long long m = std::min(n, cap);
-  if (m > 0) {
-    V3DM_BTRY(cudaMemcpyAsync(triples, b->dOut, (size_t)m * sizeof(int3), cudaMemcpyDeviceToHost, b->stream));
-    V3DM_BTRY(cudaStreamSynchronize(b->stream));
-  }
+  st = copy_triples(b, triples, std::min(n, cap));
+  if (st != V3DM_OK) return st;
   return n > cap ? V3DM_ERR_CAPACITY : V3DM_OK;
 }
 
@@ -2327,11 +2358,8 @@ int v3dm_batch_match_guided(v3dm_batch* b, int type, const double* M, const floa
   if (st != V3DM_OK) return st;
   const long long nT = b->hInfo[kInfoWords + kCntOut];
   *nOut = nT;
-  const long long m = std::min(nT, cap);
-  if (m > 0) {
-    V3DM_BTRY(cudaMemcpyAsync(triples, b->dOut, (size_t)m * sizeof(int3), cudaMemcpyDeviceToHost, b->stream));
-    V3DM_BTRY(cudaStreamSynchronize(b->stream));
-  }
+  st = copy_triples(b, triples, std::min(nT, cap));
+  if (st != V3DM_OK) return st;
   return nT > cap ? V3DM_ERR_CAPACITY : V3DM_OK;
 }
 
@@ -2369,11 +2397,8 @@ int v3dm_batch_match_proposal(v3dm_batch* b, v3dm_projection* proj, int probesLe
   if (st != V3DM_OK) return st;
   const long long n = b->hInfo[kInfoWords + kCntOut];
   *nOut = n;
-  const long long m = std::min(n, cap);
-  if (m > 0) {
-    V3DM_BTRY(cudaMemcpyAsync(triples, b->dOut, (size_t)m * sizeof(int3), cudaMemcpyDeviceToHost, b->stream));
-    V3DM_BTRY(cudaStreamSynchronize(b->stream));
-  }
+  st = copy_triples(b, triples, std::min(n, cap));
+  if (st != V3DM_OK) return st;
   return n > cap ? V3DM_ERR_CAPACITY : V3DM_OK;
 }
 

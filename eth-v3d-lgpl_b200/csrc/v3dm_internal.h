@@ -330,8 +330,15 @@ cudaError_t launch_choose_planes(const int32_t* leftDec, int nL, int* chosenFlag
                                  cudaStream_t s);
 // Mutual filter and ordered compaction (blockCount: nL/2048 + 1 ints of scratch); clears chosenFlag.
 // The pair count goes to info[kInfoPairs] and, when countOut is set, to *countOut.
+// Results in pinned host memory, written by the kernel that ends a call: the host only waits for the
+// stream.  info: the info block; pairs: the first cap pairs (null: none).
+struct HostResult {
+  int32_t* info;
+  int2* pairs;
+  int cap;
+};
 cudaError_t launch_mutual(const int32_t* leftDec, int nL, const int32_t* rightDec, int* chosenFlag, int* blockCount,
-                          int2* pairs, int32_t* info, int32_t* countOut, cudaStream_t s);
+                          int2* pairs, int32_t* info, int32_t* countOut, const HostResult& host, cudaStream_t s);
 int mutual_launches(int nL);  // kernels of launch_mutual
 
 // Candidate threshold (v3dm_api.cu).

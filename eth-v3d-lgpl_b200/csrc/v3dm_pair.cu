@@ -262,6 +262,17 @@ __global__ void k_choose(const int32_t* __restrict__ leftDec, int nL, int* chose
 constexpr int kMutThreads = 256;
 constexpr int kMutPerBlock = kMutThreads;  // one left per thread: every load of a thread in flight at once
 
+__device__ __forceinline__ void put_pair(int2* pairs, const HostResult& host, int at, int2 p) {
+  pairs[at] = p;
+  if (host.pairs && at < host.cap) host.pairs[at] = p;
+}
+// The end of a call: its count, and the info block (its other words are from the kernels before).
+__device__ __forceinline__ void put_count(int32_t* info, int32_t* countOut, const HostResult& host, int total) {
+  info[kInfoPairs] = total;
+  if (countOut) *countOut = total;
+  for (int w = 0; w < kInfoWords; ++w) host.info[w] = w == kInfoPairs ? total : info[w];
+}
+
 // Pass 1: number of mutual pairs among each block's contiguous range of lefts.
 __global__ void __launch_bounds__(kMutThreads)
 k_mutual_count(const int32_t* __restrict__ leftDec, int nL, const int32_t* __restrict__ rightDec,
@@ -288,7 +299,7 @@ k_mutual_count(const int32_t* __restrict__ leftDec, int nL, const int32_t* __res
 __global__ void __launch_bounds__(kMutThreads)
 k_mutual_write(const int32_t* __restrict__ leftDec, int nL, const int32_t* __restrict__ rightDec, int* chosenFlag,
                const int* __restrict__ blockCount, int nBlocks, int2* __restrict__ pairs, int32_t* info,
-               int32_t* countOut) {
+               int32_t* countOut, HostResult host) {
   pdl_wait();
   pdl_launch_dependents();
   __shared__ int wsum[kMutThreads / 32];
@@ -317,12 +328,9 @@ k_mutual_write(const int32_t* __restrict__ leftDec, int nL, const int32_t* __res
     blockOff += wbefore[w];
     if (w < wid) before += wsum[w];
   }
-  if (ok) pairs[blockOff + before + inc - cnt] = make_int2(k, r);
-  if (threadIdx.x == kMutThreads - 1 && blockIdx.x == nBlocks - 1) {
-    const int total = blockOff + before + inc;
-    info[kInfoPairs] = total;
-    if (countOut) *countOut = total;
-  }
+  if (ok) put_pair(pairs, host, blockOff + before + inc - cnt, make_int2(k, r));
+  if (threadIdx.x == kMutThreads - 1 && blockIdx.x == nBlocks - 1)
+    put_count(info, countOut, host, blockOff + before + inc);
 }
 
 // Up to kMutSmall lefts: one block does both passes, kMutSmallPer consecutive lefts per thread with
@@ -333,7 +341,7 @@ constexpr int kMutSmallPer = 8;
 constexpr int kMutSmall = kMutSmallThreads * kMutSmallPer;
 __global__ void __launch_bounds__(kMutSmallThreads)
 k_mutual_small(const int32_t* __restrict__ leftDec, int nL, const int32_t* __restrict__ rightDec, int* chosenFlag,
-               int2* __restrict__ pairs, int32_t* info, int32_t* countOut) {
+               int2* pairs, int32_t* info, int32_t* countOut, HostResult host) {
   pdl_wait();
   pdl_launch_dependents();
   __shared__ int wsum[kMutSmallThreads / 32];
@@ -370,10 +378,11 @@ k_mutual_small(const int32_t* __restrict__ leftDec, int nL, const int32_t* __res
 #pragma unroll
   for (int i = 0; i < kMutSmallPer; ++i)
     if (ok[i]) pairs[at++] = make_int2(k0 + i, r[i]);
-  if (threadIdx.x == kMutSmallThreads - 1) {
-    info[kInfoPairs] = at;
-    if (countOut) *countOut = at;
-  }
+  if (threadIdx.x == kMutSmallThreads - 1) put_count(info, countOut, host, at);
+  if (!host.pairs) return;
+  const int n = min(__shfl_sync(0xffffffffu, v, 31), host.cap);
+  __syncthreads();
+  for (int k = threadIdx.x; k < n; k += kMutSmallThreads) host.pairs[k] = pairs[k];  // whole lines over PCIe
 }
 static_assert(kMutSmallThreads == 1024, "one warp sums the warps' counts");
 
@@ -422,16 +431,16 @@ cudaError_t launch_choose_planes(const int32_t* leftDec, int nL, int* chosenFlag
 int mutual_launches(int nL) { return nL == 0 ? 0 : nL <= kMutSmall ? 1 : 2; }
 
 cudaError_t launch_mutual(const int32_t* leftDec, int nL, const int32_t* rightDec, int* chosenFlag, int* blockCount,
-                          int2* pairs, int32_t* info, int32_t* countOut, cudaStream_t s) {
+                          int2* pairs, int32_t* info, int32_t* countOut, const HostResult& host, cudaStream_t s) {
   const int nBlocks = (nL + kMutPerBlock - 1) / kMutPerBlock;
   if (nBlocks == 0) return cudaSuccess;
   if (nL <= kMutSmall)
     return launch_pdl(k_mutual_small, dim3(1), dim3(kMutSmallThreads), 0, s, leftDec, nL, rightDec, chosenFlag, pairs,
-                      info, countOut);
+                      info, countOut, host);
   cudaError_t e = launch_pdl(k_mutual_count, dim3(nBlocks), dim3(kMutThreads), 0, s, leftDec, nL, rightDec, blockCount);
   if (e != cudaSuccess) return e;
   return launch_pdl(k_mutual_write, dim3(nBlocks), dim3(kMutThreads), 0, s, leftDec, nL, rightDec, chosenFlag,
-                    blockCount, nBlocks, pairs, info, countOut);
+                    blockCount, nBlocks, pairs, info, countOut, host);
 }
 
 }  // namespace v3dm
