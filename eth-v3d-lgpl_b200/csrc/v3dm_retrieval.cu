@@ -70,72 +70,113 @@ __device__ __forceinline__ float rt_unorder(uint32_t o) {
 
 // Bit-sliced column counters: bit k of plane p holds bit p of image k's count.  Sixteen rows at
 // a time go through a carry-save adder tree (Harley-Seal) into the planes of weight 1, 2, 4 and
-// 8; the carries of weight 16 ripple into the planes above.
-constexpr int kRtHigh = 11;          // planes of weight 16 .. 2^14
-constexpr int kRtSegment = 32752;    // rows per flush: a count stays below 2^15
+// 8; four such carries of weight 16 go through the planes of 16 and 32, and the carry of weight 64
+// ripples into the planes above (a ripple after every sixteen rows took a quarter of the kernel).
+constexpr int kRtPlaneCount = 15;    // weights 1 .. 2^14
+constexpr int kRtSegment = 32752;    // rows per flush, over all groups: a count stays below 2^15
 constexpr int kRtChunk = 4096;       // row offsets staged in shared memory at a time
 
 struct RtPlanes {
-  uint32_t ones, twos, fours, eights, hi[kRtHigh];
+  uint32_t v[kRtPlaneCount];
 };
 
 __device__ __forceinline__ void rt_csa(uint32_t& hi, uint32_t& lo, uint32_t a, uint32_t b, uint32_t c) {
-  const uint32_t u = a ^ b;
-  hi = (a & b) | (u & c);
-  lo = u ^ c;
+  uint32_t h, l;  // majority and parity, one instruction each
+  asm("lop3.b32 %0, %1, %2, %3, 0xe8;" : "=r"(h) : "r"(a), "r"(b), "r"(c));
+  asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(l) : "r"(a), "r"(b), "r"(c));
+  hi = h;
+  lo = l;
 }
 
 __device__ __forceinline__ void rt_clear(RtPlanes& p) {
-  p.ones = p.twos = p.fours = p.eights = 0;
 #pragma unroll
-  for (int q = 0; q < kRtHigh; ++q) p.hi[q] = 0;
+  for (int q = 0; q < kRtPlaneCount; ++q) p.v[q] = 0;
 }
 
 // Adds the counts of the images of 'mask' to kdCol[0..31] and clears the planes.
 __device__ __forceinline__ void rt_flush(RtPlanes& p, uint32_t mask, uint32_t* kdCol) {
-  uint32_t any = p.ones | p.twos | p.fours | p.eights;
+  uint32_t any = 0;
 #pragma unroll
-  for (int q = 0; q < kRtHigh; ++q) any |= p.hi[q];
+  for (int q = 0; q < kRtPlaneCount; ++q) any |= p.v[q];
   any &= mask;
   while (any) {
     const int k = __ffs(any) - 1;
     any &= any - 1u;
-    uint32_t cnt = ((p.ones >> k) & 1u) | (((p.twos >> k) & 1u) << 1) | (((p.fours >> k) & 1u) << 2) |
-                   (((p.eights >> k) & 1u) << 3);
+    uint32_t cnt = 0;
 #pragma unroll
-    for (int q = 0; q < kRtHigh; ++q) cnt |= ((p.hi[q] >> k) & 1u) << (q + 4);
-    atomicAdd(&kdCol[k], cnt);
+    for (int q = 0; q < kRtPlaneCount; ++q) cnt |= ((p.v[q] >> k) & 1u) << q;
+    kdCol[k] += cnt;
   }
   rt_clear(p);
 }
 
-// Sixteen rows of one column into the planes.
-__device__ __forceinline__ void rt_add16(RtPlanes& p, const uint32_t (&x)[16]) {
-  uint32_t twosA, twosB, foursA, foursB, eightsA, eightsB, sixteens;
-  rt_csa(twosA, p.ones, p.ones, x[0], x[1]);
-  rt_csa(twosB, p.ones, p.ones, x[2], x[3]);
-  rt_csa(foursA, p.twos, p.twos, twosA, twosB);
-  rt_csa(twosA, p.ones, p.ones, x[4], x[5]);
-  rt_csa(twosB, p.ones, p.ones, x[6], x[7]);
-  rt_csa(foursB, p.twos, p.twos, twosA, twosB);
-  rt_csa(eightsA, p.fours, p.fours, foursA, foursB);
-  rt_csa(twosA, p.ones, p.ones, x[8], x[9]);
-  rt_csa(twosB, p.ones, p.ones, x[10], x[11]);
-  rt_csa(foursA, p.twos, p.twos, twosA, twosB);
-  rt_csa(twosA, p.ones, p.ones, x[12], x[13]);
-  rt_csa(twosB, p.ones, p.ones, x[14], x[15]);
-  rt_csa(foursB, p.twos, p.twos, twosA, twosB);
-  rt_csa(eightsB, p.fours, p.fours, foursA, foursB);
-  rt_csa(sixteens, p.eights, p.eights, eightsA, eightsB);
+// Another group's counts of the same column.
+__device__ __forceinline__ void rt_add_planes(RtPlanes& p, const uint32_t* other, int stride) {
+  uint32_t carry = 0;
 #pragma unroll
-  for (int q = 0; q < kRtHigh; ++q) {
-    if (!sixteens) break;
-    const uint32_t t = p.hi[q] & sixteens;
-    p.hi[q] ^= sixteens;
-    sixteens = t;
+  for (int q = 0; q < kRtPlaneCount; ++q) rt_csa(carry, p.v[q], p.v[q], other[q * stride], carry);
+}
+
+// 'carry' of weight 2^FROM into the planes from there on.
+template <int FROM>
+__device__ __forceinline__ void rt_ripple(RtPlanes& p, uint32_t carry) {
+#pragma unroll
+  for (int q = FROM; q < kRtPlaneCount; ++q) {
+    if (!carry) break;
+    const uint32_t t = p.v[q] & carry;
+    p.v[q] ^= carry;
+    carry = t;
   }
 }
 
+// The word of a column in a row of the bitmap: word offsets of both with kWide, byte offsets while the bitmap
+// has less than 4 GB.  With these the kernel's pointer stays in a uniform register and the address is one
+// 32-bit addition, where 64-bit word addresses took four instructions for every load.
+template <bool kWide>
+__device__ __forceinline__ uint32_t rt_word(const uint32_t* bits, uint32_t row, uint32_t col) {
+  if (kWide) return __ldg(bits + col + (size_t)row);
+  return __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(bits) + (row + col)));
+}
+
+// Sixteen rows of one column into the planes of weight 1 to 8; the carry of weight 16.
+template <bool kWide>
+__device__ __forceinline__ uint32_t rt_add16(RtPlanes& p, const uint32_t* bits, uint32_t col, const uint32_t* rowOff) {
+  const uint4* ro = reinterpret_cast<const uint4*>(rowOff);
+  uint32_t x[16];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint4 o = ro[q];
+    x[4 * q + 0] = rt_word<kWide>(bits, o.x, col);
+    x[4 * q + 1] = rt_word<kWide>(bits, o.y, col);
+    x[4 * q + 2] = rt_word<kWide>(bits, o.z, col);
+    x[4 * q + 3] = rt_word<kWide>(bits, o.w, col);
+  }
+  uint32_t twosA, twosB, foursA, foursB, eightsA, eightsB, sixteens;
+  rt_csa(twosA, p.v[0], p.v[0], x[0], x[1]);
+  rt_csa(twosB, p.v[0], p.v[0], x[2], x[3]);
+  rt_csa(foursA, p.v[1], p.v[1], twosA, twosB);
+  rt_csa(twosA, p.v[0], p.v[0], x[4], x[5]);
+  rt_csa(twosB, p.v[0], p.v[0], x[6], x[7]);
+  rt_csa(foursB, p.v[1], p.v[1], twosA, twosB);
+  rt_csa(eightsA, p.v[2], p.v[2], foursA, foursB);
+  rt_csa(twosA, p.v[0], p.v[0], x[8], x[9]);
+  rt_csa(twosB, p.v[0], p.v[0], x[10], x[11]);
+  rt_csa(foursA, p.v[1], p.v[1], twosA, twosB);
+  rt_csa(twosA, p.v[0], p.v[0], x[12], x[13]);
+  rt_csa(twosB, p.v[0], p.v[0], x[14], x[15]);
+  rt_csa(foursB, p.v[1], p.v[1], twosA, twosB);
+  rt_csa(eightsB, p.v[2], p.v[2], foursA, foursB);
+  rt_csa(sixteens, p.v[3], p.v[3], eightsA, eightsB);
+  return sixteens;
+}
+
+// What bounds it: the reads of the bitmap from L2 (4 bytes per 32 images and word of a query: 4.2 GB for
+// 4096 images of 2000 - 6000 words, 7 TB/s) and the logic instructions of the counters, about equally.  A
+// group's planes are added to the next group's bit-sliced, through shared memory, so that each count is
+// taken apart once and not once per group (that, 1600 instructions per thread, was as much as the counting).
+// That call took 887 us, 730 now, of which this kernel 739 and 580.  Two columns per thread (8-byte loads, 277 million
+// instructions against 348) need 80 registers and were slower with the fewer warps, 587.
+template <bool kWide>
 __global__ void __launch_bounds__(kRtThreads, 2)
 k_rt_score(const int32_t* __restrict__ offsets, const int32_t* __restrict__ words, int nLeaves, int nImages, int w32,
            const uint32_t* __restrict__ bits, const RtLogs* __restrict__ logs, int nBest,
@@ -145,6 +186,7 @@ k_rt_score(const int32_t* __restrict__ offsets, const int32_t* __restrict__ word
   uint32_t* kd = reinterpret_cast<uint32_t*>(rtSh + nBest);    // k(d), then the order bits of d's score
   __shared__ uint32_t hist[256];
   __shared__ __align__(16) uint32_t rowOff[kRtChunk];
+  static_assert(kRtChunk >= kRtPlaneCount * kRtThreads / 2, "the groups' planes take the offsets' place");
   __shared__ unsigned long long shPrefix;
   __shared__ int shRem, shCnt;
 
@@ -168,50 +210,68 @@ k_rt_score(const int32_t* __restrict__ offsets, const int32_t* __restrict__ word
   const int g = threadIdx.x / colsPerPass;
   const bool active = g < groups;
   const int chunkRows = (kRtChunk / (16 * groups)) * 16 * groups;  // >= 16 * groups, a multiple of it
-  const uint32_t zeroRow = (uint32_t)nLeaves * (uint32_t)w32;
+  const uint32_t unit = kWide ? 1u : 4u;  // of the offsets: rt_word
+  const uint32_t rowUnits = (uint32_t)w32 * unit, zeroRow = (uint32_t)nLeaves * rowUnits;
   for (int c0 = 0; c0 < nw; c0 += colsPerPass) {
     const int col = c0 + (int)threadIdx.x % colsPerPass;
     const bool mine = active && col < nw;
-    const uint32_t* bitsCol = bits + (mine ? col : 0);
+    const uint32_t colOff = (mine ? (uint32_t)col : 0u) * unit;
     const uint32_t mask = col == nw - 1 ? tailMask : 0xffffffffu;
     RtPlanes p;
     rt_clear(p);
+    // The groups' counts of the column to kd, and the planes to zero (all threads; the chunk has been read).
+    auto flush = [&]() {
+      for (int ng = groups; ng > 1; ng = (ng + 1) / 2) {
+        const int half = (ng + 1) / 2, width = (ng - half) * colsPerPass;  // groups half .. ng - 1 hand over
+        __syncthreads();
+        if (mine && g >= half && g < ng) {
+          uint32_t* o = rowOff + (g - half) * colsPerPass + (int)threadIdx.x % colsPerPass;
+#pragma unroll
+          for (int q = 0; q < kRtPlaneCount; ++q) o[q * width] = p.v[q];
+          rt_clear(p);
+        }
+        __syncthreads();
+        if (mine && g < ng - half) rt_add_planes(p, rowOff + g * colsPerPass + (int)threadIdx.x % colsPerPass, width);
+      }
+      if (mine && g == 0) rt_flush(p, mask, kd + (col << 5));
+    };
     int inSegment = 0;  // rows added since the last flush
     for (int f0 = b; f0 < e; f0 += chunkRows) {
+      const int step = 16 * groups;
+      const int rows = min(chunkRows, (e - f0 + step - 1) / step * step);
+      if (inSegment + rows > kRtSegment) {
+        flush();
+        inSegment = 0;
+      }
+      inSegment += rows;
       __syncthreads();  // the previous chunk has been read
       for (int r = threadIdx.x; r < chunkRows; r += blockDim.x) {
         const int j = f0 + r;
         uint32_t off = zeroRow;
         if (j < e) {
           const int w = __ldg(words + j);
-          if (w >= 0 && w < nLeaves) off = (uint32_t)w * (uint32_t)w32;  // else reported by k_rt_presence
+          if (w >= 0 && w < nLeaves) off = (uint32_t)w * rowUnits;  // else reported by k_rt_presence
         }
         rowOff[r] = off;
       }
       __syncthreads();
       if (mine) {
-        const int rows = min(chunkRows, ((e - f0) + 16 * groups - 1) / (16 * groups) * (16 * groups));
-        if (inSegment + rows / groups > kRtSegment) {
-          rt_flush(p, mask, kd + (col << 5));
-          inSegment = 0;
+        int r0 = 16 * g;  // a multiple of 16
+        for (; r0 + 3 * step < rows; r0 += 4 * step) {
+          uint32_t thirtyA, thirtyB, sixty, a = rt_add16<kWide>(p, bits, colOff, rowOff + r0);
+          uint32_t c = rt_add16<kWide>(p, bits, colOff, rowOff + r0 + step);
+          rt_csa(thirtyA, p.v[4], p.v[4], a, c);
+          a = rt_add16<kWide>(p, bits, colOff, rowOff + r0 + 2 * step);
+          c = rt_add16<kWide>(p, bits, colOff, rowOff + r0 + 3 * step);
+          rt_csa(thirtyB, p.v[4], p.v[4], a, c);
+          rt_csa(sixty, p.v[5], p.v[5], thirtyA, thirtyB);
+          rt_ripple<6>(p, sixty);
         }
-        inSegment += rows / groups;
-        for (int r0 = 16 * g; r0 < rows; r0 += 16 * groups) {
-          const uint4* ro = reinterpret_cast<const uint4*>(rowOff + r0);  // r0 is a multiple of 16
-          uint32_t x[16];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint4 o = ro[q];
-            x[4 * q + 0] = __ldg(bitsCol + o.x);
-            x[4 * q + 1] = __ldg(bitsCol + o.y);
-            x[4 * q + 2] = __ldg(bitsCol + o.z);
-            x[4 * q + 3] = __ldg(bitsCol + o.w);
-          }
-          rt_add16(p, x);
-        }
+        for (; r0 < rows; r0 += step) rt_ripple<4>(p, rt_add16<kWide>(p, bits, colOff, rowOff + r0));
       }
     }
-    if (mine) rt_flush(p, mask, kd + (col << 5));
+    flush();
+    __syncthreads();  // the next pass stages its offsets where the planes were
   }
   __syncthreads();
 
@@ -433,10 +493,11 @@ int rt_enqueue(v3dm_retrieval* r, int nLeaves, int nImages, const int32_t* offse
   V3DM_RT_TRY(cudaMemcpyAsync(r->dLogs, hLogs, (size_t)nImages * sizeof(RtLogs), cudaMemcpyHostToDevice, r->stream));
   V3DM_RT_TRY(cudaEventRecord(r->slotDone[s], r->stream));
   const size_t smem = (size_t)nBest * sizeof(unsigned long long) + (size_t)nImages * sizeof(uint32_t);
-  V3DM_RT_TRY(cudaFuncSetAttribute(k_rt_score, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto score = bitWords * sizeof(uint32_t) < (1ull << 32) ? k_rt_score<false> : k_rt_score<true>;
+  V3DM_RT_TRY(cudaFuncSetAttribute(score, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   V3DM_RT_TRY(rt_mark(r, 1));
-  k_rt_score<<<nImages, kRtThreads, smem, r->stream>>>(r->dOffsets, dWords, nLeaves, nImages, w32, r->dBits, r->dLogs,
-                                                       nBest, dDocs, dScores);
+  score<<<nImages, kRtThreads, smem, r->stream>>>(r->dOffsets, dWords, nLeaves, nImages, w32, r->dBits, r->dLogs, nBest,
+                                                  dDocs, dScores);
   V3DM_RT_TRY(cudaGetLastError());
   V3DM_RT_TRY(rt_mark(r, 1));
   V3DM_RT_TRY(cudaMemcpyAsync(r->hErr, r->dErr, sizeof(int), cudaMemcpyDeviceToHost, r->stream));
