@@ -144,16 +144,8 @@ __device__ long long block_scan(int n, V val, O out, long long* sh) {
   const int b = min(n, tid * per), e = min(n, b + per);
   long long s = 0;
   for (int i = b; i < e; ++i) s += val(i);
-  sh[tid] = s;
-  __syncthreads();
-  for (int o = 1; o < T; o <<= 1) {
-    const long long v = tid >= o ? sh[tid - o] : 0;
-    __syncthreads();
-    sh[tid] += v;
-    __syncthreads();
-  }
-  const long long total = sh[T - 1];
-  long long run = sh[tid] - s;
+  long long total;
+  long long run = block_prefix(s, sh, &total);
   for (int i = b; i < e; ++i) {
     const long long v = val(i);
     out(i, run);
@@ -169,7 +161,7 @@ __global__ void __launch_bounds__(kScanThreads)
 k_bscan(const int* __restrict__ cnt, int nPairs, const BImage* __restrict__ im, int nImages, int GM, int BN,
         long long capStates, long long capRows, long long capTable, long long* __restrict__ prefC,
         BImageB* __restrict__ imgB, BatchRow* __restrict__ rowsB, int* __restrict__ counters) {
-  __shared__ long long sh[kScanThreads];
+  __shared__ long long sh[33];
   const long long SB = block_scan(
       nPairs, [&](int i) { return (long long)cnt[i]; }, [&](int i, long long x) { prefC[i] = x; }, sh);
   if (threadIdx.x == 0) prefC[nPairs] = SB;
@@ -480,7 +472,7 @@ __global__ void k_pcount(const BImage* __restrict__ im, int nImages, const uint8
 __global__ void __launch_bounds__(kScanThreads)
 k_pscan_cells(const int* __restrict__ cntA, const int* __restrict__ cntB, int n, int* __restrict__ offA,
               int* __restrict__ offB, int* __restrict__ curA, int* __restrict__ curB) {
-  __shared__ long long sh[kScanThreads];
+  __shared__ long long sh[33];
   block_scan(n, [&](int i) { return (long long)cntA[i]; }, [&](int i, long long x) { offA[i] = curA[i] = (int)x; }, sh);
   block_scan(n, [&](int i) { return (long long)cntB[i]; }, [&](int i, long long x) { offB[i] = curB[i] = (int)x; }, sh);
 }
@@ -573,7 +565,7 @@ __global__ void k_prowcount(const BPair* __restrict__ pairs, const BImage* __res
 __global__ void __launch_bounds__(kScanThreads)
 k_pscan_rows(const int* __restrict__ rowCnt, int nUnits, long long capRows, int* __restrict__ rowStart,
              int* __restrict__ counters) {
-  __shared__ long long sh[kScanThreads];
+  __shared__ long long sh[33];
   const long long total = block_scan(
       nUnits, [&](int i) { return (long long)rowCnt[i]; }, [&](int i, long long x) { rowStart[i] = (int)x; }, sh);
   if (threadIdx.x == 0) {
@@ -627,7 +619,7 @@ __global__ void k_prows(const BPair* __restrict__ pairs, const BImage* __restric
 __global__ void __launch_bounds__(kScanThreads)
 k_pscan_states(const int* __restrict__ cnt, int nPairs, long long capStates, long long* __restrict__ prefC,
                int* __restrict__ counters) {
-  __shared__ long long sh[kScanThreads];
+  __shared__ long long sh[33];
   const long long SB = block_scan(
       nPairs, [&](int i) { return (long long)cnt[i]; }, [&](int i, long long x) { prefC[i] = x; }, sh);
   if (threadIdx.x == 0) {
@@ -723,7 +715,7 @@ __global__ void __launch_bounds__(kScanThreads)
 k_vscan(const int* __restrict__ cntJ, const BImage* __restrict__ im, int nImages, const long long* __restrict__ prefC,
         int GR, long long capRows, int* __restrict__ offJ, int* __restrict__ rowStartL, int* __restrict__ rowStartR,
         int* __restrict__ counters) {
-  __shared__ long long sh[kScanThreads];
+  __shared__ long long sh[33];
   const long long total = block_scan(
       nImages, [&](int j) { return (long long)cntJ[j]; }, [&](int j, long long x) { offJ[j] = (int)x; }, sh);
   __syncthreads();

@@ -22,6 +22,35 @@ __device__ __forceinline__ void merge_chunk_best(unsigned long long* best, unsig
   if (old && old != cb) atomicMax(sec, (unsigned)((old < cb ? old : cb) >> kIndexBits));
 }
 
+// Exclusive prefix of the block's values (thread order) and their total; sh holds 33 of them.  Whole warps,
+// at most 32.  Two barriers, where a scan by doubling over the block's threads takes twenty (4 us of a
+// one-block kernel's 9 to 12).
+__device__ __forceinline__ long long block_prefix(long long v, long long* sh, long long* total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  long long inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) sh[wid] = inc;
+  __syncthreads();
+  if (wid == 0) {
+    const long long w = lane < warps ? sh[lane] : 0;
+    long long t = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += u;
+    }
+    sh[lane] = t - w;
+    if (lane == 31) sh[32] = t;
+  }
+  __syncthreads();
+  *total = sh[32];
+  return sh[wid] + inc - v;
+}
+
 // A candidate (l, r, S): both best keys take it with an atomicMax whose result is unused
 // (a fire-and-forget reduction, so the issuing warp does not wait for L2).
 __device__ __forceinline__ void record_best(const MatchArgs& a, int l, int r, int32_t S) {

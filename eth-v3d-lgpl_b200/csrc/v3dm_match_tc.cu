@@ -425,34 +425,16 @@ __global__ void __launch_bounds__(kThreads, 1)
 k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int nTiles, SideArgs a) {
   static_assert(!kGather || kBatch, "gathered A blocks only in the batched pass");
   const long long lim = a.waitLimit > 0 ? a.waitLimit : kWaitCycles;
-  pdl_wait();
-  pdl_launch_dependents();
   extern __shared__ uint8_t smemRaw[];
   Smem<C>& s = *reinterpret_cast<Smem<C>*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   static_assert(C::kStages + C::kAcc + 2 <= kRunRing, "the producer does not lap a reader of the ring of runs");
   using ProducerCursor = typename std::conditional<kBatch, BatchCursor, WorkCursor>::type;
   using Cursor = typename std::conditional<kBatch, RunCursor, WorkCursor>::type;
+  // Barriers and TMEM do not depend on the kernel before: their set-up overlaps its end.
   int nA = 0, nRows = 0;
   TcShape sh{};
   long long w0 = 0, w1 = 0;
-  if constexpr (kBatch) {
-    nRows = a.nRowsPtr ? *a.nRowsPtr : a.nRows;
-    if (nRows <= 0) {  // nothing to score: uniform early exit
-      if (!kMerge && warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
-      return;
-    }
-  } else {
-    nA = a.nAptr ? *a.nAptr : a.nA;
-    sh.nGroups = (nA + C::GM - 1) / C::GM;
-    sh.nTiles = nTiles;
-    sh.nWork = (long long)sh.nGroups * nTiles;
-    if (sh.nWork == 0) {  // nothing to score (e.g. no right was chosen): uniform early exit
-      if (!kMerge && warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
-      return;
-    }
-    cta_range(sh, w0, w1);
-  }
   auto producer_cursor = [&]() -> ProducerCursor {
     if constexpr (kBatch) return BatchCursor(a.rows, nRows, a.schedule);
     else return WorkCursor(w0, w1, sh.nTiles);
@@ -488,15 +470,33 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s.tmemBase;
-  if ((tmem & 0xFFFFu) != 0 && threadIdx.x == 0) {  // 512 columns must start at column 0
-    atomicOr(a.err, kErrTmem);
-    s.abort = 1;
+  pdl_wait();
+  pdl_launch_dependents();
+  bool work;  // uniform over the block: something to score (a pass of the chosen rights may have none)
+  if constexpr (kBatch) {
+    nRows = a.nRowsPtr ? *a.nRowsPtr : a.nRows;
+    work = nRows > 0;
+  } else {
+    nA = a.nAptr ? *a.nAptr : a.nA;
+    sh.nGroups = (nA + C::GM - 1) / C::GM;
+    sh.nTiles = nTiles;
+    sh.nWork = (long long)sh.nGroups * nTiles;
+    work = sh.nWork > 0;
+    if (work) cta_range(sh, w0, w1);
   }
-  __syncthreads();
+  if ((tmem & 0xFFFFu) != 0) {  // 512 columns must start at column 0
+    if (threadIdx.x == 0) {
+      atomicOr(a.err, kErrTmem);
+      s.abort = 1;
+    }
+    __syncthreads();
+  }
 
   // Ring uses are numbered from 0 in every role: tile i has B stage i % kStages and accumulator
   // i % kAcc, the run's A block number j slot j % kASlots.
-  if (warp == 0) {
+  if (!work) {
+    if (!kMerge && warp >= kEpiWarp0 && lane == 0) a.segCount[blockIdx.x * kEpiWarps + (warp - kEpiWarp0)] = 0;
+  } else if (warp == 0) {
    if constexpr (kGather) {
     // ---------------- producer, gathered A: the whole warp ----------------
     if (!s.abort) {

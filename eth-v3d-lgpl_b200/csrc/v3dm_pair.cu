@@ -104,15 +104,6 @@ __device__ __forceinline__ void clear_segments(const PostArgs& a) {
   }
 }
 
-// Copies right r's descriptor row to slot k of the pass-B operand.
-__device__ __forceinline__ void gather_chosen(const PostArgs& a, int r, int k) {
-  a.chooseList[k] = r;
-  const uint4* src = reinterpret_cast<const uint4*>(a.chooseSrc + (size_t)r * kDescBytes);
-  uint4* dst = reinterpret_cast<uint4*>(a.chooseDst + (size_t)k * kDescBytes);
-#pragma unroll
-  for (int w = 0; w < kDescBytes / 16; ++w) dst[w] = src[w];
-}
-
 // Decisions of the pass's descriptors; flags the ones whose gated bound straddles the
 // decision, clears the state of the others.  With a.chooseFlag set, accepted partners are
 // chosen for pass B right away: the first left to name a right claims it (flag exchange),
@@ -140,6 +131,14 @@ __global__ void k_decide(PostArgs a) {
     }
     a.decision[idx] = d;
     if (a.chooseFlag) {
+      // the descriptor row, read while the claim and the slot are on their way
+      constexpr int kQuads = kDescBytes / 16;
+      uint4 row[kQuads];
+      if (d >= 0) {
+        const uint4* src = reinterpret_cast<const uint4*>(a.chooseSrc + (size_t)d * kDescBytes);
+#pragma unroll
+        for (int w = 0; w < kQuads; ++w) row[w] = src[w];
+      }
       const bool claim = d >= 0 && atomicExch(&a.chooseFlag[d], 1) == 0;
       const unsigned act = __activemask();
       const unsigned m = __ballot_sync(act, claim);
@@ -148,7 +147,13 @@ __global__ void k_decide(PostArgs a) {
         int base = 0;
         if (lane == leader) base = atomicAdd(a.chooseCount, __popc(m));
         base = __shfl_sync(act, base, leader);
-        if (claim) gather_chosen(a, d, base + __popc(m & ((1u << lane) - 1u)));
+        if (claim) {
+          const int k = base + __popc(m & ((1u << lane) - 1u));
+          a.chooseList[k] = d;
+          uint4* dst = reinterpret_cast<uint4*>(a.chooseDst + (size_t)k * kDescBytes);
+#pragma unroll
+          for (int w = 0; w < kQuads; ++w) dst[w] = row[w];
+        }
       }
     }
   }

@@ -42,6 +42,7 @@
 #include <cstring>
 #include <new>
 
+#include "v3dm_device.cuh"
 #include "v3dm_internal.h"
 
 using namespace v3dm;
@@ -129,8 +130,7 @@ constexpr int kVtLocalBins = 16384;     // bucket counts kept in shared memory b
 __global__ void __launch_bounds__(1024)
 k_vt_scan(const int* __restrict__ hist, int bins, int itemKeys, int* __restrict__ off, int4* __restrict__ items,
           int* __restrict__ nItems) {
-  __shared__ long long sh[1024];
-  __shared__ long long shI[1024];
+  __shared__ long long sh[33], shI[33];
   const int T = blockDim.x, tid = threadIdx.x;
   const int per = (bins + T - 1) / T;
   const int b0 = min(bins, tid * per), b1 = min(bins, b0 + per);
@@ -140,17 +140,8 @@ k_vt_scan(const int* __restrict__ hist, int bins, int itemKeys, int* __restrict_
     sk += cnt(b);
     si += (cnt(b) + itemKeys - 1) / itemKeys;
   }
-  sh[tid] = sk;
-  shI[tid] = si;
-  __syncthreads();
-  for (int o = 1; o < T; o <<= 1) {
-    const long long v = tid >= o ? sh[tid - o] : 0, w = tid >= o ? shI[tid - o] : 0;
-    __syncthreads();
-    sh[tid] += v;
-    shI[tid] += w;
-    __syncthreads();
-  }
-  long long k = sh[tid] - sk, it = shI[tid] - si;
+  long long keys, nIt;
+  long long k = block_prefix(sk, sh, &keys), it = block_prefix(si, shI, &nIt);
   for (int b = b0; b < b1; ++b) {
     const int c = cnt(b);
     off[b] = (int)k;
@@ -158,8 +149,8 @@ k_vt_scan(const int* __restrict__ hist, int bins, int itemKeys, int* __restrict_
     k += c;
   }
   if (tid == T - 1) {
-    off[bins] = (int)sh[T - 1];
-    *nItems = (int)shI[T - 1];
+    off[bins] = (int)keys;
+    *nItems = (int)nIt;
   }
 }
 
