@@ -266,6 +266,8 @@ struct BatchCursor {
     newA = raw.x.x != cur.aRow;
     take();
   }
+  // the next row, where there is one with another A block
+  __device__ __forceinline__ bool next_new_a() const { return step_from(R) < Rend && raw.x.x != cur.aRow; }
   __device__ __forceinline__ int next_a_row() const { return raw.x.x; }
   __device__ __forceinline__ int next_valid_rows() const { return raw.x.y; }
 };
@@ -503,10 +505,6 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
       uint32_t i = 0, j = 0;             // tiles, A blocks
       int pend[kGatherDepth + 1] = {};  // slots whose gather still needs its arrive, oldest first
       int nPend = 0;
-      int preRow = -1;                   // A block whose entry indices pre[] holds
-      int pre[C::GM / 32];
-#pragma unroll
-      for (int k = 0; k < C::GM / 32; ++k) pre[k] = -1;
       auto arrive_oldest = [&]() {
         fence_proxy_async_smem();
         __syncwarp();
@@ -522,54 +520,50 @@ k_side(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensor
       // blocking wait by lane 0 (after handing over every pending gather, so that the MMA
       // can drain what the wait depends on); the result is broadcast
       auto wait_slot = [&](unsigned long long* bar, uint32_t par) -> bool {
-        if (mbar_try(bar, par)) return true;
+        if (__all_sync(0xffffffffu, mbar_try(bar, par))) return true;
         arrive_all();
         int okl = 1;
         if (lane == 0) okl = mbar_wait(bar, par, &s.abort, a.err, lim) ? 1 : 0;
         return __shfl_sync(0xffffffffu, okl, 0) != 0;
       };
+      // The copies of A block j (rows aRow .. of the entry table) into its slot.
+      auto gather = [&](int aRow, int nValid) -> bool {
+        const uint32_t slot = ring_slot<C::kASlots>(j);
+        if (!wait_slot(&s.emptyA[slot], ring_parity<C::kASlots>(j) ^ 1)) return false;
+        ++j;
+        int src[C::GM / 32];
+#pragma unroll
+        for (int k = 0; k < C::GM / 32; ++k) {
+          const int rr = lane + 32 * k;
+          src[k] = rr < nValid ? __ldg(a.aSrcRow + aRow + rr) : -1;
+        }
+        const uint32_t dst0 = smem_u32(s.a[slot]);
+#pragma unroll
+        for (int k = 0; k < C::GM / 32; ++k) {
+          const int rr = lane + 32 * k;
+          const uint8_t* g = a.aSrc + (src[k] >= 0 ? (size_t)src[k] * kDescBytes : (size_t)0);
+          const uint32_t nb = src[k] >= 0 ? 16u : 0u;  // 0: zero fill
+          const uint32_t d = dst0 + (uint32_t)rr * 128u;
+#pragma unroll
+          for (int ch = 0; ch < 8; ++ch) cp_async16(d + (uint32_t)((ch ^ (rr & 7)) << 4), g + 16 * ch, nb);
+        }
+        cp_async_commit();
+        pend[nPend++] = (int)slot;
+        if (nPend > kGatherDepth) {
+          cp_async_wait<kGatherDepth>();
+          arrive_oldest();
+        }
+        return true;
+      };
       bool go = true;
       uint32_t r = 0;                    // runs
       for (ProducerCursor wc = producer_cursor(); wc.more() && go; wc.next()) {
         if (lane == 0) put_run(s.runs, s.runFull, r, &wc.cur, wc.newA);
-        ++r;
-        if (wc.newA) {
-          const uint32_t slot = ring_slot<C::kASlots>(j);
-          if (!wait_slot(&s.emptyA[slot], ring_parity<C::kASlots>(j) ^ 1)) break;
-          ++j;
-          const int aRow = wc.cur.aRow, nValid = wc.cur.validRows;
-          int src[C::GM / 32];
-#pragma unroll
-          for (int k = 0; k < C::GM / 32; ++k) {
-            const int rr = lane + 32 * k;
-            src[k] = aRow == preRow ? pre[k] : (rr < nValid ? __ldg(a.aSrcRow + aRow + rr) : -1);
-          }
-          const uint32_t dst0 = smem_u32(s.a[slot]);
-#pragma unroll
-          for (int k = 0; k < C::GM / 32; ++k) {
-            const int rr = lane + 32 * k;
-            const uint8_t* g = a.aSrc + (src[k] >= 0 ? (size_t)src[k] * kDescBytes : (size_t)0);
-            const uint32_t nb = src[k] >= 0 ? 16u : 0u;  // 0: zero fill
-            const uint32_t d = dst0 + (uint32_t)rr * 128u;
-#pragma unroll
-            for (int ch = 0; ch < 8; ++ch) cp_async16(d + (uint32_t)((ch ^ (rr & 7)) << 4), g + 16 * ch, nb);
-          }
-          cp_async_commit();
-          // the next row's entry indices, read now and used at its turn (the loads overlap)
-          if (wc.next_a_row() != aRow) {
-            preRow = wc.next_a_row();
-#pragma unroll
-            for (int k = 0; k < C::GM / 32; ++k) {
-              const int rr = lane + 32 * k;
-              pre[k] = rr < wc.next_valid_rows() ? __ldg(a.aSrcRow + preRow + rr) : -1;
-            }
-          }
-          pend[nPend++] = (int)slot;
-          if (nPend > kGatherDepth) {
-            cp_async_wait<kGatherDepth>();
-            arrive_oldest();
-          }
-        }
+        // A block by A block a run ahead: the copies of the next one run under this run's tiles (gathered
+        // at its own turn, six tiles ahead, a block was waited for 8800 cycles, a fifth of the pass).
+        if (r++ == 0) go = gather(wc.cur.aRow, wc.cur.validRows);
+        if (go && wc.next_new_a()) go = gather(wc.next_a_row(), wc.next_valid_rows());
+        if (!go) break;
         for (int t = 0; t < wc.nT; ++t, ++i) {
           const uint32_t st = ring_slot<C::kStages>(i);
           if (!wait_slot(&s.done[st], ring_parity<C::kStages>(i) ^ 1)) {
