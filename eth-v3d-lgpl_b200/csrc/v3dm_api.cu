@@ -58,6 +58,7 @@ struct v3dm_matcher {
   int32_t* dPairs = nullptr;      // 2 * min(nMaxL, nMaxR)
   int32_t* dInfo = nullptr;       // kInfoWords: pair count, error flags, largest segment
   int32_t* hInfo = nullptr;       // pinned mirror of dInfo, then a call's results (kHostResultWords)
+  bool infoClean = false;         // the last call has left dInfo and the counters zero
   bool resInHost = false;         // the last enqueue writes its results there itself
   bool pairsToHost = false;       // the call's pairs go to the host
   int lastPairs = 0;              // pairs of the last call, once read_info has returned
@@ -402,6 +403,7 @@ int v3dm_allocate(v3dm_matcher* h, int nMaxL, int nMaxR, int useGuided) {
   if (nMaxL > V3DM_MAX_FEATURES || nMaxR > V3DM_MAX_FEATURES) return V3DM_ERR_SIZE;
   DeviceGuard g(h->device);
   cudaStreamSynchronize(h->stream);
+  h->infoClean = false;
   free_buffers(h);
   h->nMaxL = nMaxL;
   h->nMaxR = nMaxR;
@@ -415,7 +417,7 @@ int v3dm_allocate(v3dm_matcher* h, int nMaxL, int nMaxR, int useGuided) {
             dalloc(&h->dLBest, (size_t)nMaxL + 1) == cudaSuccess && dalloc(&h->dLSec, (size_t)nMaxL + 1) == cudaSuccess &&
             dalloc(&h->dRBest, (size_t)nMaxR + 1) == cudaSuccess && dalloc(&h->dRSec, (size_t)nMaxR + 1) == cudaSuccess &&
             dalloc(&h->dScratch, (size_t)nMaxL + nMaxR + 1) == cudaSuccess &&
-            dalloc(&h->dPairs, 2 * (size_t)nMin + 2) == cudaSuccess && dalloc(&h->dInfo, kInfoWords + 4) == cudaSuccess &&
+            dalloc(&h->dPairs, 2 * (size_t)nMin + 2) == cudaSuccess && dalloc(&h->dInfo, kInfoWords + kCallCounters) == cudaSuccess &&
             cudaMallocHost(reinterpret_cast<void**>(&h->hInfo),
                            (kInfoWords + kHostResultWords) * sizeof(int32_t)) == cudaSuccess;
   if (ok && h->guidedAlloc)
@@ -936,9 +938,14 @@ int enqueue_match(v3dm_matcher* h, float minScore, float minRatio, int32_t* dPai
   h->lastLaunches = 0;
   h->countWritten = false;
   h->resInHost = false;
-  // the info block and, right after it on the tcgen05 path, the call's counters
-  V3DM_CUDA_TRY(cudaMemsetAsync(h->dInfo, 0, (h->dCounters ? kInfoWords + 4 : kInfoWords) * sizeof(int32_t),
-                                h->stream));
+  // The info block and, right after it on the tcgen05 path, the call's counters.  A call that ends leaves
+  // them zero; one that is captured does not run now and may run after any other, so it clears them itself.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  V3DM_CUDA_TRY(cudaStreamIsCapturing(h->stream, &capture));
+  const bool captured = capture != cudaStreamCaptureStatusNone, wasClean = h->infoClean;
+  if (captured || !wasClean)
+    V3DM_CUDA_TRY(cudaMemsetAsync(h->dInfo, 0, (kInfoWords + kCallCounters) * sizeof(int32_t), h->stream));
+  h->infoClean = captured && wasClean;
   if (h->nGates > 0)
     V3DM_CUDA_TRY(cudaMemcpyAsync(h->dGates, h->gates, sizeof(GateParams) * h->nGates, cudaMemcpyHostToDevice,
                                   h->stream));
@@ -952,7 +959,10 @@ int enqueue_match(v3dm_matcher* h, float minScore, float minRatio, int32_t* dPai
   } else {
     st = enqueue_match_tc(h, minScore, minRatio, dPairs);
   }
-  if (st == V3DM_OK) h->pendingCheck = true;
+  if (st == V3DM_OK) {
+    h->pendingCheck = true;
+    if (!captured && h->resInHost) h->infoClean = true;
+  }
   return st;
 }
 
@@ -1087,6 +1097,7 @@ int v3dm_scores_f32(v3dm_matcher* h, float* scores) {
   const long long n = (long long)h->nL * h->nR;
   if (n > (1LL << 26)) return V3DM_ERR_SIZE;
   if (n == 0) return V3DM_OK;
+  h->infoClean = false;  // an error flag may stay
   DeviceGuard g(h->device);
   V3DM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   {

@@ -36,6 +36,7 @@ constexpr int kInfoPairs = 0;     // number of mutual pairs
 constexpr int kInfoErr = 1;       // device error flags
 constexpr int kInfoMaxSeg = 2;    // largest candidate count of one list segment
 constexpr int kInfoWords = 4;
+constexpr int kCallCounters = 4;  // a pair call's counters, behind the info block
 
 struct MatchArgs {
   int nL, nR;

@@ -271,11 +271,12 @@ __device__ __forceinline__ void put_pair(int2* pairs, const HostResult& host, in
   pairs[at] = p;
   if (host.pairs && at < host.cap) host.pairs[at] = p;
 }
-// The end of a call: its count, and the info block (its other words are from the kernels before).
+// The end of a call: its count and the info block (whose other words are from the kernels before) to the
+// host, and the block and the counters behind it to zero for the next call, which then needs no memset.
 __device__ __forceinline__ void put_count(int32_t* info, int32_t* countOut, const HostResult& host, int total) {
-  info[kInfoPairs] = total;
   if (countOut) *countOut = total;
   for (int w = 0; w < kInfoWords; ++w) host.info[w] = w == kInfoPairs ? total : info[w];
+  for (int w = 0; w < kInfoWords + kCallCounters; ++w) info[w] = 0;
 }
 
 // Pass 1: number of mutual pairs among each block's contiguous range of lefts.
