@@ -973,6 +973,7 @@ struct v3dm_batch {
   bool havePositions = false;
   float* dGate = nullptr;           // kBGateFloats per pair (caller's order)
   long long gateCap = 0;
+  bool gatePairsValid = false;      // the three tables below hold the current pair table
   int2* dPairLR = nullptr;          // per pair (caller's order): left, right image
   long long pairLRCap = 0;
   long long* dStateA0 = nullptr;    // per pair (batch order): first pass-A state
@@ -1477,6 +1478,35 @@ int finish_call(v3dm_batch* b) {
     V3DM_BTRY(cudaStreamSynchronize(b->stream));
     return V3DM_ERR_CANDIDATES;
   }
+  return V3DM_OK;
+}
+
+// What a guided call needs of the pair table: the pairs' images; per batch-order pair its first state and
+// caller index.
+int upload_gate_pairs(v3dm_batch* b) {
+  const int n = b->nPairs;
+  std::vector<int2> lr(n);
+  std::vector<long long> s0(n);
+  std::vector<int> oo(n);
+  for (int p = 0; p < n; ++p) {
+    lr[p] = make_int2(b->pairLi[p], b->pairRi[p]);
+    s0[p] = b->bp[p].stateA0;
+    oo[p] = b->bp[p].orig;
+  }
+  V3DM_BTRY(ensure(&b->dPairLR, &b->pairLRCap, (long long)n));
+  if ((long long)n > b->pairAuxCap) {
+    bfree(b->dStateA0);
+    bfree(b->dOrigOf);
+    b->pairAuxCap = 0;
+    V3DM_BTRY(cudaMalloc(reinterpret_cast<void**>(&b->dStateA0), (size_t)n * sizeof(long long)));
+    V3DM_BTRY(cudaMalloc(reinterpret_cast<void**>(&b->dOrigOf), (size_t)n * sizeof(int)));
+    b->pairAuxCap = n;
+  }
+  V3DM_BTRY(cudaMemcpyAsync(b->dPairLR, lr.data(), lr.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
+  V3DM_BTRY(cudaMemcpyAsync(b->dStateA0, s0.data(), s0.size() * sizeof(long long), cudaMemcpyHostToDevice, b->stream));
+  V3DM_BTRY(cudaMemcpyAsync(b->dOrigOf, oo.data(), oo.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+  V3DM_BTRY(cudaStreamSynchronize(b->stream));
+  b->gatePairsValid = true;
   return V3DM_OK;
 }
 
@@ -2210,6 +2240,7 @@ int v3dm_batch_set_pairs(v3dm_batch* b, int nPairs, const int32_t* pairs) {
   V3DM_BTRY(cudaStreamSynchronize(b->stream));
   drop_graph(b);
   b->havePairs = false;
+  b->gatePairsValid = false;
   for (int i = 0; i < nI; ++i) b->bim[i].pairBeg = b->bim[i].pairEnd = 0;
   for (int k = 0; k < n;) {
     int e = k;
@@ -2309,37 +2340,20 @@ int v3dm_batch_match_guided(v3dm_batch* b, int type, const double* M, const floa
   V3DM_BTRY(cudaStreamSynchronize(b->stream));
   const int n = b->nPairs;
   if (n > 0) {
-    // per pair: the matrix as the reference's float3 rows (.cu:592-595), then thr^2 in float
-    // (.cu:591); the pair's images; per batch-order pair its first state and caller index
+    // per pair: the matrix as the reference's float3 rows (.cu:592-595), then thr^2 in float (.cu:591)
     std::vector<float> gm((size_t)n * kBGateFloats);
-    std::vector<int2> lr(n);
     for (int p = 0; p < n; ++p) {
       for (int i = 0; i < 9; ++i) gm[(size_t)p * kBGateFloats + i] = (float)M[9 * (size_t)p + i];
       gm[(size_t)p * kBGateFloats + 9] = thr[p] * thr[p];
-      lr[p] = make_int2(b->pairLi[p], b->pairRi[p]);
-    }
-    std::vector<long long> s0(n);
-    std::vector<int> oo(n);
-    for (int k = 0; k < n; ++k) {
-      s0[k] = b->bp[k].stateA0;
-      oo[k] = b->bp[k].orig;
     }
     V3DM_BTRY(ensure(&b->dGate, &b->gateCap, (long long)n * kBGateFloats));
-    V3DM_BTRY(ensure(&b->dPairLR, &b->pairLRCap, (long long)n));
-    if ((long long)n > b->pairAuxCap) {
-      bfree(b->dStateA0);
-      bfree(b->dOrigOf);
-      b->pairAuxCap = 0;
-      V3DM_BTRY(cudaMalloc(reinterpret_cast<void**>(&b->dStateA0), (size_t)n * sizeof(long long)));
-      V3DM_BTRY(cudaMalloc(reinterpret_cast<void**>(&b->dOrigOf), (size_t)n * sizeof(int)));
-      b->pairAuxCap = n;
-    }
+    // pageable memory: the copy has left gm when it returns
     V3DM_BTRY(cudaMemcpyAsync(b->dGate, gm.data(), gm.size() * sizeof(float), cudaMemcpyHostToDevice, b->stream));
-    V3DM_BTRY(cudaMemcpyAsync(b->dPairLR, lr.data(), lr.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
-    V3DM_BTRY(cudaMemcpyAsync(b->dStateA0, s0.data(), s0.size() * sizeof(long long), cudaMemcpyHostToDevice,
-                              b->stream));
-    V3DM_BTRY(cudaMemcpyAsync(b->dOrigOf, oo.data(), oo.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-    V3DM_BTRY(cudaStreamSynchronize(b->stream));  // pageable host vectors
+    // the pair table's part is uploaded with the first guided call after set_pairs
+    if (!b->gatePairsValid) {
+      const int st = upload_gate_pairs(b);
+      if (st != V3DM_OK) return st;
+    }
   }
   int st = V3DM_ERR_CANDIDATES;
   for (int attempt = 0; attempt < 6 && st == V3DM_ERR_CANDIDATES; ++attempt) {
