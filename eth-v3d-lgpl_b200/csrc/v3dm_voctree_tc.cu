@@ -186,14 +186,27 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
   // i % kVtcASlots, accumulator i % kAcc, epilogue half i % 2, B buffer j % kBBufs.  (The walk was a
   // cursor advanced at every tile, with two producers and a lane-0 issuer: the waits, branches and
   // operand moves of one tile took longer than its 16 KB of keys.  2M keys on the BF 10, depth 6 tree:
-  // 358 us a call then, 315 now; the streamed phase 54 us, 4.7 TB/s, the gathered ones 103 and 157.)
+  // 358 us a call then, 313 after; the streamed phase 54 us, 4.7 TB/s, the gathered ones 103 and 157, and with
+  // the next items loaded ahead 81 and 133: 273 us a call.)
+  // Every role loads its next item while it works on one (with two tiles to an item, as in a last phase,
+  // the item's load and then its keys' indices were waited for each time).
+  const int4 none = make_int4(0, 0, 0, 0);
+  auto next_item = [&](int it) { return it + (int)gridDim.x < nIt ? item_at(it + (int)gridDim.x) : none; };
+  const int4 first = (int)blockIdx.x < nIt ? item_at(blockIdx.x) : none;
   if (warp < kVtcProducers) {
     // ---------------- producers ----------------
     const int row0 = warp * 32;
     uint32_t i = 0, j = 0;
     bool ok = run;
-    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j) {
-      const int4 item = item_at(it);
+    // the lane's row of tile t of an item: its key
+    auto load_key = [&](const int4& item, int t) -> int {
+      const int pos = t * kVtcRows + row0 + lane;
+      return pos < item.z ? __ldg(a.perm + item.y + pos) : 0;
+    };
+    int4 item = first, after;
+    int mine = gathered ? load_key(item, 0) : 0;
+    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j, item = after) {
+      after = next_item(it);
       if (warp == 0) {
         const uint32_t buf = j % S::kBBufs;
         ok = mbar_wait_warp(&s.emptyB[buf], ((j / S::kBBufs) & 1u) ^ 1u, &s.abort, a.err);
@@ -227,15 +240,9 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
           }
         continue;
       }
-      // the lane's row of tile t: its key
-      auto load_key = [&](int t) -> int {
-        const int pos = t * kVtcRows + row0 + lane;
-        return pos < item.z ? __ldg(a.perm + item.y + pos) : 0;
-      };
-      int mine = load_key(0);
       for (int t = 0; t < tiles; ++t, ++i) {
         const uint32_t slot = i % kVtcASlots;
-        const int next = t + 1 < tiles ? load_key(t + 1) : 0;
+        const int next = t + 1 < tiles ? load_key(item, t + 1) : load_key(after, 0);
         ok = mbar_wait_warp(&s.done[slot], ((i / kVtcASlots) & 1u) ^ 1u, &s.abort, a.err);
         if (!ok) break;
         // eight lanes per 128-byte row, four rows per instruction; rows past the item keep what is there
@@ -276,8 +283,9 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
     const uint32_t aBase = sdesc_lo(smem_u32(s.a[0])), bBase = sdesc_lo(smem_u32(s.b[0]));
     uint32_t i = 0, j = 0;
     bool ok = run;
-    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j) {
-      const int4 item = item_at(it);
+    int4 item = first, after;
+    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j, item = after) {
+      after = next_item(it);
       const uint32_t buf = j % S::kBBufs;
       ok = mbar_wait_warp(&s.fullB[buf], (j / S::kBBufs) & 1u, &s.abort, a.err);
       const uint32_t bd = bBase + buf * (uint32_t)(S::kBBytes >> 4);
@@ -321,8 +329,9 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
     const int row = q * 32 + lane;
     uint32_t i0 = 0;                         // the item's first tile
     bool ok = run;
-    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x) {
-      const int4 item = item_at(it);
+    int4 item = first, after;
+    for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, item = after) {
+      after = next_item(it);
       const int tiles = (item.z + kVtcRows - 1) / kVtcRows;
       const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + item.x;
       const long long g1 = (r + 1) * BF;
