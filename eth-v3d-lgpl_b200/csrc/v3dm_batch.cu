@@ -25,7 +25,7 @@
 // second value the side pass could only bound.
 // Float descriptors that are not all of the form u/512 (v3dm_batch_set_images_f32) take the same
 // passes on the BF16 hi/lo layouts of the single-pair float matcher (v3dm_match_f.cu): groups of
-// 128 lefts against tiles of 128 columns, each descriptor's exact best and second over the other
+// up to 256 lefts against tiles of 128 columns, each descriptor's exact best and second over the other
 // image kept in registers (a guided call masks them with the pair's gate) and decided with the
 // float rules, so each pair's result equals that matcher's.
 // Every launch after the first reads its sizes from device memory, so the whole sequence is
@@ -92,7 +92,7 @@ constexpr int kBMutPerBlock = 2048;
 
 // Copies each image's descriptors to its padded place and zeroes its padding rows.  Block (x, y):
 // rows 256 x .. of image y, eight loads of a thread in flight (one block per image was bound by its
-// own SM: 24 images 44 us, 200 images 226 us).
+// own SM: 24 images 44 us, 60 images 128 us; 5.5 and 17 us now).
 __global__ void __launch_bounds__(256)
 k_bscatter(const uint8_t* __restrict__ src, const long long* __restrict__ srcOff, const BImage* __restrict__ im,
            int nImages, uint8_t* __restrict__ dst) {
@@ -481,7 +481,7 @@ k_pscan_cells(const int* __restrict__ cntA, const int* __restrict__ cntB, int n,
 // result depends on the index maps, not on the order).  Block (x, y): rows 256 x .. of image y.  It
 // counts its rows per cell, takes the places of each cell with one atomic, and copies each row with
 // eight lanes, read once and written probesL + probesR times.  What bounds it is the writes; one
-// block per image, a thread per row, took 480 us for 60 images of 8000 with 4 + 4 probes, 2.2 GB/ms.
+// block per image, a thread per row, took 480 us for 60 images of 8000 with 4 + 4 probes, this 129 us.
 constexpr int kPScatterRows = 256;
 __global__ void __launch_bounds__(kPScatterRows)
 k_pscatter(const BImage* __restrict__ im, int nImages, const uint8_t* __restrict__ cell, int probes, int probesL,

@@ -172,7 +172,7 @@ __device__ __forceinline__ uint32_t f32_to_u8_checked(float v, bool& ok) {
 
 // Four float4 of a thread in flight.  Once some value is known not to be of the form u/512 the result
 // is of no use (the caller takes the float path), so blocks that start later leave at once, and a
-// warp reports with one atomic: 180000 such descriptors took 130 us with an atomic per thread.
+// warp reports with one atomic: 180000 such descriptors took 130 us with an atomic per thread, 34 now.
 constexpr int kF32PerThread = 4;
 __global__ void __launch_bounds__(256)
 k_f32_to_u8(const float4* __restrict__ src, uint32_t* __restrict__ dst, long long n4, int* err) {

@@ -11,8 +11,9 @@
 //              side that can matter, with the gates; k_rescore_decide then decides them.
 //   k_choose   rights accepted by some left, de-duplicated, descriptors gathered for the
 //              second side pass (the mutual filter only ever reads these rights).
-//   k_mutual_count / k_mutual_write
-//              mutual filter (.cu:546-551) with an ordered compaction (ascending left).
+//   k_mutual_small, or k_mutual_count / k_mutual_write
+//              mutual filter (.cu:546-551) with an ordered compaction (ascending left); the end of a
+//              call: its results to the host, its info block cleared.
 #include <algorithm>
 
 #include "v3dm_device.cuh"
@@ -233,7 +234,7 @@ __global__ void k_rescore_decide(RescoreArgs a) {
 }
 
 // A row is 'planes' blocks of 128 bytes, block p of row r at (p * cap + r) * 128 (one block:
-// uint8 descriptors; six: the planar BF16 hi/lo layout).
+// uint8 descriptors; four: the planar BF16 hi/lo layout).
 __global__ void k_choose(const int32_t* __restrict__ leftDec, int nL, int* chosenFlag, int* chosenList,
                          int* chosenCount, const uint8_t* __restrict__ dR, uint8_t* __restrict__ dRc, int planes,
                          int capSrc, int capDst) {
