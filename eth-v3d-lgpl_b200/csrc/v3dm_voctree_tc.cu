@@ -63,12 +63,18 @@ struct VtcShape {
   static constexpr int N1 = 16;                         // children columns
   static constexpr int kRowsB = N2 + N1;                // B rows: grandchildren, then children
   static constexpr int kAccCols = N2 + N1;
-  static constexpr int kAcc = kVtcTmemCols / kAccCols;  // accumulator stages
+  // accumulator stages (narrow trees would fit 10 or 16; see the assertion)
+  static constexpr int kAcc = std::min(kVtcTmemCols / kAccCols, kVtcASlots);
   static constexpr int kABytes = kVtcRows * kDescBytes;
   static constexpr int kBBytes = kRowsB * kDescBytes;
   static constexpr int kBBufs = kBBytes <= 16384 ? 4 : 2;  // subtree ring depth
   static_assert(BF >= 2 && BF <= 15, "branching factor");
   static_assert(kAcc >= 2, "two accumulator stages");
+  // The epilogue takes tile i when done[i % kVtcASlots] completes for it, so tile i + kVtcASlots must not
+  // complete before every epilogue warp has seen tile i.  The issuer goes in order and waits for tile i's
+  // hand-back before tile i + kAcc; with more stages than slots it could pass tile i + kVtcASlots first,
+  // and a late warp would wait for a phase that needs its own hand-back.
+  static_assert(kVtcASlots >= kAcc, "the done ring is at least as deep as the accumulator ring");
 };
 
 template <int BF>

@@ -232,3 +232,22 @@ def test_device_calls_reject_misaligned_buffers(v3dm_mod):
         st = L.v3dm_voctree_quantize_f32_device(t._h, n, C.c_void_p(fk.data_ptr() + 4), C.c_void_p(base_i), 0)
         assert st == v3dm_mod.ERR_ARG
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("bf,depth", [(2, 8), (3, 5), (4, 4), (5, 4)])
+def test_tensor_descent_of_narrow_trees_with_many_tiles(v3dm_mod, oracle_mod, bf, depth):
+    """Narrow byte trees with more than fifty 128-key tiles per CTA and phase: the key-tile ring turns over many times
+    (narrow trees have the most room for accumulators, and their epilogue lags the MMAs the furthest).
+    The second call finds its keys in L2."""
+    n = 1_000_003
+    rng = synth.rng_for(8100 + bf)
+    nodes = rng.integers(0, 256, (v3dm_mod.voctree_counts(bf, depth)[0], 128)).astype(np.uint8)
+    keys = rng.integers(0, 256, (n, 128), dtype=np.uint8)
+    exp = oracle_mod.voctree(bf, depth, nodes, keys, False)
+    with v3dm_mod.VocabularyTreeTraversal(bf, depth) as t:
+        t.allocate(n)
+        t.set_nodes(nodes)
+        for m in (n, 300_000):  # 38 MB of keys: in L2 for the second call of the shorter ones
+            for _ in range(2):
+                np.testing.assert_array_equal(t.traverse_tree(keys[:m], v3dm_mod.LEAF_LOCAL), exp[:m])
+                assert t.last_launches() > 1
