@@ -191,7 +191,11 @@ struct VtcArgs {
   long long nextBase;
   int* hist;
   int bins;
-  int* err;
+  int* err;                      // error word of the call: a phase after the first does nothing once it is set
+  // failure-path test hooks (zero in production): the bounded waits give up after waitLimit cycles (0: the
+  // default), and CTA 0 does not load the node rows of its skipLoad-th item (0: none)
+  long long waitLimit;
+  int skipLoad;
 };
 bool vtc_supported(int bf);
 // Rows of the tree read by the phases: a tensor map over the node rows with boxes of kVtcBoxRows;
@@ -227,7 +231,9 @@ struct VtfArgs {
   int* nFlagged;
   int32_t* weird;                // null after the first phase
   int* nWeird;
-  int* err;
+  int* err;                      // as in VtcArgs
+  long long waitLimit;
+  int skipLoad;
 };
 int vtf_levels(int bf);          // levels a phase descends (0: shape not supported)
 constexpr int kVtfRowBytes = 512;  // split planes per node or key

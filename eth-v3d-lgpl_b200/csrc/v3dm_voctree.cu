@@ -156,12 +156,14 @@ k_vt_scan(const int* __restrict__ hist, int bins, int itemKeys, int* __restrict_
 
 // Keys in bucket order.  Each CTA takes a contiguous range of keys, counts them per bucket in
 // shared memory, reserves its slots of every bucket with one global atomic per bucket, and
-// places its keys with shared-memory ranks (the order within a bucket does not matter).
+// places its keys with shared-memory ranks (the order within a bucket does not matter).  Does nothing
+// when the phase before gave up on a wait (*err): some keys then have no bucket.
 constexpr int kVtScatterThreads = 1024;
 __global__ void __launch_bounds__(kVtScatterThreads)
 k_vt_scatter(const int32_t* __restrict__ bucket, int n, const int* __restrict__ off, int* __restrict__ cursor,
-             int32_t* __restrict__ perm, int bins) {
+             int32_t* __restrict__ perm, int bins, const int* __restrict__ err) {
   extern __shared__ int vtScatterSmem[];  // 2 x bins when bins <= kVtLocalBins
+  if (*err) return;
   int* cnt = vtScatterSmem;
   int* base = vtScatterSmem + bins;
   const long long per = ((long long)n + gridDim.x - 1) / gridDim.x;
@@ -371,8 +373,11 @@ struct v3dm_voctree {
   uint8_t* dKeys = nullptr;
   float* dStage = nullptr;
   int32_t* dIds = nullptr;
-  int32_t* dErr = nullptr;
-  int32_t* hErr = nullptr;
+  int32_t* dErr = nullptr;      // flags of the one-kernel descents and conversions, until they are read
+  int32_t* dPhaseErr = nullptr; // flags of the phases; the word before dHist, cleared with its counts by each call
+  int32_t* hErr = nullptr;      // pinned mirror of both
+  long long testWaitLimit = 0;  // failure-path test hooks of the first phase (v3dm_voctree_test_wait_fault)
+  int testSkipLoad = 0;
   unsigned long long* dReplays = nullptr;  // key-levels resolved by the sequential replay
   // tensor-core descent of u8 trees in phases of two levels (tcPath false: one-kernel descent)
   bool tcPath = false;
@@ -380,9 +385,10 @@ struct v3dm_voctree {
   long long maxBins = 1;        // buckets of the last phase
   int32_t* dBucket = nullptr;   // nMax: per key, the bucket it reached
   int32_t* dPerm = nullptr;     // nMax: keys in bucket order
-  int* dHist = nullptr;         // maxBins counts, then maxBins cursors
+  int* dErrHist = nullptr;      // two spare words, dErr, dPhaseErr, dHist
+  int* dHist = nullptr;         // vt_bins counts, then as many cursors
   int* dOff = nullptr;          // maxBins + 1
-  int4* dItems = nullptr;       // nMax / kVtItemKeys + maxBins + 1
+  int4* dItems = nullptr;       // nMax / kVtMinItem + vt_bins + 1
   int* dNItems = nullptr;
   int numSMs = 148;
   int lastLaunches = 0;         // kernels launched by the last quantization
@@ -448,6 +454,14 @@ bool vt_f_wanted(const v3dm_voctree* t, long long n) { return t->fLevels > 0 && 
 
 int vt_sort(v3dm_voctree* t, int n, long long bins, int itemKeys);
 
+// The counts of the next phase's buckets to zero, and before a call's first phase its error word, which
+// only the phases after the first read.
+int vt_clear_hist(v3dm_voctree* t, long long bins, bool first) {
+  int* from = first ? t->dPhaseErr : t->dHist;
+  const size_t words = (size_t)bins + (first ? 1 : 0);
+  return cudaMemsetAsync(from, 0, words * sizeof(int), t->stream) == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
+}
+
 int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int idMode) {
   t->lastLaunches = 0;
   if (n == 0) return V3DM_OK;
@@ -490,7 +504,8 @@ int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int i
   va.leafBase = t->leafBase;
   va.next = t->dBucket;
   va.hist = t->dHist;
-  va.err = t->dErr;
+  va.err = t->dPhaseErr;
+  va.waitLimit = t->testWaitLimit;
   long long bins = 1;
   for (int p = 0; p < t->phases; ++p) {
     const int levels = std::min(2, t->depth - 2 * p);
@@ -501,9 +516,9 @@ int vt_launch(v3dm_voctree* t, int n, const uint8_t* dKeys, int32_t* dIds, int i
       const int st = vt_sort(t, n, bins, kVtItemKeys);
       if (st != V3DM_OK) return st;
     }
-    if (!last && cudaMemsetAsync(t->dHist, 0, (size_t)nextBins * sizeof(int), t->stream) != cudaSuccess)
-      return V3DM_ERR_CUDA;
+    if (!last && vt_clear_hist(t, nextBins, p == 0) != V3DM_OK) return V3DM_ERR_CUDA;
     va.levels = levels;
+    va.skipLoad = p == 0 ? t->testSkipLoad : 0;
     va.singleN = p == 0 ? n : 0;  // the first phase: one bucket (the root), items implied
     va.bucketBase = p == 0 ? -1 : level_start(bf, 2 * p);
     va.perm = p == 0 ? nullptr : t->dPerm;
@@ -526,7 +541,8 @@ int vt_sort(v3dm_voctree* t, int n, long long bins, int itemKeys) {
   const unsigned sg =
       (unsigned)std::max<long long>(1, std::min<long long>(((long long)n + 4095) / 4096, (long long)t->numSMs * 2));
   const size_t ssm = bins <= kVtLocalBins ? 2 * (size_t)bins * sizeof(int) : 0;
-  k_vt_scatter<<<sg, kVtScatterThreads, ssm, t->stream>>>(t->dBucket, n, t->dOff, cursor, t->dPerm, (int)bins);
+  k_vt_scatter<<<sg, kVtScatterThreads, ssm, t->stream>>>(t->dBucket, n, t->dOff, cursor, t->dPerm, (int)bins,
+                                                          t->dPhaseErr);
   return cudaGetLastError() == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
 }
 
@@ -566,7 +582,8 @@ int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int
   va.hist = t->dHist;
   va.flagged = t->dFlagged;
   va.nWeird = t->dFCounts;
-  va.err = t->dErr;
+  va.err = t->dPhaseErr;
+  va.waitLimit = t->testWaitLimit;
   long long bins = 1;
   for (int p = 0; p < t->fPhases; ++p) {
     const int d0 = p * t->fLevels;
@@ -578,9 +595,9 @@ int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int
       const int st = vt_sort(t, n, bins, va.itemKeys);
       if (st != V3DM_OK) return st;
     }
-    if (!last && cudaMemsetAsync(t->dHist, 0, (size_t)nextBins * sizeof(int), t->stream) != cudaSuccess)
-      return V3DM_ERR_CUDA;
+    if (!last && vt_clear_hist(t, nextBins, p == 0) != V3DM_OK) return V3DM_ERR_CUDA;
     va.levels = levels;
+    va.skipLoad = p == 0 ? t->testSkipLoad : 0;
     va.singleN = p == 0 ? n : 0;
     va.bucketBase = p == 0 ? -1 : level_start(t->bf, d0);
     va.perm = p == 0 ? nullptr : t->dPerm;
@@ -671,15 +688,16 @@ int vt_planes(v3dm_voctree* t) {
   return V3DM_OK;
 }
 
+// Waits for the calls enqueued so far and reports what their kernels flagged; clears the flags.
 int vt_check_err(v3dm_voctree* t) {
-  if (cudaMemcpyAsync(t->hErr, t->dErr, sizeof(int32_t), cudaMemcpyDeviceToHost, t->stream) != cudaSuccess ||
+  if (cudaMemcpyAsync(t->hErr, t->dErr, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, t->stream) != cudaSuccess ||
       cudaStreamSynchronize(t->stream) != cudaSuccess)
     return V3DM_ERR_CUDA;
-  if (*t->hErr & kErrBadTree) {
-    cudaMemsetAsync(t->dErr, 0, sizeof(int32_t), t->stream);
-    return V3DM_ERR_ARG;
-  }
-  return V3DM_OK;
+  const int32_t err = t->hErr[0] & kErrBadTree, phases = t->hErr[1];
+  if (!err && !phases) return V3DM_OK;
+  if (cudaMemsetAsync(t->dErr, 0, 2 * sizeof(int32_t), t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
+  if (phases & kErrWaitTimeout) return V3DM_ERR_TIMEOUT;
+  return (err | phases) & kErrBadTree ? V3DM_ERR_ARG : V3DM_ERR_CUDA;
 }
 
 }  // namespace
@@ -716,14 +734,13 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
   vt_plan(t);
   DeviceGuardVt g(device);
   if (cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(reinterpret_cast<void**>(&t->dErr), sizeof(int32_t)) != cudaSuccess ||
-      cudaMallocHost(reinterpret_cast<void**>(&t->hErr), sizeof(int32_t)) != cudaSuccess ||
+      cudaMalloc(reinterpret_cast<void**>(&t->dErrHist), (4 + 2 * (size_t)vt_bins(t)) * sizeof(int)) != cudaSuccess ||
+      cudaMallocHost(reinterpret_cast<void**>(&t->hErr), 2 * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&t->dReplays), sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMemsetAsync(t->dErr, 0, sizeof(int32_t), t->stream) != cudaSuccess ||
+      cudaMemsetAsync(t->dErrHist, 0, 4 * sizeof(int), t->stream) != cudaSuccess ||
       cudaMemsetAsync(t->dReplays, 0, sizeof(unsigned long long), t->stream) != cudaSuccess ||
       (vt_bins(t) > 0 &&
-       (cudaMalloc(reinterpret_cast<void**>(&t->dHist), 2 * (size_t)vt_bins(t) * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&t->dOff), ((size_t)vt_bins(t) + 1) * sizeof(int)) != cudaSuccess ||
+       (cudaMalloc(reinterpret_cast<void**>(&t->dOff), ((size_t)vt_bins(t) + 1) * sizeof(int)) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&t->dMaxNorm), sizeof(float)) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&t->dFCounts), (1 + kVtMaxPhases) * sizeof(int)) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&t->dNItems), sizeof(int)) != cudaSuccess ||
@@ -731,10 +748,9 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
                              2 * kVtLocalBins * (int)sizeof(int)) != cudaSuccess)) ||
       cudaStreamSynchronize(t->stream) != cudaSuccess) {
     if (t->stream) cudaStreamDestroy(t->stream);
-    if (t->dErr) cudaFree(t->dErr);
+    if (t->dErrHist) cudaFree(t->dErrHist);
     if (t->hErr) cudaFreeHost(t->hErr);
     if (t->dReplays) cudaFree(t->dReplays);
-    if (t->dHist) cudaFree(t->dHist);
     if (t->dOff) cudaFree(t->dOff);
     if (t->dNItems) cudaFree(t->dNItems);
     if (t->dMaxNorm) cudaFree(t->dMaxNorm);
@@ -742,6 +758,9 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
     delete t;
     return V3DM_ERR_CUDA;
   }
+  t->dErr = t->dErrHist + 2;
+  t->dPhaseErr = t->dErrHist + 3;
+  t->dHist = t->dErrHist + 4;
   *out = t;
   return V3DM_OK;
 }
@@ -754,7 +773,7 @@ int v3dm_voctree_destroy(v3dm_voctree* t) {
   if (t->dNodesF) cudaFree(t->dNodesF);
   if (t->dNorm) cudaFree(t->dNorm);
   if (t->dReplays) cudaFree(t->dReplays);
-  if (t->dHist) cudaFree(t->dHist);
+  if (t->dErrHist) cudaFree(t->dErrHist);
   if (t->dOff) cudaFree(t->dOff);
   if (t->dNItems) cudaFree(t->dNItems);
   if (t->dBucket) cudaFree(t->dBucket);
@@ -769,7 +788,6 @@ int v3dm_voctree_destroy(v3dm_voctree* t) {
   if (t->dKeys) cudaFree(t->dKeys);
   if (t->dStage) cudaFree(t->dStage);
   if (t->dIds) cudaFree(t->dIds);
-  if (t->dErr) cudaFree(t->dErr);
   if (t->hErr) cudaFreeHost(t->hErr);
   cudaStreamDestroy(t->stream);
   delete t;
@@ -929,6 +947,20 @@ int v3dm_voctree_quantize_f32_device(v3dm_voctree* t, int n, const float* d_keys
   int st = vt_ensure_float_tree(t);
   if (st != V3DM_OK) return st;
   return vt_launch_f32(t, n, d_keys, d_ids, idMode);
+}
+
+int v3dm_voctree_wait(v3dm_voctree* t) {
+  if (!t) return V3DM_ERR_ARG;
+  DeviceGuardVt g(t->device);
+  return vt_check_err(t);
+}
+
+int v3dm_voctree_test_wait_fault(v3dm_voctree* t, long long waitCycles, int skipLoad) {
+  if (!t || waitCycles < 0 || skipLoad < 0) return V3DM_ERR_ARG;
+  if (skipLoad > 0 && waitCycles == 0) return V3DM_ERR_ARG;  // a skipped load needs a short wait limit
+  t->testWaitLimit = waitCycles;
+  t->testSkipLoad = skipLoad;
+  return V3DM_OK;
 }
 
 int v3dm_voctree_replays(v3dm_voctree* t, long long* n) {

@@ -27,7 +27,8 @@
 // Roles (one persistent CTA per SM, 9 warps): warps 0-3 gather the tile's split key rows (512 bytes
 // each, through the permutation) with cp.async, 16 bytes a lane, into the MMA's swizzled planes, and
 // their norms; warp 0 also loads an item's node rows with TMA (pre-split planes); warp 4 issues;
-// warps 5-8 read the scores, one key per lane.  Every wait is bounded as in k_side.
+// warps 5-8 read the scores, one key per lane.  Every wait is bounded as in k_side; after one that
+// runs out, the phases behind it do nothing (as in the byte descent).
 //
 // What bounds it: reading the keys once per phase (and writing them once).  300,007 keys on a BF 50,
 // depth 3 tree (125,000 leaves): 184 us a call, 2166 with k_voctree_f32; the split 45 us (6.8 TB/s),
@@ -133,7 +134,8 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
   extern __shared__ uint8_t vtfRaw[];
   VtfSmem& s = *reinterpret_cast<VtfSmem*>((reinterpret_cast<uintptr_t>(vtfRaw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nIt = a.singleN > 0 ? (a.singleN + a.itemKeys - 1) / a.itemKeys : *a.nItems;
+  const long long lim = a.waitLimit > 0 ? a.waitLimit : kWaitCycles;
+  int nIt = a.singleN > 0 ? (a.singleN + a.itemKeys - 1) / a.itemKeys : *a.nItems;
   const bool localHist = !a.final && a.bins <= kVfLocalBins;
   // B rows: one level, the children (N = BF rounded up to 16); two, N2 = BF^2 rounded up to 16 rows
   // of grandchildren and then 16 of children
@@ -158,7 +160,7 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
       mbar_init(&s.emptyB[i], 1);
     }
     mbar_init(&s.mmaDone, 1);
-    s.abort = 0;
+    s.abort = a.singleN > 0 ? 0 : *a.err != 0;  // an earlier phase gave up: there are no items
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (localHist)
@@ -173,21 +175,24 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s.tmemBase;
+  const bool run = !s.abort;
+  if (!run) nIt = 0;
 
   // Tiles are numbered from 0 in every role (i), items likewise (j): A slot i % 2, accumulator and
   // done barrier i % 4, norms i % 8, B buffer j % nBufs.
   if (warp < kVfProducers) {
     // ---------------- producers: 32 rows of every tile each ----------------
     const int row0 = warp * 32;
+    const uint32_t skip = blockIdx.x == 0 ? (uint32_t)a.skipLoad - 1u : 0xffffffffu;
     uint32_t i = 0, j = 0;
-    bool ok = true;
+    bool ok = run;
     for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j) {
       const int4 item = item_at(it);
       if (warp == 0) {
         const uint32_t buf = j % nBufs;
-        ok = mbar_wait_warp(&s.emptyB[buf], ((j / nBufs) & 1u) ^ 1u, &s.abort, a.err);
+        ok = mbar_wait_warp(&s.emptyB[buf], ((j / nBufs) & 1u) ^ 1u, &s.abort, a.err, lim);
         if (!ok) break;
-        if (lane == 0) {
+        if (lane == 0 && j != skip) {
           const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + item.x;
           const long long g1 = (r + 1) * bf, g2 = (g1 + 1) * bf;
           uint8_t* b = s.b + buf * bufBytes;
@@ -215,7 +220,7 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
         // the norms of tile i - 8.
         if (i >= kVfASlots) {
           const uint32_t d = i - kVfASlots;
-          ok = mbar_wait_warp(&s.done[d % kVfAcc], (d / kVfAcc) & 1u, &s.abort, a.err);
+          ok = mbar_wait_warp(&s.done[d % kVfAcc], (d / kVfAcc) & 1u, &s.abort, a.err, lim);
           if (!ok) break;
         }
         const int next = t + 1 < tiles ? load_key(t + 1) : -1;
@@ -244,7 +249,7 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
     if (warp == 0 && lane == 0)
       for (uint32_t k = j > nBufs ? j - nBufs : 0u; k < j; ++k) {
         const long long t0 = clock64();
-        while (!mbar_try(&s.fullB[k % nBufs], (k / nBufs) & 1u) && clock64() - t0 < kWaitCycles) {
+        while (k != skip && !mbar_try(&s.fullB[k % nBufs], (k / nBufs) & 1u) && clock64() - t0 < kWaitCycles) {
         }
       }
   } else if (warp == kVfMmaWarp) {
@@ -254,16 +259,16 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
     const uint32_t aBase = sdesc_lo(smem_u32(s.a[0])), bBase = sdesc_lo(smem_u32(s.b));
     const uint32_t bPlane = (uint32_t)(N * 128) >> 4;
     uint32_t i = 0, j = 0;
-    bool ok = true;
+    bool ok = run;
     for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j) {
       const int4 item = item_at(it);
       const uint32_t buf = j % nBufs;
-      ok = mbar_wait_warp(&s.fullB[buf], (j / nBufs) & 1u, &s.abort, a.err);
+      ok = mbar_wait_warp(&s.fullB[buf], (j / nBufs) & 1u, &s.abort, a.err, lim);
       const uint32_t bd = bBase + buf * ((uint32_t)bufBytes >> 4);
       const uint32_t iEnd = i + (uint32_t)((item.z + kVfRows - 1) / kVfRows);
       for (; i < iEnd && ok; ++i) {
-        ok = mbar_wait_warp(&s.fullA[i % kVfASlots], (i / kVfASlots) & 1u, &s.abort, a.err) &&
-             mbar_wait_warp(&s.accEmpty[i % kVfAcc], ((i / kVfAcc) & 1u) ^ 1u, &s.abort, a.err);
+        ok = mbar_wait_warp(&s.fullA[i % kVfASlots], (i / kVfASlots) & 1u, &s.abort, a.err, lim) &&
+             mbar_wait_warp(&s.accEmpty[i % kVfAcc], ((i / kVfAcc) & 1u) ^ 1u, &s.abort, a.err, lim);
         if (!ok) break;
         tc_fence_after();
         const uint32_t ad = aBase + (i % kVfASlots) * (uint32_t)(kVfABytes >> 4);
@@ -297,7 +302,7 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
     const int row = q * 32 + lane;
     const float maxNorm = *a.maxNorm;
     uint32_t i = 0;
-    bool ok = true;
+    bool ok = run;
     for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x) {
       const int4 item = item_at(it);
       const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + item.x;
@@ -307,7 +312,7 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
       for (int t = 0; t < tiles; ++t, ++i) {
         const int pos = t * kVfRows + row;
         const int key = pos < item.z ? (a.perm ? __ldg(a.perm + item.y + pos) : item.y + pos) : -1;
-        ok = mbar_wait_warp(&s.done[i % kVfAcc], (i / kVfAcc) & 1u, &s.abort, a.err);
+        ok = mbar_wait_warp(&s.done[i % kVfAcc], (i / kVfAcc) & 1u, &s.abort, a.err, lim);
         if (!ok) break;
         tc_fence_after();
         const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (i % kVfAcc) * 128u;

@@ -33,7 +33,8 @@
 //               512 / (N2 + 16) accumulator stages (the warp walks, one elected lane issues);
 //   warps 5-12  epilogue, two warps per TMEM lane quadrant taking alternate tiles.
 // Every mbarrier wait is bounded (kWaitCycles); on timeout the CTA records kErrWaitTimeout,
-// drains its own copies and MMAs, frees TMEM and returns.
+// drains its own copies and MMAs, frees TMEM and returns.  Its keys then have no bucket, so the
+// phases behind it, whose items and permutation would be made of them, do nothing.
 #include <cuda.h>
 
 #include <algorithm>
@@ -146,7 +147,8 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
   extern __shared__ uint8_t vtcRaw[];
   VtcSmem<BF>& s = *reinterpret_cast<VtcSmem<BF>*>((reinterpret_cast<uintptr_t>(vtcRaw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nIt = a.singleN > 0 ? (a.singleN + kVtcItemKeys - 1) / kVtcItemKeys : *a.nItems;
+  const long long lim = a.waitLimit > 0 ? a.waitLimit : kWaitCycles;
+  int nIt = a.singleN > 0 ? (a.singleN + kVtcItemKeys - 1) / kVtcItemKeys : *a.nItems;
   const bool localHist = !a.final && a.bins <= kVtcLocalBins;
   const bool gathered = a.perm != nullptr;
   // item `it`: (bucket, first position, keys)
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
     }
     for (int i = 0; i < S::kAcc; ++i) mbar_init(&s.accEmpty[i], 4);  // the four warps of the half that takes the tile
     mbar_init(&s.mmaDone, 1);
-    s.abort = 0;
+    s.abort = a.singleN > 0 ? 0 : *a.err != 0;  // an earlier phase gave up: there are no items
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (localHist)
@@ -187,6 +189,7 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
   }
   __syncthreads();
   const bool run = !s.abort;
+  if (!run) nIt = 0;
 
   // Tiles are numbered from 0 in every role (i), items likewise (j): A slot and done barrier
   // i % kVtcASlots, accumulator i % kAcc, epilogue half i % 2, B buffer j % kBBufs.  (The walk was a
@@ -202,6 +205,7 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
   if (warp < kVtcProducers) {
     // ---------------- producers ----------------
     const int row0 = warp * 32;
+    const uint32_t skip = blockIdx.x == 0 ? (uint32_t)a.skipLoad - 1u : 0xffffffffu;
     uint32_t i = 0, j = 0;
     bool ok = run;
     // the lane's row of tile t of an item: its key
@@ -215,9 +219,9 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
       after = next_item(it);
       if (warp == 0) {
         const uint32_t buf = j % S::kBBufs;
-        ok = mbar_wait_warp(&s.emptyB[buf], ((j / S::kBBufs) & 1u) ^ 1u, &s.abort, a.err);
+        ok = mbar_wait_warp(&s.emptyB[buf], ((j / S::kBBufs) & 1u) ^ 1u, &s.abort, a.err, lim);
         if (!ok) break;
-        if (lane == 0) {
+        if (lane == 0 && j != skip) {
           // subtree of the item's bucket node r: children from g1 (buffer rows N2 ..), and
           // grandchildren from g2 (buffer rows 0 .. N2 - 1)
           const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + item.x;
@@ -236,7 +240,7 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
         if (warp == 0)  // consecutive keys: one TMA tile (rows past the last key read as zero)
           for (int t = 0; t < tiles; ++t, ++i) {
             const uint32_t slot = i % kVtcASlots;
-            ok = mbar_wait_warp(&s.done[slot], ((i / kVtcASlots) & 1u) ^ 1u, &s.abort, a.err);
+            ok = mbar_wait_warp(&s.done[slot], ((i / kVtcASlots) & 1u) ^ 1u, &s.abort, a.err, lim);
             if (!ok) break;
             if (lane == 0) {
               mbar_expect_tx(&s.fullA[slot], (uint32_t)S::kABytes);
@@ -249,7 +253,7 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
       for (int t = 0; t < tiles; ++t, ++i) {
         const uint32_t slot = i % kVtcASlots;
         const int next = t + 1 < tiles ? load_key(item, t + 1) : load_key(after, 0);
-        ok = mbar_wait_warp(&s.done[slot], ((i / kVtcASlots) & 1u) ^ 1u, &s.abort, a.err);
+        ok = mbar_wait_warp(&s.done[slot], ((i / kVtcASlots) & 1u) ^ 1u, &s.abort, a.err, lim);
         if (!ok) break;
         // eight lanes per 128-byte row, four rows per instruction; rows past the item keep what is there
         const int have = item.z - t * kVtcRows - row0;
@@ -274,7 +278,8 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
     if (warp == 0 && lane == 0) {
       for (uint32_t k = j > (uint32_t)S::kBBufs ? j - S::kBBufs : 0u; k < j; ++k) {
         const long long t0 = clock64();
-        while (!mbar_try(&s.fullB[k % S::kBBufs], (k / S::kBBufs) & 1u) && clock64() - t0 < kWaitCycles) {
+        while (k != skip && !mbar_try(&s.fullB[k % S::kBBufs], (k / S::kBBufs) & 1u) &&
+               clock64() - t0 < kWaitCycles) {
         }
       }
       for (uint32_t k = i > (uint32_t)kVtcASlots ? i - kVtcASlots : 0u; !gathered && k < i; ++k) {
@@ -293,13 +298,13 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
     for (int it = blockIdx.x; it < nIt && ok; it += gridDim.x, ++j, item = after) {
       after = next_item(it);
       const uint32_t buf = j % S::kBBufs;
-      ok = mbar_wait_warp(&s.fullB[buf], (j / S::kBBufs) & 1u, &s.abort, a.err);
+      ok = mbar_wait_warp(&s.fullB[buf], (j / S::kBBufs) & 1u, &s.abort, a.err, lim);
       const uint32_t bd = bBase + buf * (uint32_t)(S::kBBytes >> 4);
       const uint32_t iEnd = i + (uint32_t)((item.z + kVtcRows - 1) / kVtcRows);
       for (; i < iEnd && ok; ++i) {
         const uint32_t slot = i % kVtcASlots, acc = i % S::kAcc;
-        ok = mbar_wait_warp(&s.fullA[slot], (i / kVtcASlots) & 1u, &s.abort, a.err) &&
-             mbar_wait_warp(&s.accEmpty[acc], ((i / S::kAcc) & 1u) ^ 1u, &s.abort, a.err);
+        ok = mbar_wait_warp(&s.fullA[slot], (i / kVtcASlots) & 1u, &s.abort, a.err, lim) &&
+             mbar_wait_warp(&s.accEmpty[acc], ((i / S::kAcc) & 1u) ^ 1u, &s.abort, a.err, lim);
         if (!ok) break;
         tc_fence_after();
         const uint32_t ad = aBase + slot * (uint32_t)(S::kABytes >> 4);
@@ -346,7 +351,7 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
       // this row's key index, loaded before the wait for the accumulator
       const int pos = t * kVtcRows + row;
       const int key = pos < item.z ? (gathered ? __ldg(a.perm + item.y + pos) : item.y + pos) : -1;
-      ok = mbar_wait_warp(&s.done[i % kVtcASlots], (i / kVtcASlots) & 1u, &s.abort, a.err);
+      ok = mbar_wait_warp(&s.done[i % kVtcASlots], (i / kVtcASlots) & 1u, &s.abort, a.err, lim);
       if (!ok) break;
       tc_fence_after();
       const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * S::kAccCols);

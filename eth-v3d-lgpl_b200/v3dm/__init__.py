@@ -108,6 +108,8 @@ def lib() -> C.CDLL:
         L.v3dm_voctree_quantize_u8.argtypes = [vp, i32, vp, vp, i32]
         L.v3dm_voctree_quantize_u8_device.argtypes = [vp, i32, vp, vp, i32]
         L.v3dm_voctree_quantize_f32_device.argtypes = [vp, i32, vp, vp, i32]
+        L.v3dm_voctree_wait.argtypes = [vp]
+        L.v3dm_voctree_test_wait_fault.argtypes = [vp, C.c_longlong, i32]
         L.v3dm_voctree_replays.argtypes = [vp, C.POINTER(C.c_longlong)]
         L.v3dm_voctree_stream.argtypes = [vp, C.POINTER(vp)]
         L.v3dm_voctree_last_launches.argtypes = [vp, C.POINTER(i32)]
@@ -458,6 +460,14 @@ class VocabularyTreeTraversal:
         """Float keys in device memory, the reference CPU tree's sequential FP32 order."""
         _check(lib().v3dm_voctree_quantize_f32_device(self._h, n, C.c_void_p(d_keys), C.c_void_p(d_ids), id_mode),
                "quantize_f32_device")
+
+    def wait(self) -> None:
+        """Waits for the device calls enqueued so far; raises what they flagged."""
+        _check(lib().v3dm_voctree_wait(self._h), "wait")
+
+    def test_wait_fault(self, wait_cycles: int, skip_load: int) -> None:
+        """Failure-path test hook (v3dm_voctree_test_wait_fault); (0, 0) turns it off."""
+        _check(lib().v3dm_voctree_test_wait_fault(self._h, int(wait_cycles), int(skip_load)), "test_wait_fault")
 
     def replays(self) -> int:
         """Key-levels decided by the sequential replay since the tree was created."""

@@ -363,7 +363,8 @@ V3DM_API int v3dm_voctree_set_nodes_u8(v3dm_voctree* t, const uint8_t* nodes);
  * -1e30f) wins.  For u/512 data every such sum is exact, and the integer descent is used.
  * (The reference's GPU kernel, .cu:705-792, sums in a different order with fast-math and can
  * differ from its CPU tree at near ties of float data; the CPU order is the one the apps use.)
- * V3DM_ERR_ARG when the tree holds values that make a descent leave the node array. */
+ * V3DM_ERR_ARG when the tree holds values that make a descent leave the node array,
+ * V3DM_ERR_TIMEOUT when a bounded device-side wait gave up (the ids are then not valid). */
 V3DM_API int v3dm_voctree_quantize_f32(v3dm_voctree* t, int n, const float* keys, int32_t* ids, int idMode);
 V3DM_API int v3dm_voctree_quantize_u8(v3dm_voctree* t, int n, const uint8_t* keys, int32_t* ids, int idMode);
 /* Device-resident variants: keys and ids in device memory, asynchronous on the tree's stream;
@@ -372,6 +373,12 @@ V3DM_API int v3dm_voctree_quantize_u8(v3dm_voctree* t, int n, const uint8_t* key
 V3DM_API int v3dm_voctree_quantize_u8_device(v3dm_voctree* t, int n, const uint8_t* d_keys, int32_t* d_ids, int idMode);
 V3DM_API int v3dm_voctree_quantize_f32_device(v3dm_voctree* t, int n, const float* d_keys, int32_t* d_ids,
                                               int idMode);
+/* Waits for the device-resident calls enqueued so far and reports their errors as the host calls do. */
+V3DM_API int v3dm_voctree_wait(v3dm_voctree* t);
+/* Test of the failure path, as v3dm_matcher_test_wait_fault: the tensor-core descents' bounded waits give
+ * up after waitCycles SM cycles, and with skipLoad = k > 0 CTA 0 does not load the node rows of its k-th
+ * item of the first phase.  waitCycles = skipLoad = 0 (the default) turns it off. */
+V3DM_API int v3dm_voctree_test_wait_fault(v3dm_voctree* t, long long waitCycles, int skipLoad);
 /* Diagnostic: key-levels, since the tree was created, whose float scores were too close to
  * decide from the fast pass and were replayed in the reference's sequential order. */
 V3DM_API int v3dm_voctree_replays(v3dm_voctree* t, long long* n);

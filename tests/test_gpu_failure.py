@@ -62,3 +62,42 @@ def test_hook_arguments(v3dm_mod):
             with pytest.raises(v3dm_mod.V3DMError) as e:
                 m.test_wait_fault(*args)
             assert e.value.status == v3dm_mod.ERR_ARG
+
+
+@pytest.mark.parametrize("bf,depth,floats", [(4, 6, False), (10, 4, False), (3, 4, False), (10, 4, True), (50, 3, True)])
+def test_a_tree_wait_that_runs_out_reports_timeout_and_the_handle_recovers(v3dm_mod, oracle_mod, bf, depth, floats):
+    """The first phase of a vocabulary-tree descent loses an item on a handle whose sorting buffers were
+    never written: the phases behind it do nothing, the call reports V3DM_ERR_TIMEOUT (the device-resident
+    call through wait()), and the next calls give the oracle's ids."""
+    import torch
+    n = 150_001
+    rng = synth.rng_for(8200 + bf + floats)
+    count = v3dm_mod.voctree_counts(bf, depth)[0]
+    nodes, keys = synth.sift_like(rng, count), synth.sift_like(rng, n)
+    if floats:
+        nodes, keys = synth.unit_sift(rng, count), synth.unit_sift(rng, n)
+    exp = oracle_mod.voctree(bf, depth, nodes, keys, False)
+    with v3dm_mod.VocabularyTreeTraversal(bf, depth) as t:
+        t.allocate(n)
+        t.set_nodes(nodes)
+        d_keys = torch.from_numpy(keys).cuda()
+        d_ids = torch.empty(n, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        call = t.quantize_f32_device if floats else t.quantize_device
+        t.test_wait_fault(20_000_000, 1)  # ~10 ms at the B200's clocks
+        with pytest.raises(v3dm_mod.V3DMError) as e:
+            t.traverse_tree(keys, v3dm_mod.LEAF_LOCAL)
+        assert e.value.status == v3dm_mod.ERR_TIMEOUT and t.last_launches() > 1
+        call(n, d_keys.data_ptr(), d_ids.data_ptr(), v3dm_mod.LEAF_LOCAL)
+        with pytest.raises(v3dm_mod.V3DMError) as e:
+            t.wait()
+        assert e.value.status == v3dm_mod.ERR_TIMEOUT
+        t.test_wait_fault(0, 0)
+        np.testing.assert_array_equal(t.traverse_tree(keys, v3dm_mod.LEAF_LOCAL), exp)
+        call(n, d_keys.data_ptr(), d_ids.data_ptr(), v3dm_mod.LEAF_LOCAL)
+        t.wait()
+        np.testing.assert_array_equal(d_ids.cpu().numpy(), exp)
+        for args in ((-1, 0), (10, -1), (0, 2)):
+            with pytest.raises(v3dm_mod.V3DMError) as e:
+                t.test_wait_fault(*args)
+            assert e.value.status == v3dm_mod.ERR_ARG
