@@ -806,8 +806,8 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
     h->lastLaunches += 2;
   }
   if (gated) {
-    V3DM_CUDA_TRY(launch_choose(h->dLeftDec, h->nL, h->dChosenFlag, h->dChosenList, h->dCounters, h->dR, h->dRc,
-                                h->stream));
+    V3DM_CUDA_TRY(launch_choose(h->dLeftDec, h->nL, h->nR, h->dChosenFlag, h->dChosenList, h->dCounters, h->dR,
+                                h->dRc, h->stream));
     h->lastLaunches += 1;
   }
   // pass B: the chosen rights against every left
@@ -852,7 +852,7 @@ int enqueue_match_tc(v3dm_matcher* h, float minScore, float minRatio, int32_t* d
     V3DM_CUDA_TRY(launch_rescore(ra, 64, h->stream));
     h->lastLaunches += 2;
   }
-  V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->dRightDec, h->dChosenFlag, h->dScratch,
+  V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->nR, h->dRightDec, h->dChosenFlag, h->dScratch,
                               reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, host_result(h), h->stream));
   h->resInHost = true;
   h->countWritten = h->countOut != nullptr;
@@ -905,11 +905,15 @@ int enqueue_match_f(v3dm_matcher* h, float minScore, float minRatio, int32_t* dP
     if (e != V3DM_OK) return e;
     V3DM_CUDA_TRY(cudaEventRecord(evA[0], h->stream));
   }
+  sa.waitLimit = h->testWaitLimit;
+  sa.skipLoad = h->testSkipLoad;
   V3DM_CUDA_TRY(launch_side_f(h->fmL, h->fmR, sa, Tf, nullptr, h->numSMs, h->stream));
+  sa.waitLimit = 0;
+  sa.skipLoad = 0;
   if (h->profile) V3DM_CUDA_TRY(cudaEventRecord(evA[1], h->stream));
   // the accepted rights, once each, gathered (four planes) for pass B
-  V3DM_CUDA_TRY(launch_choose_planes(h->dLeftDec, h->nL, h->dChosenFlag, h->dChosenList, h->dCounters, h->dRf,
-                                     h->dRcf, kFloatRowBytes / kDescBytes, h->capFR, h->capFR, h->stream));
+  V3DM_CUDA_TRY(launch_choose_planes(h->dLeftDec, h->nL, h->nR, h->dChosenFlag, h->dChosenList, h->dCounters,
+                                     h->dRf, h->dRcf, kFloatRowBytes / kDescBytes, h->capFR, h->capFR, h->stream));
   // pass B: the chosen rights against every left
   sa.nAptr = h->dCounters;
   sa.nA = h->nR;
@@ -924,7 +928,7 @@ int enqueue_match_f(v3dm_matcher* h, float minScore, float minRatio, int32_t* dP
   }
   V3DM_CUDA_TRY(launch_side_f(h->fmRc, h->fmL, sa, Tf, nullptr, h->numSMs, h->stream));
   if (h->profile) V3DM_CUDA_TRY(cudaEventRecord(evB[1], h->stream));
-  V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->dRightDec, h->dChosenFlag, h->dScratch,
+  V3DM_CUDA_TRY(launch_mutual(h->dLeftDec, h->nL, h->nR, h->dRightDec, h->dChosenFlag, h->dScratch,
                               reinterpret_cast<int2*>(dPairs), h->dInfo, h->countOut, host_result(h), h->stream));
   h->resInHost = true;
   h->countWritten = h->countOut != nullptr;

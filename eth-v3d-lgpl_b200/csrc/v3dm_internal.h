@@ -329,11 +329,11 @@ struct RescoreArgs {
 };
 cudaError_t launch_rescore(const RescoreArgs& a, int grid, cudaStream_t s);
 // Rights accepted by some left: de-duplicated list, their descriptors gathered into dRc.
-cudaError_t launch_choose(const int32_t* leftDec, int nL, int* chosenFlag, int* chosenList, int* chosenCount,
+cudaError_t launch_choose(const int32_t* leftDec, int nL, int nR, int* chosenFlag, int* chosenList, int* chosenCount,
                           const uint8_t* dR, uint8_t* dRc, cudaStream_t s);
 // The same for rows of 'planes' 128-byte blocks (block p of row r at (p * cap + r) * 128).
-cudaError_t launch_choose_planes(const int32_t* leftDec, int nL, int* chosenFlag, int* chosenList, int* chosenCount,
-                                 const uint8_t* src, uint8_t* dst, int planes, int capSrc, int capDst,
+cudaError_t launch_choose_planes(const int32_t* leftDec, int nL, int nR, int* chosenFlag, int* chosenList,
+                                 int* chosenCount, const uint8_t* src, uint8_t* dst, int planes, int capSrc, int capDst,
                                  cudaStream_t s);
 // Mutual filter and ordered compaction (blockCount: nL/2048 + 1 ints of scratch); clears chosenFlag.
 // The pair count goes to info[kInfoPairs] and, when countOut is set, to *countOut.
@@ -344,8 +344,9 @@ struct HostResult {
   int2* pairs;
   int cap;
 };
-cudaError_t launch_mutual(const int32_t* leftDec, int nL, const int32_t* rightDec, int* chosenFlag, int* blockCount,
-                          int2* pairs, int32_t* info, int32_t* countOut, const HostResult& host, cudaStream_t s);
+cudaError_t launch_mutual(const int32_t* leftDec, int nL, int nR, const int32_t* rightDec, int* chosenFlag,
+                          int* blockCount, int2* pairs, int32_t* info, int32_t* countOut, const HostResult& host,
+                          cudaStream_t s);
 int mutual_launches(int nL);  // kernels of launch_mutual
 
 // Candidate threshold (v3dm_api.cu).

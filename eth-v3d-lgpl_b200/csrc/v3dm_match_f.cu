@@ -194,7 +194,8 @@ __device__ __forceinline__ bool gates_reject(const GateParams* gates, int n, int
 //   warp 1      MMA issuer (the warp walks, one elected lane issues): the A blocks into TMEM, then per
 //               tile 24 MMAs for each block;
 //   warps 2-9   epilogue, four per block: one A row per lane.
-// Bounded waits as in k_side.  With 'dump' set (a small diagnostic call without gates) every score is
+// Bounded waits as in k_side; the rows of a CTA that gives up keep whatever a.decision held, which the
+// kernels that read it allow for.  With 'dump' set (a small diagnostic call without gates) every score is
 // also written to dump[state * nB + column].
 // What bounds it: the tensor pipe, 24 x 64 = 1536 cycles per block and tile, of which it takes 1760.
 // Before, with 128-row groups and the hi planes stored twice (96 KB of L2 reads per block and tile
@@ -211,6 +212,7 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
   extern __shared__ uint8_t smemRaw[];
   SmemF& s = *reinterpret_cast<SmemF*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long lim = a.waitLimit > 0 ? a.waitLimit : kWaitCycles;
   const FWalk start(a);
   if (!start.more()) return;
   if (threadIdx.x == 0) {
@@ -242,12 +244,18 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       uint32_t u = 0;
+      uint32_t skipped = 0xffffffffu;  // test hook: the use that was not loaded
+      int bLoads = 0;
       bool ok = true;
       auto load = [&](const CUtensorMap* m, int r) {
         const uint32_t st = u % kFStages;
-        if (!mbar_wait(&s.empty[st], ((u / kFStages) & 1u) ^ 1u, &s.abort, a.err)) return false;
-        mbar_expect_tx(&s.full[st], (uint32_t)kFStageBytes);
-        tma_load_3d(s.b[st], m, &s.full[st], 0, r, 0);
+        if (!mbar_wait(&s.empty[st], ((u / kFStages) & 1u) ^ 1u, &s.abort, a.err, lim)) return false;
+        if (m == &tmB && ++bLoads == a.skipLoad && blockIdx.x == 0) {
+          skipped = u;
+        } else {
+          mbar_expect_tx(&s.full[st], (uint32_t)kFStageBytes);
+          tma_load_3d(s.b[st], m, &s.full[st], 0, r, 0);
+        }
         ++u;
         return true;
       };
@@ -258,7 +266,7 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
       // Drain: every load this thread issued has landed before the CTA may exit.
       for (uint32_t k = u > (uint32_t)kFStages ? u - kFStages : 0u; k < u; ++k) {
         const long long t0c = clock64();
-        while (!mbar_try(&s.full[k % kFStages], (k / kFStages) & 1u) && clock64() - t0c < kWaitCycles) {
+        while (k != skipped && !mbar_try(&s.full[k % kFStages], (k / kFStages) & 1u) && clock64() - t0c < kWaitCycles) {
         }
       }
     }
@@ -268,7 +276,7 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
     const uint32_t base = sdesc_lo(smem_u32(s.b[0]));
     uint32_t u = 0, i[kFGroups] = {};
     bool ok = true;
-    auto wait = [&](unsigned long long* b, uint32_t par) { return mbar_wait_warp(b, par, &s.abort, a.err); };
+    auto wait = [&](unsigned long long* b, uint32_t par) { return mbar_wait_warp(b, par, &s.abort, a.err, lim); };
     for (FWalk wk = start; wk.more() && ok; wk.next()) {
       const int groups = wk.groups();
       // the group into TMEM (after the previous group's MMAs, which were issued first); a stage is
@@ -376,7 +384,7 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
         if (st >= 0) enter = f32_unorder(b2);
       };
       for (int t = 0; t < wk.nT; ++t, ++i) {
-        ok = mbar_wait_warp(&s.accFull[g], i & 1u, &s.abort, a.err);
+        ok = mbar_wait_warp(&s.accFull[g], i & 1u, &s.abort, a.err, lim);
         if (!ok) break;
         tc_fence_after();
         const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * kFN);

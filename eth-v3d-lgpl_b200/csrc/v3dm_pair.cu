@@ -234,8 +234,9 @@ __global__ void k_rescore_decide(RescoreArgs a) {
 }
 
 // A row is 'planes' blocks of 128 bytes, block p of row r at (p * cap + r) * 128 (one block:
-// uint8 descriptors; four: the planar BF16 hi/lo layout).
-__global__ void k_choose(const int32_t* __restrict__ leftDec, int nL, int* chosenFlag, int* chosenList,
+// uint8 descriptors; four: the planar BF16 hi/lo layout).  A float pass that gave up on a wait leaves rows
+// undecided: here and in the mutual filter what such a row holds is no right when it is not below nR.
+__global__ void k_choose(const int32_t* __restrict__ leftDec, int nL, int nR, int* chosenFlag, int* chosenList,
                          int* chosenCount, const uint8_t* __restrict__ dR, uint8_t* __restrict__ dRc, int planes,
                          int capSrc, int capDst) {
   pdl_wait();
@@ -245,7 +246,7 @@ __global__ void k_choose(const int32_t* __restrict__ leftDec, int nL, int* chose
     const int r = leftDec[l];
     // the first left to name a right claims it; the claiming lanes of a warp take
     // consecutive list slots with one counter update
-    const bool claim = r >= 0 && atomicExch(&chosenFlag[r], 1) == 0;
+    const bool claim = (unsigned)r < (unsigned)nR && atomicExch(&chosenFlag[r], 1) == 0;
     const unsigned act = __activemask();
     const unsigned m = __ballot_sync(act, claim);
     if (!m) continue;
@@ -282,14 +283,14 @@ __device__ __forceinline__ void put_count(int32_t* info, int32_t* countOut, cons
 
 // Pass 1: number of mutual pairs among each block's contiguous range of lefts.
 __global__ void __launch_bounds__(kMutThreads)
-k_mutual_count(const int32_t* __restrict__ leftDec, int nL, const int32_t* __restrict__ rightDec,
+k_mutual_count(const int32_t* __restrict__ leftDec, int nL, int nR, const int32_t* __restrict__ rightDec,
                int* __restrict__ blockCount) {
   pdl_wait();
   pdl_launch_dependents();
   __shared__ int wsum[kMutThreads / 32];
   const int k = blockIdx.x * kMutPerBlock + threadIdx.x;
   const int r = k < nL ? leftDec[k] : -1;
-  int cnt = r >= 0 && rightDec[r] == k;
+  int cnt = (unsigned)r < (unsigned)nR && rightDec[r] == k;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = cnt;
@@ -304,9 +305,9 @@ k_mutual_count(const int32_t* __restrict__ leftDec, int nL, const int32_t* __res
 // Pass 2: each block offsets its pairs by the counts of the blocks before it (summed by the
 // whole block) and writes them in ascending left order; clears the chosen-right flags.
 __global__ void __launch_bounds__(kMutThreads)
-k_mutual_write(const int32_t* __restrict__ leftDec, int nL, const int32_t* __restrict__ rightDec, int* chosenFlag,
-               const int* __restrict__ blockCount, int nBlocks, int2* __restrict__ pairs, int32_t* info,
-               int32_t* countOut, HostResult host) {
+k_mutual_write(const int32_t* __restrict__ leftDec, int nL, int nR, const int32_t* __restrict__ rightDec,
+               int* chosenFlag, const int* __restrict__ blockCount, int nBlocks, int2* __restrict__ pairs,
+               int32_t* info, int32_t* countOut, HostResult host) {
   pdl_wait();
   pdl_launch_dependents();
   __shared__ int wsum[kMutThreads / 32];
@@ -314,8 +315,8 @@ k_mutual_write(const int32_t* __restrict__ leftDec, int nL, const int32_t* __res
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int k = blockIdx.x * kMutPerBlock + threadIdx.x;
   const int r = k < nL ? leftDec[k] : -1;
-  const bool ok = r >= 0 && rightDec[r] == k;
-  if (r >= 0) chosenFlag[r] = 0;
+  const bool right = (unsigned)r < (unsigned)nR, ok = right && rightDec[r] == k;
+  if (right) chosenFlag[r] = 0;
   int t = 0;
   for (int b = threadIdx.x; b < (int)blockIdx.x; b += kMutThreads) t += blockCount[b];
   const int cnt = ok ? 1 : 0;
@@ -347,8 +348,8 @@ constexpr int kMutSmallThreads = 1024;
 constexpr int kMutSmallPer = 8;
 constexpr int kMutSmall = kMutSmallThreads * kMutSmallPer;
 __global__ void __launch_bounds__(kMutSmallThreads)
-k_mutual_small(const int32_t* __restrict__ leftDec, int nL, const int32_t* __restrict__ rightDec, int* chosenFlag,
-               int2* pairs, int32_t* info, int32_t* countOut, HostResult host) {
+k_mutual_small(const int32_t* __restrict__ leftDec, int nL, int nR, const int32_t* __restrict__ rightDec,
+               int* chosenFlag, int2* pairs, int32_t* info, int32_t* countOut, HostResult host) {
   pdl_wait();
   pdl_launch_dependents();
   __shared__ int wsum[kMutSmallThreads / 32];
@@ -360,10 +361,10 @@ k_mutual_small(const int32_t* __restrict__ leftDec, int nL, const int32_t* __res
   bool ok[kMutSmallPer];
   int cnt = 0;
 #pragma unroll
-  for (int i = 0; i < kMutSmallPer; ++i) ok[i] = r[i] >= 0 && rightDec[r[i]] == k0 + i;
+  for (int i = 0; i < kMutSmallPer; ++i) ok[i] = (unsigned)r[i] < (unsigned)nR && rightDec[r[i]] == k0 + i;
 #pragma unroll
   for (int i = 0; i < kMutSmallPer; ++i) {
-    if (r[i] >= 0) chosenFlag[r[i]] = 0;
+    if ((unsigned)r[i] < (unsigned)nR) chosenFlag[r[i]] = 0;
     cnt += ok[i];
   }
   int inc = cnt;
@@ -416,37 +417,39 @@ cudaError_t launch_rescore(const RescoreArgs& a, int grid, cudaStream_t s) {
   return launch_pdl(k_rescore_decide, dim3(16), dim3(256), 0, s, a);
 }
 
-cudaError_t launch_choose(const int32_t* leftDec, int nL, int* chosenFlag, int* chosenList, int* chosenCount,
+cudaError_t launch_choose(const int32_t* leftDec, int nL, int nR, int* chosenFlag, int* chosenList, int* chosenCount,
                           const uint8_t* dR, uint8_t* dRc, cudaStream_t s) {
   if (nL == 0) return cudaSuccess;
   int blocks = (nL + 255) / 256;
   if (blocks > 148) blocks = 148;
-  return launch_pdl(k_choose, dim3(blocks), dim3(256), 0, s, leftDec, nL, chosenFlag, chosenList, chosenCount, dR, dRc,
-                    1, 0, 0);
+  return launch_pdl(k_choose, dim3(blocks), dim3(256), 0, s, leftDec, nL, nR, chosenFlag, chosenList, chosenCount, dR,
+                    dRc, 1, 0, 0);
 }
 
-cudaError_t launch_choose_planes(const int32_t* leftDec, int nL, int* chosenFlag, int* chosenList, int* chosenCount,
-                                 const uint8_t* src, uint8_t* dst, int planes, int capSrc, int capDst,
+cudaError_t launch_choose_planes(const int32_t* leftDec, int nL, int nR, int* chosenFlag, int* chosenList,
+                                 int* chosenCount, const uint8_t* src, uint8_t* dst, int planes, int capSrc, int capDst,
                                  cudaStream_t s) {
   if (nL == 0) return cudaSuccess;
   int blocks = (nL + 255) / 256;
   if (blocks > 148) blocks = 148;
-  return launch_pdl(k_choose, dim3(blocks), dim3(256), 0, s, leftDec, nL, chosenFlag, chosenList, chosenCount, src,
+  return launch_pdl(k_choose, dim3(blocks), dim3(256), 0, s, leftDec, nL, nR, chosenFlag, chosenList, chosenCount, src,
                     dst, planes, capSrc, capDst);
 }
 
 int mutual_launches(int nL) { return nL == 0 ? 0 : nL <= kMutSmall ? 1 : 2; }
 
-cudaError_t launch_mutual(const int32_t* leftDec, int nL, const int32_t* rightDec, int* chosenFlag, int* blockCount,
-                          int2* pairs, int32_t* info, int32_t* countOut, const HostResult& host, cudaStream_t s) {
+cudaError_t launch_mutual(const int32_t* leftDec, int nL, int nR, const int32_t* rightDec, int* chosenFlag,
+                          int* blockCount, int2* pairs, int32_t* info, int32_t* countOut, const HostResult& host,
+                          cudaStream_t s) {
   const int nBlocks = (nL + kMutPerBlock - 1) / kMutPerBlock;
   if (nBlocks == 0) return cudaSuccess;
   if (nL <= kMutSmall)
-    return launch_pdl(k_mutual_small, dim3(1), dim3(kMutSmallThreads), 0, s, leftDec, nL, rightDec, chosenFlag, pairs,
-                      info, countOut, host);
-  cudaError_t e = launch_pdl(k_mutual_count, dim3(nBlocks), dim3(kMutThreads), 0, s, leftDec, nL, rightDec, blockCount);
+    return launch_pdl(k_mutual_small, dim3(1), dim3(kMutSmallThreads), 0, s, leftDec, nL, nR, rightDec, chosenFlag,
+                      pairs, info, countOut, host);
+  cudaError_t e = launch_pdl(k_mutual_count, dim3(nBlocks), dim3(kMutThreads), 0, s, leftDec, nL, nR, rightDec,
+                             blockCount);
   if (e != cudaSuccess) return e;
-  return launch_pdl(k_mutual_write, dim3(nBlocks), dim3(kMutThreads), 0, s, leftDec, nL, rightDec, chosenFlag,
+  return launch_pdl(k_mutual_write, dim3(nBlocks), dim3(kMutThreads), 0, s, leftDec, nL, nR, rightDec, chosenFlag,
                     blockCount, nBlocks, pairs, info, countOut, host);
 }
 

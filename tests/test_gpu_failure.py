@@ -101,3 +101,35 @@ def test_a_tree_wait_that_runs_out_reports_timeout_and_the_handle_recovers(v3dm_
             with pytest.raises(v3dm_mod.V3DMError) as e:
                 t.test_wait_fault(*args)
             assert e.value.status == v3dm_mod.ERR_ARG
+
+
+@pytest.mark.parametrize("nL,nR", [(300, 6000), (7000, 500), (9000, 9000)])
+def test_a_float_wait_that_runs_out_reports_timeout_and_the_handle_recovers(v3dm_mod, oracle_mod, nL, nR):
+    """Float descriptors: the rows of a CTA that gives up are not decided, and the kernels that read the
+    decisions (never written on this handle, or left by a call with more rights) take none of them for
+    an index past the rights.  300 lefts: a row in segments, whose merge never comes; 9000: two mutual kernels."""
+    rng = synth.rng_for(8300 + nL)
+    L, R = synth.unit_sift(rng, nL), synth.unit_sift(rng, nR)
+    k = min(nL, nR) // 3
+    R[:k] = L[rng.permutation(nL)[:k]]
+    with v3dm_mod.SIFTMatching(0) as m:
+        m.allocate(nL, nR)
+        m.set_left_features(L)
+        m.set_right_features(R)
+        for _ in range(2):
+            m.test_wait_fault(20_000_000, 1)
+            with pytest.raises(v3dm_mod.V3DMError) as e:
+                m.find_putative_matches(0.7, 0.8)
+            assert e.value.status == v3dm_mod.ERR_TIMEOUT
+            m.test_wait_fault(0, 0)
+            got = m.find_putative_matches(0.7, 0.8)
+            assert got.shape[0] >= 0.9 * k
+            # fewer rights: the decisions of the call before name rights past them
+            m.set_right_features(R[:40])
+            m.test_wait_fault(20_000_000, 1)
+            with pytest.raises(v3dm_mod.V3DMError) as e:
+                m.find_putative_matches(0.7, 0.8)
+            assert e.value.status == v3dm_mod.ERR_TIMEOUT
+            m.test_wait_fault(0, 0)
+            m.set_right_features(R)
+            np.testing.assert_array_equal(m.find_putative_matches(0.7, 0.8), got)
