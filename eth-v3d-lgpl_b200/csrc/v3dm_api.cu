@@ -459,6 +459,8 @@ int v3dm_allocate(v3dm_matcher* h, int nMaxL, int nMaxR, int useGuided) {
     free_buffers(h);
     return V3DM_ERR_CUDA;
   }
+  // a wait may come before anything has written there: after a call that was only captured
+  std::memset(h->hInfo, 0, (kInfoWords + kHostResultWords) * sizeof(int32_t));
   h->allocated = true;
   return V3DM_OK;
 }
