@@ -971,6 +971,7 @@ struct v3dm_batch {
   float2* dPos = nullptr;
   long long posCap = 0;
   bool havePositions = false;
+  std::vector<float> hGate;         // the gates being uploaded; not changed before the call that uses them has ended
   float* dGate = nullptr;           // kBGateFloats per pair (caller's order)
   long long gateCap = 0;
   bool gatePairsValid = false;      // the three tables below hold the current pair table
@@ -2341,13 +2342,13 @@ int v3dm_batch_match_guided(v3dm_batch* b, int type, const double* M, const floa
   const int n = b->nPairs;
   if (n > 0) {
     // per pair: the matrix as the reference's float3 rows (.cu:592-595), then thr^2 in float (.cu:591)
-    std::vector<float> gm((size_t)n * kBGateFloats);
+    std::vector<float>& gm = b->hGate;
+    gm.resize((size_t)n * kBGateFloats);
     for (int p = 0; p < n; ++p) {
       for (int i = 0; i < 9; ++i) gm[(size_t)p * kBGateFloats + i] = (float)M[9 * (size_t)p + i];
       gm[(size_t)p * kBGateFloats + 9] = thr[p] * thr[p];
     }
     V3DM_BTRY(ensure(&b->dGate, &b->gateCap, (long long)n * kBGateFloats));
-    // pageable memory: the copy has left gm when it returns
     V3DM_BTRY(cudaMemcpyAsync(b->dGate, gm.data(), gm.size() * sizeof(float), cudaMemcpyHostToDevice, b->stream));
     // the pair table's part is uploaded with the first guided call after set_pairs
     if (!b->gatePairsValid) {
