@@ -77,10 +77,10 @@ constexpr int kCntFlagB = 12;     // and pass-B states
 constexpr int kCntAll = 16;      // batch and proposal counter words
 static_assert(kInfoWords + kCntAll <= 32, "one warp hands them to the host");
 
-// The kernel that ends a call leaves its info and counter words, and the first kHostTriples triples, in
-// pinned memory, where a host call takes them without asking for a copy (each copy that is waited for
-// is 10 - 15 us; 65536 take 16 us to cross PCIe either way, and of a call with more of them the copy is
-// a few per cent).
+// The kernel that ends a call leaves its info and counter words, and a host call's first kHostTriples
+// triples, in pinned memory, where the host call takes them without asking for a copy (each copy that is
+// waited for is 10 - 15 us; 65536 take 16 us to cross PCIe either way, and of a call with more of them the
+// copy of the others is a few per cent).
 constexpr int kHostTriples = 65536;
 constexpr size_t kHostInfoBytes = 128;  // the words, then the triples
 
@@ -354,10 +354,10 @@ k_bmutual_write(int* counters, const int32_t* __restrict__ decB, const int* __re
       const int s = beg + i;
       out[off++] = make_int3(chosenPair[s], chosenLeft[s], chosenRight[s]);
     }
-  // the block's triples that go to the host, word by word in order: whole lines over PCIe (triples
-  // stored by the threads that found them took 40 us for 16384)
+  // the block's triples that go to the host (a host call's), word by word in order: whole lines over PCIe
+  // (triples stored by the threads that found them took 40 us for 16384)
   const int first = blockOff;
-  if (first >= kHostTriples) return;
+  if (!hostOut || first >= kHostTriples) return;
   int total = 0;
   for (int k = 0; k < kBMutThreads / 32; ++k) total += wsum[k];
   __syncthreads();
@@ -909,9 +909,10 @@ struct v3dm_batch {
   TcMaps mapsA, mapsB;
   bool mapsValid = false;
   int lastLaunches = 0;
-  // graph of one call
+  bool toHost = false;              // the call's triples go to the host
+  // graphs of one call, [0] of a device call and [1] of a host call
   bool useGraph = true;
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph[2] = {};
   uint32_t graphMs = 0, graphMr = 0;
   int graphLaunches = 0;
   bool pendingCheck = false;
@@ -962,7 +963,7 @@ struct v3dm_batch {
   long long mapImgGrows = 0;
   const uint8_t* mapsPla = nullptr;
   const uint8_t* mapsPlb = nullptr;
-  cudaGraphExec_t graphP = nullptr;
+  cudaGraphExec_t graphP[2] = {};
   uint32_t gpMs = 0, gpMr = 0;
   int gpProbes = 0, gpCells = 0, gpLaunches = 0;
   const v3dm_projection* gpProj = nullptr;
@@ -1051,11 +1052,19 @@ cudaError_t ensure(T** p, long long* cap, long long need) {
   return cudaSuccess;
 }
 
+void drop_graph_p(v3dm_batch* b) {
+  for (cudaGraphExec_t& g : b->graphP) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
+
 void drop_graph(v3dm_batch* b) {
-  if (b->graph) cudaGraphExecDestroy(b->graph);
-  b->graph = nullptr;
-  if (b->graphP) cudaGraphExecDestroy(b->graphP);
-  b->graphP = nullptr;
+  for (cudaGraphExec_t& g : b->graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+  drop_graph_p(b);
 }
 
 cudaError_t alloc_records(v3dm_batch* b, long long segCap) {
@@ -1156,16 +1165,24 @@ int ensure_maps(v3dm_batch* b) {
 int3* host_triples(v3dm_batch* b) {
   return reinterpret_cast<int3*>(reinterpret_cast<uint8_t*>(b->hInfo) + kHostInfoBytes);
 }
+// Where the call being enqueued leaves its triples for the host (null: nowhere).
+int3* call_triples(v3dm_batch* b) { return b->toHost ? host_triples(b) : nullptr; }
 
-// The first m triples of a call that the stream has finished.
+struct HostCall {
+  v3dm_batch* b;
+  explicit HostCall(v3dm_batch* b_) : b(b_) { b->toHost = true; }
+  ~HostCall() { b->toHost = false; }
+};
+
+// The first m triples of a host call that the stream has finished.
 int copy_triples(v3dm_batch* b, int32_t* triples, long long m) {
   if (m <= 0) return V3DM_OK;
-  if (m <= kHostTriples) {
-    std::memcpy(triples, host_triples(b), (size_t)m * sizeof(int3));
-    return V3DM_OK;
-  }
-  V3DM_BTRY(cudaMemcpyAsync(triples, b->dOut, (size_t)m * sizeof(int3), cudaMemcpyDeviceToHost, b->stream));
-  V3DM_BTRY(cudaStreamSynchronize(b->stream));
+  const long long pinned = std::min<long long>(m, kHostTriples), rest = m - pinned;
+  if (rest > 0)
+    V3DM_BTRY(cudaMemcpyAsync(triples + 3 * pinned, b->dOut + pinned, (size_t)rest * sizeof(int3),
+                              cudaMemcpyDeviceToHost, b->stream));
+  std::memcpy(triples, host_triples(b), (size_t)pinned * sizeof(int3));
+  if (rest > 0) V3DM_BTRY(cudaStreamSynchronize(b->stream));
   return V3DM_OK;
 }
 
@@ -1276,7 +1293,7 @@ int enqueue_batch(v3dm_batch* b, float minScore, float minRatio, bool withEvents
   V3DM_BTRY(cudaGetLastError());
   k_bmutual_write<<<mutBlocks, kBMutThreads, 0, b->stream>>>(b->dCounters, b->dDecB, b->dChosenLeft,
                                                              b->dChosenRight, b->dChosenPair, b->dBlockCount,
-                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, host_triples(b));
+                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, call_triples(b));
   V3DM_BTRY(cudaGetLastError());
   launches += 2;
   b->lastLaunches = launches;
@@ -1340,7 +1357,7 @@ int enqueue_batch_f(v3dm_batch* b, float minScore, float minRatio, bool withEven
   V3DM_BTRY(cudaGetLastError());
   k_bmutual_write<<<mutBlocks, kBMutThreads, 0, b->stream>>>(b->dCounters, b->dDecB, b->dChosenLeft,
                                                              b->dChosenRight, b->dChosenPair, b->dBlockCount,
-                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, host_triples(b));
+                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, call_triples(b));
   V3DM_BTRY(cudaGetLastError());
   launches += 2;
   b->lastLaunches = launches;
@@ -1413,8 +1430,9 @@ int launch_call(v3dm_batch* b, float minScore, float minRatio) {
     return st;
   }
   if (!b->useGraph) return enqueue_call(b, minScore, minRatio, false);
-  if (!b->graph || b->graphMs != ms || b->graphMr != mr) {
-    drop_graph(b);
+  cudaGraphExec_t& graph = b->graph[b->toHost];
+  if (!graph || b->graphMs != ms || b->graphMr != mr) {
+    if (b->graphMs != ms || b->graphMr != mr) drop_graph(b);  // the other one is of the old parameters too
     cudaGraph_t g = nullptr;
     V3DM_BTRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     st = enqueue_call(b, minScore, minRatio, false);
@@ -1424,17 +1442,17 @@ int launch_call(v3dm_batch* b, float minScore, float minRatio) {
       return st;
     }
     if (e != cudaSuccess) return bfail(e, "cudaStreamEndCapture", __LINE__);
-    e = cudaGraphInstantiate(&b->graph, g, 0);
+    e = cudaGraphInstantiate(&graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
-      b->graph = nullptr;
+      graph = nullptr;
       return bfail(e, "cudaGraphInstantiate", __LINE__);
     }
     b->graphMs = ms;
     b->graphMr = mr;
     b->graphLaunches = b->lastLaunches;
   }
-  V3DM_BTRY(cudaGraphLaunch(b->graph, b->stream));
+  V3DM_BTRY(cudaGraphLaunch(graph, b->stream));
   b->lastLaunches = b->graphLaunches;
   return V3DM_OK;
 }
@@ -1647,15 +1665,13 @@ int prepare_proposal(v3dm_batch* b, int probesL, int probesR, int C) {
     b->mapsPValid = true;
     b->laRows = laRows;
     b->lbRows = lbRows;
-    if (b->graphP) cudaGraphExecDestroy(b->graphP);
-    b->graphP = nullptr;
+    drop_graph_p(b);
   }
   if (b->mapImgGimg != b->dImg || b->mapImgGrows != b->totalRows) {
     V3DM_BTRY(tc_gather_map(&b->mapImgG, b->dImg, (int)std::max<long long>(b->totalRows, 1)));
     b->mapImgGimg = b->dImg;
     b->mapImgGrows = b->totalRows;
-    if (b->graphP) cudaGraphExecDestroy(b->graphP);
-    b->graphP = nullptr;
+    drop_graph_p(b);
   }
   return V3DM_OK;
 }
@@ -1824,7 +1840,7 @@ int enqueue_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL, in
   V3DM_BTRY(cudaGetLastError());
   k_bmutual_write<<<mutBlocks, kBMutThreads, 0, b->stream>>>(b->dCounters, b->dDecB, b->dChosenLeft,
                                                              b->dChosenRight, b->dChosenPair, b->dBlockCount,
-                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, host_triples(b));
+                                                             mutBlocks, b->dOut, b->dInfo, b->hInfo, call_triples(b));
   V3DM_BTRY(cudaGetLastError());
   launches += 5;  // pass-B states (count, scan, choose), mutual filter (two)
   b->lastLaunches = launches;
@@ -1864,9 +1880,11 @@ int launch_call_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL
     return st;
   }
   if (!b->useGraph) return enqueue_proposal(b, proj, probesL, probesR, minScore, minRatio, false);
-  if (!b->graphP || b->gpMs != ms || b->gpMr != mr || b->gpProbes != probes || b->gpCells != C || b->gpProj != proj) {
-    if (b->graphP) cudaGraphExecDestroy(b->graphP);
-    b->graphP = nullptr;
+  const bool sameCall =
+      b->gpMs == ms && b->gpMr == mr && b->gpProbes == probes && b->gpCells == C && b->gpProj == proj;
+  cudaGraphExec_t& graphP = b->graphP[b->toHost];
+  if (!graphP || !sameCall) {
+    if (!sameCall) drop_graph_p(b);
     cudaGraph_t g = nullptr;
     V3DM_BTRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     st = enqueue_proposal(b, proj, probesL, probesR, minScore, minRatio, false);
@@ -1876,10 +1894,10 @@ int launch_call_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL
       return st;
     }
     if (e != cudaSuccess) return bfail(e, "cudaStreamEndCapture", __LINE__);
-    e = cudaGraphInstantiate(&b->graphP, g, 0);
+    e = cudaGraphInstantiate(&graphP, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
-      b->graphP = nullptr;
+      graphP = nullptr;
       return bfail(e, "cudaGraphInstantiate", __LINE__);
     }
     b->gpMs = ms;
@@ -1889,7 +1907,7 @@ int launch_call_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL
     b->gpProj = proj;
     b->gpLaunches = b->lastLaunches;
   }
-  V3DM_BTRY(cudaGraphLaunch(b->graphP, b->stream));
+  V3DM_BTRY(cudaGraphLaunch(graphP, b->stream));
   b->lastLaunches = b->gpLaunches;
   return V3DM_OK;
 }
@@ -2303,6 +2321,7 @@ int v3dm_batch_set_pairs(v3dm_batch* b, int nPairs, const int32_t* pairs) {
 int v3dm_batch_match(v3dm_batch* b, float minScore, float minRatio, int32_t* triples, long long cap, long long* nOut) {
   if (!b || !nOut || cap < 0 || (cap > 0 && !triples)) return V3DM_ERR_ARG;
   BDeviceGuard g(b->device);
+  HostCall host(b);
   int st = run_host(b, minScore, minRatio);
   if (st != V3DM_OK) return st;
   const long long n = b->hInfo[kInfoWords + kCntOut];
@@ -2356,6 +2375,7 @@ int v3dm_batch_match_guided(v3dm_batch* b, int type, const double* M, const floa
       if (st != V3DM_OK) return st;
     }
   }
+  HostCall host(b);
   int st = V3DM_ERR_CANDIDATES;
   for (int attempt = 0; attempt < 6 && st == V3DM_ERR_CANDIDATES; ++attempt) {
     st = launch_call_guided(b, type, minScore, minRatio);
@@ -2395,6 +2415,7 @@ int v3dm_batch_match_proposal(v3dm_batch* b, v3dm_projection* proj, int probesLe
                               float minRatio, int32_t* triples, long long cap, long long* nOut) {
   if (!b || !nOut || cap < 0 || (cap > 0 && !triples)) return V3DM_ERR_ARG;
   BDeviceGuard g(b->device);
+  HostCall host(b);
   int st = V3DM_ERR_CANDIDATES;
   for (int attempt = 0; attempt < 6 && st == V3DM_ERR_CANDIDATES; ++attempt) {
     st = launch_call_proposal(b, proj, probesLeft, probesRight, minScore, minRatio);

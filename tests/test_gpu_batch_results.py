@@ -1,4 +1,7 @@
-"""What a batch handle keeps from call to call: the pair table's part of guided calls."""
+"""What a batch handle keeps from call to call: the pair table's part of guided calls, graphs and the pinned
+memory that host calls take their triples from."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -36,3 +39,46 @@ def test_guided_calls_with_changing_pair_tables_and_gates(v3dm_mod, oracle_mod):
         b.set_images(desc[: offs[4]], counts[:4])
         with pytest.raises(v3dm_mod.V3DMError):
             b.match_guided(F, thr, 0.7, 0.8)
+
+
+@pytest.mark.parametrize("k", [1000, 32768, 32769, 40000])
+def test_triples_around_the_pinned_memory_and_device_calls(v3dm_mod, k):
+    """Host calls with 2 k triples, around the 65536 that a call leaves in pinned memory, between device calls on
+    the same handle: two pairs of images, each the other's rows in reverse order."""
+    import torch
+    rng = synth.rng_for(43)
+    L = synth.sift_like(rng, k)
+    R = L[::-1].copy()
+    desc, counts = np.concatenate([L, R, R]), np.array([k, k, k], np.int32)
+    one = np.stack([np.arange(k), k - 1 - np.arange(k)], 1)
+    exp = np.concatenate([np.c_[np.zeros(k, np.int64), one], np.c_[np.ones(k, np.int64), one]])
+    count = torch.zeros(1, dtype=torch.int32, device="cuda")
+    with v3dm_mod.BatchMatching() as b:
+        b.set_images(desc, counts)
+        b.set_pairs([(0, 1), (0, 2)])
+
+        def device_call():
+            count.zero_()
+            torch.cuda.synchronize()
+            for _ in range(2):  # a first call may have to grow the buffers
+                b.match_device(0.7, 0.8, count.data_ptr())
+                if b.wait() == v3dm_mod.OK:
+                    break
+            torch.cuda.synchronize()
+            assert int(count[0]) == 2 * k
+
+        device_call()
+        for _ in range(2):
+            np.testing.assert_array_equal(b.match(0.7, 0.8), exp)
+            device_call()
+        b.use_graph(False)
+        np.testing.assert_array_equal(b.match(0.7, 0.8), exp)
+        device_call()
+        # the first rows, when the caller's buffer is smaller
+        out = np.full((70000, 3), -1, np.int32)
+        n = C.c_longlong(0)
+        for cap in (5, min(2 * k, 65537) - 1):
+            st = v3dm_mod.lib().v3dm_batch_match(b._h, 0.7, 0.8, out.ctypes.data, cap, C.byref(n))
+            assert st == v3dm_mod.ERR_CAPACITY and n.value == 2 * k
+            np.testing.assert_array_equal(out[:cap], exp[:cap])
+            assert (out[cap:] == -1).all()
