@@ -55,7 +55,7 @@ using namespace v3dm;
 namespace {
 
 constexpr int kRsScoreThreads = 128;
-constexpr int kRsMinSlots = 131072;  // sample slots of a round at least (190 MB)
+constexpr int kRsMinSlots = 131072;  // sample slots of a round at least, where there are as many draws (190 MB)
 constexpr int kRsStage = 1024;       // correspondences staged at a time in k_rs_score
 constexpr int kRsUnroll = 4;         // correspondences a thread of k_rs_score scores at a time
 
@@ -613,8 +613,10 @@ cudaError_t rs_mark(v3dm_ransac* r, int k) {
 // Everything from normalisation to inlier flags, on r's stream; inputs already on the device.
 int rs_enqueue(v3dm_ransac* r, int nPairs, int nCorrs, int nDraw, int nSamples, bool draw, uint64_t seed,
                double thr2, const float4* dCorrs, int32_t* dSamples, double* dOut, int32_t* dNIn, uint8_t* dFlags) {
-  // sample slots of one round: 128 per pair, and enough for the later rounds of few pairs
-  const size_t nR = std::max((size_t)nPairs * kRsRound, (size_t)kRsMinSlots);
+  // sample slots of one round: 128 per pair, and enough for the later rounds of few pairs, whose draws
+  // may all fit (a single pair of 1001 draws then holds 2 MB)
+  const size_t nR =
+      std::max((size_t)nPairs * kRsRound, std::min((size_t)kRsMinSlots, (size_t)nPairs * (size_t)nDraw));
   const size_t maxItems = nR * kRsMaxSol / kRsScoreThreads + (size_t)nPairs;
   V3DM_RS_TRY(rs_grow(r->dPlan, r->planCap, 2 * (size_t)nPairs + 2));
   V3DM_RS_TRY(rs_grow(r->dItems, r->itemsCap, maxItems));
@@ -643,7 +645,8 @@ int rs_enqueue(v3dm_ransac* r, int nPairs, int nCorrs, int nDraw, int nSamples, 
     V3DM_RS_TRY(rs_grow(r->dTaskIdx, r->taskIdxCap, (size_t)nPairs * kRsTasks));
     V3DM_RS_TRY(rs_grow(r->dTaskN, r->taskNCap, (size_t)nPairs + 3));
     V3DM_RS_TRY(rs_grow(r->dTasks, r->tasksCap, (size_t)nPairs * kRsTasks));
-    rw.ctas = 2 * r->numSMs;  // two CTAs of k_rs_refine fit an SM
+    // two CTAs of k_rs_refine fit an SM; each holds room for a pair's inliers, so no more than there can be tasks
+    rw.ctas = (int)std::min<size_t>(2 * (size_t)r->numSMs, (size_t)nPairs * kRsTasks);
     V3DM_RS_TRY(rs_grow(r->dRefined, r->refinedCap, (size_t)nPairs * kRsTasks + rw.ctas));
     for (int p = 0; p < nPairs; ++p)
       rw.listRoom = std::max(rw.listRoom, (long long)(r->hOffsets[p + 1] - r->hOffsets[p]));
