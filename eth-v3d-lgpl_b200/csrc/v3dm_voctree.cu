@@ -397,6 +397,7 @@ struct v3dm_voctree {
   long long fMaxBins = 1;       // buckets of its last phase
   void* dPlanes = nullptr;      // split node planes, kVtfRowBytes per node (valid when planesReady)
   bool planesReady = false;
+  bool fNoRoom = false;         // the float descent's buffers did not fit; tried again after allocate and set_nodes
   float* dMaxNorm = nullptr;
   float* dChildNorm = nullptr;  // in dPlanes' block
   int4* dFlagged = nullptr;     // 2 x nMax
@@ -453,6 +454,7 @@ constexpr int kVtMinPerBin = 16;
 bool vt_f_wanted(const v3dm_voctree* t, long long n) { return t->fLevels > 0 && n >= kVtMinPerBin * t->fMaxBins; }
 
 int vt_sort(v3dm_voctree* t, int n, long long bins, int itemKeys);
+int vt_float_descent(v3dm_voctree* t);
 
 // The counts of the next phase's buckets to zero, and before a call's first phase its error word, which
 // only the phases after the first read.
@@ -549,6 +551,10 @@ int vt_sort(v3dm_voctree* t, int n, long long bins, int itemKeys) {
 int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int idMode) {
   t->lastLaunches = 0;
   if (n == 0) return V3DM_OK;
+  if (vt_f_wanted(t, n) && n <= t->nMax) {
+    const int st = vt_float_descent(t);
+    if (st != V3DM_OK) return st;
+  }
   if (!vt_f_wanted(t, n) || !t->planesReady || !t->dSplit || n > t->nMax) {
     t->lastLaunches = 1;
     long long threads = (long long)n * kTpk;
@@ -635,8 +641,6 @@ int vt_to_u8(v3dm_voctree* t, const float* dSrc, size_t count, uint8_t* dst, boo
   return V3DM_OK;
 }
 
-int vt_planes(v3dm_voctree* t);
-
 // Node norms of the float tree.
 int vt_norms(v3dm_voctree* t) {
   if (!t->dNorm && cudaMalloc(reinterpret_cast<void**>(&t->dNorm), (size_t)t->nodeCount * sizeof(float)) != cudaSuccess)
@@ -665,19 +669,38 @@ int vt_ensure_float_tree(v3dm_voctree* t) {
   st = vt_norms(t);
   if (st != V3DM_OK) return st;
   t->nodesF = true;
-  return vt_planes(t);
+  return V3DM_OK;
 }
 
-// The split node planes, once the float tree is set and calls can be large enough for them.  A tree
-// whose planes do not fit in memory keeps the one-kernel descent.
-int vt_planes(v3dm_voctree* t) {
-  if (!t->nodesF || t->planesReady || !vt_f_wanted(t, t->nMax)) return V3DM_OK;
+// What the tensor-core descent of float keys needs beside the sorting buffers: the split node planes, and
+// for nMax keys its lists and the split keys (548 bytes per key).  Made once the tree is a float tree and calls can
+// be large enough: when a tree of other values than u/512 is set or allocated for, and otherwise with the
+// first float keys that want it, since byte trees and keys never use them.  What does not fit in memory, or
+// would have to be made while the stream is being captured, leaves the one-kernel descent.
+int vt_float_descent(v3dm_voctree* t) {
+  if (!t->nodesF || !vt_f_wanted(t, t->nMax) || (t->planesReady && t->dSplit) || t->fNoRoom) return V3DM_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(t->stream, &capture) != cudaSuccess) return V3DM_ERR_CUDA;
+  if (capture != cudaStreamCaptureStatusNone) return V3DM_OK;
+  const size_t m = (size_t)t->nMax;
+  if (!t->dSplit && ((!t->dFlagged &&
+                      cudaMalloc(reinterpret_cast<void**>(&t->dFlagged), 2 * m * sizeof(int4)) != cudaSuccess) ||
+                     (!t->dWeird &&
+                      cudaMalloc(reinterpret_cast<void**>(&t->dWeird), m * sizeof(int32_t)) != cudaSuccess) ||
+                     cudaMalloc(&t->dSplit, m * (kVtfRowBytes + sizeof(float))) != cudaSuccess)) {
+    cudaGetLastError();
+    t->dSplit = nullptr;
+    t->fNoRoom = true;
+    return V3DM_OK;
+  }
+  if (t->planesReady) return V3DM_OK;
   // one block: the planes, then the children's norms (nodeCount / BF parents, the root among them)
   const size_t planeBytes = (size_t)t->nodeCount * kVtfRowBytes;
   if (!t->dPlanes &&
       cudaMalloc(&t->dPlanes, planeBytes + (size_t)(t->nodeCount / t->bf) * sizeof(float)) != cudaSuccess) {
     cudaGetLastError();
     t->dPlanes = nullptr;
+    t->fNoRoom = true;
     return V3DM_OK;
   }
   t->dChildNorm = reinterpret_cast<float*>(static_cast<uint8_t*>(t->dPlanes) + planeBytes);
@@ -827,16 +850,9 @@ int v3dm_voctree_allocate(v3dm_voctree* t, int nMax) {
        cudaMalloc(reinterpret_cast<void**>(&t->dItems), (m / kVtMinItem + vt_bins(t) + 1) * sizeof(int4)) !=
            cudaSuccess))
     return V3DM_ERR_CUDA;
-  // the float descent's lists and split keys (548 bytes per key; without them calls take k_voctree_f32)
-  if (vt_f_wanted(t, nMax) &&
-      (cudaMalloc(reinterpret_cast<void**>(&t->dFlagged), 2 * m * sizeof(int4)) != cudaSuccess ||
-       cudaMalloc(reinterpret_cast<void**>(&t->dWeird), m * sizeof(int32_t)) != cudaSuccess ||
-       cudaMalloc(&t->dSplit, m * (kVtfRowBytes + sizeof(float))) != cudaSuccess)) {
-    cudaGetLastError();
-    t->dSplit = nullptr;
-  }
   t->nMax = nMax;
-  return vt_planes(t);
+  t->fNoRoom = false;
+  return t->nodesU8 ? V3DM_OK : vt_float_descent(t);
 }
 
 int v3dm_voctree_set_nodes_u8(v3dm_voctree* t, const uint8_t* nodes) {
@@ -844,7 +860,7 @@ int v3dm_voctree_set_nodes_u8(v3dm_voctree* t, const uint8_t* nodes) {
   DeviceGuardVt g(t->device);
   if (!t->dNodes && cudaMalloc(reinterpret_cast<void**>(&t->dNodes), (size_t)t->nodeCount * kDescBytes) != cudaSuccess)
     return V3DM_ERR_CUDA;
-  t->nodesU8 = t->nodesF = t->planesReady = false;
+  t->nodesU8 = t->nodesF = t->planesReady = t->fNoRoom = false;
   if (cudaMemcpyAsync(t->dNodes, nodes, (size_t)t->nodeCount * kDescBytes, cudaMemcpyHostToDevice, t->stream) !=
           cudaSuccess ||
       cudaStreamSynchronize(t->stream) != cudaSuccess)
@@ -856,7 +872,7 @@ int v3dm_voctree_set_nodes_u8(v3dm_voctree* t, const uint8_t* nodes) {
 int v3dm_voctree_set_nodes_f32(v3dm_voctree* t, const float* nodes) {
   if (!t || !nodes) return V3DM_ERR_ARG;
   DeviceGuardVt g(t->device);
-  t->nodesU8 = t->nodesF = t->planesReady = false;
+  t->nodesU8 = t->nodesF = t->planesReady = t->fNoRoom = false;
   int st = vt_alloc_float_tree(t);
   if (st != V3DM_OK) return st;
   if (!t->dNodes && cudaMalloc(reinterpret_cast<void**>(&t->dNodes), (size_t)t->nodeCount * kDescBytes) != cudaSuccess)
@@ -871,7 +887,7 @@ int v3dm_voctree_set_nodes_f32(v3dm_voctree* t, const float* nodes) {
   if (st != V3DM_OK) return st;
   t->nodesF = true;
   t->nodesU8 = exact;  // u/512 trees also keep the faster integer descent
-  return vt_planes(t);
+  return exact ? V3DM_OK : vt_float_descent(t);
 }
 
 int v3dm_voctree_quantize_u8(v3dm_voctree* t, int n, const uint8_t* keys, int32_t* ids, int idMode) {
