@@ -163,12 +163,13 @@ __global__ void __launch_bounds__(kVtScatterThreads)
 k_vt_scatter(const int32_t* __restrict__ bucket, int n, const int* __restrict__ off, int* __restrict__ cursor,
              int32_t* __restrict__ perm, int bins, const int* __restrict__ err) {
   extern __shared__ int vtScatterSmem[];  // 2 x bins when bins <= kVtLocalBins
-  if (*err) return;
+  const int failed = *err;
   int* cnt = vtScatterSmem;
   int* base = vtScatterSmem + bins;
   const long long per = ((long long)n + gridDim.x - 1) / gridDim.x;
   const int k0 = (int)min((long long)n, per * blockIdx.x), k1 = (int)min((long long)n, per * (blockIdx.x + 1));
   if (bins > kVtLocalBins) {  // too many buckets for shared memory: one global atomic per key
+    if (failed) return;
     for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
       const int b = bucket[k];
       perm[off[b] + atomicAdd(&cursor[b], 1)] = k;
@@ -177,6 +178,7 @@ k_vt_scatter(const int32_t* __restrict__ bucket, int n, const int* __restrict__ 
   }
   for (int b = threadIdx.x; b < bins; b += blockDim.x) cnt[b] = 0;
   __syncthreads();
+  if (failed) return;
   for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) atomicAdd(&cnt[bucket[k]], 1);
   __syncthreads();
   for (int b = threadIdx.x; b < bins; b += blockDim.x) {
@@ -374,7 +376,7 @@ struct v3dm_voctree {
   float* dStage = nullptr;
   int32_t* dIds = nullptr;
   int32_t* dErr = nullptr;      // flags of the one-kernel descents and conversions, until they are read
-  int32_t* dPhaseErr = nullptr; // flags of the phases; the word before dHist, cleared with its counts by each call
+  int32_t* dPhaseErr = nullptr; // flags of the phases; before dHist, cleared with its counts by each call
   int32_t* hErr = nullptr;      // pinned mirror of both
   long long testWaitLimit = 0;  // failure-path test hooks of the first phase (v3dm_voctree_test_wait_fault)
   int testSkipLoad = 0;
@@ -385,7 +387,7 @@ struct v3dm_voctree {
   long long maxBins = 1;        // buckets of the last phase
   int32_t* dBucket = nullptr;   // nMax: per key, the bucket it reached
   int32_t* dPerm = nullptr;     // nMax: keys in bucket order
-  int* dErrHist = nullptr;      // two spare words, dErr, dPhaseErr, dHist
+  int* dErrHist = nullptr;      // three spare words, dErr, dPhaseErr, three spare words, dHist
   int* dHist = nullptr;         // vt_bins counts, then as many cursors
   int* dOff = nullptr;          // maxBins + 1
   int4* dItems = nullptr;       // nMax / kVtMinItem + vt_bins + 1
@@ -460,7 +462,7 @@ int vt_float_descent(v3dm_voctree* t);
 // only the phases after the first read.
 int vt_clear_hist(v3dm_voctree* t, long long bins, bool first) {
   int* from = first ? t->dPhaseErr : t->dHist;
-  const size_t words = (size_t)bins + (first ? 1 : 0);
+  const size_t words = (size_t)bins + (first ? t->dHist - t->dPhaseErr : 0);
   return cudaMemsetAsync(from, 0, words * sizeof(int), t->stream) == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
 }
 
@@ -757,10 +759,10 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
   vt_plan(t);
   DeviceGuardVt g(device);
   if (cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(reinterpret_cast<void**>(&t->dErrHist), (4 + 2 * (size_t)vt_bins(t)) * sizeof(int)) != cudaSuccess ||
+      cudaMalloc(reinterpret_cast<void**>(&t->dErrHist), (8 + 2 * (size_t)vt_bins(t)) * sizeof(int)) != cudaSuccess ||
       cudaMallocHost(reinterpret_cast<void**>(&t->hErr), 2 * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&t->dReplays), sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMemsetAsync(t->dErrHist, 0, 4 * sizeof(int), t->stream) != cudaSuccess ||
+      cudaMemsetAsync(t->dErrHist, 0, 8 * sizeof(int), t->stream) != cudaSuccess ||
       cudaMemsetAsync(t->dReplays, 0, sizeof(unsigned long long), t->stream) != cudaSuccess ||
       (vt_bins(t) > 0 &&
        (cudaMalloc(reinterpret_cast<void**>(&t->dOff), ((size_t)vt_bins(t) + 1) * sizeof(int)) != cudaSuccess ||
@@ -781,9 +783,9 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
     delete t;
     return V3DM_ERR_CUDA;
   }
-  t->dErr = t->dErrHist + 2;
-  t->dPhaseErr = t->dErrHist + 3;
-  t->dHist = t->dErrHist + 4;
+  t->dErr = t->dErrHist + 3;
+  t->dPhaseErr = t->dErrHist + 4;
+  t->dHist = t->dErrHist + 8;
   *out = t;
   return V3DM_OK;
 }

@@ -135,6 +135,7 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
   VtfSmem& s = *reinterpret_cast<VtfSmem*>((reinterpret_cast<uintptr_t>(vtfRaw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long lim = a.waitLimit > 0 ? a.waitLimit : kWaitCycles;
+  const int failed = a.singleN > 0 || threadIdx.x != 0 ? 0 : *a.err != 0;
   int nIt = a.singleN > 0 ? (a.singleN + a.itemKeys - 1) / a.itemKeys : *a.nItems;
   const bool localHist = !a.final && a.bins <= kVfLocalBins;
   // B rows: one level, the children (N = BF rounded up to 16); two, N2 = BF^2 rounded up to 16 rows
@@ -160,7 +161,7 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
       mbar_init(&s.emptyB[i], 1);
     }
     mbar_init(&s.mmaDone, 1);
-    s.abort = a.singleN > 0 ? 0 : *a.err != 0;  // an earlier phase gave up: there are no items
+    s.abort = failed;  // an earlier phase gave up: there are no items
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (localHist)

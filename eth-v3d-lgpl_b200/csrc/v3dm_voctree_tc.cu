@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
   VtcSmem<BF>& s = *reinterpret_cast<VtcSmem<BF>*>((reinterpret_cast<uintptr_t>(vtcRaw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long lim = a.waitLimit > 0 ? a.waitLimit : kWaitCycles;
+  const int failed = a.singleN > 0 || threadIdx.x != 0 ? 0 : *a.err != 0;
   int nIt = a.singleN > 0 ? (a.singleN + kVtcItemKeys - 1) / kVtcItemKeys : *a.nItems;
   const bool localHist = !a.final && a.bins <= kVtcLocalBins;
   const bool gathered = a.perm != nullptr;
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
     }
     for (int i = 0; i < S::kAcc; ++i) mbar_init(&s.accEmpty[i], 4);  // the four warps of the half that takes the tile
     mbar_init(&s.mmaDone, 1);
-    s.abort = a.singleN > 0 ? 0 : *a.err != 0;  // an earlier phase gave up: there are no items
+    s.abort = failed;  // an earlier phase gave up: there are no items
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (localHist)
