@@ -229,6 +229,7 @@ struct VtfArgs {
   int bins;
   int4* flagged;                 // two per listed key: (key, node, levels, 0), the candidate children's mask
   int* nFlagged;
+  int* ticket;                   // resolution: zero, and its last block leaves it and *nFlagged zero (null: as they are)
   int32_t* weird;                // null after the first phase
   int* nWeird;
   int* err;                      // as in VtcArgs
@@ -244,6 +245,9 @@ cudaError_t launch_vtf_split(const float* keys, int n, void* split, float* norm,
 // The phase and the resolution of what it listed.
 cudaError_t launch_vtf(const VtfArgs& a, const CUtensorMap& m, const float* nodes, unsigned long long* exactCount,
                        int grid, cudaStream_t st);
+// The resolution alone, by programmatic launch: `blocks` blocks of eight warps, a warp per listed key at a time.
+cudaError_t launch_vtf_resolve(const VtfArgs& a, const float* nodes, unsigned long long* exactCount, int blocks,
+                               cudaStream_t st);
 // 2-D map over rows x 128 bytes with a box of boxRows rows and the 128-byte swizzle (v3dm_match_tc.cu).
 cudaError_t tc_rows_map(CUtensorMap* m, const uint8_t* base, int rows, int boxRows);
 

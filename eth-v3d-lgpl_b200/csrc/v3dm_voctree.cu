@@ -14,7 +14,7 @@
 //   - k_voctree otherwise: one launch, four threads per key (below).
 // Float nodes and keys of any value:
 //   - the tensor-core descent with exact replay of near ties (v3dm_voctree_f.cu) for shapes and
-//     calls with enough keys per bucket (vt_f_wanted);
+//     calls with enough keys (vt_f_wanted);
 //   - k_voctree_f32 otherwise: float nodes and keys (the apps' trees are float k-means
 //     centres of unit-L2 descriptors, v3d_voctree.h:38-52).  The leaf ids equal those of the
 //     reference's CPU tree, VocabularyTree::findBestNodeIndex (v3d_voctree.h:82-99), which sums
@@ -29,7 +29,8 @@
 //     precomputed node norms rounded up.  When one child's lower bound is above every other
 //     child's upper bound (and above -1e30f), it is the sequential rule's choice.  Otherwise
 //     (near ties, equal children, non-finite values) one thread of the key replays the
-//     reference's sequential FP32 loop over all children, with __fmul_rn / __fadd_rn.
+//     reference's sequential FP32 loop over all children, with __fmul_rn / __fadd_rn, or the key is
+//     listed and k_vtf_resolve does, a child per lane (vt_f_listed).
 //
 // k_voctree: four threads per key, each holding 32 bytes of the key in registers; a warp
 // descends eight keys.  At each level a thread loads its 32-byte slice of every child (each
@@ -219,12 +220,17 @@ __device__ __forceinline__ int seq_best_child(const float* __restrict__ key, con
 // q = 0..7, so the four threads of a key read 64 contiguous bytes of a node row per load.
 // nodeNorm[i] >= |node i| (L2).  exactCount (optional) counts the key-levels resolved by the
 // sequential replay.  err gets kErrBadTree when a child block would leave the tree.  With list, the
-// keys are list[0 .. *listN) instead of 0 .. n - 1.
+// keys are list[0 .. *listN) instead of 0 .. n - 1.  With undecided, a key whose level the bounds cannot
+// decide is not replayed by one of its threads while the warp waits, 10 us and more a level, but listed with
+// the levels it has left (as VtfArgs::flagged), and k_vtf_resolve descends them; keys of no finite or of huge
+// scores are still replayed here.
 __global__ void __launch_bounds__(kVtThreads, 2)
 k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNorm, long long nodeCount, int bf,
               int depth, long long leafBase, const float* __restrict__ keys, int n, int32_t* __restrict__ out,
               int idMode, unsigned long long* __restrict__ exactCount, int32_t* __restrict__ err,
-              const int32_t* __restrict__ list, const int* __restrict__ listN) {
+              const int32_t* __restrict__ list, const int* __restrict__ listN, int4* __restrict__ undecided,
+              int* __restrict__ nUndecided) {
+  pdl_launch_dependents();
   const int gt = blockIdx.x * kVtThreads + threadIdx.x;
   const int part = gt % kTpk;
   const int lane = threadIdx.x & 31;
@@ -249,9 +255,9 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
   ss += __shfl_xor_sync(0xffffffffu, ss, 1);
   ss += __shfl_xor_sync(0xffffffffu, ss, 2);
   const float kn = __fmul_ru(__fsqrt_ru(ss), 1.000001f);
-  long long nextId = 0, leafId = 0;
+  long long nextId = 0, leafId = -1;
   unsigned long long replays = 0;
-  bool ok = true;
+  bool ok = true, listed = false;
   for (int d = 0; d < depth; ++d) {
     if (nextId < 0 || nextId + bf > nodeCount) {  // cannot happen for a finite tree; leaves the loop safely
       ok = false;
@@ -261,6 +267,7 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
     float lo1 = -INFINITY, up1 = -INFINITY, up2 = -INFINITY;
     int c1 = -1, cu1 = -1;
     bool finite = true;
+    float eMax = 0.0f;
 #pragma unroll 2
     for (int c = 0; c < bf; ++c) {
       const float4* row = reinterpret_cast<const float4*>(base + (size_t)c * kDescBytes) + part;
@@ -277,6 +284,7 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
       acc += __shfl_xor_sync(0xffffffffu, acc, 2);
       const float e = __fadd_ru(__fmul_ru(__fmul_ru(kSeqRel, kn), __ldg(nodeNorm + nextId + c)), kSeqAbs);
       const float lo = __fsub_rd(acc, e), up = __fadd_ru(acc, e);
+      eMax = fmaxf(eMax, e);
       finite = finite && isfinite(lo) && isfinite(up);
       if (lo > lo1) {
         lo1 = lo;
@@ -293,7 +301,15 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
     const float othersUp = cu1 == c1 ? up2 : up1;
     int best = c1;
     // the same on the four lanes of the key: their scores and bounds are bit-identical
-    if (!(finite && c1 >= 0 && othersUp < lo1 && lo1 > -1e30f)) {
+    const bool usual = finite && c1 >= 0 && lo1 > -1e30f;
+    if (undecided && usual && !(othersUp < lo1) && eMax < kSeqRel * 1e30f) {
+      if (part == 0 && valid && !listed) {
+        const int slot = atomicAdd(nUndecided, 1);
+        undecided[2 * slot] = make_int4(key, (int)leafId, depth - d, 0);
+        undecided[2 * slot + 1] = make_int4(-1, -1, -1, -1);  // all children
+      }
+      listed = true;
+    } else if (!(usual && othersUp < lo1) && !listed) {
       int b = -1;
       if (part == 0 && valid) {
         b = seq_best_child(krow, base, bf);
@@ -301,12 +317,12 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
       }
       best = __shfl_sync(grp, b, lane & ~3);
     }
-    if (!valid) best = 0;
+    if (!valid || listed) best = 0;
     leafId = nextId + best;
     nextId = (leafId + 1) * bf;
   }
   if (!ok && part == 0 && valid) atomicOr(err, kErrBadTree);
-  if (valid && part == 0) out[key] = (int32_t)(idMode == V3DM_LEAF_LOCAL ? leafId - leafBase : leafId);
+  if (valid && part == 0 && !listed) out[key] = (int32_t)(idMode == V3DM_LEAF_LOCAL ? leafId - leafBase : leafId);
   if (exactCount && part == 0 && replays) atomicAdd(exactCount, replays);
   }
 }
@@ -406,6 +422,7 @@ struct v3dm_voctree {
   void* dSplit = nullptr;       // nMax split keys, then their norms
   int32_t* dWeird = nullptr;    // nMax
   int* dFCounts = nullptr;      // [0] weird keys, [1 + p] listed keys of phase p
+  int* dListCount = nullptr;    // behind them: keys the one-kernel descent listed, then a ticket; zero between calls
   CUtensorMap tmPlanes;
   CUtensorMap tmNodes;          // the u8 node rows for the tensor path's TMA loads
   bool tmValid = false;
@@ -449,11 +466,29 @@ long long vt_bins(const v3dm_voctree* t) {
   return std::max(t->tcPath ? t->maxBins : 0, t->fLevels ? t->fMaxBins : 0);
 }
 
-// A call of n keys takes the float tensor descent when the last phase has at least kVtMinPerBin keys
-// per bucket: below that the tiles of 128 keys are mostly empty (and the node planes, 512 bytes a node,
-// are not made for trees whose calls cannot reach it).
+// The ways of a call of n float keys.  Below kVtMinPerBin keys per bucket of the last phase, the tiles of 128
+// keys would be mostly empty: k_voctree_f32, which replays near ties itself.  From there on k_voctree_f32
+// lists them for k_vtf_resolve, until the phases are faster: the two kernels take about 5 us, 0.45 us per child
+// row of a path (bf * depth of them) and 41 ps per key and row, the phases 28 us each, 150 ps per key each and
+// 100 ps per key.  Measured on k-means trees, us (one kernel, two, phases):
+//   BF 10, depth 4:   4000 keys 62, 31, 61;   16000 88, 39, 67;   25600 92, 64, 67;   64000 174, 114, 89
+//   BF 5, depth 4:    4000 keys 27, 25, 57;   64000 83, 68, 72;   200000 213, 166, 142
+//   BF 16, depth 1:   4000 keys 31, 15, 25;   64000 60, 38, 34
+//   BF 33, depth 1:   256 keys 14, 15, 24;    4000 61, 25, 26;    64000 115, 68, 36
+//   BF 50, depth 3:   40000 keys 574, 291, 149
+//   BF 128, depth 2:  2048 keys 523, 128, 58
+//   BF 2, depth 8:    4096 keys 17, 33, 116;  64000 57, 76, 139: with so few children a replay costs less than the
+//                     second kernel, but phases never pay.
+// (The node planes, 512 bytes a node, and the split keys are not made for trees whose calls cannot reach
+// the phases.)
 constexpr int kVtMinPerBin = 16;
-bool vt_f_wanted(const v3dm_voctree* t, long long n) { return t->fLevels > 0 && n >= kVtMinPerBin * t->fMaxBins; }
+bool vt_f_listed(const v3dm_voctree* t, long long n) { return t->fLevels > 0 && n >= kVtMinPerBin * t->fMaxBins; }
+bool vt_f_wanted(const v3dm_voctree* t, long long n) {
+  const long long rows = (long long)t->bf * t->depth;
+  const long long perKey = 41 * rows - 150 * t->fPhases - 100;                     // ps
+  const long long once = 28000000LL * t->fPhases - 5000000LL - 450000LL * rows;  // ps
+  return vt_f_listed(t, n) && n * perKey >= once;
+}
 
 int vt_sort(v3dm_voctree* t, int n, long long bins, int itemKeys);
 int vt_float_descent(v3dm_voctree* t);
@@ -553,20 +588,39 @@ int vt_sort(v3dm_voctree* t, int n, long long bins, int itemKeys) {
 int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int idMode) {
   t->lastLaunches = 0;
   if (n == 0) return V3DM_OK;
-  if (vt_f_wanted(t, n) && n <= t->nMax) {
+  if (vt_f_listed(t, n) && n <= t->nMax) {
     const int st = vt_float_descent(t);
     if (st != V3DM_OK) return st;
   }
-  if (!vt_f_wanted(t, n) || !t->planesReady || !t->dSplit || n > t->nMax) {
+  const bool lists = vt_f_listed(t, n) && n <= t->nMax && t->dFlagged && t->dWeird;
+  if (!lists || !vt_f_wanted(t, n) || !t->planesReady || !t->dSplit) {
     t->lastLaunches = 1;
     long long threads = (long long)n * kTpk;
     unsigned blocks = (unsigned)((threads + kVtThreads - 1) / kVtThreads);
     k_voctree_f32<<<blocks, kVtThreads, 0, t->stream>>>(t->dNodesF, t->dNorm, t->nodeCount, t->bf, t->depth,
                                                         t->leafBase, dKeys, n, dIds, idMode, t->dReplays, t->dErr,
-                                                        nullptr, nullptr);
-    return cudaGetLastError() == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
+                                                        nullptr, nullptr, lists ? t->dFlagged : nullptr,
+                                                        lists ? t->dListCount : nullptr);
+    if (cudaGetLastError() != cudaSuccess) return V3DM_ERR_CUDA;
+    if (!lists) return V3DM_OK;
+    VtfArgs va;
+    std::memset(&va, 0, sizeof(va));
+    va.keys = dKeys;
+    va.bf = t->bf;
+    va.final = 1;
+    va.out = dIds;
+    va.idMode = idMode;
+    va.leafBase = t->leafBase;
+    va.flagged = t->dFlagged;
+    va.nFlagged = t->dListCount;
+    va.ticket = t->dListCount + 1;
+    va.err = t->dErr;
+    t->lastLaunches = 2;
+    const int warps8 = std::max(1, std::min(8 * t->numSMs, n / 64));
+    if (launch_vtf_resolve(va, t->dNodesF, t->dReplays, warps8, t->stream) == cudaSuccess) return V3DM_OK;
+    cudaMemsetAsync(t->dListCount, 0, 2 * sizeof(int), t->stream);  // nothing else will
+    return V3DM_ERR_CUDA;
   }
-  if (cudaMemsetAsync(t->dFCounts, 0, (1 + kVtMaxPhases) * sizeof(int), t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
   float* keyNorm = reinterpret_cast<float*>(static_cast<uint8_t*>(t->dSplit) + (size_t)t->nMax * kVtfRowBytes);
   if (launch_vtf_split(dKeys, n, t->dSplit, keyNorm, t->numSMs, t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
   t->lastLaunches += 1;
@@ -592,6 +646,7 @@ int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int
   va.nWeird = t->dFCounts;
   va.err = t->dPhaseErr;
   va.waitLimit = t->testWaitLimit;
+  if (cudaMemsetAsync(t->dFCounts, 0, (1 + kVtMaxPhases) * sizeof(int), t->stream) != cudaSuccess) return V3DM_ERR_CUDA;
   long long bins = 1;
   for (int p = 0; p < t->fPhases; ++p) {
     const int d0 = p * t->fLevels;
@@ -622,7 +677,7 @@ int vt_launch_f32(v3dm_voctree* t, int n, const float* dKeys, int32_t* dIds, int
   // keys that are not finite (or overflow): the whole descent in one kernel, over what the phases wrote
   k_voctree_f32<<<2 * t->numSMs, kVtThreads, 0, t->stream>>>(t->dNodesF, t->dNorm, t->nodeCount, t->bf, t->depth,
                                                             t->leafBase, dKeys, n, dIds, idMode, t->dReplays, t->dErr,
-                                                            t->dWeird, t->dFCounts);
+                                                            t->dWeird, t->dFCounts, nullptr, nullptr);
   t->lastLaunches += 1;
   return cudaGetLastError() == cudaSuccess ? V3DM_OK : V3DM_ERR_CUDA;
 }
@@ -674,42 +729,38 @@ int vt_ensure_float_tree(v3dm_voctree* t) {
   return V3DM_OK;
 }
 
-// What the tensor-core descent of float keys needs beside the sorting buffers: the split node planes, and
-// for nMax keys its lists and the split keys (548 bytes per key).  Made once the tree is a float tree and calls can
-// be large enough: when a tree of other values than u/512 is set or allocated for, and otherwise with the
-// first float keys that want it, since byte trees and keys never use them.  What does not fit in memory, or
+// What calls of float keys need beside the tree: for nMax keys the lists (36 bytes per key) and, where they can be
+// large enough for the phases, the split keys (516 bytes per key) and the split node planes.  Made once the tree is a
+// float tree: when a tree of other values than u/512 is set or allocated for, and otherwise with the
+// first float keys that want them, since byte trees and keys never use them.  What does not fit in memory, or
 // would have to be made while the stream is being captured, leaves the one-kernel descent.
 int vt_float_descent(v3dm_voctree* t) {
-  if (!t->nodesF || !vt_f_wanted(t, t->nMax) || (t->planesReady && t->dSplit) || t->fNoRoom) return V3DM_OK;
+  const bool phases = vt_f_wanted(t, t->nMax);
+  if (!t->nodesF || !vt_f_listed(t, t->nMax) || t->fNoRoom) return V3DM_OK;
+  if (t->dFlagged && t->dWeird && (!phases || (t->planesReady && t->dSplit))) return V3DM_OK;
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(t->stream, &capture) != cudaSuccess) return V3DM_ERR_CUDA;
   if (capture != cudaStreamCaptureStatusNone) return V3DM_OK;
   const size_t m = (size_t)t->nMax;
-  if (!t->dSplit && ((!t->dFlagged &&
-                      cudaMalloc(reinterpret_cast<void**>(&t->dFlagged), 2 * m * sizeof(int4)) != cudaSuccess) ||
-                     (!t->dWeird &&
-                      cudaMalloc(reinterpret_cast<void**>(&t->dWeird), m * sizeof(int32_t)) != cudaSuccess) ||
-                     cudaMalloc(&t->dSplit, m * (kVtfRowBytes + sizeof(float))) != cudaSuccess)) {
-    cudaGetLastError();
-    t->dSplit = nullptr;
-    t->fNoRoom = true;
+  auto make = [&](void** p, size_t bytes) {  // whether it is there
+    if (!*p && cudaMalloc(p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+      t->fNoRoom = true;
+    }
+    return *p != nullptr;
+  };
+  if (!make(reinterpret_cast<void**>(&t->dFlagged), 2 * m * sizeof(int4)) ||
+      !make(reinterpret_cast<void**>(&t->dWeird), m * sizeof(int32_t)) || !phases ||
+      !make(&t->dSplit, m * (kVtfRowBytes + sizeof(float))) || t->planesReady)
     return V3DM_OK;
-  }
-  if (t->planesReady) return V3DM_OK;
   // one block: the planes, then the children's norms (nodeCount / BF parents, the root among them)
   const size_t planeBytes = (size_t)t->nodeCount * kVtfRowBytes;
-  if (!t->dPlanes &&
-      cudaMalloc(&t->dPlanes, planeBytes + (size_t)(t->nodeCount / t->bf) * sizeof(float)) != cudaSuccess) {
-    cudaGetLastError();
-    t->dPlanes = nullptr;
-    t->fNoRoom = true;
-    return V3DM_OK;
-  }
+  if (!make(&t->dPlanes, planeBytes + (size_t)(t->nodeCount / t->bf) * sizeof(float))) return V3DM_OK;
   t->dChildNorm = reinterpret_cast<float*>(static_cast<uint8_t*>(t->dPlanes) + planeBytes);
-  if (vtf_prepare(t->dNodesF, t->dNorm, t->nodeCount, t->bf, t->dPlanes, t->dChildNorm, t->dMaxNorm, &t->tmPlanes,
-                  t->stream) != cudaSuccess)
-    return V3DM_ERR_CUDA;
-  t->planesReady = true;
+  t->planesReady = vtf_prepare(t->dNodesF, t->dNorm, t->nodeCount, t->bf, t->dPlanes, t->dChildNorm, t->dMaxNorm,
+                               &t->tmPlanes, t->stream) == cudaSuccess;
+  t->fNoRoom = !t->planesReady;
   return V3DM_OK;
 }
 
@@ -767,7 +818,8 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
       (vt_bins(t) > 0 &&
        (cudaMalloc(reinterpret_cast<void**>(&t->dOff), ((size_t)vt_bins(t) + 1) * sizeof(int)) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&t->dMaxNorm), sizeof(float)) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&t->dFCounts), (1 + kVtMaxPhases) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(reinterpret_cast<void**>(&t->dFCounts), (3 + kVtMaxPhases) * sizeof(int)) != cudaSuccess ||
+        cudaMemsetAsync(t->dFCounts, 0, (3 + kVtMaxPhases) * sizeof(int), t->stream) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&t->dNItems), sizeof(int)) != cudaSuccess ||
         cudaFuncSetAttribute(k_vt_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              2 * kVtLocalBins * (int)sizeof(int)) != cudaSuccess)) ||
@@ -786,6 +838,7 @@ int v3dm_voctree_create(v3dm_voctree** out, int device, int bf, int depth) {
   t->dErr = t->dErrHist + 3;
   t->dPhaseErr = t->dErrHist + 4;
   t->dHist = t->dErrHist + 8;
+  if (t->dFCounts) t->dListCount = t->dFCounts + 1 + kVtMaxPhases;
   *out = t;
   return V3DM_OK;
 }

@@ -251,3 +251,34 @@ def test_tensor_descent_of_narrow_trees_with_many_tiles(v3dm_mod, oracle_mod, bf
             for _ in range(2):
                 np.testing.assert_array_equal(t.traverse_tree(keys[:m], v3dm_mod.LEAF_LOCAL), exp[:m])
                 assert t.last_launches() > 1
+
+
+@pytest.mark.parametrize("bf,depth,n,launches", [(5, 1, 16, 2), (2, 8, 4097, 2), (5, 4, 20000, 2), (10, 3, 1601, 2),
+                                                 (10, 4, 26000, 2), (10, 4, 27000, 8), (16, 1, 33, 2), (32, 2, 513, 2),
+                                                 (33, 1, 64, 2), (50, 1, 16, 2), (50, 1, 2000, 4), (50, 2, 801, 2),
+                                                 (128, 2, 2048, 8), (3, 5, 1295, 1), (300, 2, 3000, 1)])
+@pytest.mark.parametrize("ties", [False, True])
+def test_float_ways_of_small_calls(v3dm_mod, oracle_mod, bf, depth, n, launches, ties):
+    """Float calls on both sides of the line between the one-kernel descent, that descent with its undecided keys
+    listed, and the phases: ids of the oracle's sequential FP32 descent for unit descriptors, for nodes of which a
+    third are copies of their neighbours (equal scores), and for zero, NaN, infinite and overflowing keys; every
+    way twice, since the lists' counters are left clean by the kernel that reads them."""
+    rng = synth.rng_for(9500 + 100 * bf + depth)
+    count = v3dm_mod.voctree_counts(bf, depth)[0]
+    nodes, keys = synth.unit_sift(rng, count), synth.unit_sift(rng, n)
+    if ties:
+        nodes[1::3] = nodes[0::3][: len(nodes[1::3])]
+        keys[1] = 0.0
+        keys[2] = np.nan
+        keys[3, 5] = np.inf
+        keys[4] = 3e38
+        keys[5] = -keys[5]
+        keys[6] *= 1e18
+    exp = oracle_mod.voctree(bf, depth, nodes, keys, False)
+    with v3dm_mod.VocabularyTreeTraversal(bf, depth) as t:
+        t.allocate(n)
+        t.set_nodes(nodes)
+        for _ in range(2):
+            np.testing.assert_array_equal(t.traverse_tree(keys, v3dm_mod.LEAF_LOCAL), exp)
+            assert t.last_launches() == launches
+        assert not ties or t.replays() > 0
