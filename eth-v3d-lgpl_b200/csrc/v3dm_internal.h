@@ -238,6 +238,9 @@ struct VtfArgs {
 };
 int vtf_levels(int bf);          // levels a phase descends (0: shape not supported)
 constexpr int kVtfRowBytes = 512;  // split planes per node or key
+// A key's norm from FP32 squares is good to 1e-6 above 3e-19 (a square loses at most 2^-150); a key below this
+// line, well above that one, has no bound to decide a level with.
+constexpr float kVtTinyNorm = 1e-15f;
 // The split node planes, the norms above (childNorm: rows / bf entries) and the planes' tensor map.
 cudaError_t vtf_prepare(const float* nodes, const float* norm, long long rows, int bf, void* planes, float* childNorm,
                         float* maxNorm, CUtensorMap* map, cudaStream_t st);

@@ -26,7 +26,7 @@
 //     gamma_128 * sum|k_i n_i| <= 7.63e-6 * |k| |n| of the exact dot product (the standard bound
 //     for recursive summation, n = 128 terms; the FMA pass has at most 34 roundings per term),
 //     so |fast - sequential| <= 1.53e-5 * |k| |n|; the kernel uses 2e-5 * |k| |n| + 1e-36 with
-//     precomputed node norms rounded up.  When one child's lower bound is above every other
+//     precomputed node norms rounded up (and nothing for keys whose squares may underflow).  When one child's lower bound is above every other
 //     child's upper bound (and above -1e30f), it is the sequential rule's choice.  Otherwise
 //     (near ties, equal children, non-finite values) one thread of the key replays the
 //     reference's sequential FP32 loop over all children, with __fmul_rn / __fadd_rn, or the key is
@@ -255,6 +255,7 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
   ss += __shfl_xor_sync(0xffffffffu, ss, 1);
   ss += __shfl_xor_sync(0xffffffffu, ss, 2);
   const float kn = __fmul_ru(__fsqrt_ru(ss), 1.000001f);
+  const bool bounded = kn >= kVtTinyNorm;
   long long nextId = 0, leafId = -1;
   unsigned long long replays = 0;
   bool ok = true, listed = false;
@@ -302,14 +303,15 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
     int best = c1;
     // the same on the four lanes of the key: their scores and bounds are bit-identical
     const bool usual = finite && c1 >= 0 && lo1 > -1e30f;
-    if (undecided && usual && !(othersUp < lo1) && eMax < kSeqRel * 1e30f) {
+    const bool decided = usual && othersUp < lo1 && bounded;
+    if (undecided && usual && !decided && eMax < kSeqRel * 1e30f) {
       if (part == 0 && valid && !listed) {
         const int slot = atomicAdd(nUndecided, 1);
         undecided[2 * slot] = make_int4(key, (int)leafId, depth - d, 0);
         undecided[2 * slot + 1] = make_int4(-1, -1, -1, -1);  // all children
       }
       listed = true;
-    } else if (!(usual && othersUp < lo1) && !listed) {
+    } else if (!decided && !listed) {
       int b = -1;
       if (part == 0 && valid) {
         b = seq_best_child(krow, base, bf);

@@ -17,6 +17,8 @@
 //     largest norm among the node's children); else the key goes to a list and k_vtf_resolve evaluates
 //     the reference's sequential sums over all the children, one child per lane: 1 to 4% of the
 //     key-levels on k-means trees of unit descriptors.
+//   - Keys of a norm below kVtTinyNorm are listed at every level: their bound would be relative to a norm that
+//     FP32 squares do not give.
 //   - Keys whose norm times the largest node norm is not below 1e30 (NaN, infinities, overflow) are
 //     listed and descend with k_voctree_f32 at the end, whatever the phases made of them.
 // A phase descends one level (BF <= 128), or two where BF^2 grandchildren and BF children fit 128
@@ -356,7 +358,7 @@ k_vtf(VtfArgs a, const __grid_constant__ CUtensorMap tmNodes) {
           }
         }
         const float tiny = 1e-30f * (1.0f + kn + maxNorm);  // underflow
-        const float e1 = kTcRel * kn * childNorm + tiny;
+        const float e1 = kn >= kVtTinyNorm ? kTcRel * kn * childNorm + tiny : INFINITY;
         const bool weird = !(kn * maxNorm < 1e30f);
         long long node = g1 + ta.c;
         int undecided = 0;  // levels left to the replay, from node `from` down

@@ -282,3 +282,25 @@ def test_float_ways_of_small_calls(v3dm_mod, oracle_mod, bf, depth, n, launches,
             np.testing.assert_array_equal(t.traverse_tree(keys, v3dm_mod.LEAF_LOCAL), exp)
             assert t.last_launches() == launches
         assert not ties or t.replays() > 0
+
+
+@pytest.mark.parametrize("bf,depth,n,launches", [(10, 4, 40000, 8), (50, 2, 6000, 8), (5, 4, 20000, 2), (300, 2, 3000, 1)])
+def test_float_keys_of_tiny_norm(v3dm_mod, oracle_mod, bf, depth, n, launches):
+    """Keys whose squares underflow (norms from 1e-14 down to subnormal values), on nodes within 1% of each other: the
+    bounds that decide a level are relative to a norm that such a key does not have in FP32, so its levels are
+    evaluated in order.  Ids of the oracle's sequential FP32 descent."""
+    rng = synth.rng_for(9700 + bf)
+    count = v3dm_mod.voctree_counts(bf, depth)[0]
+    nodes = (synth.unit_sift(rng, 1) * (1 + rng.normal(0, 0.01, (count, 128)))).astype(np.float32)
+    keys = synth.unit_sift(rng, n)
+    scale = np.array([1.0, 1e-14, 1e-16, 1e-18, 1e-19, 1e-20, 1e-21, 1e-22, 1e-25, 1e-30, 1e-36, 1e-39])
+    keys = (keys.astype(np.float64) * scale[np.arange(n) % len(scale), None]).astype(np.float32)
+    exp = oracle_mod.voctree(bf, depth, nodes, keys, False)
+    with v3dm_mod.VocabularyTreeTraversal(bf, depth) as t:
+        t.allocate(n)
+        t.set_nodes(nodes)
+        got = t.traverse_tree(keys, v3dm_mod.LEAF_LOCAL)
+        assert t.last_launches() == launches
+    for k, s in enumerate(scale):
+        print(s, int((got[k::len(scale)] != exp[k::len(scale)]).sum()))
+    np.testing.assert_array_equal(got, exp)
