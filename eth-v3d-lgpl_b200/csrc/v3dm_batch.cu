@@ -966,7 +966,7 @@ struct v3dm_batch {
   cudaGraphExec_t graphP[2] = {};
   uint32_t gpMs = 0, gpMr = 0;
   int gpProbes = 0, gpCells = 0, gpLaunches = 0;
-  const v3dm_projection* gpProj = nullptr;
+  unsigned long long gpProj = 0;    // proj_id
   long long exhaustivePairs = 0;    // sum over pairs of nL * nR
   // guided calls: positions of the images' descriptors and one gate per pair
   float2* dPos = nullptr;
@@ -1881,7 +1881,7 @@ int launch_call_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL
   }
   if (!b->useGraph) return enqueue_proposal(b, proj, probesL, probesR, minScore, minRatio, false);
   const bool sameCall =
-      b->gpMs == ms && b->gpMr == mr && b->gpProbes == probes && b->gpCells == C && b->gpProj == proj;
+      b->gpMs == ms && b->gpMr == mr && b->gpProbes == probes && b->gpCells == C && b->gpProj == proj_id(proj);
   cudaGraphExec_t& graphP = b->graphP[b->toHost];
   if (!graphP || !sameCall) {
     if (!sameCall) drop_graph_p(b);
@@ -1904,7 +1904,7 @@ int launch_call_proposal(v3dm_batch* b, const v3dm_projection* proj, int probesL
     b->gpMr = mr;
     b->gpProbes = probes;
     b->gpCells = C;
-    b->gpProj = proj;
+    b->gpProj = proj_id(proj);
     b->gpLaunches = b->lastLaunches;
   }
   V3DM_BTRY(cudaGraphLaunch(graphP, b->stream));

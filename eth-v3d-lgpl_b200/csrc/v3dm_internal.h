@@ -363,6 +363,7 @@ int host_candidate_threshold(float minScore, float minRatio, bool gated, int32_t
 cudaError_t proj_assign(const v3dm_projection* p, const uint8_t* dDesc, long long n, int probes, uint8_t* dCells,
                         cudaStream_t s);
 int proj_cells(const v3dm_projection* p);
+unsigned long long proj_id(const v3dm_projection* p);  // another for every projection made
 cudaStream_t proj_stream(const v3dm_projection* p);
 
 // Whether a caller's device buffer meets the alignment its kernels access it with (a power of two).

@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -472,7 +473,15 @@ struct PGuard {
 
 using namespace v3dm;
 
+// Numbers of the projections made so far: a captured call belongs to one of them, not to an address that the
+// next one may get.
+static unsigned long long proj_next_id() {
+  static std::atomic<unsigned long long> last{0};
+  return ++last;
+}
+
 struct v3dm_projection {
+  const unsigned long long id = proj_next_id();
   int device = 0;
   cudaStream_t stream = nullptr;
   float* dW = nullptr;                 // FP32 master parameters
@@ -591,6 +600,7 @@ cudaError_t proj_assign(const v3dm_projection* p, const uint8_t* dDesc, long lon
                         p->dCells, p->nCells, probes, dCells, s);
 }
 int proj_cells(const v3dm_projection* p) { return p->nCells; }
+unsigned long long proj_id(const v3dm_projection* p) { return p->id; }
 cudaStream_t proj_stream(const v3dm_projection* p) { return p->stream; }
 }  // namespace v3dm
 

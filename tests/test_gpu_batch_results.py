@@ -82,3 +82,27 @@ def test_triples_around_the_pinned_memory_and_device_calls(v3dm_mod, k):
             assert st == v3dm_mod.ERR_CAPACITY and n.value == 2 * k
             np.testing.assert_array_equal(out[:cap], exp[:cap])
             assert (out[cap:] == -1).all()
+
+
+def test_proposal_calls_with_projections_made_in_turn(v3dm_mod):
+    """Projections made and closed one after the other (each may get the address of the last, but not its device
+    buffers): a batch handle's captured call is used only for the projection it was captured with."""
+    desc, counts, offs, pos, cams = synth.scene(44, 5, 300, 900)
+    rng = synth.rng_for(45)
+    with v3dm_mod.BatchMatching() as kept:
+        kept.set_images(desc, counts)
+        kept.set_pairs(None)
+        hold = []
+        for k in range(6):
+            net = v3dm_mod.Projection(0, seed=100 + k)
+            hold.append(v3dm_mod.Projection(0, seed=1))  # takes the buffers that the last one gave back
+            cells = rng.normal(0, 1, (16, 32)).astype(np.float32)
+            net.set_cells(cells / np.linalg.norm(cells, axis=1, keepdims=True))
+            got = kept.match_proposal(net, 2, 0.7, 0.8, probes_right=2)
+            with v3dm_mod.BatchMatching() as fresh:
+                fresh.set_images(desc, counts)
+                fresh.set_pairs(None)
+                np.testing.assert_array_equal(got, fresh.match_proposal(net, 2, 0.7, 0.8, probes_right=2))
+            net.close()
+        for h in hold:
+            h.close()
