@@ -9,6 +9,8 @@
 
 namespace v3dm {
 
+constexpr int kB200SMs = 148;  // for grids that are sized without a handle's own count
+
 // Launches kernel k with programmatic stream serialization (see pdl_wait in v3dm_device.cuh).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
@@ -342,8 +344,6 @@ cudaError_t launch_choose(const int32_t* leftDec, int nL, int nR, int* chosenFla
 cudaError_t launch_choose_planes(const int32_t* leftDec, int nL, int nR, int* chosenFlag, int* chosenList,
                                  int* chosenCount, const uint8_t* src, uint8_t* dst, int planes, int capSrc, int capDst,
                                  cudaStream_t s);
-// Mutual filter and ordered compaction (blockCount: nL/2048 + 1 ints of scratch); clears chosenFlag.
-// The pair count goes to info[kInfoPairs] and, when countOut is set, to *countOut.
 // Results in pinned host memory, written by the kernel that ends a call: the host only waits for the
 // stream.  info: the info block; pairs: the first cap pairs (null: none).
 struct HostResult {
@@ -351,6 +351,9 @@ struct HostResult {
   int2* pairs;
   int cap;
 };
+// Mutual filter and ordered compaction (blockCount: nL / 256 + 1 ints of scratch); clears chosenFlag.  The
+// pair count goes to *countOut, when that is set, and with the info block to host; the info block and the
+// call's counters behind it are left zero.
 cudaError_t launch_mutual(const int32_t* leftDec, int nL, int nR, const int32_t* rightDec, int* chosenFlag,
                           int* blockCount, int2* pairs, int32_t* info, int32_t* countOut, const HostResult& host,
                           cudaStream_t s);

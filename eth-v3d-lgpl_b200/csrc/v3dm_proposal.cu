@@ -279,9 +279,9 @@ cudaError_t launch_forward(const uint8_t* x, long long n, const __nv_bfloat16* w
   if (n <= 0) return cudaSuccess;
   // Two descriptors per thread once that still gives every SM the two blocks it holds; below that more
   // threads matter more.  As many blocks as are resident at once: each stages the weights.
-  const bool two = n >= 148LL * 2 * 2 * kFwdThreads;
+  const bool two = n >= (long long)kB200SMs * 2 * 2 * kFwdThreads;
   const int tile = kFwdThreads * (two ? 2 : 1);
-  const long long blocks = std::min((n + tile - 1) / tile, 148LL * (two ? 2 : 3));
+  const long long blocks = std::min((n + tile - 1) / tile, (long long)kB200SMs * (two ? 2 : 3));
   auto f = probes <= 4 ? (two ? k_proj_forward<4, 2> : k_proj_forward<4, 1>)
                        : (two ? k_proj_forward<V3DM_PROJ_MAX_PROBES, 2> : k_proj_forward<V3DM_PROJ_MAX_PROBES, 1>);
   f<<<(unsigned)blocks, kFwdThreads, kFwdSmem, s>>>(x, (int)n, w1b, b1, w2b, b2, hOut, zOut, normOut, cells, nCells,

@@ -32,13 +32,13 @@
 //                   to the next round;
 // and at the end
 //   k_rs_finish     pose, error and inlier flags of the chosen candidate.
-// With the loop's iterative refinement (mode.iterativeRefinement, v3dm_ransac_set_refinement),
-// k_rs_select refines each accepted pose as reconstruction_common.cpp:255-314 does: the pose of the
-// accepted sample is refined by refineRelativePose (v3d_poseutilities.cpp:1063-1101: Levenberg-
-// Marquardt on the weighted Sampson residuals of the candidate's inliers; ess::refine_pose restates
-// it, here with its sums over the inliers split across the warp), the refined F is scored over all
-// correspondences in the loop's order, and the loop keeps min(cost, refined cost), the refined
-// model and the refined inlier count for its sample budget.
+// With the loop's iterative refinement (mode.iterativeRefinement, v3dm_ransac_set_refinement) the selection
+// is v3dm_ransac_refine.cu's, as reconstruction_common.cpp:255-314: an accepted candidate's pose is refined by
+// refineRelativePose (v3d_poseutilities.cpp:1063-1101) on the candidate's inliers, the refined F is scored over
+// all correspondences in the loop's order, and the loop keeps min(cost, refined cost), the refined model and the
+// refined inlier count for its sample budget.  k_rs_refine_tasks lists the candidates that a round can accept,
+// k_rs_refine refines each on a CTA of its own, every sum over the inliers in index order in one lane of a
+// warp (that order is what makes the result the reference's), and k_rs_select_refine walks the loop.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -333,64 +333,64 @@ k_rs_score(const int32_t* __restrict__ offsets, const float4* __restrict__ corrs
   __shared__ double4 st[kRsStage];  // the positions converted once per CTA
   const int total = *nItems;
   for (int it = blockIdx.x; it < total; it += gridDim.x) {
-  const int p = items[it].x;
-  const int h = items[it].y + (int)threadIdx.x;
-  const int b = offsets[p], n = offsets[p + 1] - b;
-  const bool mine = h < listN[p];
-  const double bound = states[p].minError;
-  long long slot = 0;
-  double F[9];
-  if (mine) {
-    slot = (long long)plan.start[p] * kRsMaxSol + list[(long long)plan.start[p] * kRsMaxSol + h];
-    for (int k = 0; k < 9; ++k) F[k] = slots[slot * kRsSlotDoubles + 9 + k];
-  }
-  double sum = 0.0;
-  int cnt = 0;
-  bool open = mine;  // the candidate can still be accepted
-  for (int c0 = 0; c0 < n; c0 += kRsStage) {
-    const int m = min(kRsStage, n - c0);
-    if (!__syncthreads_or(open)) break;
-    for (int k = threadIdx.x; k < m; k += blockDim.x) {
-      const float4 c = corrs[b + c0 + k];
-      st[k] = make_double4(c.x, c.y, c.z, c.w);
+    const int p = items[it].x;
+    const int h = items[it].y + (int)threadIdx.x;
+    const int b = offsets[p], n = offsets[p + 1] - b;
+    const bool mine = h < listN[p];
+    const double bound = states[p].minError;
+    long long slot = 0;
+    double F[9];
+    if (mine) {
+      slot = (long long)plan.start[p] * kRsMaxSol + list[(long long)plan.start[p] * kRsMaxSol + h];
+      for (int k = 0; k < 9; ++k) F[k] = slots[slot * kRsSlotDoubles + 9 + k];
     }
-    __syncthreads();
-    if (open) {
-      // kRsUnroll terms at a time: their operations are independent and hide each other's latency.  The
-      // division is unconditional: among a warp's 32 candidates one nearly always needs it, and a branch
-      // around it would order the terms one after the other (6.3 ms of scoring in a 256-pair call).
-      int k = 0;
-      for (; k + kRsUnroll <= m; k += kRsUnroll) {
-        double num[kRsUnroll], den[kRsUnroll], d[kRsUnroll];
+    double sum = 0.0;
+    int cnt = 0;
+    bool open = mine;  // the candidate can still be accepted
+    for (int c0 = 0; c0 < n; c0 += kRsStage) {
+      const int m = min(kRsStage, n - c0);
+      if (!__syncthreads_or(open)) break;
+      for (int k = threadIdx.x; k < m; k += blockDim.x) {
+        const float4 c = corrs[b + c0 + k];
+        st[k] = make_double4(c.x, c.y, c.z, c.w);
+      }
+      __syncthreads();
+      if (open) {
+        // kRsUnroll terms at a time: their operations are independent and hide each other's latency.  The
+        // division is unconditional: among a warp's 32 candidates one nearly always needs it, and a branch
+        // around it would order the terms one after the other (6.3 ms of scoring in a 256-pair call).
+        int k = 0;
+        for (; k + kRsUnroll <= m; k += kRsUnroll) {
+          double num[kRsUnroll], den[kRsUnroll], d[kRsUnroll];
 #pragma unroll
-        for (int u = 0; u < kRsUnroll; ++u) {
-          const double4 c = st[k + u];
-          ess::sampson_parts(F, c.x, c.y, c.z, c.w, num[u], den[u]);
+          for (int u = 0; u < kRsUnroll; ++u) {
+            const double4 c = st[k + u];
+            ess::sampson_parts(F, c.x, c.y, c.z, c.w, num[u], den[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < kRsUnroll; ++u) d[u] = ess::ddiv(num[u], den[u]);
+#pragma unroll
+          for (int u = 0; u < kRsUnroll; ++u) {
+            cnt += d[u] < thr2;
+            sum = ess::dadd(sum, thr2 < d[u] ? thr2 : d[u]);  // std::min(d, thr2)
+          }
+          if ((k & 31) == 0 && !(sum < bound)) {  // the terms to come only add to it
+            open = false;
+            break;
+          }
         }
-#pragma unroll
-        for (int u = 0; u < kRsUnroll; ++u) d[u] = ess::ddiv(num[u], den[u]);
-#pragma unroll
-        for (int u = 0; u < kRsUnroll; ++u) {
-          cnt += d[u] < thr2;
-          sum = ess::dadd(sum, thr2 < d[u] ? thr2 : d[u]);  // std::min(d, thr2)
-        }
-        if ((k & 31) == 0 && !(sum < bound)) {  // the terms to come only add to it
-          open = false;
-          break;
+        for (; open && k < m; ++k) {
+          const double4 c = st[k];
+          bool in;
+          sum = ess::dadd(sum, ess::sampson_truncated(F, c.x, c.y, c.z, c.w, thr2, in));
+          cnt += in;
         }
       }
-      for (; open && k < m; ++k) {
-        const double4 c = st[k];
-        bool in;
-        sum = ess::dadd(sum, ess::sampson_truncated(F, c.x, c.y, c.z, c.w, thr2, in));
-        cnt += in;
-      }
     }
-  }
-  if (mine) {
-    cost[slot] = sum;
-    inl[slot] = cnt;
-  }
+    if (mine) {
+      cost[slot] = sum;
+      inl[slot] = cnt;
+    }
   }
 }
 

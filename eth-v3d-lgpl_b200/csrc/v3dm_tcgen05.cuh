@@ -89,14 +89,8 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
 }
 
 // Shared-memory matrix descriptor of a K-major operand stored as 128-byte rows with the
-// 128-byte swizzle: 8-row core groups 1024 bytes apart (SBO), version 1, layout SWIZZLE_128B.
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-         (2ull << 61);
-}
-
-// The same in two words: the low one for a shared-memory address (it advances by bytes >> 4), and
-// the descriptor of a low word.
+// 128-byte swizzle: 8-row core groups 1024 bytes apart (SBO), version 1, layout SWIZZLE_128B.  Its low
+// word for a shared-memory address (it advances by bytes >> 4), and the descriptor of a low word.
 __device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr) { return ((saddr >> 4) & 0x3FFFu) | (1u << 16); }
 __device__ __forceinline__ uint64_t sdesc_of(uint32_t lo) {
   constexpr uint64_t hi = ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);

@@ -237,95 +237,95 @@ k_voctree_f32(const float* __restrict__ nodes, const float* __restrict__ nodeNor
   const unsigned grp = 0xfu << (lane & ~3);
   const int total = list ? *listN : n;
   for (int at = gt / kTpk; at - lane / kTpk < total; at += gridDim.x * kVtThreads / kTpk) {  // whole warps
-  const bool valid = at < total;
-  const int key = list ? (valid ? list[at] : 0) : at;
-  const float* krow = keys + (size_t)(valid ? key : 0) * kDescBytes;
-  float4 kv[8];
+    const bool valid = at < total;
+    const int key = list ? (valid ? list[at] : 0) : at;
+    const float* krow = keys + (size_t)(valid ? key : 0) * kDescBytes;
+    float4 kv[8];
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
-    kv[q] = valid ? __ldg(reinterpret_cast<const float4*>(krow) + q * 4 + part) : make_float4(0.f, 0.f, 0.f, 0.f);
-  float ss = 0.0f;
+    for (int q = 0; q < 8; ++q)
+      kv[q] = valid ? __ldg(reinterpret_cast<const float4*>(krow) + q * 4 + part) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float ss = 0.0f;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    ss = fmaf(kv[q].x, kv[q].x, ss);
-    ss = fmaf(kv[q].y, kv[q].y, ss);
-    ss = fmaf(kv[q].z, kv[q].z, ss);
-    ss = fmaf(kv[q].w, kv[q].w, ss);
-  }
-  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-  ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-  const float kn = __fmul_ru(__fsqrt_ru(ss), 1.000001f);
-  const bool bounded = kn >= kVtTinyNorm;
-  long long nextId = 0, leafId = -1;
-  unsigned long long replays = 0;
-  bool ok = true, listed = false;
-  for (int d = 0; d < depth; ++d) {
-    if (nextId < 0 || nextId + bf > nodeCount) {  // cannot happen for a finite tree; leaves the loop safely
-      ok = false;
-      break;
+    for (int q = 0; q < 8; ++q) {
+      ss = fmaf(kv[q].x, kv[q].x, ss);
+      ss = fmaf(kv[q].y, kv[q].y, ss);
+      ss = fmaf(kv[q].z, kv[q].z, ss);
+      ss = fmaf(kv[q].w, kv[q].w, ss);
     }
-    const float* base = nodes + (size_t)nextId * kDescBytes;
-    float lo1 = -INFINITY, up1 = -INFINITY, up2 = -INFINITY;
-    int c1 = -1, cu1 = -1;
-    bool finite = true;
-    float eMax = 0.0f;
+    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+    const float kn = __fmul_ru(__fsqrt_ru(ss), 1.000001f);
+    const bool bounded = kn >= kVtTinyNorm;
+    long long nextId = 0, leafId = -1;
+    unsigned long long replays = 0;
+    bool ok = true, listed = false;
+    for (int d = 0; d < depth; ++d) {
+      if (nextId < 0 || nextId + bf > nodeCount) {  // cannot happen for a finite tree; leaves the loop safely
+        ok = false;
+        break;
+      }
+      const float* base = nodes + (size_t)nextId * kDescBytes;
+      float lo1 = -INFINITY, up1 = -INFINITY, up2 = -INFINITY;
+      int c1 = -1, cu1 = -1;
+      bool finite = true;
+      float eMax = 0.0f;
 #pragma unroll 2
-    for (int c = 0; c < bf; ++c) {
-      const float4* row = reinterpret_cast<const float4*>(base + (size_t)c * kDescBytes) + part;
-      float acc = 0.0f;
+      for (int c = 0; c < bf; ++c) {
+        const float4* row = reinterpret_cast<const float4*>(base + (size_t)c * kDescBytes) + part;
+        float acc = 0.0f;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 w = __ldg(row + q * 4);
-        acc = fmaf(kv[q].x, w.x, acc);
-        acc = fmaf(kv[q].y, w.y, acc);
-        acc = fmaf(kv[q].z, w.z, acc);
-        acc = fmaf(kv[q].w, w.w, acc);
+        for (int q = 0; q < 8; ++q) {
+          const float4 w = __ldg(row + q * 4);
+          acc = fmaf(kv[q].x, w.x, acc);
+          acc = fmaf(kv[q].y, w.y, acc);
+          acc = fmaf(kv[q].z, w.z, acc);
+          acc = fmaf(kv[q].w, w.w, acc);
+        }
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);  // fadd commutes: the four lanes agree exactly
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+        const float e = __fadd_ru(__fmul_ru(__fmul_ru(kSeqRel, kn), __ldg(nodeNorm + nextId + c)), kSeqAbs);
+        const float lo = __fsub_rd(acc, e), up = __fadd_ru(acc, e);
+        eMax = fmaxf(eMax, e);
+        finite = finite && isfinite(lo) && isfinite(up);
+        if (lo > lo1) {
+          lo1 = lo;
+          c1 = c;
+        }
+        if (up > up1) {
+          up2 = up1;
+          up1 = up;
+          cu1 = c;
+        } else if (up > up2) {
+          up2 = up;
+        }
       }
-      acc += __shfl_xor_sync(0xffffffffu, acc, 1);  // fadd commutes: the four lanes agree exactly
-      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-      const float e = __fadd_ru(__fmul_ru(__fmul_ru(kSeqRel, kn), __ldg(nodeNorm + nextId + c)), kSeqAbs);
-      const float lo = __fsub_rd(acc, e), up = __fadd_ru(acc, e);
-      eMax = fmaxf(eMax, e);
-      finite = finite && isfinite(lo) && isfinite(up);
-      if (lo > lo1) {
-        lo1 = lo;
-        c1 = c;
+      const float othersUp = cu1 == c1 ? up2 : up1;
+      int best = c1;
+      // the same on the four lanes of the key: their scores and bounds are bit-identical
+      const bool usual = finite && c1 >= 0 && lo1 > -1e30f;
+      const bool decided = usual && othersUp < lo1 && bounded;
+      if (undecided && usual && !decided && eMax < kSeqRel * 1e30f) {
+        if (part == 0 && valid && !listed) {
+          const int slot = atomicAdd(nUndecided, 1);
+          undecided[2 * slot] = make_int4(key, (int)leafId, depth - d, 0);
+          undecided[2 * slot + 1] = make_int4(-1, -1, -1, -1);  // all children
+        }
+        listed = true;
+      } else if (!decided && !listed) {
+        int b = -1;
+        if (part == 0 && valid) {
+          b = seq_best_child(krow, base, bf);
+          ++replays;
+        }
+        best = __shfl_sync(grp, b, lane & ~3);
       }
-      if (up > up1) {
-        up2 = up1;
-        up1 = up;
-        cu1 = c;
-      } else if (up > up2) {
-        up2 = up;
-      }
+      if (!valid || listed) best = 0;
+      leafId = nextId + best;
+      nextId = (leafId + 1) * bf;
     }
-    const float othersUp = cu1 == c1 ? up2 : up1;
-    int best = c1;
-    // the same on the four lanes of the key: their scores and bounds are bit-identical
-    const bool usual = finite && c1 >= 0 && lo1 > -1e30f;
-    const bool decided = usual && othersUp < lo1 && bounded;
-    if (undecided && usual && !decided && eMax < kSeqRel * 1e30f) {
-      if (part == 0 && valid && !listed) {
-        const int slot = atomicAdd(nUndecided, 1);
-        undecided[2 * slot] = make_int4(key, (int)leafId, depth - d, 0);
-        undecided[2 * slot + 1] = make_int4(-1, -1, -1, -1);  // all children
-      }
-      listed = true;
-    } else if (!decided && !listed) {
-      int b = -1;
-      if (part == 0 && valid) {
-        b = seq_best_child(krow, base, bf);
-        ++replays;
-      }
-      best = __shfl_sync(grp, b, lane & ~3);
-    }
-    if (!valid || listed) best = 0;
-    leafId = nextId + best;
-    nextId = (leafId + 1) * bf;
-  }
-  if (!ok && part == 0 && valid) atomicOr(err, kErrBadTree);
-  if (valid && part == 0 && !listed) out[key] = (int32_t)(idMode == V3DM_LEAF_LOCAL ? leafId - leafBase : leafId);
-  if (exactCount && part == 0 && replays) atomicAdd(exactCount, replays);
+    if (!ok && part == 0 && valid) atomicOr(err, kErrBadTree);
+    if (valid && part == 0 && !listed) out[key] = (int32_t)(idMode == V3DM_LEAF_LOCAL ? leafId - leafBase : leafId);
+    if (exactCount && part == 0 && replays) atomicAdd(exactCount, replays);
   }
 }
 

@@ -601,7 +601,7 @@ cudaError_t vtf_prepare(const float* nodes, const float* norm, long long rows, i
                                                                   static_cast<uint2*>(planes));
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(maxNorm, 0, sizeof(float), st)) != cudaSuccess) return e;
-  k_vtf_max_norm<<<148, 256, 0, st>>>(norm, rows / bf, bf, reinterpret_cast<unsigned int*>(childNorm),
+  k_vtf_max_norm<<<kB200SMs, 256, 0, st>>>(norm, rows / bf, bf, reinterpret_cast<unsigned int*>(childNorm),
                                       reinterpret_cast<unsigned int*>(maxNorm));
   return cudaGetLastError();
 }

@@ -348,48 +348,48 @@ __global__ void __launch_bounds__(kVtcThreads, 1)
       const long long r = a.bucketBase < 0 ? -1 : a.bucketBase + item.x;
       const long long g1 = (r + 1) * BF;
       for (int t = (int)((i0 ^ half) & 1u); t < tiles; t += 2) {
-      const uint32_t i = i0 + (uint32_t)t, acc = i % S::kAcc;
-      // this row's key index, loaded before the wait for the accumulator
-      const int pos = t * kVtcRows + row;
-      const int key = pos < item.z ? (gathered ? __ldg(a.perm + item.y + pos) : item.y + pos) : -1;
-      ok = mbar_wait_warp(&s.done[i % kVtcASlots], (i / kVtcASlots) & 1u, &s.abort, a.err, lim);
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * S::kAccCols);
-      // D2 in columns 0 .. N2 - 1, D1 in N2 .. N2 + 15
-      uint32_t d1[16];
-      tmem_ld16(tb + S::N2, d1);
-      tmem_wait(d1);
-      const int c1 = vtc_argmax<BF>(d1);
-      uint32_t g[BF];  // the chosen child's BF children: columns BF c1 .. BF c1 + BF - 1 of D2
-      if (a.levels == 2) {
+        const uint32_t i = i0 + (uint32_t)t, acc = i % S::kAcc;
+        // this row's key index, loaded before the wait for the accumulator
+        const int pos = t * kVtcRows + row;
+        const int key = pos < item.z ? (gathered ? __ldg(a.perm + item.y + pos) : item.y + pos) : -1;
+        ok = mbar_wait_warp(&s.done[i % kVtcASlots], (i / kVtcASlots) & 1u, &s.abort, a.err, lim);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * S::kAccCols);
+        // D2 in columns 0 .. N2 - 1, D1 in N2 .. N2 + 15
+        uint32_t d1[16];
+        tmem_ld16(tb + S::N2, d1);
+        tmem_wait(d1);
+        const int c1 = vtc_argmax<BF>(d1);
+        uint32_t g[BF];  // the chosen child's BF children: columns BF c1 .. BF c1 + BF - 1 of D2
+        if (a.levels == 2) {
 #pragma unroll
-        for (int k = 0; k < BF; ++k) g[k] = 0u;
+          for (int k = 0; k < BF; ++k) g[k] = 0u;
 #pragma unroll
-        for (int c0 = 0; c0 < BF * BF; c0 += 64) {
-          uint32_t v[64];
-          tmem_ld32(tb + (uint32_t)c0, v);
-          if (c0 + 32 < BF * BF) tmem_ld32(tb + (uint32_t)(c0 + 32), v + 32);
-          tmem_wait(v);
+          for (int c0 = 0; c0 < BF * BF; c0 += 64) {
+            uint32_t v[64];
+            tmem_ld32(tb + (uint32_t)c0, v);
+            if (c0 + 32 < BF * BF) tmem_ld32(tb + (uint32_t)(c0 + 32), v + 32);
+            tmem_wait(v);
 #pragma unroll
-          for (int k = 0; k < 64; ++k)
-            if (c0 + k < BF * BF) g[(c0 + k) % BF] = c1 == (c0 + k) / BF ? v[k] : g[(c0 + k) % BF];
+            for (int k = 0; k < 64; ++k)
+              if (c0 + k < BF * BF) g[(c0 + k) % BF] = c1 == (c0 + k) / BF ? v[k] : g[(c0 + k) % BF];
+          }
         }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s.accEmpty[acc]);
-      if (key < 0) continue;
-      const long long node = a.levels == 2 ? (g1 + 1) * BF + (long long)BF * c1 + vtc_argmax<BF>(g) : g1 + c1;
-      if (a.final) {
-        a.out[key] = (int32_t)(a.idMode == V3DM_LEAF_LOCAL ? node - a.leafBase : node);
-      } else {
-        const int bkt = (int)(node - a.nextBase);
-        a.next[key] = bkt;
-        // one update per distinct bucket of the warp (keys of a tile often share buckets)
-        const unsigned peers = __match_any_sync(__activemask(), bkt);
-        if (lane == __ffs(peers) - 1) atomicAdd(localHist ? &s.hist[bkt] : &a.hist[bkt], __popc(peers));
-      }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s.accEmpty[acc]);
+        if (key < 0) continue;
+        const long long node = a.levels == 2 ? (g1 + 1) * BF + (long long)BF * c1 + vtc_argmax<BF>(g) : g1 + c1;
+        if (a.final) {
+          a.out[key] = (int32_t)(a.idMode == V3DM_LEAF_LOCAL ? node - a.leafBase : node);
+        } else {
+          const int bkt = (int)(node - a.nextBase);
+          a.next[key] = bkt;
+          // one update per distinct bucket of the warp (keys of a tile often share buckets)
+          const unsigned peers = __match_any_sync(__activemask(), bkt);
+          if (lane == __ffs(peers) - 1) atomicAdd(localHist ? &s.hist[bkt] : &a.hist[bkt], __popc(peers));
+        }
       }
       i0 += (uint32_t)tiles;
     }
