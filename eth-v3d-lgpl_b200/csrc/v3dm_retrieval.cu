@@ -93,7 +93,9 @@ __device__ __forceinline__ void rt_clear(RtPlanes& p) {
   for (int q = 0; q < kRtPlaneCount; ++q) p.v[q] = 0;
 }
 
-// Adds the counts of the images of 'mask' to kdCol[0..31] and clears the planes.
+// Adds the counts of the images of 'mask' to kdCol[0..31] (kAtomic: that other groups add to as well) and
+// clears the planes.
+template <bool kAtomic>
 __device__ __forceinline__ void rt_flush(RtPlanes& p, uint32_t mask, uint32_t* kdCol) {
   uint32_t any = 0;
 #pragma unroll
@@ -105,9 +107,16 @@ __device__ __forceinline__ void rt_flush(RtPlanes& p, uint32_t mask, uint32_t* k
     uint32_t cnt = 0;
 #pragma unroll
     for (int q = 0; q < kRtPlaneCount; ++q) cnt |= ((p.v[q] >> k) & 1u) << q;
-    kdCol[k] += cnt;
+    if (kAtomic) atomicAdd(&kdCol[k], cnt);
+    else kdCol[k] += cnt;
   }
   rt_clear(p);
+}
+
+// By value and not inlined: the registers of the counting loop do not have to make room for it (inlined, 4096
+// images of 2000 - 6000 words, which hardly use it, took 743 us a call instead of 718).
+__device__ __noinline__ void rt_flush_shared(RtPlanes p, uint32_t mask, uint32_t* kdCol) {
+  rt_flush<true>(p, mask, kdCol);
 }
 
 // Another group's counts of the same column.
@@ -173,8 +182,9 @@ __device__ __forceinline__ uint32_t rt_add16(RtPlanes& p, const uint32_t* bits, 
 // What bounds it: the reads of the bitmap from L2 (4 bytes per 32 images and word of a query: 4.2 GB for
 // 4096 images of 2000 - 6000 words, 7 TB/s) and the logic instructions of the counters, about equally.  A
 // group's planes are added to the next group's bit-sliced, through shared memory, so that each count is
-// taken apart once and not once per group (that, 1600 instructions per thread, was as much as the counting).
-// That call took 887 us, 730 now, of which this kernel 739 and 580.  Two columns per thread (8-byte loads, 277 million
+// taken apart once and not once per group (that, 1600 instructions per thread, was as much as the counting),
+// where there are more than a few (`direct` below).
+// That call took 887 us, of which this kernel 739, and takes 718 now.  Two columns per thread (8-byte loads, 277 million
 // instructions against 348) need 80 registers and were slower with the fewer warps, 587.
 template <bool kWide>
 __global__ void __launch_bounds__(kRtThreads, 2)
@@ -210,6 +220,11 @@ k_rt_score(const int32_t* __restrict__ offsets, const int32_t* __restrict__ word
   const int g = threadIdx.x / colsPerPass;
   const bool active = g < groups;
   const int chunkRows = (kRtChunk / (16 * groups)) * 16 * groups;  // >= 16 * groups, a multiple of it
+  // A group has nq / groups rows, and of each of a column's images about nq / nLeaves of them: while that is 0.4 or
+  // less, few counts are set and each group adds its own to k(d).  Adding up the groups' planes takes two barriers
+  // for every halving of the groups whatever they hold: always done, 512 images of 600 words (100000 leaves) took
+  // 78 us a call and 200 of 600 59, with this rule 69 and 53; never done, 400 images of 4000 words 111, with it 97.
+  const bool direct = 5LL * (e - b) * (e - b) <= 2LL * groups * nLeaves;
   const uint32_t unit = kWide ? 1u : 4u;  // of the offsets: rt_word
   const uint32_t rowUnits = (uint32_t)w32 * unit, zeroRow = (uint32_t)nLeaves * rowUnits;
   for (int c0 = 0; c0 < nw; c0 += colsPerPass) {
@@ -221,6 +236,11 @@ k_rt_score(const int32_t* __restrict__ offsets, const int32_t* __restrict__ word
     rt_clear(p);
     // The groups' counts of the column to kd, and the planes to zero (all threads; the chunk has been read).
     auto flush = [&]() {
+      if (direct) {
+        if (mine) rt_flush_shared(p, mask, kd + (col << 5));
+        rt_clear(p);
+        return;
+      }
       for (int ng = groups; ng > 1; ng = (ng + 1) / 2) {
         const int half = (ng + 1) / 2, width = (ng - half) * colsPerPass;  // groups half .. ng - 1 hand over
         __syncthreads();
@@ -233,7 +253,7 @@ k_rt_score(const int32_t* __restrict__ offsets, const int32_t* __restrict__ word
         __syncthreads();
         if (mine && g < ng - half) rt_add_planes(p, rowOff + g * colsPerPass + (int)threadIdx.x % colsPerPass, width);
       }
-      if (mine && g == 0) rt_flush(p, mask, kd + (col << 5));
+      if (mine && g == 0) rt_flush<false>(p, mask, kd + (col << 5));
     };
     int inSegment = 0;  // rows added since the last flush
     for (int f0 = b; f0 < e; f0 += chunkRows) {
