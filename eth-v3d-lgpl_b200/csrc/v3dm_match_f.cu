@@ -212,7 +212,6 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
   extern __shared__ uint8_t smemRaw[];
   SmemF& s = *reinterpret_cast<SmemF*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long lim = a.waitLimit > 0 ? a.waitLimit : kWaitCycles;
   const FWalk start(a);
   if (!start.more()) return;
   if (threadIdx.x == 0) {
@@ -249,7 +248,7 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
       bool ok = true;
       auto load = [&](const CUtensorMap* m, int r) {
         const uint32_t st = u % kFStages;
-        if (!mbar_wait(&s.empty[st], ((u / kFStages) & 1u) ^ 1u, &s.abort, a.err, lim)) return false;
+        if (!mbar_wait(&s.empty[st], ((u / kFStages) & 1u) ^ 1u, &s.abort, a.err)) return false;
         if (m == &tmB && ++bLoads == a.skipLoad && blockIdx.x == 0) {
           skipped = u;
         } else {
@@ -276,6 +275,7 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
     const uint32_t base = sdesc_lo(smem_u32(s.b[0]));
     uint32_t u = 0, i[kFGroups] = {};
     bool ok = true;
+    const long long lim = a.waitLimit > 0 ? a.waitLimit : kWaitCycles;  // the other roles follow its abort
     auto wait = [&](unsigned long long* b, uint32_t par) { return mbar_wait_warp(b, par, &s.abort, a.err, lim); };
     for (FWalk wk = start; wk.more() && ok; wk.next()) {
       const int groups = wk.groups();
@@ -384,7 +384,7 @@ k_side_f(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtens
         if (st >= 0) enter = f32_unorder(b2);
       };
       for (int t = 0; t < wk.nT; ++t, ++i) {
-        ok = mbar_wait_warp(&s.accFull[g], i & 1u, &s.abort, a.err, lim);
+        ok = mbar_wait_warp(&s.accFull[g], i & 1u, &s.abort, a.err);
         if (!ok) break;
         tc_fence_after();
         const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * kFN);
