@@ -220,11 +220,12 @@ k_rt_score(const int32_t* __restrict__ offsets, const int32_t* __restrict__ word
   const int g = threadIdx.x / colsPerPass;
   const bool active = g < groups;
   const int chunkRows = (kRtChunk / (16 * groups)) * 16 * groups;  // >= 16 * groups, a multiple of it
-  // A group has nq / groups rows, and of each of a column's images about nq / nLeaves of them: while that is 0.4 or
+  // A group has nq / groups rows, and of each of a column's images about nq / nLeaves of them: while that is 0.3 or
   // less, few counts are set and each group adds its own to k(d).  Adding up the groups' planes takes two barriers
   // for every halving of the groups whatever they hold: always done, 512 images of 600 words (100000 leaves) took
   // 78 us a call and 200 of 600 59, with this rule 69 and 53; never done, 400 images of 4000 words 111, with it 97.
-  const bool direct = 5LL * (e - b) * (e - b) <= 2LL * groups * nLeaves;
+  // In between: 300 images of 1500 words (0.44) 61 added up and 68 not, 363 of 1500 (0.49) 77 and 72.
+  const bool direct = 10LL * (e - b) * (e - b) <= 3LL * groups * nLeaves;
   const uint32_t unit = kWide ? 1u : 4u;  // of the offsets: rt_word
   const uint32_t rowUnits = (uint32_t)w32 * unit, zeroRow = (uint32_t)nLeaves * rowUnits;
   for (int c0 = 0; c0 < nw; c0 += colsPerPass) {

@@ -36,9 +36,9 @@ def test_bitmap_around_four_gigabytes(v3dm_mod, oracle_mod, leaves):
     _check(v3dm_mod, oracle_mod, leaves, counts, words, 7)
 
 
-@pytest.mark.parametrize("n_images,n,leaves", [(1100, 400, 400_000), (1100, 400, 10_000), (33, 1023, 10_000), (33, 1023, 12_000),
-                                               (3, 4097, 150_000), (3, 33_000, 200_000), (3, 66_000, 100_000),
-                                               (3, 66_000, 100_000_000)])
+@pytest.mark.parametrize("n_images,n,leaves", [(1100, 400, 400_000), (1100, 400, 10_000), (33, 1023, 10_000), (33, 1023, 16_000),
+                                               (3, 4097, 150_000), (3, 4097, 300_000), (3, 33_000, 200_000), (3, 66_000, 100_000),
+                                               (3, 66_000, 120_000_000)])
 def test_counts_where_groups_add_for_themselves_and_where_they_are_added_up(v3dm_mod, oracle_mod, n_images, n, leaves):
     """Both ways of emptying the counters, chosen by words, groups and leaves, with queries of more rows than the
     counters hold (32752) among them; n / leaves + 0.1 < 1, so that the scores are finite."""
