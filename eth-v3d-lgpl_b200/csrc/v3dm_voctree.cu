@@ -26,11 +26,11 @@
 //     gamma_128 * sum|k_i n_i| <= 7.63e-6 * |k| |n| of the exact dot product (the standard bound
 //     for recursive summation, n = 128 terms; the FMA pass has at most 34 roundings per term),
 //     so |fast - sequential| <= 1.53e-5 * |k| |n|; the kernel uses 2e-5 * |k| |n| + 1e-36 with
-//     precomputed node norms rounded up (and nothing for keys whose squares may underflow).  When one child's lower bound is above every other
+//     precomputed node norms rounded up.  When one child's lower bound is above every other
 //     child's upper bound (and above -1e30f), it is the sequential rule's choice.  Otherwise
-//     (near ties, equal children, non-finite values) one thread of the key replays the
-//     reference's sequential FP32 loop over all children, with __fmul_rn / __fadd_rn, or the key is
-//     listed and k_vtf_resolve does, a child per lane (vt_f_listed).
+//     (near ties, equal children, non-finite values, keys whose squares may underflow) one thread
+//     of the key replays the reference's sequential FP32 loop over all children, with __fmul_rn /
+//     __fadd_rn, or the key is listed and k_vtf_resolve does, a child per lane (vt_f_listed).
 //
 // k_voctree: four threads per key, each holding 32 bytes of the key in registers; a warp
 // descends eight keys.  At each level a thread loads its 32-byte slice of every child (each
