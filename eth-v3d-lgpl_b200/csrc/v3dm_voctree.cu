@@ -469,7 +469,8 @@ long long vt_bins(const v3dm_voctree* t) {
 }
 
 // The ways of a call of n float keys.  Below kVtMinPerBin keys per bucket of the last phase, the tiles of 128
-// keys would be mostly empty: k_voctree_f32, which replays near ties itself.  From there on k_voctree_f32
+// keys would be mostly empty, and a second kernel is too much for the smallest calls (BF 10, depth 1, 16 to 1000
+// keys: 6.5 us without, 10.5 with it): k_voctree_f32, which replays near ties itself.  From there on k_voctree_f32
 // lists them for k_vtf_resolve, until the phases are faster: the two kernels take about 5 us, 0.45 us per child
 // row of a path (bf * depth of them) and 41 ps per key and row, the phases 28 us each, 150 ps per key each and
 // 100 ps per key.  Measured on k-means trees, us (one kernel, two, phases):
